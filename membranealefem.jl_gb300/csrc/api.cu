@@ -342,6 +342,13 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
     pp.neu_type[k] = (int)d->neu_type[k];
     pp.neu_val[k] = d->neu_val[k];
   }
+  {  // Neumann entries that can meet on one element: both of two opposite sides only across a single element
+    int cnt[4] = {0, 0, 0, 0};
+    for (int k = 0; k < pp.n_neu; ++k) ++cnt[pp.neu_bdry[k]];
+    const int bt = d->num2el == 1 ? cnt[0] + cnt[2] : std::max(cnt[0], cnt[2]);
+    const int lr = d->num1el == 1 ? cnt[1] + cnt[3] : std::max(cnt[1], cnt[3]);
+    pp.max_btask = 3 * (bt + lr);
+  }
 
   // integer maps (0-based int32)
   std::vector<int> ix((size_t)numel * 9), lm((size_t)numel * nq), uel(numel), bref((size_t)numel * 4, -1);
@@ -1575,7 +1582,7 @@ static int tan_tune(mafem_handle* h, const AsmJob* d_ajobs, int slot, unsigned c
     float t = INFINITY;
     for (int r = 0; r < 4 && e == cudaSuccess; ++r) {
       e = cudaEventRecord(e0, st);
-      if (e == cudaSuccess) e = launch_batch_tan(h->pp.motion, epb, d_ajobs, d_item, d_off, 1, off[1], h->pp.nq, st);
+      if (e == cudaSuccess) e = launch_batch_tan(epb, d_ajobs, d_item, d_off, 1, off[1], h->pp, st);
       if (e == cudaSuccess) e = cudaEventRecord(e1, st);
       if (e == cudaSuccess) e = cudaEventSynchronize(e1);
       float ms = 0.0f;
@@ -1795,6 +1802,12 @@ static cudaError_t run_round(RoundRunner& R, const PatchJob* d_jobs, const AsmJo
     if (k + 1 < m && gkey(it[k + 1]) != gkey(it[k])) groups.push_back(k + 1);
   }
   groups.push_back(m);
+  std::vector<PhysParams> gpp;  // a group's launch parameters
+  for (size_t g = 0; g + 1 < groups.size(); ++g) {
+    gpp.push_back(hv[it[groups[g]]]->pp);
+    for (int k = groups[g]; k < groups[g + 1]; ++k)
+      gpp.back().max_btask = std::max(gpp.back().max_btask, hv[it[k]]->pp.max_btask);
+  }
   const size_t bytes = dir_off + (size_t)(m + 1) * sizeof(int);
   for (int k = 0; k < m; ++k) R.h_order[k] = slot_of[pj[k]];
   const unsigned char* dr = R.d_round;
@@ -1825,8 +1838,8 @@ static cudaError_t run_round(RoundRunner& R, const PatchJob* d_jobs, const AsmJo
       e = launch_batch_resid(h->pp.motion, d_ajobs, d_items + g0, d_off(0, g0), g1 - g0, off[0][g1] - off[0][g0],
                              h->pp.nq, st);
       if (e == cudaSuccess)
-        e = launch_batch_tan(h->pp.motion, epb[g0], d_ajobs, d_items + g0, d_off(1, g0), g1 - g0,
-                             off[1][g1] - off[1][g0], h->pp.nq, st);
+        e = launch_batch_tan(epb[g0], d_ajobs, d_items + g0, d_off(1, g0), g1 - g0, off[1][g1] - off[1][g0],
+                             gpp[g], st);
     }
     if (e == cudaSuccess) {
       launch_batch_gather(d_ajobs, d_items, d_off(2, 0), m, off[2][m], st);
@@ -1858,7 +1871,7 @@ static cudaError_t run_round(RoundRunner& R, const PatchJob* d_jobs, const AsmJo
     key.push_back((int64_t)items[k].job * 4 + items[k].start);
     key.push_back(((int64_t)h->numel << 32) | (uint32_t)h->numnp);
     key.push_back((h->nmdf << 24) | ((int64_t)h->n_dir << 8) | (h->pp.motion << 4) | (h->ndf & 15));
-    key.push_back(epb[k]);
+    key.push_back(((int64_t)h->pp.max_btask << 8) | epb[k]);
   }
   for (int k = 0; k < m; ++k) key.push_back(R.h_order[k]);
   auto found = R.graphs.find(key);

@@ -1,5 +1,5 @@
 // elem.cu -- element residual + tangent (calc_r_K's element loop) and the
-// atomics-free gather of element blocks into the banded global tangent.
+// element kernels of the batched rounds.
 //
 // Reference: src/analysis/FiniteElement.jl:75-200 (calc_r_K), :208-242
 // (calc_elem_residual), :253-330 (calc_elem_dof_residuals), :338-400
@@ -8,37 +8,56 @@
 //
 // The reference differentiates the element residual by complex steps, one
 // residual evaluation per active element dof (FiniteElement.jl:109-126).  Here
-// the same derivative is computed in forward mode: each thread of an element
-// owns one element dof q = (node a*, dof d*) and evaluates the residual on dual
-// numbers (primal FP64, tangent T = double or float) seeded with
-// ∂cps[a*, d*] = 1 and, when d* is a mesh-motion dof of component j,
-// ∂xms[a*, j] = Δt -- the reference's two complex steps of one column merged by
-// linearity (FiniteElement.jl:113-122).  The derivative of |τ| is dropped in
-// the boundary term, exactly as the reference's conjugating `dot` drops it
-// (FiniteElement.jl:448).
+// the same derivative is formed at the Gauss points.  A residual row of node b
+// is linear in node b's basis values, r_(b,i) = sum_s phi_s[b] c_(i,s) with
+// phi = (N_,1, N_,2, nn_11, nn_22, nn_12, N), nn the covariant second
+// derivatives, and the coefficients c depend on
+// the unknowns only through the fields' interpolants sum_a phi_t[a] u_a.  So
+// the element tangent is
+//   K_(b,i),(a,f) = sum_points sum_s sum_t phi_s[b] D_(i,s),(f,t) phi_t[a],
+// with D = dc / d(interpolant t of field f): at most 29 directions (field,
+// interpolant) per point instead of the element's 72 dofs.  Mesh-motion fields
+// carry the node positions with them, dx = dt du, which is the reference's two
+// complex steps of one column merged by linearity (FiniteElement.jl:113-122).
+// The derivative of |τ| is dropped in the boundary term, exactly as the
+// reference's conjugating `dot` drops it (FiniteElement.jl:448).
 //
-// Two precisions.  The plain FP64 form evaluates primal and tangent in FP64
-// (P = T = double) and takes the residual from the same pass (each thread keeps
-// the primal value of its own row).  The FP32 form splits the work by pipe:
-// elem_tan_kernel evaluates primal and tangent in FP32 (P = T = float, staged
-// inputs converted once per element), and elem_resid_kernel evaluates the
-// primal alone in FP64, one thread per (element, Gauss point), so that the
-// FP64 pipe -- 1/64 of the FP32 rate on this GPU -- does 1/72 of the plain
-// form's FP64 work.  The residual's summation order (Gauss points 0..8, the
-// Dohrmann-Bochev term, then the Neumann points) is the plain form's.
+// One CTA per element (elem_body), in phases:
+//   0  nodes, Gauss-point tables; the interpolants of every point;
+//   1  the primal values of every point, one thread per point, kept in shared
+//      memory (each is needed by every direction; formed once);
+//   2  D, one lane per direction and one warp per point (two points per warp
+//      in the Lagrangian motion's 16 directions): forward-mode derivatives on
+//      the stored primal values;
+//   3  the two contractions: a thread owns one (row field i, column (a, f))
+//      pair, forms W_s = sum_t D_(i,s),(f,t) phi_t[a] and adds sum_s phi_s[b]
+//      W_s to its nine rows b, kept in registers over the points;
+//   4  the block through shared memory to K_el[e][col][row], coalesced.
+// What bounds it: FP64 issue in the plain form (one warp-wide FP64 instruction
+// per 64 cycles and sub-partition), FP32 issue and shared-memory reads in the
+// FP32 form.  Work per ALEVB element: 9 x ~400 warp instructions in phase 2
+// and 9 x ~700 in phase 3, against 72 x 9 dual residual evaluations of ~2400
+// (FP64) when every element dof is a direction of its own.
+// Measured on a GB300, against one dual residual evaluation per dof: assembly
+// with its gathers (mafem_calc_r_K) in FP64 3.16 -> 0.92 ms on 32 x 32 ALEVB,
+// 0.58 -> 0.09 ms on 8 x 8 LAG; the FP32 tangent of 32 x 32 ALEVB alone
+// 171 -> 72 us.
 //
-// Layout: elements are independent, so one CTA processes EPB elements with
-// nq = 9*ndf threads each; the element's tangent columns accumulate in shared
-// memory ([row][q], conflict-free) and are written once, column-major, to a
-// staging buffer K_el[e][q][row].  A second kernel gathers, for every band
-// entry, the <= 9 element contributions that land on it (a biquadratic node
-// lies in up to 3 x 3 elements; no atomics: each
-// output is written by exactly one thread), zero-filling the rest of the band.
+// Two precisions.  The plain FP64 form evaluates everything in FP64 and takes
+// the residual from the primal values.  The FP32 form splits the work by pipe:
+// the tangent in FP32 (inputs converted once per element), and the residual
+// alone in FP64 by elem_resid_kernel, one thread per (element, Gauss point).
+// The residual's summation order (Gauss points 0..8, the Dohrmann-Bochev term,
+// then the Neumann points) is the same in both.
+//
+// A second kernel (assemble.cu) gathers, for every band entry, the <= 9 element
+// contributions that land on it.
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "batch_common.cuh"
 #include "mafem_internal.h"
@@ -106,59 +125,10 @@ struct Coef {
       : kb(P(pp.kb)), kg(P(pp.kg)), zv(P(pp.zv)), pn(P(pp.pn)), adb_zv(P(pp.adb / pp.zv)), am(P(pp.am)) {}
 };
 
-// Row accumulators.  A residual row at one Gauss point is linear in node b's
-// basis values (N, N_,α, N_,αβ): lin() receives the row's coefficient duals
-// c[s] and the basis values phi[s] of node b and adds sum_s phi[s] c[s].  The
-// tangent pass adds the tangent part to column q of the element block (and, in
-// the plain form, the primal of row q alone); the residual pass adds the
-// primal of every row into a per-task array.
-template <class P, class T, bool WANT_R>
-struct AccTan {
-  T* Ks;
-  int ldk, q;
-  P rsum;
-  __device__ __forceinline__ void operator()(int row, Dual<P, T> val) {
-    if (WANT_R && row == q) rsum += val.v;
-    Ks[row * ldk + q] += val.d;
-  }
-  template <int NS>
-  __device__ __forceinline__ void lin(int row, const Dual<P, T> (&c)[NS], const P (&phi)[NS]) {
-    T d = T(phi[0]) * c[0].d;
-#pragma unroll
-    for (int s = 1; s < NS; ++s) d += T(phi[s]) * c[s].d;
-    Ks[row * ldk + q] += d;
-    if (WANT_R && row == q) {
-      P v = phi[0] * c[0].v;
-#pragma unroll
-      for (int s = 1; s < NS; ++s) v += phi[s] * c[s].v;
-      rsum += v;
-    }
-  }
-};
-struct AccRes {
-  double* R;  // [row]
-  template <int NS>
-  __device__ __forceinline__ void lin(int row, const Dual<double, Nil> (&c)[NS], const double (&phi)[NS]) {
-    double v = phi[0] * c[0].v;
-#pragma unroll
-    for (int s = 1; s < NS; ++s) v += phi[s] * c[s].v;
-    R[row] += v;
-  }
-};
-// boundary rows are velocity rows only: R[b*3 + i] for row vd[i] + ndf*b
-struct AccResV {
-  double* R;
-  int ndf, vd0, vd1;
-  __device__ __forceinline__ void operator()(int row, Dual<double, Nil> val) {
-    const int b = row / ndf, d = row - b * ndf;
-    R[b * 3 + (d == vd0 ? 0 : d == vd1 ? 1 : 2)] += val.v;
-  }
-};
-
-// Primal values of one (element, area Gauss point) that every tangent
-// direction shares, formed once: a_α and x_,αβ (sums over the 9 nodes of the
-// mesh positions) and the interpolants of the 8 unknowns -- u N for u = 0..7,
-// u N_,1 and u N_,2 for u = 0..5 (zero for an unknown the motion lacks).
+// Primal values of one (element, area Gauss point) formed from the nodes: a_α
+// and x_,αβ (sums over the 9 nodes of the mesh positions) and the interpolants
+// of the 8 unknowns -- u N for u = 0..7, u N_,1 and u N_,2 for u = 0..5 (zero
+// for an unknown the motion lacks).
 constexpr int kPreA = 0, kPreX = 6, kPreN = 15, kPreD0 = 23, kPreD1 = 29, kPre = 35;
 template <class P>
 __device__ __forceinline__ P gp_pre_value(int j, const PhysParams& pp, const P* X, const P* C, const P* f) {
@@ -188,437 +158,899 @@ __device__ __forceinline__ P gp_pre_value(int j, const PhysParams& pp, const P* 
   return s;
 }
 
-// ---- element kernel --------------------------------------------------------------
+// ---- one Gauss point ---------------------------------------------------------------
 // motion is a template parameter; the dof maps are runtime (PhysParams).
 enum { STATIC_ = 1, EUL_ = 2, LAG_ = 3, ALEV_ = 4, ALEVB_ = 5 };
+// basis kinds t (and s): N_,1, N_,2, nn_11, nn_22, nn_12, N
+constexpr int kN = 5;
+
+// A direction of differentiation at a point: interpolant t of one field.
+// comp: its vector component; v, m, l, p: which field; geo: the field moves the
+// mesh (component comp), so the positions follow with dt.
+template <class T>
+struct Seed {
+  int comp, t;
+  bool v, m, l, p, geo;
+  T dt;
+  __device__ __forceinline__ T x(int i, int k) const { return (geo && comp == i && t == k) ? dt : T(0); }
+  __device__ __forceinline__ T vel(int i, int k) const { return (v && comp == i && t == k) ? T(1) : T(0); }
+  __device__ __forceinline__ T mesh(int i, int k) const { return (m && comp == i && t == k) ? T(1) : T(0); }
+  __device__ __forceinline__ T lam() const { return l ? T(1) : T(0); }
+  __device__ __forceinline__ T pres() const { return p ? T(1) : T(0); }
+};
+template <>
+struct Seed<Nil> {
+  __device__ __forceinline__ Nil x(int, int) const { return Nil(); }
+  __device__ __forceinline__ Nil vel(int, int) const { return Nil(); }
+  __device__ __forceinline__ Nil mesh(int, int) const { return Nil(); }
+  __device__ __forceinline__ Nil lam() const { return Nil(); }
+  __device__ __forceinline__ Nil pres() const { return Nil(); }
+};
+
+// What happens to the primal value of a named intermediate: kept as computed,
+// stored for the tangent pass, or (tangent pass) read back -- the compiler then
+// drops its computation.  The index follows the order of evaluation.
+struct Keep {
+  template <class D>
+  __device__ __forceinline__ void operator()(D&) {}
+};
+template <class P>
+struct Store {
+  P* p;
+  int id;
+  __device__ __forceinline__ void operator()(Dual<P, Nil>& x) { p[id++] = x.v; }
+};
+template <class P>
+struct Load {
+  const P* p;
+  int id;
+  template <class T>
+  __device__ __forceinline__ void operator()(Dual<P, T>& x) { x.v = p[id++]; }
+};
+constexpr int kNamed = 74;              // named intermediates of gp_eval at most (ALE, ALEVB)
+constexpr int kPreGam = kPre + 14;     // where Γ^1_k, Γ^2_k, b_k (k = 11, 22, 12) stand in the table
+constexpr int kPrim = kPre + kNamed;   // table stride per point (odd: conflict-free over points)
 
 // One area Gauss point: calc_elem_dof_residuals' GP body (FiniteElement.jl:284-321)
-// with geo_dyn_stress (GeoDynStress.jl:91-178) inlined, on dual numbers.
-template <class P, class T, int MOTION, class Acc>
-__device__ __forceinline__ void area_gp(const PhysParams& pp, const Coef<P>& cf, const P* pre, const P* f, int as,
-                                        int js, int us, P dt, Acc& acc) {
-  const int ndf = pp.ndf;
-  const P w = f[0];
-  const P* N = f + 1;
-  const P* dN0 = f + 10;
-  const P* dN1 = f + 19;
-  const P* dd[3] = {f + 28, f + 37, f + 46};
-  const T sN = T(N[as]), sd0 = T(dN0[as]), sd1 = T(dN1[as]);
-
-  // geometry: a_α, x_,αβ (x itself is not used by the residual); the seed of a
-  // mesh-motion direction is ∂xms[as, js] = Δt
-  Dual<P, T> a[3][2], xab[3][3];
+// with geo_dyn_stress (GeoDynStress.jl:91-178) inlined, on dual numbers.  The
+// residual rows (node-major packing of calc_elem_residual, FiniteElement.jl:
+// 225-239) are linear in the node's basis values -- with the covariant second
+// derivatives nn_k = N_,k - Γ^α_k N_,α,
+//   r_v,i = (a_i,1 S1 + a_i,2 S3) N_,1 + (a_i,1 S3 + a_i,2 S2) N_,2
+//           + n_i M_k J w nn_k - n_i pn J w N,     S = (σ11, σ22, σ12) J w,
+// and likewise for the mesh, pressure and λ rows -- and `out` receives each
+// row's coefficients of (N_,1, N_,2, nn_11, nn_22, nn_12, N): v(i, c[6], Gam),
+// m6(i, c[6], Gam) / m3(i, c of N_,1, N_,2, N) / m1(i, c of N), p(c of N), l(c of N).
+//
+// The directions use the same covariant basis: a position direction t = γ < 2
+// moves a_γ by e_j and x_,k by Γ^γ_k e_j, one with t = 2 + k moves x_,k alone,
+// with weights N_,γ and nn_k of the node.  The derivatives of the geometry are
+// then closed forms without cancellation,
+//   ∂a^αβ = -(a^α_j a^γβ + a^αγ a^β_j), ∂n = -n_j a^γ, ∂J = J a^γ_j,
+//   ∂a^α = a^αγ n_j n - a^α_j a^γ, ∂b_k = 0, ∂Γ^α_k = a^αγ n_j b_k    (t = γ),
+//   ∂b_k = n_j, ∂Γ^α_k = a^α_j, nothing else                       (t = 2 + k)
+// where N_,k-based directions would leave differences of terms of the size of
+// the parametrisation's Γ N_,α to the rounding.  The row coefficients of N_,α
+// carry the change of nn_k: -n_i M_k J w ∂Γ^α_k.
+template <class P, class T, int MOTION, class Named, class Out>
+__device__ __forceinline__ void gp_eval(const Coef<P>& cf, const P* pre, const P w, const Seed<T>& sd, Named nm,
+                                        Out& out) {
+  using D = Dual<P, T>;
+  constexpr bool kTan = !std::is_same<T, Nil>::value;
+  auto val = [](P v) { return cst<P, T>(v); };
+  // geometry: a_α, x_,αβ (x itself is not used by the residual)
+  D a[3][2];
+  P xab[3][3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    T g = (i == js) ? T(dt) : T(0);
-    a[i][0] = mk<P, T>(pre[kPreA + 2 * i], g * sd0);
-    a[i][1] = mk<P, T>(pre[kPreA + 2 * i + 1], g * sd1);
+    a[i][0] = mk<P, T>(pre[kPreA + 2 * i], sd.x(i, 0));
+    a[i][1] = mk<P, T>(pre[kPreA + 2 * i + 1], sd.x(i, 1));
 #pragma unroll
-    for (int k = 0; k < 3; ++k) xab[i][k] = mk<P, T>(pre[kPreX + 3 * i + k], g * T(dd[k][as]));
+    for (int k = 0; k < 3; ++k) xab[i][k] = pre[kPreX + 3 * i + k];
   }
-  Dual<P, T> a11 = a[0][0] * a[0][0] + a[1][0] * a[1][0] + a[2][0] * a[2][0];
-  Dual<P, T> a12 = a[0][0] * a[0][1] + a[1][0] * a[1][1] + a[2][0] * a[2][1];
-  Dual<P, T> a22 = a[0][1] * a[0][1] + a[1][1] * a[1][1] + a[2][1] * a[2][1];
-  Dual<P, T> det = a11 * a22 - a12 * a12;
-  Dual<P, T> idet = inv(det);
-  Dual<P, T> i11 = a22 * idet, i12 = -(a12 * idet), i22 = a11 * idet;  // a^αβ
-  Dual<P, T> aup[3][2];
+  D J, i11, i12, i22, aup[3][2], n[3], bf[3];
+  P Gam[3][2];
+  {
+    auto dot = [&](int k, int l) { return a[0][k].v * a[0][l].v + a[1][k].v * a[1][l].v + a[2][k].v * a[2][l].v; };
+    const P a11 = dot(0, 0), a12 = dot(0, 1), a22 = dot(1, 1);
+    const P det = a11 * a22 - a12 * a12;
+    D idet = val(P(1) / det);
+    nm(idet);
+    J = val(sqrt(det));
+    nm(J);
+    const P iJ = P(1) / J.v;
+    i11 = val(a22 * idet.v), i12 = val(-(a12 * idet.v)), i22 = val(a11 * idet.v);  // a^αβ
+    nm(i11), nm(i12), nm(i22);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    aup[i][0] = a[i][0] * i11 + a[i][1] * i12;
-    aup[i][1] = a[i][0] * i12 + a[i][1] * i22;
+    for (int i = 0; i < 3; ++i) {
+      aup[i][0] = val(a[i][0].v * i11.v + a[i][1].v * i12.v);
+      aup[i][1] = val(a[i][0].v * i12.v + a[i][1].v * i22.v);
+      nm(aup[i][0]), nm(aup[i][1]);
+    }
+    n[0] = val((a[1][0].v * a[2][1].v - a[2][0].v * a[1][1].v) * iJ);
+    n[1] = val((a[2][0].v * a[0][1].v - a[0][0].v * a[2][1].v) * iJ);
+    n[2] = val((a[0][0].v * a[1][1].v - a[1][0].v * a[0][1].v) * iJ);
+    nm(n[0]), nm(n[1]), nm(n[2]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      D g0 = val(xab[0][k] * aup[0][0].v + xab[1][k] * aup[1][0].v + xab[2][k] * aup[2][0].v);
+      D g1 = val(xab[0][k] * aup[0][1].v + xab[1][k] * aup[1][1].v + xab[2][k] * aup[2][1].v);
+      bf[k] = val(xab[0][k] * n[0].v + xab[1][k] * n[1].v + xab[2][k] * n[2].v);
+      nm(g0), nm(g1), nm(bf[k]);
+      Gam[k][0] = g0.v;
+      Gam[k][1] = g1.v;
+    }
   }
-  Dual<P, T> J = dsqrt(det);
-  Dual<P, T> iJ = inv(J);
-  Dual<P, T> n[3];
-  n[0] = (a[1][0] * a[2][1] - a[2][0] * a[1][1]) * iJ;
-  n[1] = (a[2][0] * a[0][1] - a[0][0] * a[2][1]) * iJ;
-  n[2] = (a[0][0] * a[1][1] - a[1][0] * a[0][1]) * iJ;
-  Dual<P, T> Gam[3][2], bf[3];
+  // the direction's scalars: a^α_j and n_j (0 unless it moves the mesh), a^αγ
+  [[maybe_unused]] T u0{}, u1{}, nj{}, ig0{}, ig1{};
+  if constexpr (kTan) {
+    const bool g1 = sd.t == 1;
+    const T gj = sd.geo ? sd.dt : T(0);
+    u0 = gj * T(sd.comp == 0 ? aup[0][0].v : sd.comp == 1 ? aup[1][0].v : aup[2][0].v);
+    u1 = gj * T(sd.comp == 0 ? aup[0][1].v : sd.comp == 1 ? aup[1][1].v : aup[2][1].v);
+    nj = gj * T(sd.comp == 0 ? n[0].v : sd.comp == 1 ? n[1].v : n[2].v);
+    const T fa = sd.t < 2 ? T(1) : T(0);  // moves a_γ
+    const T v0 = fa * u0, v1 = fa * u1, vn = fa * nj;
+    ig0 = T(g1 ? i12.v : i11.v);  // a^0γ
+    ig1 = T(g1 ? i22.v : i12.v);  // a^1γ
+    i11.d = T(-2) * v0 * ig0;
+    i12.d = -(v0 * ig1 + ig0 * v1);
+    i22.d = T(-2) * v1 * ig1;
+    J.d = T(J.v) * (g1 ? v1 : v0);
+    const T p0 = ig0 * vn, p1 = ig1 * vn;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    Gam[k][0] = xab[0][k] * aup[0][0] + xab[1][k] * aup[1][0] + xab[2][k] * aup[2][0];
-    Gam[k][1] = xab[0][k] * aup[0][1] + xab[1][k] * aup[1][1] + xab[2][k] * aup[2][1];
-    bf[k] = xab[0][k] * n[0] + xab[1][k] * n[1] + xab[2][k] * n[2];
+    for (int i = 0; i < 3; ++i) {
+      const T ag = T(g1 ? aup[i][1].v : aup[i][0].v);  // a^γ_i
+      aup[i][0].d = p0 * T(n[i].v) - v0 * ag;
+      aup[i][1].d = p1 * T(n[i].v) - v1 * ag;
+      n[i].d = -(vn * ag);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) bf[k].d = sd.t == 2 + k ? nj : T(0);
   }
   // b^αβ = a⁻¹ b a⁻¹ (symmetric)
-  Dual<P, T> t11 = i11 * bf[0] + i12 * bf[2], t12 = i11 * bf[2] + i12 * bf[1];
-  Dual<P, T> t21 = i12 * bf[0] + i22 * bf[2], t22 = i12 * bf[2] + i22 * bf[1];
-  Dual<P, T> bu11 = t11 * i11 + t12 * i12, bu12 = t11 * i12 + t12 * i22, bu22 = t21 * i12 + t22 * i22;
-  Dual<P, T> H = (i11 * bf[0] + i12 * bf[2] + i12 * bf[2] + i22 * bf[1]) * P(0.5);
-  Dual<P, T> K = (bf[0] * bf[1] - bf[2] * bf[2]) * idet;
+  D t11 = i11 * bf[0] + i12 * bf[2], t12 = i11 * bf[2] + i12 * bf[1];
+  D t21 = i12 * bf[0] + i22 * bf[2], t22 = i12 * bf[2] + i22 * bf[1];
+  nm(t11), nm(t12), nm(t21), nm(t22);
+  D bu11 = t11 * i11 + t12 * i12, bu12 = t11 * i12 + t12 * i22, bu22 = t21 * i12 + t22 * i22;
+  nm(bu11), nm(bu12), nm(bu22);
+  D H = (t11 + t22) * P(0.5);  // tr(a⁻¹ b) / 2
+  nm(H);
+  // K = det b / det a, as a determinant of the mixed components
+  D K = t11 * t22 - t12 * t21;
 
-  // dynamics: interpolants of unknown u (pre-formed), seeded when u is this
-  // direction's unknown; kind 0: N, 1: N_,1, 2: N_,2
-  auto interp = [&](int u, int kind, T swt) -> Dual<P, T> {
-    const P s = pre[(kind == 0 ? kPreN : kind == 1 ? kPreD0 : kPreD1) + u];
-    return mk<P, T>(s, (u == us) ? swt : T(0));
-  };
-  Dual<P, T> dv[3][2];
+  // dynamics
+  D dv[3][2];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    dv[i][0] = interp(i, 1, sd0);
-    dv[i][1] = interp(i, 2, sd1);
+    dv[i][0] = mk<P, T>(pre[kPreD0 + i], sd.vel(i, 0));
+    dv[i][1] = mk<P, T>(pre[kPreD1 + i], sd.vel(i, 1));
   }
-  Dual<P, T> lam = interp(6, 0, sN);
+  D lam = mk<P, T>(pre[kPreN + 6], sd.lam());
 
   // π^αβ = ζv sym(a^αᵀ v_,α a⁻¹)  (GeoDynStress.jl:148-149)
-  auto visc = [&](Dual<P, T> g[3][2], Dual<P, T>& p11, Dual<P, T>& p12, Dual<P, T>& p22) {
-    Dual<P, T> u[3][2];
+  auto visc = [&](const D (&g)[3][2], D& p11, D& p12, D& p22) {
+    D u[3][2];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       u[i][0] = g[i][0] * i11 + g[i][1] * i12;
       u[i][1] = g[i][0] * i12 + g[i][1] * i22;
+      nm(u[i][0]), nm(u[i][1]);
     }
-    Dual<P, T> P11 = aup[0][0] * u[0][0] + aup[1][0] * u[1][0] + aup[2][0] * u[2][0];
-    Dual<P, T> P12 = aup[0][0] * u[0][1] + aup[1][0] * u[1][1] + aup[2][0] * u[2][1];
-    Dual<P, T> P21 = aup[0][1] * u[0][0] + aup[1][1] * u[1][0] + aup[2][1] * u[2][0];
-    Dual<P, T> P22 = aup[0][1] * u[0][1] + aup[1][1] * u[1][1] + aup[2][1] * u[2][1];
+    D P11 = aup[0][0] * u[0][0] + aup[1][0] * u[1][0] + aup[2][0] * u[2][0];
+    D P12 = aup[0][0] * u[0][1] + aup[1][0] * u[1][1] + aup[2][0] * u[2][1];
+    D P21 = aup[0][1] * u[0][0] + aup[1][1] * u[1][0] + aup[2][1] * u[2][0];
+    D P22 = aup[0][1] * u[0][1] + aup[1][1] * u[1][1] + aup[2][1] * u[2][1];
     p11 = (P11 + P11) * cf.zv;
     p12 = (P12 + P21) * cf.zv;
     p22 = (P22 + P22) * cf.zv;
   };
-  Dual<P, T> p11, p12, p22;
+  D p11, p12, p22;
   visc(dv, p11, p12, p22);
   // tr(a^αᵀ v_,α) for rλ (FiniteElement.jl:298)
-  Dual<P, T> tr = aup[0][0] * dv[0][0] + aup[1][0] * dv[1][0] + aup[2][0] * dv[2][0] + aup[0][1] * dv[0][1] +
-               aup[1][1] * dv[1][1] + aup[2][1] * dv[2][1];
+  D tr = aup[0][0] * dv[0][0] + aup[1][0] * dv[1][0] + aup[2][0] * dv[2][0] + aup[0][1] * dv[0][1] +
+         aup[1][1] * dv[1][1] + aup[2][1] * dv[2][1];
+  nm(tr);
   // σ, M in Voigt form (GeoDynStress.jl:150-154)
-  Dual<P, T> cb = cf.kb * (H * H) - cf.kg * K;
-  Dual<P, T> cs = cb + lam;
-  Dual<P, T> hb = H * (P(2) * cf.kb);
-  Dual<P, T> sg0 = i11 * cs - bu11 * hb + p11;
-  Dual<P, T> sg1 = i22 * cs - bu22 * hb + p22;
-  Dual<P, T> sg2 = (i12 * cs - bu12 * hb + p12) * P(2);
-  Dual<P, T> hm = H * (cf.kb + P(2) * cf.kg);
-  Dual<P, T> M0 = i11 * hm - bu11 * cf.kg;
-  Dual<P, T> M1 = i22 * hm - bu22 * cf.kg;
-  Dual<P, T> M2 = (i12 * hm - bu12 * cf.kg) * P(2);
-  Dual<P, T> JW = J * w;
-
-  // mesh-motion quantities
-  Dual<P, T> sm0, sm1, sm2, pm_, vmv[3], nd_;
-  if (MOTION == ALEV_ || MOTION == ALEVB_) {
-    Dual<P, T> dvm[3][2];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      dvm[i][0] = interp(3 + i, 1, sd0);
-      dvm[i][1] = interp(3 + i, 2, sd1);
-    }
-    Dual<P, T> m11, m12, m22;
-    visc(dvm, m11, m12, m22);
-    sm0 = i11 * cb - bu11 * hb + m11;  // GeoDynStress.jl:156-159
-    sm1 = i22 * cb - bu22 * hb + m22;
-    sm2 = (i12 * cb - bu12 * hb + m12) * P(2);
-    pm_ = interp(7, 0, sN);
-    Dual<P, T> nd = cst<P, T>(P(0));
-#pragma unroll
-    for (int i = 0; i < 3; ++i) nd = nd + n[i] * (interp(3 + i, 0, sN) - interp(i, 0, sN));
-    nd_ = nd;
+  D cb = cf.kb * (H * H) - cf.kg * K;
+  D cs = cb + lam;
+  D hb = H * (P(2) * cf.kb);
+  nm(cb), nm(cs), nm(hb);
+  D sg0 = i11 * cs - bu11 * hb + p11;
+  D sg1 = i22 * cs - bu22 * hb + p22;
+  D sg2 = i12 * cs - bu12 * hb + p12;
+  D hm = H * (cf.kb + P(2) * cf.kg);
+  nm(hm);
+  D M0 = i11 * hm - bu11 * cf.kg;
+  D M1 = i22 * hm - bu22 * cf.kg;
+  D M2 = (i12 * hm - bu12 * cf.kg) * P(2);
+  nm(sg0), nm(sg1), nm(sg2), nm(M0), nm(M1), nm(M2);
+  D JW = J * w;
+  nm(JW);
+  D MJ[3] = {M0 * JW, M1 * JW, M2 * JW};  // bending: nn·M J w = sum_k N_,k MJ_k - N_,α GM_α
+  nm(MJ[0]), nm(MJ[1]), nm(MJ[2]);
+  D qm = val(bf[0].v * MJ[0].v + bf[1].v * MJ[1].v + bf[2].v * MJ[2].v);  // M_k J w b_k
+  nm(qm);
+  [[maybe_unused]] T dg0{}, dg1{};  // M_k J w ∂Γ^α_k
+  if constexpr (kTan) {
+    const T mk_ = sd.t == 2 ? T(MJ[0].v) : sd.t == 3 ? T(MJ[1].v) : sd.t == 4 ? T(MJ[2].v) : T(0);
+    const T qn = sd.t < 2 ? nj * T(qm.v) : T(0);
+    dg0 = ig0 * qn + u0 * mk_;
+    dg1 = ig1 * qn + u1 * mk_;
   }
-  Dual<P, T> nv;
-  if (MOTION == EUL_) {
-    Dual<P, T> v[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      v[i] = interp(i, 0, sN);
-      vmv[i] = interp(3 + i, 0, sN);
-    }
-    nv = n[0] * v[0] + n[1] * v[1] + n[2] * v[2];
-  }
-
-  // Residual rows (node-major packing of calc_elem_residual,
-  // FiniteElement.jl:225-239).  Row (node b, dof) of this point is linear in
-  // node b's basis values -- with nn_k(b) = N_,k[b] - Γ^α_k N_,α[b],
-  //   r_v,i = a_i,1 c1 + a_i,2 c2 + n_i (nn·M) J w - n_i pn N J w,
-  //   c1 = (σ11 N_,1 + σ12 N_,2) J w, c2 = (σ22 N_,2 + σ12 N_,1) J w,
-  // and likewise for the mesh, pressure and λ rows -- so each row's
-  // coefficients of (N_,1, N_,2, N_,11, N_,22, N_,12, N) are formed once per
-  // point and the node loop is a 6-term sum per row.
-  const int vd[3] = {pp.dof_of[0], pp.dof_of[1], pp.dof_of[2]};
-  const int mo[3] = {pp.dof_of[3], pp.dof_of[4], pp.dof_of[5]};
-  const int lo = pp.dof_of[6], po = pp.dof_of[7];
-  auto phi6 = [&](int b, P (&ph)[6]) {
-    ph[0] = dN0[b];
-    ph[1] = dN1[b];
-    ph[2] = dd[0][b];
-    ph[3] = dd[1][b];
-    ph[4] = dd[2][b];
-    ph[5] = N[b];
+  auto bend = [&](int i, D c, [[maybe_unused]] T dg) {  // the change of nn_k in the row's coefficient of N_,α
+    if constexpr (kTan) c.d -= T(n[i].v) * dg;
+    return c;
   };
-  const Dual<P, T> JWh = JW * P(0.5);
-  const Dual<P, T> MJ[3] = {M0 * JW, M1 * JW, M2 * JW};  // bending: nn·M J w = sum_k N_,k MJ_k - N_,α GM_α
-  const Dual<P, T> GM0 = Gam[0][0] * MJ[0] + Gam[1][0] * MJ[1] + Gam[2][0] * MJ[2];
-  const Dual<P, T> GM1 = Gam[0][1] * MJ[0] + Gam[1][1] * MJ[1] + Gam[2][1] * MJ[2];
   {
-    const Dual<P, T> S0 = sg0 * JW, S1 = sg1 * JW, S2 = sg2 * JWh, PN = JW * cf.pn;
+    D S0 = sg0 * JW, S1 = sg1 * JW, S2 = sg2 * JW;
+    nm(S0), nm(S1), nm(S2);
+    const D PN = JW * cf.pn;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      if (vd[i] < 0) continue;
-      const Dual<P, T> c[6] = {a[i][0] * S0 + a[i][1] * S2 - n[i] * GM0, a[i][0] * S2 + a[i][1] * S1 - n[i] * GM1,
-                               n[i] * MJ[0], n[i] * MJ[1], n[i] * MJ[2], -(n[i] * PN)};
-#pragma unroll 1
-      for (int b = 0; b < 9; ++b) {
-        P ph[6];
-        phi6(b, ph);
-        acc.lin(vd[i] + ndf * b, c, ph);
-      }
+      const D c[6] = {bend(i, a[i][0] * S0 + a[i][1] * S2, dg0), bend(i, a[i][0] * S2 + a[i][1] * S1, dg1),
+                      n[i] * MJ[0], n[i] * MJ[1], n[i] * MJ[2], -(n[i] * PN)};
+      out.v(i, c, Gam);
     }
   }
-  if (MOTION == ALEV_ || MOTION == ALEVB_) {
-    const Dual<P, T> E0 = sm0 * JW, E1 = sm1 * JW, E2 = sm2 * JWh, PJ = pm_ * JW;
+  if constexpr (MOTION == ALEV_ || MOTION == ALEVB_) {
+    D dvm[3][2];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      if (MOTION == ALEVB_) {  // the mesh rows carry the bending term too
-        const Dual<P, T> c[6] = {a[i][0] * E0 + a[i][1] * E2 - n[i] * GM0, a[i][0] * E2 + a[i][1] * E1 - n[i] * GM1,
-                                 n[i] * MJ[0], n[i] * MJ[1], n[i] * MJ[2], -(n[i] * PJ)};
-#pragma unroll 1
-        for (int b = 0; b < 9; ++b) {
-          P ph[6];
-          phi6(b, ph);
-          acc.lin(mo[i] + ndf * b, c, ph);
-        }
+      dvm[i][0] = mk<P, T>(pre[kPreD0 + 3 + i], sd.mesh(i, 0));
+      dvm[i][1] = mk<P, T>(pre[kPreD1 + 3 + i], sd.mesh(i, 1));
+    }
+    D m11, m12, m22;
+    visc(dvm, m11, m12, m22);
+    D sm0 = i11 * cb - bu11 * hb + m11;  // GeoDynStress.jl:156-159
+    D sm1 = i22 * cb - bu22 * hb + m22;
+    D sm2 = i12 * cb - bu12 * hb + m12;
+    nm(sm0), nm(sm1), nm(sm2);
+    D pm = mk<P, T>(pre[kPreN + 7], sd.pres());
+    D nd = cst<P, T>(P(0));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      D dvn = mk<P, T>(pre[kPreN + 3 + i], sd.mesh(i, kN)) - mk<P, T>(pre[kPreN + i], sd.vel(i, kN));
+      nd = nd + n[i] * dvn;
+    }
+    nm(nd);
+    D E0 = sm0 * JW, E1 = sm1 * JW, E2 = sm2 * JW, PJ = pm * JW;
+    nm(E0), nm(E1), nm(E2), nm(PJ);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      if constexpr (MOTION == ALEVB_) {  // the mesh rows carry the bending term too
+        const D c[6] = {bend(i, a[i][0] * E0 + a[i][1] * E2, dg0), bend(i, a[i][0] * E2 + a[i][1] * E1, dg1),
+                        n[i] * MJ[0], n[i] * MJ[1], n[i] * MJ[2], -(n[i] * PJ)};
+        out.m6(i, c, Gam);
       } else {
-        const Dual<P, T> c[3] = {a[i][0] * E0 + a[i][1] * E2, a[i][0] * E2 + a[i][1] * E1, -(n[i] * PJ)};
-#pragma unroll 1
-        for (int b = 0; b < 9; ++b) {
-          const P ph[3] = {dN0[b], dN1[b], N[b]};
-          acc.lin(mo[i] + ndf * b, c, ph);
-        }
+        const D c[3] = {a[i][0] * E0 + a[i][1] * E2, a[i][0] * E2 + a[i][1] * E1, -(n[i] * PJ)};
+        out.m3(i, c);
       }
     }
-    const Dual<P, T> c[1] = {-(JW * nd_) - pm_ * (w * cf.adb_zv)};
-#pragma unroll 1
-    for (int b = 0; b < 9; ++b) {
-      const P ph[1] = {N[b]};
-      acc.lin(po + ndf * b, c, ph);
-    }
+    out.p(-(JW * nd) - pm * (w * cf.adb_zv));
   }
-  if (MOTION == EUL_) {
+  if constexpr (MOTION == EUL_) {
+    D v[3], vmv[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      const Dual<P, T> c[1] = {(vmv[i] - n[i] * nv) * JW * cf.am};
-#pragma unroll 1
-      for (int b = 0; b < 9; ++b) {
-        const P ph[1] = {N[b]};
-        acc.lin(mo[i] + ndf * b, c, ph);
-      }
+      v[i] = mk<P, T>(pre[kPreN + i], sd.vel(i, kN));
+      vmv[i] = mk<P, T>(pre[kPreN + 3 + i], sd.mesh(i, kN));
+    }
+    D nv = n[0] * v[0] + n[1] * v[1] + n[2] * v[2];
+    nm(nv);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      D s = vmv[i] - n[i] * nv;
+      nm(s);
+      out.m1(i, s * JW * cf.am);
     }
   }
-  {
-    const Dual<P, T> c[1] = {(J * tr - cf.adb_zv * lam) * w};
-#pragma unroll 1
-    for (int b = 0; b < 9; ++b) {
-      const P ph[1] = {N[b]};
-      acc.lin(lo + ndf * b, c, ph);
-    }
-  }
+  out.l((J * tr - cf.adb_zv * lam) * w);
 }
 
-// One boundary Gauss point of calc_bdry_element_residual (FiniteElement.jl:363-384).
-template <class P, class T, class Acc>
-__device__ __forceinline__ void bdry_gp(const PhysParams& pp, const P* X, const P* f, int bdry, int ntype, P nval,
-                                        P mscale, int as, int js, P dt, Acc& acc) {
-  const int ndf = pp.ndf;
-  const P w = f[0];
-  const P* N = f + 1;
-  const P* dN0 = f + 10;
-  const P* dN1 = f + 19;
-  const T sd0 = T(dN0[as]), sd1 = T(dN1[as]);
-  Dual<P, T> a[3][2];
+// ---- one boundary Gauss point ------------------------------------------------------
+// calc_bdry_element_residual (FiniteElement.jl:363-384): the coefficients of
+// N_,1, N_,2 and N of the three velocity rows at one point of boundary `bdry`,
+// out(i, c[3]).  f: the point's table (w, N, N_,1, N_,2); X: the nodes.
+template <class P, class T, class Tab, class Out>
+__device__ __forceinline__ void bdry_eval(const P* X, const Tab* f, int bdry, int ntype, P nval, P mscale,
+                                          const Seed<T>& sd, Out& out) {
+  using D = Dual<P, T>;
+  const P w = P(f[0]);
+  D a[3][2];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     P s0 = 0, s1 = 0;
 #pragma unroll
     for (int b = 0; b < 9; ++b) {
-      s0 += dN0[b] * X[b * 3 + i];
-      s1 += dN1[b] * X[b * 3 + i];
+      s0 += P(f[10 + b]) * X[b * 3 + i];
+      s1 += P(f[19 + b]) * X[b * 3 + i];
     }
-    T g = (i == js) ? T(dt) : T(0);
-    a[i][0] = mk<P, T>(s0, g * sd0);
-    a[i][1] = mk<P, T>(s1, g * sd1);
+    a[i][0] = mk<P, T>(s0, sd.x(i, 0));
+    a[i][1] = mk<P, T>(s1, sd.x(i, 1));
   }
-  Dual<P, T> a11 = a[0][0] * a[0][0] + a[1][0] * a[1][0] + a[2][0] * a[2][0];
-  Dual<P, T> a12 = a[0][0] * a[0][1] + a[1][0] * a[1][1] + a[2][0] * a[2][1];
-  Dual<P, T> a22 = a[0][1] * a[0][1] + a[1][1] * a[1][1] + a[2][1] * a[2][1];
-  Dual<P, T> det = a11 * a22 - a12 * a12;
-  Dual<P, T> idet = inv(det);
-  Dual<P, T> i11 = a22 * idet, i12 = -(a12 * idet), i22 = a11 * idet;
-  Dual<P, T> aup[3][2];
+  D a11 = a[0][0] * a[0][0] + a[1][0] * a[1][0] + a[2][0] * a[2][0];
+  D a12 = a[0][0] * a[0][1] + a[1][0] * a[1][1] + a[2][0] * a[2][1];
+  D a22 = a[0][1] * a[0][1] + a[1][1] * a[1][1] + a[2][1] * a[2][1];
+  D det = a11 * a22 - a12 * a12;
+  D idet = inv(det);
+  D i11 = a22 * idet, i12 = -(a12 * idet), i22 = a11 * idet;
+  D aup[3][2];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     aup[i][0] = a[i][0] * i11 + a[i][1] * i12;
     aup[i][1] = a[i][0] * i12 + a[i][1] * i22;
   }
-  Dual<P, T> iJ = inv(dsqrt(det));
-  Dual<P, T> n[3];
+  D iJ = inv(dsqrt(det));
+  D n[3];
   n[0] = (a[1][0] * a[2][1] - a[2][0] * a[1][1]) * iJ;
   n[1] = (a[2][0] * a[0][1] - a[0][0] * a[2][1]) * iJ;
   n[2] = (a[0][0] * a[1][1] - a[1][0] * a[0][1]) * iJ;
   // τ = ±a_α / |a_α|; the norm is a primal constant (conjugating dot, FiniteElement.jl:448)
-  int col = (bdry == 0 || bdry == 2) ? 0 : 1;
-  const float sgn = (bdry == 0 || bdry == 1) ? 1.0f : -1.0f;
-  P nrm = sqrt(a[0][col].v * a[0][col].v + a[1][col].v * a[1][col].v + a[2][col].v * a[2][col].v);
-  P sc = P(sgn) / nrm;
-  Dual<P, T> tau[3];
+  const bool c0 = bdry == 0 || bdry == 2;
+  const P sgn = (bdry == 0 || bdry == 1) ? P(1) : P(-1);
+  D ac[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) tau[i] = a[i][col] * sc;
-  Dual<P, T> nu[3];
+  for (int i = 0; i < 3; ++i) ac[i] = c0 ? a[i][0] : a[i][1];
+  const P sc = sgn / sqrt(ac[0].v * ac[0].v + ac[1].v * ac[1].v + ac[2].v * ac[2].v);
+  D tau[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) tau[i] = ac[i] * sc;
+  D nu[3];
   nu[0] = tau[1] * n[2] - tau[2] * n[1];
   nu[1] = tau[2] * n[0] - tau[0] * n[2];
   nu[2] = tau[0] * n[1] - tau[1] * n[0];
-  Dual<P, T> t0 = aup[0][0] * tau[0] + aup[1][0] * tau[1] + aup[2][0] * tau[2];
-  Dual<P, T> t1 = aup[0][1] * tau[0] + aup[1][1] * tau[1] + aup[2][1] * tau[2];
-  Dual<P, T> JG = inv(dsqrt(t0 * t0 + t1 * t1));
-  const int vd[3] = {pp.dof_of[0], pp.dof_of[1], pp.dof_of[2]};
+  D t0 = aup[0][0] * tau[0] + aup[1][0] * tau[1] + aup[2][0] * tau[2];
+  D t1 = aup[0][1] * tau[0] + aup[1][1] * tau[1] + aup[2][1] * tau[2];
+  D JG = inv(dsqrt(t0 * t0 + t1 * t1));
+  const D zero = cst<P, T>(P(0));
   if (ntype == MAFEM_STRETCH || ntype == MAFEM_SHEAR) {
-    Dual<P, T> fv[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) fv[i] = (ntype == MAFEM_STRETCH ? nu[i] : tau[i]) * (nval * w);
-    Dual<P, T> fj[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) fj[i] = fv[i] * JG;
-#pragma unroll 1
-    for (int b = 0; b < 9; ++b)
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-        if (vd[i] >= 0) acc(vd[i] + ndf * b, -(fj[i] * N[b]));
+    for (int i = 0; i < 3; ++i) {
+      const D fi = (ntype == MAFEM_STRETCH ? nu[i] : tau[i]) * (nval * w) * JG;
+      const D c[3] = {zero, zero, -fi};
+      out(i, c);
+    }
   } else {  // MOMENT (F_BEND only; other types are rejected on the host)
-    Dual<P, T> nu0 = aup[0][0] * nu[0] + aup[1][0] * nu[1] + aup[2][0] * nu[2];
-    Dual<P, T> nu1 = aup[0][1] * nu[0] + aup[1][1] * nu[1] + aup[2][1] * nu[2];
-    Dual<P, T> s = JG * (nval * mscale * w);
-#pragma unroll 1
-    for (int b = 0; b < 9; ++b) {
-      Dual<P, T> dn = (nu0 * dN0[b] + nu1 * dN1[b]) * s;
+    D s = JG * (nval * mscale * w);
+    D nu0 = (aup[0][0] * nu[0] + aup[1][0] * nu[1] + aup[2][0] * nu[2]) * s;
+    D nu1 = (aup[0][1] * nu[0] + aup[1][1] * nu[1] + aup[2][1] * nu[2]) * s;
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-        if (vd[i] >= 0) acc(vd[i] + ndf * b, -(n[i] * dn));
+    for (int i = 0; i < 3; ++i) {
+      const D c[3] = {-(n[i] * nu0), -(n[i] * nu1), zero};
+      out(i, c);
     }
   }
 }
 
-// Plain form (P = T = double, WANT_R): primal and tangent of every element dof
-// in one pass.  FP32 form (P = T = float, !WANT_R): the tangent alone.
-// elist (optional): evaluate only elements elist[0 .. nlist) and write their
-// rows to r_el[k][q]; area_only: the area Gauss points alone
+// ---- layout of D -------------------------------------------------------------------
+// Per area point: "heavy" blocks of 6 x 5 (s over all six kinds, t over the five
+// derivative kinds) for the pairs of a row field that carries the bending term
+// and a field that moves the mesh, [pair 3 i + j][s][t], padded to kHS values
+// per pair (16-byte reads; the three pairs of a warp in different banks); then
+// "light" pairs of at most 2 x 3, kLS values each.
+template <class P>
+constexpr int kHS = sizeof(P) == 8 ? 30 : 36;
+constexpr int kLS = 6;
+template <int MOTION>
+struct Lay {
+  static constexpr bool ale = MOTION == ALEV_ || MOTION == ALEVB_;
+  static constexpr bool lag = MOTION == LAG_, eul = MOTION == EUL_;
+  static constexpr int nheavy = ale ? 2 : (lag || eul) ? 1 : 0;  // blocks of 9 pairs: v rows, then mesh rows
+  static constexpr int dirs = lag ? 16 : 32;                     // lanes per point in phase 2
+  static constexpr int warps = lag ? 5 : 9;
+  static constexpr int threads = 32 * warps;
+  // light groups of three pairs, in units of pairs
+  static constexpr int vv = 0;                          // (v_i, v_j), i major: 9 pairs (not LAG)
+  static constexpr int vl = lag ? 0 : 9;                // (v_i, λ)
+  static constexpr int lv = vl + 3, ll = lv + 3;        // (λ, v_j), (λ, λ)
+  static constexpr int lm = ll + 1;                     // (λ, m_j) (ALE, EUL)
+  static constexpr int mp = lm + 3, pv = mp + 3, pm = pv + 3, pp = pm + 3;  // ALE: (m_i, p), (p, v_j), (p, m_j), (p, p)
+  static constexpr int mv = lm + 3, mm = mv + 9;        // EUL: (m_i, v_j), (m_i, m_j)
+  static constexpr int nlight = ale ? pp + 1 : eul ? mm + 9 : ll + 1;
+  template <class P>
+  __host__ __device__ static constexpr int light0() { return nheavy * 9 * kHS<P>; }
+  template <class P>
+  __host__ __device__ static constexpr int dsize() { return (light0<P>() + nlight * kLS + 1) & ~1; }
+};
+
+// Phase 2's output: the lane's direction selects where its derivatives go.
+template <class P, int MOTION>
+struct OutD {
+  using LY = Lay<MOTION>;
+  P* D;                 // the point's block
+  int ov, sv, qv, nv;   // v rows: offset, stride per i and per s, number of s (0: none)
+  int om, sm, qm;       // mesh rows (om < 0: none); qm = 0: only the last kind (N) is kept
+  int op, ol;           // pressure, λ rows (< 0: none)
+  template <class T>
+  __device__ __forceinline__ void v(int i, const Dual<P, T> (&c)[6], const P (&)[3][2]) {
+#pragma unroll
+    for (int s = 0; s < 6; ++s)
+      if (s < nv) D[ov + i * sv + s * qv] = c[s].d;
+  }
+  template <class T>
+  __device__ __forceinline__ void m6(int i, const Dual<P, T> (&c)[6], const P (&)[3][2]) {
+    if (om < 0) return;
+#pragma unroll
+    for (int s = 0; s < 6; ++s)
+      if (qm || s == 5) D[om + i * sm + s * qm] = c[s].d;
+  }
+  template <class T>
+  __device__ __forceinline__ void m3(int i, const Dual<P, T> (&c)[3]) {
+    if (om < 0) return;
+    if (qm) {
+      D[om + i * sm] = c[0].d;
+      D[om + i * sm + qm] = c[1].d;
+#pragma unroll
+      for (int s = 2; s < 5; ++s) D[om + i * sm + s * qm] = T(0);
+    }
+    D[om + i * sm + 5 * qm] = c[2].d;
+  }
+  template <class T>
+  __device__ __forceinline__ void m1(int i, const Dual<P, T>& c) {
+    if (om >= 0) D[om + i * sm] = c.d;
+  }
+  template <class T>
+  __device__ __forceinline__ void p(const Dual<P, T>& c) {
+    if (op >= 0) D[op] = c.d;
+  }
+  template <class T>
+  __device__ __forceinline__ void l(const Dual<P, T>& c) {
+    if (ol >= 0) D[ol] = c.d;
+  }
+};
+
+// The direction of lane `dl` (0 .. dirs - 1) and where its derivatives go.
+// LAG: v_j's five derivative kinds (3 x 5), λ; the other motions: v_j with
+// N_,1, N_,2, N (3 x 3), m_j with all six kinds (3 x 6), λ, p.
+template <class P, class T, int MOTION>
+__host__ __device__ __forceinline__ bool direction(int dl, T dt, Seed<T>& sd, OutD<P, MOTION>& o) {
+  using LY = Lay<MOTION>;
+  constexpr int L0 = LY::template light0<P>();
+  sd.dt = dt;
+  sd.comp = 0;
+  sd.t = kN;
+  sd.v = sd.m = sd.l = sd.p = sd.geo = false;
+  o.ov = o.sv = o.qv = o.nv = 0;
+  o.om = -1;
+  o.sm = o.qm = 0;
+  o.op = o.ol = -1;
+  if constexpr (LY::lag) {
+    if (dl < 15) {
+      sd.comp = dl / 5;
+      sd.t = dl - 5 * sd.comp;
+      sd.v = sd.geo = true;
+    } else {
+      sd.l = true;
+    }
+  } else {
+    if (dl < 9) {
+      sd.comp = dl / 3;
+      const int r = dl - 3 * sd.comp;
+      sd.t = r == 2 ? kN : r;
+      sd.v = true;
+    } else if (dl < 27) {
+      sd.comp = (dl - 9) / 6;
+      sd.t = dl - 9 - 6 * sd.comp;
+      sd.m = sd.geo = MOTION != STATIC_;
+      if (MOTION == STATIC_) return false;
+    } else if (dl == 27) {
+      sd.l = true;
+    } else if (dl == 28 && LY::ale) {
+      sd.p = true;
+    } else {
+      return false;
+    }
+  }
+  const int j = sd.comp, t = sd.t;
+  if (sd.geo && t < 5) {
+    o.ov = j * kHS<P> + t;
+    o.sv = 3 * kHS<P>;
+    o.qv = 5;
+    o.nv = 6;
+    if constexpr (LY::ale) {
+      o.om = 9 * kHS<P> + j * kHS<P> + t;
+      o.sm = 3 * kHS<P>;
+      o.qm = 5;
+    }
+  } else if (sd.v && t < 2) {
+    o.ov = L0 + (LY::vv + j) * kLS + t;
+    o.sv = 3 * kLS;
+    o.qv = 3;
+    o.nv = 2;
+  } else if (sd.l) {
+    o.ov = L0 + LY::vl * kLS;
+    o.sv = kLS;
+    o.qv = 3;
+    o.nv = 2;
+  }
+  if constexpr (LY::ale) {
+    if (sd.p) {
+      o.om = L0 + LY::mp * kLS;
+      o.sm = kLS;
+      o.qm = 0;
+      o.op = L0 + LY::pp * kLS;
+    } else if (sd.v && t == kN) {
+      o.op = L0 + (LY::pv + j) * kLS;
+    } else if (sd.m && (t < 2 || t == kN)) {
+      o.op = L0 + (LY::pm + j) * kLS + (t == kN ? 2 : t);
+    }
+  }
+  if constexpr (LY::eul) {
+    if (sd.v && t == kN) {
+      o.om = L0 + (LY::mv + j) * kLS;
+      o.sm = 3 * kLS;
+    } else if (sd.m && (t < 2 || t == kN)) {
+      o.om = L0 + (LY::mm + j) * kLS + (t == kN ? 2 : t);
+      o.sm = 3 * kLS;
+    }
+  }
+  if (sd.l) o.ol = L0 + LY::ll * kLS;
+  else if (sd.v && t < 2) o.ol = L0 + (LY::lv + j) * kLS + t;
+  else if (sd.m && t < 2) o.ol = L0 + (LY::lm + j) * kLS + t;
+  return true;
+}
+
+// Phase 3's light units: a warp takes up to three pairs (27 lanes: pair x node
+// a) of one group.  Row unknown r0 + q dr, column unknown c0 + q dc for pair q;
+// s0, s1 and t0..t2: the kinds (absent ones meet stored zeros).
+struct LightUnit {
+  short pair, npair, r0, dr, c0, dc, s0, s1, t0, t1, t2;
+};
+template <int MOTION>
+__host__ __device__ __forceinline__ LightUnit light_unit(int k) {
+  using LY = Lay<MOTION>;
+  // groups in order; LAG has no (v, v) group of its own
+  if constexpr (!LY::lag) {
+    if (k < 3) return LightUnit{(short)(LY::vv + 3 * k), 3, (short)k, 0, 0, 1, 0, 1, 0, 1, 0};
+    k -= 3;
+  }
+  if (k == 0) return LightUnit{LY::vl, 3, 0, 1, 6, 0, 0, 1, kN, 0, 0};
+  if (k == 1) return LightUnit{LY::lv, 3, 6, 0, 0, 1, kN, 0, 0, 1, 0};
+  if (k == 2) return LightUnit{LY::ll, 1, 6, 0, 6, 0, kN, 0, kN, 0, 0};
+  if constexpr (LY::ale || LY::eul) {
+    if (k == 3) return LightUnit{LY::lm, 3, 6, 0, 3, 1, kN, 0, 0, 1, 0};
+  }
+  if constexpr (LY::eul) {
+    if (k < 7) return LightUnit{(short)(LY::mv + 3 * (k - 4)), 3, (short)(3 + k - 4), 0, 0, 1, kN, 0, kN, 0, 0};
+    return LightUnit{(short)(LY::mm + 3 * (k - 7)), 3, (short)(3 + k - 7), 0, 3, 1, kN, 0, 0, 1, kN};
+  }
+  if (k == 4) return LightUnit{LY::mp, 3, 3, 1, 7, 0, kN, 0, kN, 0, 0};
+  if (k == 5) return LightUnit{LY::pv, 3, 7, 0, 0, 1, kN, 0, kN, 0, 0};
+  if (k == 6) return LightUnit{LY::pm, 3, 7, 0, 3, 1, kN, 0, 0, 1, kN};
+  return LightUnit{LY::pp, 1, 7, 0, 7, 0, kN, 0, kN, 0, 0};
+}
+template <int MOTION>
+__host__ __device__ constexpr int light_units() {
+  return Lay<MOTION>::lag ? 3 : Lay<MOTION>::ale ? 11 : Lay<MOTION>::eul ? 13 : 6;
+}
+
+// Residual rows from the primal coefficients (plain form): c[row field][s] of
+// every point; kCf per point: v 3 x 6, mesh 3 x 6, p, λ.
+constexpr int kCf = 38;
+template <class P>
+struct OutCoef {
+  P* c;
+  __device__ __forceinline__ void v(int i, const Dual<P, Nil> (&x)[6], const P (&)[3][2]) {
+#pragma unroll
+    for (int s = 0; s < 6; ++s) c[i * 6 + s] = x[s].v;
+  }
+  __device__ __forceinline__ void m6(int i, const Dual<P, Nil> (&x)[6], const P (&)[3][2]) {
+#pragma unroll
+    for (int s = 0; s < 6; ++s) c[18 + i * 6 + s] = x[s].v;
+  }
+  __device__ __forceinline__ void m3(int i, const Dual<P, Nil> (&x)[3]) {
+    c[18 + i * 6] = x[0].v;
+    c[18 + i * 6 + 1] = x[1].v;
+#pragma unroll
+    for (int s = 2; s < 5; ++s) c[18 + i * 6 + s] = P(0);
+    c[18 + i * 6 + 5] = x[2].v;
+  }
+  __device__ __forceinline__ void m1(int i, const Dual<P, Nil>& x) {
+#pragma unroll
+    for (int s = 0; s < 5; ++s) c[18 + i * 6 + s] = P(0);
+    c[18 + i * 6 + 5] = x.v;
+  }
+  __device__ __forceinline__ void p(const Dual<P, Nil>& x) { c[36] = x.v; }
+  __device__ __forceinline__ void l(const Dual<P, Nil>& x) { c[37] = x.v; }
+};
+struct OutNone {
+  template <class X, class G>
+  __device__ __forceinline__ void v(int, const X&, const G&) {}
+  template <class X, class G>
+  __device__ __forceinline__ void m6(int, const X&, const G&) {}
+  template <class X>
+  __device__ __forceinline__ void m3(int, const X&) {}
+  template <class X>
+  __device__ __forceinline__ void m1(int, const X&) {}
+  template <class X>
+  __device__ __forceinline__ void p(const X&) {}
+  template <class X>
+  __device__ __forceinline__ void l(const X&) {}
+};
+
+// Shared memory of elem_body, in values of P.  kBd: per boundary point, the
+// 3 x 3 pairs' 3 x 2 derivatives, the nodes' (N_,1, N_,2, N) and the three rows'
+// coefficients.
+constexpr int kBd = 54 + 27 + 9;
+constexpr int kPhi = 54;  // phi[b][s] of a point, then w (stride kTab)
+template <class P, int MOTION>
+constexpr size_t elem_smem_values(int nq, int max_bt) {
+  const size_t ks = (size_t)nq * (nq + 1), tab = 9 * kTab;  // the raw tables share the block's place
+  return 28 + 72 + 9 * kTab + (9 * kPrim + 1) + 9 * kCf + (size_t)max_bt * kBd + 9 * Lay<MOTION>::template dsize<P>() +
+         (ks > tab ? ks : tab);
+}
+
+// One element per CTA iteration: element elist[kk] (or kk), kk < nel.  Plain
+// form (P = double, WANT_R): residual and tangent.  FP32 form (!WANT_R): the
+// tangent alone.  area_only: the area Gauss points alone
 // (calc_elem_dof_residuals without the Dohrmann-Bochev projection or boundary
-// terms, as PullForce.jl uses it); K_el may be null (no tangent written).
-// The element loop of one CTA (CTA number blk of the patch), shared by the
-// single-patch kernel and the batched kernel, which reads Pt / pp from a job
-// table into shared memory.
-template <class P, class T, bool WANT_R, int MOTION, int EPB>
-__device__ __forceinline__ void elem_body(const DevPatch& Pt, const PhysParams& pp, double time, double dt,
-                                          double* __restrict__ r_el, T* __restrict__ K_el,
-                                          const int* __restrict__ elist, int nlist, int area_only, int blk,
-                                          unsigned char* smem_raw) {
-  const int nq = pp.nq, ndf = pp.ndf;
-  const int ldk = nq + 1;
-  const int slot = threadIdx.x / nq;
-  const int q = threadIdx.x - slot * nq;
-  const int kk = blk * EPB + slot;  // element (or list) index of this slot
-  const int e = elist ? (kk < nlist ? elist[kk] : 0) : kk;
-  // per-slot shared memory: X[27], C[72], GP tables [9][kTab], the points'
-  // shared primal values [9][kPre] in P; then the blocks
-  const size_t per_slot = 27 + 72 + 9 * kTab + 9 * kPre;
-  P* base = reinterpret_cast<P*>(smem_raw);
-  P* X = base + slot * per_slot;
-  P* C = X + 27;
-  P* tab = C + 72;
-  P* pre = tab + 9 * kTab;
-  T* Ks = reinterpret_cast<T*>(base + EPB * per_slot) + (size_t)slot * nq * ldk;
-  const bool live = (slot < EPB) && (elist ? kk < nlist : e < Pt.numel);
+// terms, as PullForce.jl uses it); K_el may be null (no tangent formed).
+// Shared by the single-patch kernel and the batched kernel, which reads Pt / pp
+// from a job table into shared memory.
+template <class P, bool WANT_R, int MOTION>
+__device__ __forceinline__ void elem_one(const DevPatch& Pt, const PhysParams& pp, double time, double dt,
+                                         double* __restrict__ r_el, P* __restrict__ K_el, int e, int kk, int area_only,
+                                         unsigned char* smem_raw) {
+  using LY = Lay<MOTION>;
+  constexpr int NT = LY::threads, DS = LY::template dsize<P>(), L0 = LY::template light0<P>();
+  const int nq = pp.nq, ndf = pp.ndf, ldk = nq + 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  P* D = reinterpret_cast<P*>(smem_raw);  // [9][DS]
+  P* phi = D + 9 * DS;                    // [9][kTab]: phi[b][s], w at kPhi
+  P* C = phi + 9 * kTab;                  // [9][8]
+  P* X = C + 72;                          // [9][3]
+  P* prim = X + 28;                       // [9][kPrim]
+  P* cf9 = prim + 9 * kPrim + 1;          // [9][kCf]
+  P* bd = cf9 + 9 * kCf;                  // [boundary point][kBd]
+  P* Ks = bd + pp.max_btask * kBd;        // [nq][ldk]: column, row
+  P* tab = Ks;                            // [9][kTab]: the raw tables, until the interpolants are formed
 
-  if (live) {
-    const int u = Pt.uel[e];
-    for (int k = q; k < 9 * kTab; k += nq) tab[k] = P(Pt.tab[(size_t)u * 9 * kTab + k]);
-    for (int k = q; k < 27; k += nq) {
-      int b = k / 3, i = k - 3 * (k / 3);
-      X[k] = P(Pt.xms[(size_t)i * Pt.numnp + Pt.ix[e * 9 + b]]);
+  // phase 0
+  const int u = Pt.uel[e];
+  for (int k = tid; k < 9 * kTab; k += NT) {
+    const P v = P(Pt.tab[(size_t)u * 9 * kTab + k]);
+    tab[k] = v;
+    const int g = k / kTab, r = k - g * kTab;
+    if (r == 0) phi[g * kTab + kPhi] = v;
+    else if (r < 10) phi[g * kTab + (r - 1) * 6 + kN] = v;
+    else if (r < 55) phi[g * kTab + ((r - 10) % 9) * 6 + (r - 10) / 9] = v;
+  }
+  for (int k = tid; k < 27; k += NT) {
+    const int b = k / 3, i = k - 3 * b;
+    X[k] = P(Pt.xms[(size_t)i * Pt.numnp + Pt.ix[e * 9 + b]]);
+  }
+  for (int k = tid; k < 72; k += NT) {
+    const int b = k / 8, d = k - 8 * b;
+    C[k] = d < ndf ? P(Pt.cps[(size_t)d * Pt.numnp + Pt.ix[e * 9 + b]]) : P(0);
+  }
+  if (K_el)
+    for (int k = tid; k < 9 * LY::nlight * kLS; k += NT) {
+      const int g = k / (LY::nlight * kLS);
+      D[g * DS + L0 + k - g * LY::nlight * kLS] = P(0);
     }
-    for (int k = q; k < 72; k += nq) {
-      int b = k / 8, d = k - 8 * (k / 8);
-      C[k] = d < ndf ? P(Pt.cps[(size_t)d * Pt.numnp + Pt.ix[e * 9 + b]]) : P(0);
-    }
-    for (int k = q; k < nq * ldk; k += nq) Ks[k] = T(0.0);
+  // the element's boundary points: (Neumann entry, point)
+  int nbt = 0;
+  if (!area_only)
+    for (int k = 0; k < pp.n_neu; ++k) nbt += Pt.bref[e * 4 + pp.neu_bdry[k]] >= 0 ? 3 : 0;
+  __syncthreads();
+  for (int k = tid; k < 9 * kPre; k += NT) {
+    const int gp = k / kPre;
+    prim[gp * kPrim + k - gp * kPre] = gp_pre_value<P>(k - gp * kPre, pp, X, C, tab + gp * kTab);
   }
   __syncthreads();
-  if (live)
-    for (int k = q; k < 9 * kPre; k += nq) {
-      const int gp = k / kPre;
-      pre[k] = gp_pre_value<P>(k - gp * kPre, pp, X, C, tab + gp * kTab);
+  // phase 1
+  const Coef<P> cf(pp);
+  if (tid < 9) {
+    P* pr = prim + tid * kPrim;
+    if constexpr (WANT_R) {
+      OutCoef<P> oc{cf9 + tid * kCf};
+      gp_eval<P, Nil, MOTION>(cf, pr, phi[tid * kTab + kPhi], Seed<Nil>(), Store<P>{pr, kPre}, oc);
+    } else {
+      OutNone oc;
+      gp_eval<P, Nil, MOTION>(cf, pr, phi[tid * kTab + kPhi], Seed<Nil>(), Store<P>{pr, kPre}, oc);
     }
-  __syncthreads();
-  if (live) {
-    const int as = q / ndf, ds = q - as * ndf;
-    const int us = pp.unk_of[ds];
-    const int js = (pp.mmo[0] == ds) ? 0 : (pp.mmo[1] == ds) ? 1 : (pp.mmo[2] == ds) ? 2 : -1;
-    const Coef<P> cf(pp);
-    const P pdt = P(dt);
-    AccTan<P, T, WANT_R> acc{Ks, ldk, q, P(0)};
-
-#pragma unroll 1
-    for (int gp = 0; gp < 9; ++gp)
-      area_gp<P, T, MOTION>(pp, cf, pre + gp * kPre, tab + gp * kTab, as, js, us, pdt, acc);
-
-    // Dohrmann-Bochev projection (FiniteElement.jl:323-327): rλ += Gᵀ H⁻¹ G λ αdb/ζv,
-    // and for ALEV/ALEVB rp += Gᵀ H⁻¹ G p αdb/ζv.  Linear in λ / p.
-    if (!area_only) {
-      const double* T81 = Pt.db + (size_t)Pt.uel[e] * 81;
-      const double s = pp.adb / pp.zv;
-      const int lo = pp.dof_of[6], po = pp.dof_of[7];
-      const bool alep = (MOTION == ALEV_ || MOTION == ALEVB_);
-      for (int b = 0; b < 9; ++b) {
-        const int rowl = lo + ndf * b;
-        if (us == 6) Ks[rowl * ldk + q] += T(T81[b * 9 + as] * s);
-        if (alep && us == 7) Ks[(po + ndf * b) * ldk + q] += T(T81[b * 9 + as] * s);
-        if (WANT_R) {
-          double sl = 0, sp = 0;
-          for (int c = 0; c < 9; ++c) {
-            sl += T81[b * 9 + c] * C[c * 8 + lo];
-            if (alep) sp += T81[b * 9 + c] * C[c * 8 + po];
+  }
+  if (K_el)  // the raw tables in Ks are no longer read: the block starts at zero
+    for (int k = tid; k < nq * ldk; k += NT) Ks[k] = P(0);
+  // boundary points: six directions each (component j, N_,1 / N_,2), five points a warp, taken by the last warps
+  {
+    const int bl = lane / 6, q = lane - 6 * bl;  // point slot, direction
+    for (int b0 = (LY::warps - 1 - warp) * 5; b0 < nbt; b0 += LY::warps * 5) {
+      const int bt = b0 + bl;
+      if (bl < 5 && bt < nbt) {
+        int k = 0, left = bt;  // the bt-th (entry, point)
+        for (; k < pp.n_neu; ++k) {
+          if (Pt.bref[e * 4 + pp.neu_bdry[k]] < 0) continue;
+          if (left < 3) break;
+          left -= 3;
+        }
+        const int bb = pp.neu_bdry[k], ntype = pp.neu_type[k];
+        const double* src = Pt.btab + ((size_t)Pt.bref[e * 4 + bb] * 3 + left) * kTab;
+        const P mscale = P(ntype == MAFEM_MOMENT ? fmin(time / pp.bend_tm, 1.0) : 1.0);
+        Seed<P> sd;
+        sd.comp = q >> 1;
+        sd.t = q & 1;
+        sd.v = sd.m = sd.l = sd.p = false;
+        sd.geo = MOTION != STATIC_;
+        sd.dt = P(dt);
+        P* B = bd + bt * kBd;
+        auto put = [&](int i, const Dual<P, P> (&c)[3]) {
+#pragma unroll
+          for (int s = 0; s < 3; ++s) {
+            B[(i * 3 + (q >> 1)) * 6 + s * 2 + (q & 1)] = c[s].d;
+            if (q == 0) B[81 + i * 3 + s] = c[s].v;
           }
-          if (rowl == q) acc.rsum += sl * s;
-          if (alep && po + ndf * b == q) acc.rsum += sp * s;
+        };
+        bdry_eval<P, P>(X, src, bb, ntype, P(pp.neu_val[k]), mscale, sd, put);
+        for (int k2 = q; k2 < 27; k2 += 6) {
+          const int b = k2 / 3, s = k2 - 3 * b;
+          B[54 + k2] = P(src[s == 2 ? 1 + b : 10 + 9 * s + b]);
         }
       }
     }
-
-    // Neumann boundary terms of this element (calc_r_K's boundary loop,
-    // FiniteElement.jl:150-197): same LM, so they add into the same block.
-    for (int k = 0; k < (area_only ? 0 : pp.n_neu); ++k) {
-      const int b = pp.neu_bdry[k];
-      const int row = Pt.bref[e * 4 + b];
-      if (row < 0) continue;
-      const P mscale = P(pp.neu_type[k] == MAFEM_MOMENT ? fmin(time / pp.bend_tm, 1.0) : 1.0);
-      for (int g = 0; g < 3; ++g) {
-        const double* src = Pt.btab + ((size_t)row * 3 + g) * kTab;
-        if constexpr (sizeof(P) == sizeof(double)) {
-          bdry_gp<P, T>(pp, X, src, b, pp.neu_type[k], P(pp.neu_val[k]), mscale, as, js, pdt, acc);
-        } else {
-          P fb[28];  // w, N, dN: the boundary term uses no second derivatives
-          for (int t = 0; t < 28; ++t) fb[t] = P(src[t]);
-          bdry_gp<P, T>(pp, X, fb, b, pp.neu_type[k], P(pp.neu_val[k]), mscale, as, js, pdt, acc);
-        }
-      }
-    }
-    if (WANT_R) r_el[(size_t)(elist ? kk : e) * nq + q] = acc.rsum;
   }
   __syncthreads();
-  if (live && K_el) {
-    // column-major element block K_el[e][col][row] (coalesced stores)
-    T* dst = K_el + (size_t)e * nq * nq;
-    for (int idx = q; idx < nq * nq; idx += nq) {
-      int c = idx / nq, r = idx - c * nq;
-      dst[idx] = Ks[r * ldk + c];
+  // nn_k[b] = N_,k - Γ^α_k N_,α in place of N_,k (Γ: named intermediates of gp_eval)
+  for (int k = tid; k < 243; k += NT) {
+    const int g = k / 27, r = k - 27 * g, b = r / 3, kk2 = r - 3 * b;
+    const P* G = prim + g * kPrim + kPreGam + 3 * kk2;
+    P* ph = phi + g * kTab + b * 6;
+    ph[2 + kk2] -= G[0] * ph[0] + G[1] * ph[1];
+  }
+  __syncthreads();
+  if (K_el) {
+    // phase 2
+    constexpr int PPW = 32 / LY::dirs;  // points per warp
+    const int gp = warp * PPW + lane / LY::dirs, dl = lane % LY::dirs;
+    if (gp < 9) {
+      Seed<P> sd;
+      OutD<P, MOTION> o;
+      o.D = D + gp * DS;
+      if (direction<P, P, MOTION>(dl, P(dt), sd, o)) {
+        const P* pr = prim + gp * kPrim;
+        gp_eval<P, P, MOTION>(cf, pr, phi[gp * kTab + kPhi], sd, Load<P>{pr, kPre}, o);
+      }
     }
+    __syncthreads();
+    // phase 3
+    const int q = lane / 9, na = lane - 9 * q;  // pair and column node of this lane
+    const bool on = q < 3;
+    const double dbs = pp.adb / pp.zv;
+    for (int un = warp; un < 3 * LY::nheavy; un += LY::warps) {  // heavy: row field `un`, column field m_q (LAG: v_q)
+      if (on) {
+        P acc[9];
+#pragma unroll
+        for (int b = 0; b < 9; ++b) acc[b] = P(0);
+        const P* Dp = D + (un * 3 + q) * kHS<P>;
+#pragma unroll 1
+        for (int g = 0; g < 9; ++g) {
+          const P* ph = phi + g * kTab;
+          P pt[5], W[6];
+#pragma unroll
+          for (int t = 0; t < 5; ++t) pt[t] = ph[na * 6 + t];
+#pragma unroll
+          for (int s = 0; s < 6; ++s) {
+            W[s] = Dp[g * DS + s * 5] * pt[0];
+#pragma unroll
+            for (int t = 1; t < 5; ++t) W[s] += Dp[g * DS + s * 5 + t] * pt[t];
+          }
+#pragma unroll
+          for (int b = 0; b < 9; ++b) {  // FP32: the point's sum first, one rounding at the size of acc per point
+            P v = sizeof(P) == 8 ? acc[b] + ph[b * 6] * W[0] : ph[b * 6] * W[0];
+#pragma unroll
+            for (int s = 1; s < 6; ++s) v += ph[b * 6 + s] * W[s];
+            acc[b] = sizeof(P) == 8 ? v : acc[b] + v;
+          }
+        }
+        if (un < 3)  // the velocity rows' boundary points
+          for (int bt = 0; bt < nbt; ++bt) {
+            const P* B = bd + bt * kBd;
+            const P p0 = B[54 + na * 3], p1 = B[54 + na * 3 + 1];
+            P W[3];
+#pragma unroll
+            for (int s = 0; s < 3; ++s) W[s] = B[(un * 3 + q) * 6 + 2 * s] * p0 + B[(un * 3 + q) * 6 + 2 * s + 1] * p1;
+#pragma unroll
+            for (int b = 0; b < 9; ++b)
+#pragma unroll
+              for (int s = 0; s < 3; ++s) acc[b] += B[54 + b * 3 + s] * W[s];
+          }
+        const int rd = pp.dof_of[un], cd = pp.dof_of[(LY::lag ? 0 : 3) + q];
+        if (rd >= 0 && cd >= 0) {
+          P* dst = Ks + (na * ndf + cd) * ldk + rd;
+#pragma unroll
+          for (int b = 0; b < 9; ++b) dst[b * ndf] = acc[b];
+        }
+      }
+    }
+    // light units: the warps without a heavy one (every warp when there are none)
+    constexpr int w0 = 3 * LY::nheavy;
+    for (int k = warp - w0; k >= 0 && k < light_units<MOTION>(); k += LY::warps - w0) {
+      const LightUnit U = light_unit<MOTION>(k);
+      if (on && q < U.npair) {
+        const int ru = U.r0 + q * U.dr, cu = U.c0 + q * U.dc;
+        const int rd = pp.dof_of[ru], cd = pp.dof_of[cu];
+        P acc[9];
+#pragma unroll
+        for (int b = 0; b < 9; ++b) acc[b] = P(0);
+        if (ru == cu && ru >= 6 && !area_only) {
+          // Dohrmann-Bochev projection (FiniteElement.jl:323-327): rλ += Gᵀ H⁻¹ G λ αdb/ζv,
+          // and for ALEV/ALEVB rp += Gᵀ H⁻¹ G p αdb/ζv.  Linear in λ / p.
+          const double* T81 = Pt.db + (size_t)u * 81;
+#pragma unroll
+          for (int b = 0; b < 9; ++b) acc[b] = P(T81[b * 9 + na] * dbs);
+        }
+        const P* Dp = D + L0 + (U.pair + q) * kLS;
+#pragma unroll 1
+        for (int g = 0; g < 9; ++g) {
+          const P* ph = phi + g * kTab;
+          const P p0 = ph[na * 6 + U.t0], p1 = ph[na * 6 + U.t1], p2 = ph[na * 6 + U.t2];
+          const P* Dg = Dp + g * DS;
+          const P W0 = Dg[0] * p0 + Dg[1] * p1 + Dg[2] * p2, W1 = Dg[3] * p0 + Dg[4] * p1 + Dg[5] * p2;
+#pragma unroll
+          for (int b = 0; b < 9; ++b) acc[b] += ph[b * 6 + U.s0] * W0 + ph[b * 6 + U.s1] * W1;
+        }
+        if (rd >= 0 && cd >= 0) {
+          P* dst = Ks + (na * ndf + cd) * ldk + rd;
+#pragma unroll
+          for (int b = 0; b < 9; ++b) dst[b * ndf] = acc[b];
+        }
+      }
+    }
+  }
+  if constexpr (WANT_R) {
+    for (int row = NT - 1 - tid; row < nq; row += NT) {  // the last warps: they hold the light units
+      const int b = row / ndf, d = row - b * ndf, un = pp.unk_of[d];
+      P r = P(0);
+      for (int g = 0; g < 9; ++g) {
+        const P* ph = phi + g * kTab + b * 6;
+        const P* c = cf9 + g * kCf;
+        if (un < 6) {
+          P s = ph[0] * c[un * 6];
+#pragma unroll
+          for (int k = 1; k < 6; ++k) s += ph[k] * c[un * 6 + k];
+          r += s;
+        } else {
+          r += ph[kN] * c[un == 6 ? 37 : 36];
+        }
+      }
+      if (!area_only) {
+        if (un == 6 || (un == 7 && LY::ale)) {
+          const double* T81 = Pt.db + (size_t)u * 81;
+          double s = 0;
+          for (int c = 0; c < 9; ++c) s += T81[b * 9 + c] * C[c * 8 + d];
+          r += s * (pp.adb / pp.zv);
+        }
+        if (un < 3)
+          for (int bt = 0; bt < nbt; ++bt) {
+            const P* B = bd + bt * kBd;
+            r += B[54 + b * 3] * B[81 + un * 3] + B[54 + b * 3 + 1] * B[81 + un * 3 + 1] +
+                 B[54 + b * 3 + 2] * B[81 + un * 3 + 2];
+          }
+      }
+      r_el[(size_t)kk * nq + row] = r;
+    }
+  }
+  if (K_el) {
+    // phase 4: column-major element block K_el[e][col][row]
+    __syncthreads();
+    P* dst = K_el + (size_t)e * nq * nq;
+    for (int c = warp; c < nq; c += LY::warps)
+      for (int r = lane; r < nq; r += 32) dst[c * nq + r] = Ks[c * ldk + r];
   }
 }
 
-template <class P, class T, bool WANT_R, int MOTION, int EPB>
-__global__ void elem_kernel(DevPatch Pt, PhysParams pp, double time, double dt, double* __restrict__ r_el,
-                            T* __restrict__ K_el, const int* __restrict__ elist, int nlist, int area_only) {
+// Two CTAs per SM: one's serial phases (0, 1, 4) run beside the other's FP64
+// work.  In FP64 that holds it to 96 registers, which spills 0.7 KB per thread,
+// yet 32 x 32 ALEVB is assembled in 1.00 ms against 1.11 ms with one CTA and 168
+// registers (both before the closed-form geometry derivatives).
+template <class P, bool WANT_R, int MOTION>
+__global__ void __launch_bounds__(Lay<MOTION>::threads, 2)
+    elem_kernel(DevPatch Pt, PhysParams pp, double time, double dt, double* __restrict__ r_el, P* __restrict__ K_el,
+                const int* __restrict__ elist, int area_only) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  elem_body<P, T, WANT_R, MOTION, EPB>(Pt, pp, time, dt, r_el, K_el, elist, nlist, area_only, blockIdx.x, smem_raw);
+  const int kk = blockIdx.x;
+  elem_one<P, WANT_R, MOTION>(Pt, pp, time, dt, r_el, K_el, elist ? elist[kk] : kk, kk, area_only, smem_raw);
 }
 
 // FP64 residual of the FP32 form: primal only, one thread per (element, area
@@ -627,6 +1059,43 @@ __global__ void elem_kernel(DevPatch Pt, PhysParams pp, double time, double dt, 
 // row) sums them in Gauss-point order and adds the Dohrmann-Bochev term;
 // phase 3: the Neumann points (task = element, bc, point; velocity rows only)
 // likewise, summed in (bc, point) order -- the plain form's order.
+struct OutRows {  // adds a point's rows into R[row]
+  double* R;      // [row]
+  const double* f;
+  const PhysParams& pp;
+  __device__ __forceinline__ void add(int d, const double (&c)[6]) {
+    if (d < 0) return;
+#pragma unroll 1
+    for (int b = 0; b < 9; ++b)
+      R[b * pp.ndf + d] += f[10 + b] * c[0] + f[19 + b] * c[1] + f[28 + b] * c[2] + f[37 + b] * c[3] +
+                           f[46 + b] * c[4] + f[1 + b] * c[5];
+  }
+  __device__ __forceinline__ void addn(int d, double c) {
+    if (d < 0) return;
+#pragma unroll 1
+    for (int b = 0; b < 9; ++b) R[b * pp.ndf + d] += f[1 + b] * c;
+  }
+  // sum_k c_k nn_k = sum_k c_k N_,k - (sum_k c_k Γ^α_k) N_,α
+  __device__ __forceinline__ void addc(int d, const Dual<double, Nil> (&x)[6], const double (&G)[3][2]) {
+    const double c[6] = {x[0].v - (G[0][0] * x[2].v + G[1][0] * x[3].v + G[2][0] * x[4].v),
+                         x[1].v - (G[0][1] * x[2].v + G[1][1] * x[3].v + G[2][1] * x[4].v),
+                         x[2].v, x[3].v, x[4].v, x[5].v};
+    add(d, c);
+  }
+  __device__ __forceinline__ void v(int i, const Dual<double, Nil> (&x)[6], const double (&G)[3][2]) {
+    addc(pp.dof_of[i], x, G);
+  }
+  __device__ __forceinline__ void m6(int i, const Dual<double, Nil> (&x)[6], const double (&G)[3][2]) {
+    addc(pp.dof_of[3 + i], x, G);
+  }
+  __device__ __forceinline__ void m3(int i, const Dual<double, Nil> (&x)[3]) {
+    const double c[6] = {x[0].v, x[1].v, 0.0, 0.0, 0.0, x[2].v};
+    add(pp.dof_of[3 + i], c);
+  }
+  __device__ __forceinline__ void m1(int i, const Dual<double, Nil>& x) { addn(pp.dof_of[3 + i], x.v); }
+  __device__ __forceinline__ void p(const Dual<double, Nil>& x) { addn(pp.dof_of[7], x.v); }
+  __device__ __forceinline__ void l(const Dual<double, Nil>& x) { addn(pp.dof_of[6], x.v); }
+};
 constexpr int kResEPB = 16;  // elements per CTA: 144 threads
 template <int MOTION>
 __device__ __forceinline__ void resid_body(const DevPatch& Pt, const PhysParams& pp, double time, double dt,
@@ -656,8 +1125,8 @@ __device__ __forceinline__ void resid_body(const DevPatch& Pt, const PhysParams&
       double pre[kPre];
 #pragma unroll
       for (int j = 0; j < kPre; ++j) pre[j] = gp_pre_value<double>(j, pp, X + el * 27, C + el * 72, f);
-      AccRes acc{R + (size_t)tid * nq};
-      area_gp<double, Nil, MOTION>(pp, cf, pre, f, 0, -1, -1, dt, acc);
+      OutRows acc{R + (size_t)tid * nq, f, pp};
+      gp_eval<double, Nil, MOTION>(cf, pre, f[0], Seed<Nil>(), Keep(), acc);
     }
   }
   __syncthreads();
@@ -698,9 +1167,13 @@ __device__ __forceinline__ void resid_body(const DevPatch& Pt, const PhysParams&
       const int row = Pt.bref[(e0 + el) * 4 + bd];
       if (row < 0) continue;
       const double mscale = pp.neu_type[k] == MAFEM_MOMENT ? fmin(time / pp.bend_tm, 1.0) : 1.0;
-      AccResV acc{R + (size_t)t * 27, ndf, pp.dof_of[0], pp.dof_of[1]};
-      bdry_gp<double, Nil>(pp, X + el * 27, Pt.btab + ((size_t)row * 3 + g) * kTab, bd, pp.neu_type[k],
-                           pp.neu_val[k], mscale, 0, -1, dt, acc);
+      const double* f = Pt.btab + ((size_t)row * 3 + g) * kTab;
+      double* Rt = R + (size_t)t * 27;  // velocity rows only: [b][i]
+      auto put = [&](int i, const Dual<double, Nil> (&c)[3]) {
+#pragma unroll 1
+        for (int b = 0; b < 9; ++b) Rt[b * 3 + i] += f[10 + b] * c[0].v + f[19 + b] * c[1].v + f[1 + b] * c[2].v;
+      };
+      bdry_eval<double, Nil>(X + el * 27, f, bd, pp.neu_type[k], pp.neu_val[k], mscale, Seed<Nil>(), put);
     }
     __syncthreads();
     const int vd0 = pp.dof_of[0], vd1 = pp.dof_of[1], vd2 = pp.dof_of[2];
@@ -736,8 +1209,6 @@ __global__ void __launch_bounds__(kResEPB * 9) elem_resid_kernel(DevPatch Pt, Ph
 // ---- batched element kernels of the FP32 form: every patch of a round in one launch per motion ----
 // The CTA reads its patch's tables and parameters into shared memory, then runs
 // the single-patch kernel's body on its CTA number within the patch.
-// elements per CTA of the FP32 tangent kernel: 2 or 4, chosen per motion by
-// the batch's autotuner (fewer elements per CTA, more CTAs per SM)
 template <int MOTION>
 __global__ void __launch_bounds__(kResEPB * 9) batch_resid_kernel(const AsmJob* __restrict__ jobs,
                                                                  const AsmItem* __restrict__ items,
@@ -754,9 +1225,13 @@ __global__ void __launch_bounds__(kResEPB * 9) batch_resid_kernel(const AsmJob* 
   __syncthreads();
   resid_body<MOTION>(sP, spp, it.time, it.dt, J->r_el, off[0] + (int)blockIdx.x - off[k], smem_raw);
 }
+// Elements per CTA of the FP32 tangent kernel (one after the other): 2 or 4,
+// chosen per motion by the batch's autotuner (four share a CTA's set-up, two
+// spread small rounds over more SMs).
 template <int MOTION, int EPB>
-__global__ void batch_tan_kernel(const AsmJob* __restrict__ jobs, const AsmItem* __restrict__ items,
-                                 const int* __restrict__ off, int m) {
+__global__ void __launch_bounds__(Lay<MOTION>::threads, 2)
+    batch_tan_kernel(const AsmJob* __restrict__ jobs, const AsmItem* __restrict__ items, const int* __restrict__ off,
+                     int m) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_k;
   __shared__ __align__(16) DevPatch sP;
@@ -767,34 +1242,38 @@ __global__ void batch_tan_kernel(const AsmJob* __restrict__ jobs, const AsmItem*
   batch_copy(&sP, &J->P, (int)sizeof(DevPatch));
   batch_copy(&spp, &J->pp, (int)sizeof(PhysParams));
   __syncthreads();
-  elem_body<float, float, false, MOTION, EPB>(sP, spp, it.time, it.dt, nullptr, J->K_el, nullptr, 0, 0,
-                                                  off[0] + (int)blockIdx.x - off[k], smem_raw);
+  const int e0 = (off[0] + (int)blockIdx.x - off[k]) * EPB;
+#pragma unroll 1
+  for (int e = e0; e < min(e0 + EPB, sP.numel); ++e) {
+    elem_one<float, false, MOTION>(sP, spp, it.time, it.dt, nullptr, J->K_el, e, e, 0, smem_raw);
+    __syncthreads();  // the next element overwrites the block just copied out
+  }
 }
 
 // ---- launchers -----------------------------------------------------------------------
-template <class P, class T>
-static size_t elem_smem(int nq, int epb) {
-  return (size_t)epb * (27 + 72 + 9 * kTab + 9 * kPre) * sizeof(P) + (size_t)epb * nq * (nq + 1) * sizeof(T);
+// The dynamic shared memory a kernel may ask for: the largest element (nq = 72)
+// with the most boundary points it can have (8 Neumann entries).
+template <class P, int MOTION>
+static size_t elem_smem(const PhysParams& pp) {
+  return elem_smem_values<P, MOTION>(pp.nq, pp.max_btask) * sizeof(P);
 }
-template <class T>
-size_t elem_smem_bytes(int nq, int epb) {
-  return elem_smem<T, T>(nq, epb);
+template <class P, int MOTION>
+static size_t elem_smem_cap() {
+  return elem_smem_values<P, MOTION>(72, 3 * kMaxNeu) * sizeof(P);
 }
 static size_t resid_smem(int nq) {
   return (size_t)kResEPB * (27 + 72) * 8 + (size_t)std::max(kResEPB * 9 * nq, kResEPB * 24 * 27) * 8;
 }
 
-template <class P, class T, bool WANT_R, int MOTION, int EPB>
+template <class P, bool WANT_R, int MOTION>
 static cudaError_t launch_elem_t(const DevPatch& Pt, const PhysParams& pp, double time, double dt, double* r_el,
-                                 T* K_el, cudaStream_t st, const int* elist, int nlist, int area_only) {
-  // the cap is the size needed by the largest element (nq = 72), identical for every caller
-  auto kern = elem_kernel<P, T, WANT_R, MOTION, EPB>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)elem_smem<P, T>(72, EPB));
+                                 P* K_el, cudaStream_t st, const int* elist, int nlist, int area_only) {
+  auto kern = elem_kernel<P, WANT_R, MOTION>;
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)elem_smem_cap<P, MOTION>());
   if (e != cudaSuccess) return e;
-  const int blocks = ((elist ? nlist : Pt.numel) + EPB - 1) / EPB;
-  kern<<<blocks, EPB * pp.nq, elem_smem<P, T>(pp.nq, EPB), st>>>(Pt, pp, time, dt, r_el, K_el, elist, nlist,
-                                                                   area_only);
+  const int blocks = elist ? nlist : Pt.numel;
+  kern<<<blocks, Lay<MOTION>::threads, elem_smem<P, MOTION>(pp), st>>>(Pt, pp, time, dt, r_el, K_el, elist, area_only);
   return cudaGetLastError();
 }
 
@@ -814,41 +1293,35 @@ cudaError_t launch_elem<double>(const DevPatch& Pt, const PhysParams& pp, double
                                 double* K_el, cudaStream_t st, const int* elist, int nlist, int area_only) {
   switch (pp.motion) {
     case MAFEM_STATIC:
-      return launch_elem_t<double, double, true, STATIC_, 4>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
+      return launch_elem_t<double, true, STATIC_>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
     case MAFEM_EUL:
-      return launch_elem_t<double, double, true, EUL_, 2>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
+      return launch_elem_t<double, true, EUL_>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
     case MAFEM_LAG:
-      return launch_elem_t<double, double, true, LAG_, 4>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
+      return launch_elem_t<double, true, LAG_>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
     case MAFEM_ALEV:
-      return launch_elem_t<double, double, true, ALEV_, 2>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
+      return launch_elem_t<double, true, ALEV_>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
     default:
-      return launch_elem_t<double, double, true, ALEVB_, 2>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist,
-                                                            area_only);
+      return launch_elem_t<double, true, ALEVB_>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
   }
 }
 
 // FP32 form: the FP64 residual kernel, then the FP32 tangent (whole patch only)
+template <int MOTION>
+static cudaError_t launch_elem_f(const DevPatch& Pt, const PhysParams& pp, double time, double dt, double* r_el,
+                                 float* K_el, cudaStream_t st) {
+  const cudaError_t e = launch_resid_t<MOTION>(Pt, pp, time, dt, r_el, st);
+  return e ? e : launch_elem_t<float, false, MOTION>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0);
+}
 template <>
 cudaError_t launch_elem<float>(const DevPatch& Pt, const PhysParams& pp, double time, double dt, double* r_el,
                                float* K_el, cudaStream_t st, const int* elist, int nlist, int area_only) {
   if (elist || nlist || area_only) return cudaErrorInvalidValue;
-  cudaError_t e;
   switch (pp.motion) {
-    case MAFEM_STATIC:
-      e = launch_resid_t<STATIC_>(Pt, pp, time, dt, r_el, st);
-      return e ? e : launch_elem_t<float, float, false, STATIC_, 4>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0);
-    case MAFEM_EUL:
-      e = launch_resid_t<EUL_>(Pt, pp, time, dt, r_el, st);
-      return e ? e : launch_elem_t<float, float, false, EUL_, 4>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0);
-    case MAFEM_LAG:
-      e = launch_resid_t<LAG_>(Pt, pp, time, dt, r_el, st);
-      return e ? e : launch_elem_t<float, float, false, LAG_, 4>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0);
-    case MAFEM_ALEV:
-      e = launch_resid_t<ALEV_>(Pt, pp, time, dt, r_el, st);
-      return e ? e : launch_elem_t<float, float, false, ALEV_, 4>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0);
-    default:
-      e = launch_resid_t<ALEVB_>(Pt, pp, time, dt, r_el, st);
-      return e ? e : launch_elem_t<float, float, false, ALEVB_, 4>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0);
+    case MAFEM_STATIC: return launch_elem_f<STATIC_>(Pt, pp, time, dt, r_el, K_el, st);
+    case MAFEM_EUL: return launch_elem_f<EUL_>(Pt, pp, time, dt, r_el, K_el, st);
+    case MAFEM_LAG: return launch_elem_f<LAG_>(Pt, pp, time, dt, r_el, K_el, st);
+    case MAFEM_ALEV: return launch_elem_f<ALEV_>(Pt, pp, time, dt, r_el, K_el, st);
+    default: return launch_elem_f<ALEVB_>(Pt, pp, time, dt, r_el, K_el, st);
   }
 }
 
@@ -861,10 +1334,10 @@ static cudaError_t batch_setup_t() {
                                        (int)resid_smem(72));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(batch_tan_kernel<MOTION, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)elem_smem<float, float>(72, 2));
+                             (int)elem_smem_cap<float, MOTION>());
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(batch_tan_kernel<MOTION, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)elem_smem<float, float>(72, 4));
+                             (int)elem_smem_cap<float, MOTION>());
   return e;
 }
 cudaError_t batch_asm_setup() {
@@ -889,29 +1362,25 @@ cudaError_t launch_batch_resid(int motion, const AsmJob* jobs, const AsmItem* it
   }
   return cudaGetLastError();
 }
-template <int EPB>
-static cudaError_t launch_batch_tan_t(int motion, const AsmJob* jobs, const AsmItem* items, const int* off, int m,
-                                      int ctas, int nq, cudaStream_t st) {
-  const size_t sm = elem_smem<float, float>(nq, EPB);
-  const int thr = EPB * nq;
-  switch (motion) {
-    case MAFEM_STATIC: batch_tan_kernel<STATIC_, EPB><<<ctas, thr, sm, st>>>(jobs, items, off, m); break;
-    case MAFEM_EUL: batch_tan_kernel<EUL_, EPB><<<ctas, thr, sm, st>>>(jobs, items, off, m); break;
-    case MAFEM_LAG: batch_tan_kernel<LAG_, EPB><<<ctas, thr, sm, st>>>(jobs, items, off, m); break;
-    case MAFEM_ALEV: batch_tan_kernel<ALEV_, EPB><<<ctas, thr, sm, st>>>(jobs, items, off, m); break;
-    default: batch_tan_kernel<ALEVB_, EPB><<<ctas, thr, sm, st>>>(jobs, items, off, m); break;
+template <int MOTION>
+static void launch_batch_tan_m(int epb, const AsmJob* jobs, const AsmItem* items, const int* off, int m, int ctas,
+                               const PhysParams& pp, cudaStream_t st) {
+  const size_t sm = elem_smem<float, MOTION>(pp);
+  if (epb == 2) batch_tan_kernel<MOTION, 2><<<ctas, Lay<MOTION>::threads, sm, st>>>(jobs, items, off, m);
+  else batch_tan_kernel<MOTION, 4><<<ctas, Lay<MOTION>::threads, sm, st>>>(jobs, items, off, m);
+}
+cudaError_t launch_batch_tan(int epb, const AsmJob* jobs, const AsmItem* items, const int* off, int m, int ctas,
+                             const PhysParams& pp, cudaStream_t st) {
+  if (ctas <= 0) return cudaSuccess;
+  if (epb != 2 && epb != 4) return cudaErrorInvalidValue;
+  switch (pp.motion) {
+    case MAFEM_STATIC: launch_batch_tan_m<STATIC_>(epb, jobs, items, off, m, ctas, pp, st); break;
+    case MAFEM_EUL: launch_batch_tan_m<EUL_>(epb, jobs, items, off, m, ctas, pp, st); break;
+    case MAFEM_LAG: launch_batch_tan_m<LAG_>(epb, jobs, items, off, m, ctas, pp, st); break;
+    case MAFEM_ALEV: launch_batch_tan_m<ALEV_>(epb, jobs, items, off, m, ctas, pp, st); break;
+    default: launch_batch_tan_m<ALEVB_>(epb, jobs, items, off, m, ctas, pp, st); break;
   }
   return cudaGetLastError();
 }
-cudaError_t launch_batch_tan(int motion, int epb, const AsmJob* jobs, const AsmItem* items, const int* off, int m,
-                             int ctas, int nq, cudaStream_t st) {
-  if (ctas <= 0) return cudaSuccess;
-  if (epb == 2) return launch_batch_tan_t<2>(motion, jobs, items, off, m, ctas, nq, st);
-  if (epb == 4) return launch_batch_tan_t<4>(motion, jobs, items, off, m, ctas, nq, st);
-  return cudaErrorInvalidValue;
-}
-
-template size_t elem_smem_bytes<double>(int, int);
-template size_t elem_smem_bytes<float>(int, int);
 
 }  // namespace mafem

@@ -73,6 +73,7 @@ struct PhysParams {
   int neu_type[kMaxNeu];              // SHEAR/STRETCH/MOMENT
   double neu_val[kMaxNeu];
   double bend_tm;
+  int max_btask;                      // boundary Gauss points of one element at most (3 per Neumann entry on it)
 };
 
 struct DevPatch {
@@ -113,8 +114,6 @@ BandLayout make_band_layout(int64_t n, int kl, int ku, int nb);
 #include <cuda.h>  // CUtensorMap
 #include <cuda_runtime.h>
 namespace mafem {
-template <class T>
-size_t elem_smem_bytes(int nq, int epb);
 template <class T>
 cudaError_t launch_elem(const DevPatch& P, const PhysParams& pp, double time, double dt, double* r_el, T* K_el,
                         cudaStream_t st, const int* elist = nullptr, int nlist = 0, int area_only = 0);
@@ -297,8 +296,9 @@ cudaError_t batch_asm_setup();
 // off[0 .. m]); each launch covers CTAs off[0] .. off[m] - 1.
 cudaError_t launch_batch_resid(int motion, const AsmJob* jobs, const AsmItem* items, const int* off, int m, int ctas,
                                int nq, cudaStream_t st);
-cudaError_t launch_batch_tan(int motion, int epb, const AsmJob* jobs, const AsmItem* items, const int* off, int m,
-                             int ctas, int nq, cudaStream_t st);
+// pp: the group's parameters (motion, nq; max_btask: the largest of its patches)
+cudaError_t launch_batch_tan(int epb, const AsmJob* jobs, const AsmItem* items, const int* off, int m, int ctas,
+                             const PhysParams& pp, cudaStream_t st);
 // Both bands and the residual; the residual gather also zeroes each patch's info words.
 void launch_batch_gather(const AsmJob* jobs, const AsmItem* items, const int* off, int m, int ctas, cudaStream_t st);
 void launch_batch_rgather(const AsmJob* jobs, const AsmItem* items, const int* off, int m, int ctas, cudaStream_t st);
