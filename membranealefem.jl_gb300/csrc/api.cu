@@ -139,6 +139,7 @@ struct mafem_handle {
   int* d_rstate = nullptr;              // refinement state {done, sweeps, status} (FP32 form)
   int* h_rstate = nullptr;              // its pinned host copy
   bool no_async = false;                // the next iteration waits for its solve (a redo)
+  bool band_dirty = false;              // the bands hold values outside the rows gather_column writes
   std::unique_ptr<StateWriter> writer;  // state files, created by the first write
   double* d_snap = nullptr;             // device snapshots: nsnap x [xms | cps]
   int nsnap = 0;
@@ -490,6 +491,19 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
   UP(d_tab, tab);
   UP(d_db, db);
   UP(d_btab, btab);
+  // first unknown of every control point, when the unknowns are numbered
+  // control point by control point (the reference's ID numbering)
+  int* d_nf = nullptr;
+  {
+    std::vector<int> nf((size_t)numnp + 1, 0);
+    bool mono = true;
+    for (int64_t q = 0; q < n; ++q) {
+      mono &= q == 0 || unk_node[q] >= unk_node[q - 1];
+      ++nf[(size_t)unk_node[q] + 1];
+    }
+    for (int v = 0; v < numnp; ++v) nf[(size_t)v + 1] += nf[v];
+    if (mono) UP(d_nf, nf);
+  }
   // pivot blocks: the unknowns of one node (consecutive in the ID numbering)
   std::vector<int> blk_end(n);
   int maxblk = 1;
@@ -572,6 +586,7 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
     h->d_band0 = band0;
     h->d_rdiag = rd;
   }
+  h->band_dirty = true;  // cleared by the first gather
   ce = cudaMallocHost(&h->h_out, 20 * sizeof(double));
   if (ce == cudaSuccess) h->h_rstate = reinterpret_cast<int*>(h->h_out + 16);
   if (ce != cudaSuccess) {
@@ -607,18 +622,7 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
       J.npan = h->blk.npan();
       J.num1np = (int)d->num1np;
       J.num2np = (int)d->num2np;
-      // first unknown of every control point, when the unknowns are numbered
-      // control point by control point (the reference's ID numbering)
-      std::vector<int> nf((size_t)numnp + 1, 0);
-      bool mono = true;
-      for (int64_t q = 0; q < n; ++q) {
-        mono &= q == 0 || unk_node[q] >= unk_node[q - 1];
-        ++nf[(size_t)unk_node[q] + 1];
-      }
-      for (int v = 0; v < numnp; ++v) nf[(size_t)v + 1] += nf[v];
-      if (mono) {
-        int* d_nf = nullptr;
-        UP(d_nf, nf);
+      if (d_nf) {
         J.node_first = d_nf;
         J.unk_node = d_un;
       }
@@ -630,7 +634,7 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
   P.num1np = (int)d->num1np; P.num2np = (int)d->num2np; P.nmdf = n;
   P.kl = (int)kl; P.ku = (int)kl;
   P.ix = d_ix; P.lm = d_lm; P.uel = d_uel; P.tab = d_tab; P.db = d_db; P.bref = d_bref; P.btab = d_btab;
-  P.unk_node = d_un; P.unk_dof = d_ud; P.node_unk = d_nu;
+  P.unk_node = d_un; P.unk_dof = d_ud; P.node_unk = d_nu; P.node_first = d_nf;
   P.xms = d_xms; P.cps = d_cps;
   cudaError_t e1, e2;
   if (precision == MAFEM_PLAIN_FP64) {
@@ -690,16 +694,34 @@ extern "C" int mafem_download_state(mafem_handle* h, double* xms, double* cps) {
   return MAFEM_OK;
 }
 
+// The rows of the bands that the gathers do not write (gather_column) are zero
+// unless the band is new, was factored with full partial pivoting or came from
+// the caller: then clear both bands, ordered on st before the next gather.
+static int band_clear(mafem_handle* h, cudaStream_t st) {
+  if (!h->band_dirty) return MAFEM_OK;
+  const size_t bytes = (size_t)h->L.ldb * h->nmdf * (h->precision == MAFEM_PLAIN_FP64 ? 8 : 4);
+  CK(cudaMemsetAsync(h->d_band, 0, bytes, st));
+  if (h->d_band0) CK(cudaMemsetAsync(h->d_band0, 0, bytes, st));
+  h->band_dirty = false;
+  return MAFEM_OK;
+}
+// super-diagonals the next factorisation fills: full partial pivoting fills the
+// top kl rows of the band, which band_clear empties
+static int fill_diagonals(const mafem_handle* h) { return h->use_blk ? h->blk.kuf : (int)h->L.ku; }
+
 // element kernel + gathers: r -> d_r, K -> d_band
 static int assemble(mafem_handle* h, double time, double dt, bool both_bands = false) {
   cudaError_t e;
+  const int rc = band_clear(h, h->st);
+  if (rc) return rc;
   if (h->precision == MAFEM_PLAIN_FP64) {
     e = launch_elem<double>(h->P, h->pp, time, dt, h->d_rel, (double*)h->d_Kel, h->st);
     if (e != cudaSuccess) {
       h->err = std::string("element kernel: ") + cudaGetErrorString(e);
       return MAFEM_ERR_CUDA;
     }
-    launch_band_gather<double>(h->P, h->ndf, h->nq, h->L, (const double*)h->d_Kel, (double*)h->d_band, h->st);
+    launch_band_gather<double>(h->P, h->ndf, h->nq, h->L, fill_diagonals(h), (const double*)h->d_Kel,
+                               (double*)h->d_band, h->st);
     h->launches += 2;
   } else {
     e = launch_elem<float>(h->P, h->pp, time, dt, h->d_rel, (float*)h->d_Kel, h->st);
@@ -707,8 +729,8 @@ static int assemble(mafem_handle* h, double time, double dt, bool both_bands = f
       h->err = std::string("element kernel: ") + cudaGetErrorString(e);
       return MAFEM_ERR_CUDA;
     }
-    launch_band_gather<float>(h->P, h->ndf, h->nq, h->L, (const float*)h->d_Kel, (float*)h->d_band, h->st,
-                              both_bands ? (float*)h->d_band0 : nullptr);
+    launch_band_gather<float>(h->P, h->ndf, h->nq, h->L, fill_diagonals(h), (const float*)h->d_Kel,
+                              (float*)h->d_band, h->st, both_bands ? (float*)h->d_band0 : nullptr);
     h->launches += 2;
   }
   launch_resid_gather(h->P, h->ndf, h->nq, h->d_rel, h->d_r, h->st);
@@ -799,13 +821,15 @@ static int factor(mafem_handle* h, double* x, const double* rhs0) {
       CK(cudaMemcpyAsync(h->d_band, h->host_band, (size_t)h->L.ldb * n * sizeof(double), cudaMemcpyHostToDevice,
                          h->st));
     else if (fp64)
-      launch_band_gather<double>(h->P, h->ndf, h->nq, h->L, (const double*)h->d_Kel, (double*)h->d_band, h->st);
+      launch_band_gather<double>(h->P, h->ndf, h->nq, h->L, fill_diagonals(h), (const double*)h->d_Kel,
+                                 (double*)h->d_band, h->st);
     else
       CK(cudaMemcpyAsync(h->d_band, h->d_band0, (size_t)h->L.ldb * n * sizeof(float), cudaMemcpyDeviceToDevice,
                          h->st));
     if (x && rhs0) CK(cudaMemcpyAsync(x, rhs0, n * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
   }
   CK(cudaMemsetAsync(h->d_info, 0, sizeof(int), h->st));
+  h->band_dirty = true;
   const int nl = fp64 ? band_lu_factor<double>((double*)h->d_band, h->L, h->d_ipiv, h->d_perm, h->rmax, h->d_info, x,
                                                h->apply_threads, h->apply_blocks, h->st, h->st2, h->ev_pool.data(),
                                                nullptr)
@@ -1074,12 +1098,12 @@ static int iter_enqueue(mafem_handle* h) {
   const int64_t n = h->nmdf;
   h->ss_patch = false;
   CK(cudaMemsetAsync(h->d_info, 0, 2 * sizeof(int), h->st));  // zero-pivot column, wait-ran-out word
+  h->ss_async = h->use_blk && h->lu_path != MAFEM_LU_FULL && !h->no_async;
   cudaEventRecord(h->ev[0], h->st);
-  int rc = assemble(h, h->ss_time, h->ss_dt);
+  int rc = assemble(h, h->ss_time, h->ss_dt, h->ss_async && h->precision != MAFEM_PLAIN_FP64);
   if (rc) return rc;
   cudaEventRecord(h->ev[1], h->st);
   h->ss_sweeps = 0;
-  h->ss_async = h->use_blk && h->lu_path != MAFEM_LU_FULL && !h->no_async;
   if (h->ss_async && h->precision == MAFEM_PLAIN_FP64) {
     CK(cudaMemcpyAsync(h->d_x, h->d_r, n * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
     if ((rc = factor_enqueue(h, h->d_x)) != MAFEM_OK) return rc;
@@ -1090,8 +1114,6 @@ static int iter_enqueue(mafem_handle* h) {
     // refinement sweeps (those after convergence return at once); a node block
     // without a usable pivot, or a refinement that did not converge within
     // them, leaves the state unchanged and iter_finish redoes or reports it
-    CK(cudaMemcpyAsync(h->d_band0, h->d_band, (size_t)h->L.ldb * n * sizeof(float), cudaMemcpyDeviceToDevice,
-                       h->st));
     if ((rc = factor_enqueue(h, nullptr)) != MAFEM_OK) return rc;
     cudaEventRecord(h->ev[2], h->st);
     refine_begin(h, h->d_r);
@@ -1548,6 +1570,7 @@ static AsmJob asm_job(const mafem_handle* h) {
   a.dir_idx = h->d_dir_idx;
   a.dir_val = h->d_dir_val;
   a.n_dir = h->n_dir;
+  a.kuf = h->blk.kuf;
   return a;
 }
 
@@ -1859,6 +1882,8 @@ static cudaError_t run_round(RoundRunner& R, const PatchJob* d_jobs, const AsmJo
     return e;
   };
 
+  for (int i : it)  // before the round, outside its graph
+    if (band_clear(hv[i], R.st) != MAFEM_OK) return cudaErrorUnknown;
   if (!R.graph_on) return enqueue(false);
   // the graph's key: everything its nodes bake in (grids, copy sizes, kernel arguments)
   // (a job's shape too: a slot of a server may hold another patch later)
@@ -2813,6 +2838,7 @@ extern "C" int mafem_solve_band(mafem_handle* h, const double* band, int64_t lda
   // the handle's padded layout: column j at j*ldb, the caller's row r at row nb + r
   // (rows 0..nb-1 and nb+rows..ldb-1 of every column are padding, zero)
   std::vector<double> hb64;
+  h->band_dirty = true;
   if (h->precision == MAFEM_PLAIN_FP64) {
     hb64.assign((size_t)L.ldb * n, 0.0);
     for (int64_t j = 0; j < n; ++j)
@@ -2918,9 +2944,11 @@ extern "C" int mafem_profile_factor(mafem_handle* h, double time, double dt, maf
                            nullptr, nullptr, ev.data());
     blk_after_factor(h);
   } else if (fp64) {
+    h->band_dirty = true;
     band_lu_factor<double>((double*)h->d_band, h->L, h->d_ipiv, h->d_perm, h->rmax, h->d_info, h->d_x,
                            h->apply_threads, h->apply_blocks, h->st, nullptr, nullptr, ev.data());
   } else {
+    h->band_dirty = true;
     band_lu_factor<float>((float*)h->d_band, h->L, h->d_ipiv, h->d_perm, h->rmax, h->d_info, nullptr,
                           h->apply_threads, h->apply_blocks, h->st, nullptr, nullptr, ev.data());
   }

@@ -23,49 +23,78 @@ namespace mafem {
 __host__ __device__ __forceinline__ int64_t min64(int64_t a, int64_t b) { return a < b ? a : b; }
 __host__ __device__ __forceinline__ int64_t max64(int64_t a, int64_t b) { return a > b ? a : b; }
 
-// One thread per stored entry of band column j; entries outside the element
-// stencil (structural zeros, pivoting-fill rows, padding) are written as zero,
-// so the band needs no separate clearing pass.
-// Band entry (row j + s - off, column j): the sum of the <= 3 x 3 element
-// contributions, zero outside the element stencil.
+// Band column j, by one warp.  Written are the rows the factorisation may have
+// changed since the last gather -- j - kuf - kBlkW .. j + kl: the fill of
+// node-block pivoting (kuf super-diagonals; a panel's interchanges reach at most
+// kBlkW rows further, where it stores zeros) -- first as zeros in 16-byte
+// stores, then the column's element stencil: the unknowns of 5 x 5 control
+// points, one run of rows per row of the control-point grid, a lane per row
+// adding its <= 3 x 3 element contributions (consecutive rows read consecutive
+// entries of an element's column).  All other rows of the band are zero from
+// its allocation on (full partial pivoting and a caller's band, which fill
+// them, have the whole band cleared before the next gather).  ab2 (optional):
+// the unfactored copy, which nothing overwrites: its stencil rows alone.
+// Bound: the bytes written; one thread per stored entry of the whole column, each
+// finding its control point by division, took 115 us for the 32 x 32 ALEVB FP32
+// band (58 MB, 0.5 TB/s), this MEASGATHER us.
 template <class T>
-__device__ __forceinline__ T band_entry(const DevPatch& P, int ndf, int nq, const BandLayout& L,
-                                        const T* __restrict__ K_el, int64_t j, int s1J, int s2J, int dj, int64_t s) {
-  const int64_t i = j + s - L.off;
-  T val = T(0);
-  if (i >= 0 && i < L.n && i - j >= -L.ku && i - j <= L.kl) {
-    const int NI = P.unk_node[i], di = P.unk_dof[i];
-    const int s1I = NI % P.num1np, s2I = NI / P.num1np;
-    if (abs(s1I - s1J) <= 2 && abs(s2I - s2J) <= 2) {
+__device__ __forceinline__ void gather_column(const DevPatch& P, int ndf, int nq, const BandLayout& L, int kuf,
+                                              const T* __restrict__ K_el, T* __restrict__ ab, T* __restrict__ ab2,
+                                              int64_t j) {
+  constexpr int E = 16 / (int)sizeof(T);
+  const int lane = threadIdx.x & 31;
+  const int NJ = P.unk_node[j], dj = P.unk_dof[j], W = P.num1np;
+  const int s2J = NJ / W, s1J = NJ - s2J * W;
+  {
+    const int s0 = max((int)L.off - kuf - kBlkW, 0) / E, s1 = (int)(L.off + L.kl) / E;
+    float4* col = reinterpret_cast<float4*>(ab + j * L.ldb);
+    for (int v = s0 + lane; v <= s1; v += 32) col[v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+  __syncwarp();  // a row's zero before its value
+  T* col = ab + j * L.ldb + L.off - j;  // + i: row i
+  T* col2 = ab2 ? ab2 + j * L.ldb + L.off - j : nullptr;
+  const int64_t nq2 = (int64_t)nq * nq;
+  const int step1 = (int)nq2 - ndf * nq - ndf;  // the next element along the grid row: nodes a, b one less
+  // unknowns not numbered control point by control point: every row of the band is looked at
+  const int g0 = P.node_first ? max(s2J - 2, 0) : 0, g1 = P.node_first ? min(s2J + 2, P.num2np - 1) : 0;
+  for (int s2g = g0; s2g <= g1; ++s2g) {
+    int lo, hi;
+    if (P.node_first) {
+      lo = P.node_first[s2g * W + max(s1J - 2, 0)];
+      hi = P.node_first[s2g * W + min(s1J + 2, W - 1) + 1];
+    } else {
+      lo = (int)max64(0, j - L.ku);
+      hi = (int)min64(L.n, j + L.kl + 1);
+    }
+    for (int i = lo + lane; i < hi; i += 32) {
+      const int NI = P.unk_node[i], di = P.unk_dof[i];
+      const int s2I = P.node_first ? s2g : NI / W, s1I = NI - s2I * W;
       const int e1lo = max(max(s1I, s1J) - 2, 0), e1hi = min(min(s1I, s1J), P.num1el - 1);
       const int e2lo = max(max(s2I, s2J) - 2, 0), e2hi = min(min(s2I, s2J), P.num2el - 1);
-      for (int e2 = e2lo; e2 <= e2hi; ++e2)
-        for (int e1 = e1lo; e1 <= e1hi; ++e1) {
-          const int e = e1 + P.num1el * e2;
-          const int a = (s1I - e1) + 3 * (s2I - e2), b = (s1J - e1) + 3 * (s2J - e2);
-          val += K_el[(size_t)e * nq * nq + (size_t)(b * ndf + dj) * nq + a * ndf + di];
-        }
+      T val = T(0);
+      const T* src = K_el + (int64_t)(e1lo + P.num1el * e2lo) * nq2 +
+                     (((s1J - e1lo) + 3 * (s2J - e2lo)) * ndf + dj) * nq + ((s1I - e1lo) + 3 * (s2I - e2lo)) * ndf + di;
+      const int64_t step2 = (int64_t)P.num1el * nq2 - 3 * ndf * nq - 3 * ndf;
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (e2lo + q <= e2hi && e1lo + k <= e1hi) val += src[q * step2 + (int64_t)k * step1];
+      if (P.node_first || (e1lo <= e1hi && e2lo <= e2hi)) {
+        col[i] = val;
+        if (col2) col2[i] = val;
+      }
     }
   }
-  return val;
 }
 
-// One thread per stored entry of band column j; entries outside the element
-// stencil (structural zeros, pivoting-fill rows, padding) are written as zero,
-// so the band needs no separate clearing pass.
+constexpr int kGatherWarps = 8;  // columns per CTA
 template <class T>
-__global__ void band_gather_kernel(DevPatch P, int ndf, int nq, BandLayout L, const T* __restrict__ K_el,
-                                   T* __restrict__ ab, T* __restrict__ ab2) {
-  for (int64_t j = blockIdx.y; j < L.n; j += gridDim.y) {
-    const int NJ = P.unk_node[j], dj = P.unk_dof[j];
-    const int s1J = NJ % P.num1np, s2J = NJ / P.num1np;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < L.ldb;
-         s += (int64_t)gridDim.x * blockDim.x) {
-      const T val = band_entry<T>(P, ndf, nq, L, K_el, j, s1J, s2J, dj, s);
-      ab[j * L.ldb + s] = val;
-      if (ab2) ab2[j * L.ldb + s] = val;  // the unfactored copy the refinement multiplies by
-    }
-  }
+__global__ void __launch_bounds__(32 * kGatherWarps)
+    band_gather_kernel(DevPatch P, int ndf, int nq, BandLayout L, int kuf, const T* __restrict__ K_el,
+                       T* __restrict__ ab, T* __restrict__ ab2) {
+  const int64_t j = blockIdx.x * (int64_t)kGatherWarps + (threadIdx.x >> 5);
+  if (j < L.n) gather_column<T>(P, ndf, nq, L, kuf, K_el, ab, ab2, j);
 }
 
 // r[i] = Σ_e r_el[e][(a, di)] over the elements containing node(i) (FiniteElement.jl:131)
@@ -263,24 +292,14 @@ __global__ void sqrt_pair_kernel(const double* __restrict__ part, int nblk, doub
 // order as the per-patch kernels.
 
 // Both bands of the FP32 form, kGatherCols columns per CTA.
-__global__ void __launch_bounds__(256, 4) batch_gather_kernel(const AsmJob* __restrict__ jobs,
-                                                           const AsmItem* __restrict__ items,
-                                                           const int* __restrict__ off, int m) {
+__global__ void __launch_bounds__(32 * kGatherCols) batch_gather_kernel(const AsmJob* __restrict__ jobs,
+                                                                        const AsmItem* __restrict__ items,
+                                                                        const int* __restrict__ off, int m) {
   __shared__ int s_k;
   const int k = batch_item(off, m, &s_k);
   const AsmJob& J = jobs[items[k].job];
-  const BandLayout L = J.L;
-  const int ndf = J.pp.ndf, nq = J.pp.nq;
-  const int64_t j0 = (int64_t)(off[0] + (int)blockIdx.x - off[k]) * kGatherCols;
-  for (int64_t j = j0; j < min64(j0 + kGatherCols, L.n); ++j) {
-    const int NJ = J.P.unk_node[j], dj = J.P.unk_dof[j];
-    const int s1J = NJ % J.P.num1np, s2J = NJ / J.P.num1np;
-    for (int64_t s = threadIdx.x; s < L.ldb; s += blockDim.x) {
-      const float val = band_entry<float>(J.P, ndf, nq, L, J.K_el, j, s1J, s2J, dj, s);
-      J.band[j * L.ldb + s] = val;
-      J.band0[j * L.ldb + s] = val;
-    }
-  }
+  const int64_t j = (int64_t)(off[0] + (int)blockIdx.x - off[k]) * kGatherCols + (threadIdx.x >> 5);
+  if (j < J.L.n) gather_column<float>(J.P, J.pp.ndf, J.pp.nq, J.L, J.kuf, J.K_el, J.band, J.band0, j);
 }
 
 // The residual, 256 unknowns per CTA; the patch's first CTA also zeroes its
@@ -373,7 +392,7 @@ __global__ void __launch_bounds__(256) batch_predictor_kernel(const AsmJob* __re
 
 // ---- launchers -------------------------------------------------------------------
 void launch_batch_gather(const AsmJob* jobs, const AsmItem* items, const int* off, int m, int ctas, cudaStream_t st) {
-  if (ctas > 0) batch_gather_kernel<<<ctas, 256, 0, st>>>(jobs, items, off, m);
+  if (ctas > 0) batch_gather_kernel<<<ctas, 32 * kGatherCols, 0, st>>>(jobs, items, off, m);
 }
 void launch_batch_rgather(const AsmJob* jobs, const AsmItem* items, const int* off, int m, int ctas, cudaStream_t st) {
   if (ctas > 0) batch_rgather_kernel<<<ctas, 256, 0, st>>>(jobs, items, off, m);
@@ -393,10 +412,10 @@ void launch_batch_dirichlet(const AsmJob* jobs, const AsmItem* items, const int*
   if (ctas > 0) batch_dirichlet_kernel<<<ctas, 256, 0, st>>>(jobs, items, off, m);
 }
 template <class T>
-void launch_band_gather(const DevPatch& P, int ndf, int nq, const BandLayout& L, const T* K_el, T* ab,
+void launch_band_gather(const DevPatch& P, int ndf, int nq, const BandLayout& L, int kuf, const T* K_el, T* ab,
                         cudaStream_t st, T* ab2) {
-  dim3 grid((unsigned)((L.ldb + 255) / 256), (unsigned)min64(L.n, 65535));
-  band_gather_kernel<T><<<grid, 256, 0, st>>>(P, ndf, nq, L, K_el, ab, ab2);
+  const unsigned grid = (unsigned)((L.n + kGatherWarps - 1) / kGatherWarps);
+  band_gather_kernel<T><<<grid, 32 * kGatherWarps, 0, st>>>(P, ndf, nq, L, kuf, K_el, ab, ab2);
 }
 void launch_resid_gather(const DevPatch& P, int ndf, int nq, const double* r_el, double* r, cudaStream_t st) {
   const int blocks = (int)min64(1024, (P.nmdf + 255) / 256);
@@ -506,9 +525,9 @@ void launch_axpy(int64_t n, const double* dx, double* x, cudaStream_t st) {
   axpy_kernel<<<blocks, 256, 0, st>>>(n, dx, x);
 }
 
-template void launch_band_gather<double>(const DevPatch&, int, int, const BandLayout&, const double*, double*,
+template void launch_band_gather<double>(const DevPatch&, int, int, const BandLayout&, int, const double*, double*,
                                          cudaStream_t, double*);
-template void launch_band_gather<float>(const DevPatch&, int, int, const BandLayout&, const float*, float*,
+template void launch_band_gather<float>(const DevPatch&, int, int, const BandLayout&, int, const float*, float*,
                                         cudaStream_t, float*);
 template void launch_band_residual<double>(const double*, const BandLayout&, const double*, const double*, double*,
                                            double*, double*, cudaStream_t, const int*);

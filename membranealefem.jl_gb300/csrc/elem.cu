@@ -22,7 +22,7 @@
 // The derivative of |τ| is dropped in the boundary term, exactly as the
 // reference's conjugating `dot` drops it (FiniteElement.jl:448).
 //
-// One CTA per element (elem_body), in phases:
+// One to four elements per CTA (elem_body), in phases:
 //   0  nodes, Gauss-point tables; the interpolants of every point;
 //   1  the primal values of every point, one thread per point, kept in shared
 //      memory (each is needed by every direction; formed once);
@@ -540,6 +540,10 @@ struct Lay {
   static constexpr int dirs = lag ? 16 : 32;                     // lanes per point in phase 2
   static constexpr int warps = lag ? 5 : 9;
   static constexpr int threads = 32 * warps;
+  template <class P>
+  __host__ __device__ static constexpr int ctas() {  // resident CTAs per SM to compile for
+    return lag ? (sizeof(P) == 8 ? 3 : 4) : 2;
+  }
   // light groups of three pairs, in units of pairs
   static constexpr int vv = 0;                          // (v_i, v_j), i major: 9 pairs (not LAG)
   static constexpr int vl = lag ? 0 : 9;                // (v_i, λ)
@@ -551,7 +555,7 @@ struct Lay {
   template <class P>
   __host__ __device__ static constexpr int light0() { return nheavy * 9 * kHS<P>; }
   template <class P>
-  __host__ __device__ static constexpr int dsize() { return (light0<P>() + nlight * kLS + 1) & ~1; }
+  __host__ __device__ static constexpr int dsize() { return (light0<P>() + nlight * kLS + 3) & ~3; }
 };
 
 // Phase 2's output: the lane's direction selects where its derivatives go.
@@ -693,32 +697,33 @@ __host__ __device__ __forceinline__ bool direction(int dl, T dt, Seed<T>& sd, Ou
 
 // Phase 3's light units: a warp takes up to three pairs (27 lanes: pair x node
 // a) of one group.  Row unknown r0 + q dr, column unknown c0 + q dc for pair q;
-// s0, s1 and t0..t2: the kinds (absent ones meet stored zeros).
+// s0: kN, or 0 for the two kinds N_,1, N_,2; t0..t2: the column's kinds (absent
+// ones meet stored zeros).
 struct LightUnit {
-  short pair, npair, r0, dr, c0, dc, s0, s1, t0, t1, t2;
+  short pair, npair, r0, dr, c0, dc, s0, t0, t1, t2;
 };
 template <int MOTION>
 __host__ __device__ __forceinline__ LightUnit light_unit(int k) {
   using LY = Lay<MOTION>;
   // groups in order; LAG has no (v, v) group of its own
   if constexpr (!LY::lag) {
-    if (k < 3) return LightUnit{(short)(LY::vv + 3 * k), 3, (short)k, 0, 0, 1, 0, 1, 0, 1, 0};
+    if (k < 3) return LightUnit{(short)(LY::vv + 3 * k), 3, (short)k, 0, 0, 1, 0, 0, 1, 0};
     k -= 3;
   }
-  if (k == 0) return LightUnit{LY::vl, 3, 0, 1, 6, 0, 0, 1, kN, 0, 0};
-  if (k == 1) return LightUnit{LY::lv, 3, 6, 0, 0, 1, kN, 0, 0, 1, 0};
-  if (k == 2) return LightUnit{LY::ll, 1, 6, 0, 6, 0, kN, 0, kN, 0, 0};
+  if (k == 0) return LightUnit{LY::vl, 3, 0, 1, 6, 0, 0, kN, 0, 0};
+  if (k == 1) return LightUnit{LY::lv, 3, 6, 0, 0, 1, kN, 0, 1, 0};
+  if (k == 2) return LightUnit{LY::ll, 1, 6, 0, 6, 0, kN, kN, 0, 0};
   if constexpr (LY::ale || LY::eul) {
-    if (k == 3) return LightUnit{LY::lm, 3, 6, 0, 3, 1, kN, 0, 0, 1, 0};
+    if (k == 3) return LightUnit{LY::lm, 3, 6, 0, 3, 1, kN, 0, 1, 0};
   }
   if constexpr (LY::eul) {
-    if (k < 7) return LightUnit{(short)(LY::mv + 3 * (k - 4)), 3, (short)(3 + k - 4), 0, 0, 1, kN, 0, kN, 0, 0};
-    return LightUnit{(short)(LY::mm + 3 * (k - 7)), 3, (short)(3 + k - 7), 0, 3, 1, kN, 0, 0, 1, kN};
+    if (k < 7) return LightUnit{(short)(LY::mv + 3 * (k - 4)), 3, (short)(3 + k - 4), 0, 0, 1, kN, kN, 0, 0};
+    return LightUnit{(short)(LY::mm + 3 * (k - 7)), 3, (short)(3 + k - 7), 0, 3, 1, kN, 0, 1, kN};
   }
-  if (k == 4) return LightUnit{LY::mp, 3, 3, 1, 7, 0, kN, 0, kN, 0, 0};
-  if (k == 5) return LightUnit{LY::pv, 3, 7, 0, 0, 1, kN, 0, kN, 0, 0};
-  if (k == 6) return LightUnit{LY::pm, 3, 7, 0, 3, 1, kN, 0, 0, 1, kN};
-  return LightUnit{LY::pp, 1, 7, 0, 7, 0, kN, 0, kN, 0, 0};
+  if (k == 4) return LightUnit{LY::mp, 3, 3, 1, 7, 0, kN, kN, 0, 0};
+  if (k == 5) return LightUnit{LY::pv, 3, 7, 0, 0, 1, kN, kN, 0, 0};
+  if (k == 6) return LightUnit{LY::pm, 3, 7, 0, 3, 1, kN, 0, 1, kN};
+  return LightUnit{LY::pp, 1, 7, 0, 7, 0, kN, kN, 0, 0};
 }
 template <int MOTION>
 __host__ __device__ constexpr int light_units() {
@@ -771,90 +776,133 @@ struct OutNone {
 
 // Shared memory of elem_body, in values of P.  kBd: per boundary point, the
 // 3 x 3 pairs' 3 x 2 derivatives, the nodes' (N_,1, N_,2, N) and the three rows'
-// coefficients.
+// coefficients.  Per element of the CTA: phi, unknowns, positions, primal table,
+// coefficients (plain form) and boundary points; D and the block once.
 constexpr int kBd = 54 + 27 + 9;
 constexpr int kPhi = 54;  // phi[b][s] of a point, then w (stride kTab)
-template <class P, int MOTION>
+template <class P>
+__host__ __device__ constexpr int elem_slot(int max_bt) {
+  return (9 * kTab + 72 + 28 + 9 * kPrim + 1 + (sizeof(P) == 8 ? 9 * kCf : 0) + max_bt * kBd + 3) & ~3;
+}
+template <class P, int MOTION, int EPB>
 constexpr size_t elem_smem_values(int nq, int max_bt) {
-  const size_t ks = (size_t)nq * (nq + 1), tab = 9 * kTab;  // the raw tables share the block's place
-  return 28 + 72 + 9 * kTab + (9 * kPrim + 1) + 9 * kCf + (size_t)max_bt * kBd + 9 * Lay<MOTION>::template dsize<P>() +
-         (ks > tab ? ks : tab);
+  const size_t ks = (size_t)nq * (nq + 1), tab = (size_t)EPB * 9 * kTab;  // the raw tables share the block's place
+  return 9 * Lay<MOTION>::template dsize<P>() + (size_t)EPB * elem_slot<P>(max_bt) + (ks > tab ? ks : tab);
 }
 
-// One element per CTA iteration: element elist[kk] (or kk), kk < nel.  Plain
-// form (P = double, WANT_R): residual and tangent.  FP32 form (!WANT_R): the
-// tangent alone.  area_only: the area Gauss points alone
-// (calc_elem_dof_residuals without the Dohrmann-Bochev projection or boundary
-// terms, as PullForce.jl uses it); K_el may be null (no tangent formed).
-// Shared by the single-patch kernel and the batched kernel, which reads Pt / pp
-// from a job table into shared memory.
-template <class P, bool WANT_R, int MOTION>
-__device__ __forceinline__ void elem_one(const DevPatch& Pt, const PhysParams& pp, double time, double dt,
-                                         double* __restrict__ r_el, P* __restrict__ K_el, int e, int kk, int area_only,
-                                         unsigned char* smem_raw) {
+// 16-byte (N values from a 16-byte boundary) and 2-value shared-memory reads
+template <class P, int N, int M>
+__device__ __forceinline__ void ld_quads(P (&r)[M], const P* p) {
+  constexpr int E = 16 / (int)sizeof(P);
+  using V = typename std::conditional<sizeof(P) == 8, double2, float4>::type;
+#pragma unroll
+  for (int k = 0; k < N / E; ++k) {
+    const V v = reinterpret_cast<const V*>(p)[k];
+    const P* e = reinterpret_cast<const P*>(&v);
+#pragma unroll
+    for (int i = 0; i < E; ++i) r[k * E + i] = e[i];
+  }
+}
+template <class P, int N, int M>
+__device__ __forceinline__ void ld_pairs(P (&r)[M], const P* p) {
+  using V = typename std::conditional<sizeof(P) == 8, double2, float2>::type;
+#pragma unroll
+  for (int k = 0; k < N / 2; ++k) {
+    const V v = reinterpret_cast<const V*>(p)[k];
+    r[2 * k] = v.x;
+    r[2 * k + 1] = v.y;
+  }
+}
+
+// EPB elements per CTA, list positions kk0 .. kk0 + EPB - 1 below nel: elements
+// elist[kk] (or kk).  Phases 0 and 1 run for all of them at once (phase 1 is a
+// chain of ~250 instructions in nine lanes: a warp per element), phases 2 to 4
+// one element after another.  Plain form (P = double, WANT_R): residual and
+// tangent.  FP32 form (!WANT_R): the tangent alone.  area_only: the area Gauss
+// points alone (calc_elem_dof_residuals without the Dohrmann-Bochev projection
+// or boundary terms, as PullForce.jl uses it); K_el may be null (no tangent
+// formed).  Shared by the single-patch kernel and the batched kernel, which
+// reads Pt / pp from a job table into shared memory.
+template <class P, bool WANT_R, int MOTION, int EPB>
+__device__ __forceinline__ void elem_body(const DevPatch& Pt, const PhysParams& pp, double time, double dt,
+                                          double* __restrict__ r_el, P* __restrict__ K_el,
+                                          const int* __restrict__ elist, int kk0, int nel, int area_only,
+                                          unsigned char* smem_raw) {
   using LY = Lay<MOTION>;
+  static_assert(EPB <= LY::warps, "a warp per element in phase 1");
   constexpr int NT = LY::threads, DS = LY::template dsize<P>(), L0 = LY::template light0<P>();
   const int nq = pp.nq, ndf = pp.ndf, ldk = nq + 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ne = min(EPB, nel - kk0), slot = elem_slot<P>(pp.max_btask);
+  auto elem_of = [&](int l) { return elist ? elist[kk0 + l] : kk0 + l; };
   P* D = reinterpret_cast<P*>(smem_raw);  // [9][DS]
-  P* phi = D + 9 * DS;                    // [9][kTab]: phi[b][s], w at kPhi
-  P* C = phi + 9 * kTab;                  // [9][8]
-  P* X = C + 72;                          // [9][3]
-  P* prim = X + 28;                       // [9][kPrim]
-  P* cf9 = prim + 9 * kPrim + 1;          // [9][kCf]
-  P* bd = cf9 + 9 * kCf;                  // [boundary point][kBd]
-  P* Ks = bd + pp.max_btask * kBd;        // [nq][ldk]: column, row
-  P* tab = Ks;                            // [9][kTab]: the raw tables, until the interpolants are formed
+  P* S0 = D + 9 * DS;                     // [EPB][slot]
+  P* Ks = S0 + EPB * slot;                // [nq][ldk]: column, row
+  P* tab = Ks;                            // [EPB][9][kTab]: the raw tables, until the interpolants are formed
+  // places in a slot
+  constexpr int oC = 9 * kTab, oX = oC + 72, oP = oX + 28, oF = oP + 9 * kPrim + 1,
+                oB = oF + (sizeof(P) == 8 ? 9 * kCf : 0);
 
   // phase 0
-  const int u = Pt.uel[e];
-  for (int k = tid; k < 9 * kTab; k += NT) {
-    const P v = P(Pt.tab[(size_t)u * 9 * kTab + k]);
-    tab[k] = v;
+  for (int k0 = tid; k0 < ne * 9 * kTab; k0 += NT) {
+    const int l = k0 / (9 * kTab), k = k0 - l * 9 * kTab;
+    P* phi = S0 + l * slot;  // [9][kTab]: phi[b][s], w at kPhi
+    const P v = P(Pt.tab[(size_t)Pt.uel[elem_of(l)] * 9 * kTab + k]);
+    tab[k0] = v;
     const int g = k / kTab, r = k - g * kTab;
     if (r == 0) phi[g * kTab + kPhi] = v;
     else if (r < 10) phi[g * kTab + (r - 1) * 6 + kN] = v;
     else if (r < 55) phi[g * kTab + ((r - 10) % 9) * 6 + (r - 10) / 9] = v;
   }
-  for (int k = tid; k < 27; k += NT) {
-    const int b = k / 3, i = k - 3 * b;
-    X[k] = P(Pt.xms[(size_t)i * Pt.numnp + Pt.ix[e * 9 + b]]);
+  for (int k0 = tid; k0 < ne * 27; k0 += NT) {
+    const int l = k0 / 27, k = k0 - 27 * l, b = k / 3, i = k - 3 * b;
+    S0[l * slot + oX + k] = P(Pt.xms[(size_t)i * Pt.numnp + Pt.ix[elem_of(l) * 9 + b]]);
   }
-  for (int k = tid; k < 72; k += NT) {
-    const int b = k / 8, d = k - 8 * b;
-    C[k] = d < ndf ? P(Pt.cps[(size_t)d * Pt.numnp + Pt.ix[e * 9 + b]]) : P(0);
+  for (int k0 = tid; k0 < ne * 72; k0 += NT) {
+    const int l = k0 / 72, k = k0 - 72 * l, b = k / 8, d = k - 8 * b;
+    S0[l * slot + oC + k] = d < ndf ? P(Pt.cps[(size_t)d * Pt.numnp + Pt.ix[elem_of(l) * 9 + b]]) : P(0);
   }
-  if (K_el)
+  if (K_el)  // the light pairs' unused places stay zero
     for (int k = tid; k < 9 * LY::nlight * kLS; k += NT) {
       const int g = k / (LY::nlight * kLS);
       D[g * DS + L0 + k - g * LY::nlight * kLS] = P(0);
     }
-  // the element's boundary points: (Neumann entry, point)
-  int nbt = 0;
-  if (!area_only)
-    for (int k = 0; k < pp.n_neu; ++k) nbt += Pt.bref[e * 4 + pp.neu_bdry[k]] >= 0 ? 3 : 0;
+  __shared__ int s_nbt[EPB], s_u[EPB];  // an element's boundary points (Neumann entry, point); its tables
+  if (tid < ne) {
+    const int e = elem_of(tid);
+    int n = 0;
+    if (!area_only)
+      for (int k = 0; k < pp.n_neu; ++k) n += Pt.bref[e * 4 + pp.neu_bdry[k]] >= 0 ? 3 : 0;
+    s_nbt[tid] = n;
+    s_u[tid] = Pt.uel[e];
+  }
   __syncthreads();
-  for (int k = tid; k < 9 * kPre; k += NT) {
-    const int gp = k / kPre;
-    prim[gp * kPrim + k - gp * kPre] = gp_pre_value<P>(k - gp * kPre, pp, X, C, tab + gp * kTab);
+  for (int k0 = tid; k0 < ne * 9 * kPre; k0 += NT) {
+    const int l = k0 / (9 * kPre), k = k0 - l * 9 * kPre, gp = k / kPre;
+    P* S = S0 + l * slot;
+    S[oP + gp * kPrim + k - gp * kPre] =
+        gp_pre_value<P>(k - gp * kPre, pp, S + oX, S + oC, tab + (l * 9 + gp) * kTab);
   }
   __syncthreads();
   // phase 1
   const Coef<P> cf(pp);
-  if (tid < 9) {
-    P* pr = prim + tid * kPrim;
+  if (warp < ne && lane < 9) {
+    P* S = S0 + warp * slot;
+    P* pr = S + oP + lane * kPrim;
     if constexpr (WANT_R) {
-      OutCoef<P> oc{cf9 + tid * kCf};
-      gp_eval<P, Nil, MOTION>(cf, pr, phi[tid * kTab + kPhi], Seed<Nil>(), Store<P>{pr, kPre}, oc);
+      OutCoef<P> oc{S + oF + lane * kCf};
+      gp_eval<P, Nil, MOTION>(cf, pr, S[lane * kTab + kPhi], Seed<Nil>(), Store<P>{pr, kPre}, oc);
     } else {
       OutNone oc;
-      gp_eval<P, Nil, MOTION>(cf, pr, phi[tid * kTab + kPhi], Seed<Nil>(), Store<P>{pr, kPre}, oc);
+      gp_eval<P, Nil, MOTION>(cf, pr, S[lane * kTab + kPhi], Seed<Nil>(), Store<P>{pr, kPre}, oc);
     }
   }
-  if (K_el)  // the raw tables in Ks are no longer read: the block starts at zero
+  if (K_el)  // the raw tables in Ks are no longer read; blocks of uncoupled fields stay zero
     for (int k = tid; k < nq * ldk; k += NT) Ks[k] = P(0);
   // boundary points: six directions each (component j, N_,1 / N_,2), five points a warp, taken by the last warps
-  {
+  for (int l = 0; l < ne; ++l) {
+    const int e = elem_of(l), nbt = s_nbt[l];
+    P* S = S0 + l * slot;
     const int bl = lane / 6, q = lane - 6 * bl;  // point slot, direction
     for (int b0 = (LY::warps - 1 - warp) * 5; b0 < nbt; b0 += LY::warps * 5) {
       const int bt = b0 + bl;
@@ -874,7 +922,7 @@ __device__ __forceinline__ void elem_one(const DevPatch& Pt, const PhysParams& p
         sd.v = sd.m = sd.l = sd.p = false;
         sd.geo = MOTION != STATIC_;
         sd.dt = P(dt);
-        P* B = bd + bt * kBd;
+        P* B = S + oB + bt * kBd;
         auto put = [&](int i, const Dual<P, P> (&c)[3]) {
 #pragma unroll
           for (int s = 0; s < 3; ++s) {
@@ -882,7 +930,7 @@ __device__ __forceinline__ void elem_one(const DevPatch& Pt, const PhysParams& p
             if (q == 0) B[81 + i * 3 + s] = c[s].v;
           }
         };
-        bdry_eval<P, P>(X, src, bb, ntype, P(pp.neu_val[k]), mscale, sd, put);
+        bdry_eval<P, P>(S + oX, src, bb, ntype, P(pp.neu_val[k]), mscale, sd, put);
         for (int k2 = q; k2 < 27; k2 += 6) {
           const int b = k2 / 3, s = k2 - 3 * b;
           B[54 + k2] = P(src[s == 2 ? 1 + b : 10 + 9 * s + b]);
@@ -892,151 +940,178 @@ __device__ __forceinline__ void elem_one(const DevPatch& Pt, const PhysParams& p
   }
   __syncthreads();
   // nn_k[b] = N_,k - Γ^α_k N_,α in place of N_,k (Γ: named intermediates of gp_eval)
-  for (int k = tid; k < 243; k += NT) {
-    const int g = k / 27, r = k - 27 * g, b = r / 3, kk2 = r - 3 * b;
-    const P* G = prim + g * kPrim + kPreGam + 3 * kk2;
-    P* ph = phi + g * kTab + b * 6;
+  for (int k0 = tid; k0 < ne * 243; k0 += NT) {
+    const int l = k0 / 243, k = k0 - 243 * l, g = k / 27, r = k - 27 * g, b = r / 3, kk2 = r - 3 * b;
+    P* S = S0 + l * slot;
+    const P* G = S + oP + g * kPrim + kPreGam + 3 * kk2;
+    P* ph = S + g * kTab + b * 6;
     ph[2 + kk2] -= G[0] * ph[0] + G[1] * ph[1];
   }
   __syncthreads();
-  if (K_el) {
-    // phase 2
-    constexpr int PPW = 32 / LY::dirs;  // points per warp
-    const int gp = warp * PPW + lane / LY::dirs, dl = lane % LY::dirs;
-    if (gp < 9) {
-      Seed<P> sd;
-      OutD<P, MOTION> o;
-      o.D = D + gp * DS;
-      if (direction<P, P, MOTION>(dl, P(dt), sd, o)) {
-        const P* pr = prim + gp * kPrim;
-        gp_eval<P, P, MOTION>(cf, pr, phi[gp * kTab + kPhi], sd, Load<P>{pr, kPre}, o);
-      }
-    }
-    __syncthreads();
-    // phase 3
-    const int q = lane / 9, na = lane - 9 * q;  // pair and column node of this lane
-    const bool on = q < 3;
-    const double dbs = pp.adb / pp.zv;
-    for (int un = warp; un < 3 * LY::nheavy; un += LY::warps) {  // heavy: row field `un`, column field m_q (LAG: v_q)
-      if (on) {
-        P acc[9];
-#pragma unroll
-        for (int b = 0; b < 9; ++b) acc[b] = P(0);
-        const P* Dp = D + (un * 3 + q) * kHS<P>;
 #pragma unroll 1
-        for (int g = 0; g < 9; ++g) {
-          const P* ph = phi + g * kTab;
-          P pt[5], W[6];
-#pragma unroll
-          for (int t = 0; t < 5; ++t) pt[t] = ph[na * 6 + t];
-#pragma unroll
-          for (int s = 0; s < 6; ++s) {
-            W[s] = Dp[g * DS + s * 5] * pt[0];
-#pragma unroll
-            for (int t = 1; t < 5; ++t) W[s] += Dp[g * DS + s * 5 + t] * pt[t];
-          }
-#pragma unroll
-          for (int b = 0; b < 9; ++b) {  // FP32: the point's sum first, one rounding at the size of acc per point
-            P v = sizeof(P) == 8 ? acc[b] + ph[b * 6] * W[0] : ph[b * 6] * W[0];
-#pragma unroll
-            for (int s = 1; s < 6; ++s) v += ph[b * 6 + s] * W[s];
-            acc[b] = sizeof(P) == 8 ? v : acc[b] + v;
-          }
-        }
-        if (un < 3)  // the velocity rows' boundary points
-          for (int bt = 0; bt < nbt; ++bt) {
-            const P* B = bd + bt * kBd;
-            const P p0 = B[54 + na * 3], p1 = B[54 + na * 3 + 1];
-            P W[3];
-#pragma unroll
-            for (int s = 0; s < 3; ++s) W[s] = B[(un * 3 + q) * 6 + 2 * s] * p0 + B[(un * 3 + q) * 6 + 2 * s + 1] * p1;
-#pragma unroll
-            for (int b = 0; b < 9; ++b)
-#pragma unroll
-              for (int s = 0; s < 3; ++s) acc[b] += B[54 + b * 3 + s] * W[s];
-          }
-        const int rd = pp.dof_of[un], cd = pp.dof_of[(LY::lag ? 0 : 3) + q];
-        if (rd >= 0 && cd >= 0) {
-          P* dst = Ks + (na * ndf + cd) * ldk + rd;
-#pragma unroll
-          for (int b = 0; b < 9; ++b) dst[b * ndf] = acc[b];
+  for (int l = 0; l < ne; ++l) {
+    const int e = elem_of(l), nbt = s_nbt[l], u = s_u[l];
+    const P* S = S0 + l * slot;
+    const P* phi = S;
+    const P* bd = S + oB;
+    if (K_el) {
+      // phase 2
+      constexpr int PPW = 32 / LY::dirs;  // points per warp
+      const int gp = warp * PPW + lane / LY::dirs, dl = lane % LY::dirs;
+      if (gp < 9) {
+        Seed<P> sd;
+        OutD<P, MOTION> o;
+        o.D = D + gp * DS;
+        if (direction<P, P, MOTION>(dl, P(dt), sd, o)) {
+          const P* pr = S + oP + gp * kPrim;
+          gp_eval<P, P, MOTION>(cf, pr, phi[gp * kTab + kPhi], sd, Load<P>{pr, kPre}, o);
         }
       }
-    }
-    // light units: the warps without a heavy one (every warp when there are none)
-    constexpr int w0 = 3 * LY::nheavy;
-    for (int k = warp - w0; k >= 0 && k < light_units<MOTION>(); k += LY::warps - w0) {
-      const LightUnit U = light_unit<MOTION>(k);
-      if (on && q < U.npair) {
-        const int ru = U.r0 + q * U.dr, cu = U.c0 + q * U.dc;
-        const int rd = pp.dof_of[ru], cd = pp.dof_of[cu];
-        P acc[9];
+      __syncthreads();
+      // phase 3
+      const int q = lane / 9, na = lane - 9 * q;  // pair and column node of this lane
+      const bool on = q < 3;
+      const double dbs = pp.adb / pp.zv;
+      for (int un = warp; un < 3 * LY::nheavy; un += LY::warps) {  // heavy: row field `un`, column field m_q (LAG: v_q)
+        if (on) {
+          P acc[9];
 #pragma unroll
-        for (int b = 0; b < 9; ++b) acc[b] = P(0);
-        if (ru == cu && ru >= 6 && !area_only) {
-          // Dohrmann-Bochev projection (FiniteElement.jl:323-327): rλ += Gᵀ H⁻¹ G λ αdb/ζv,
-          // and for ALEV/ALEVB rp += Gᵀ H⁻¹ G p αdb/ζv.  Linear in λ / p.
-          const double* T81 = Pt.db + (size_t)u * 81;
-#pragma unroll
-          for (int b = 0; b < 9; ++b) acc[b] = P(T81[b * 9 + na] * dbs);
-        }
-        const P* Dp = D + L0 + (U.pair + q) * kLS;
+          for (int b = 0; b < 9; ++b) acc[b] = P(0);
+          const P* Dp = D + (un * 3 + q) * kHS<P>;
 #pragma unroll 1
-        for (int g = 0; g < 9; ++g) {
-          const P* ph = phi + g * kTab;
-          const P p0 = ph[na * 6 + U.t0], p1 = ph[na * 6 + U.t1], p2 = ph[na * 6 + U.t2];
-          const P* Dg = Dp + g * DS;
-          const P W0 = Dg[0] * p0 + Dg[1] * p1 + Dg[2] * p2, W1 = Dg[3] * p0 + Dg[4] * p1 + Dg[5] * p2;
+          for (int g = 0; g < 9; ++g) {
+            const P* ph = phi + g * kTab;
+            P pt[6], W[6], Dg[32];
+            ld_pairs<P, 6>(pt, ph + na * 6);
+            ld_quads<P, sizeof(P) == 8 ? 30 : 32>(Dg, Dp + g * DS);
 #pragma unroll
-          for (int b = 0; b < 9; ++b) acc[b] += ph[b * 6 + U.s0] * W0 + ph[b * 6 + U.s1] * W1;
-        }
-        if (rd >= 0 && cd >= 0) {
-          P* dst = Ks + (na * ndf + cd) * ldk + rd;
+            for (int s = 0; s < 6; ++s) {
+              W[s] = Dg[s * 5] * pt[0];
 #pragma unroll
-          for (int b = 0; b < 9; ++b) dst[b * ndf] = acc[b];
-        }
-      }
-    }
-  }
-  if constexpr (WANT_R) {
-    for (int row = NT - 1 - tid; row < nq; row += NT) {  // the last warps: they hold the light units
-      const int b = row / ndf, d = row - b * ndf, un = pp.unk_of[d];
-      P r = P(0);
-      for (int g = 0; g < 9; ++g) {
-        const P* ph = phi + g * kTab + b * 6;
-        const P* c = cf9 + g * kCf;
-        if (un < 6) {
-          P s = ph[0] * c[un * 6];
+              for (int t = 1; t < 5; ++t) W[s] += Dg[s * 5 + t] * pt[t];
+            }
 #pragma unroll
-          for (int k = 1; k < 6; ++k) s += ph[k] * c[un * 6 + k];
-          r += s;
-        } else {
-          r += ph[kN] * c[un == 6 ? 37 : 36];
-        }
-      }
-      if (!area_only) {
-        if (un == 6 || (un == 7 && LY::ale)) {
-          const double* T81 = Pt.db + (size_t)u * 81;
-          double s = 0;
-          for (int c = 0; c < 9; ++c) s += T81[b * 9 + c] * C[c * 8 + d];
-          r += s * (pp.adb / pp.zv);
-        }
-        if (un < 3)
-          for (int bt = 0; bt < nbt; ++bt) {
-            const P* B = bd + bt * kBd;
-            r += B[54 + b * 3] * B[81 + un * 3] + B[54 + b * 3 + 1] * B[81 + un * 3 + 1] +
-                 B[54 + b * 3 + 2] * B[81 + un * 3 + 2];
+            for (int b2 = 0; b2 < 10; b2 += 2) {  // two rows' basis values: 12 values, 16-byte aligned
+              P f[12];
+              ld_quads<P, 12>(f, ph + b2 * 6);  // (b = 9: the point's weight and the next point's first values, unused)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int b = b2 + h;
+                if (b > 8) continue;
+                // FP32: the point's sum first, one rounding at the size of acc per point
+                P v = sizeof(P) == 8 ? acc[b] + f[h * 6] * W[0] : f[h * 6] * W[0];
+#pragma unroll
+                for (int s = 1; s < 6; ++s) v += f[h * 6 + s] * W[s];
+                acc[b] = sizeof(P) == 8 ? v : acc[b] + v;
+              }
+            }
           }
+          if (un < 3)  // the velocity rows' boundary points
+            for (int bt = 0; bt < nbt; ++bt) {
+              const P* B = bd + bt * kBd;
+              const P p0 = B[54 + na * 3], p1 = B[54 + na * 3 + 1];
+              P W[3];
+#pragma unroll
+              for (int s = 0; s < 3; ++s) W[s] = B[(un * 3 + q) * 6 + 2 * s] * p0 + B[(un * 3 + q) * 6 + 2 * s + 1] * p1;
+#pragma unroll
+              for (int b = 0; b < 9; ++b)
+#pragma unroll
+                for (int s = 0; s < 3; ++s) acc[b] += B[54 + b * 3 + s] * W[s];
+            }
+          const int rd = pp.dof_of[un], cd = pp.dof_of[(LY::lag ? 0 : 3) + q];
+          if (rd >= 0 && cd >= 0) {
+            P* dst = Ks + (na * ndf + cd) * ldk + rd;
+#pragma unroll
+            for (int b = 0; b < 9; ++b) dst[b * ndf] = acc[b];
+          }
+        }
       }
-      r_el[(size_t)kk * nq + row] = r;
+      // light units: the warps without a heavy one (every warp when there are none)
+      constexpr int w0 = 3 * LY::nheavy;
+      for (int k = warp - w0; k >= 0 && k < light_units<MOTION>(); k += LY::warps - w0) {
+        const LightUnit U = light_unit<MOTION>(k);
+        if (on && q < U.npair) {
+          const int ru = U.r0 + q * U.dr, cu = U.c0 + q * U.dc;
+          const int rd = pp.dof_of[ru], cd = pp.dof_of[cu];
+          P acc[9];
+#pragma unroll
+          for (int b = 0; b < 9; ++b) acc[b] = P(0);
+          if (ru == cu && ru >= 6 && !area_only) {
+            // Dohrmann-Bochev projection (FiniteElement.jl:323-327): rλ += Gᵀ H⁻¹ G λ αdb/ζv,
+            // and for ALEV/ALEVB rp += Gᵀ H⁻¹ G p αdb/ζv.  Linear in λ / p.
+            const double* T81 = Pt.db + (size_t)u * 81;
+#pragma unroll
+            for (int b = 0; b < 9; ++b) acc[b] = P(T81[b * 9 + na] * dbs);
+          }
+          const P* Dp = D + L0 + (U.pair + q) * kLS;
+#pragma unroll 1
+          for (int g = 0; g < 9; ++g) {
+            const P* ph = phi + g * kTab;
+            const P p0 = ph[na * 6 + U.t0], p1 = ph[na * 6 + U.t1], p2 = ph[na * 6 + U.t2];
+            P Dg[6];
+            ld_pairs<P, 6>(Dg, Dp + g * DS);
+            const P W0 = Dg[0] * p0 + Dg[1] * p1 + Dg[2] * p2;
+            if (U.s0 == kN) {  // rows with the basis values alone
+#pragma unroll
+              for (int b = 0; b < 9; ++b) acc[b] += ph[b * 6 + kN] * W0;
+            } else {  // N_,1 and N_,2
+              const P W1 = Dg[3] * p0 + Dg[4] * p1 + Dg[5] * p2;
+#pragma unroll
+              for (int b = 0; b < 9; ++b) {
+                P f[2];
+                ld_pairs<P, 2>(f, ph + b * 6);
+                acc[b] += f[0] * W0 + f[1] * W1;
+              }
+            }
+          }
+          if (rd >= 0 && cd >= 0) {
+            P* dst = Ks + (na * ndf + cd) * ldk + rd;
+#pragma unroll
+            for (int b = 0; b < 9; ++b) dst[b * ndf] = acc[b];
+          }
+        }
+      }
     }
-  }
-  if (K_el) {
-    // phase 4: column-major element block K_el[e][col][row]
-    __syncthreads();
-    P* dst = K_el + (size_t)e * nq * nq;
-    for (int c = warp; c < nq; c += LY::warps)
-      for (int r = lane; r < nq; r += 32) dst[c * nq + r] = Ks[c * ldk + r];
+    if constexpr (WANT_R) {
+      for (int row = NT - 1 - tid; row < nq; row += NT) {  // the last warps: they hold the light units
+        const int b = row / ndf, d = row - b * ndf, un = pp.unk_of[d];
+        P r = P(0);
+        for (int g = 0; g < 9; ++g) {
+          const P* ph = phi + g * kTab + b * 6;
+          const P* c = S + oF + g * kCf;
+          if (un < 6) {
+            P s = ph[0] * c[un * 6];
+#pragma unroll
+            for (int k = 1; k < 6; ++k) s += ph[k] * c[un * 6 + k];
+            r += s;
+          } else {
+            r += ph[kN] * c[un == 6 ? 37 : 36];
+          }
+        }
+        if (!area_only) {
+          if (un == 6 || (un == 7 && LY::ale)) {
+            const double* T81 = Pt.db + (size_t)u * 81;
+            double s = 0;
+            for (int c = 0; c < 9; ++c) s += T81[b * 9 + c] * S[oC + c * 8 + d];
+            r += s * (pp.adb / pp.zv);
+          }
+          if (un < 3)
+            for (int bt = 0; bt < nbt; ++bt) {
+              const P* B = bd + bt * kBd;
+              r += B[54 + b * 3] * B[81 + un * 3] + B[54 + b * 3 + 1] * B[81 + un * 3 + 1] +
+                   B[54 + b * 3 + 2] * B[81 + un * 3 + 2];
+            }
+        }
+        r_el[(size_t)(kk0 + l) * nq + row] = r;
+      }
+    }
+    if (K_el) {
+      // phase 4: column-major element block K_el[e][col][row]
+      __syncthreads();
+      P* dst = K_el + (size_t)e * nq * nq;
+      for (int c = warp; c < nq; c += LY::warps)
+        for (int r = lane; r < nq; r += 32) dst[c * nq + r] = Ks[c * ldk + r];
+    }
   }
 }
 
@@ -1044,13 +1119,12 @@ __device__ __forceinline__ void elem_one(const DevPatch& Pt, const PhysParams& p
 // work.  In FP64 that holds it to 96 registers, which spills 0.7 KB per thread,
 // yet 32 x 32 ALEVB is assembled in 1.00 ms against 1.11 ms with one CTA and 168
 // registers (both before the closed-form geometry derivatives).
-template <class P, bool WANT_R, int MOTION>
-__global__ void __launch_bounds__(Lay<MOTION>::threads, 2)
+template <class P, bool WANT_R, int MOTION, int EPB>
+__global__ void __launch_bounds__(Lay<MOTION>::threads, (Lay<MOTION>::template ctas<P>()))
     elem_kernel(DevPatch Pt, PhysParams pp, double time, double dt, double* __restrict__ r_el, P* __restrict__ K_el,
-                const int* __restrict__ elist, int area_only) {
+                const int* __restrict__ elist, int nel, int area_only) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int kk = blockIdx.x;
-  elem_one<P, WANT_R, MOTION>(Pt, pp, time, dt, r_el, K_el, elist ? elist[kk] : kk, kk, area_only, smem_raw);
+  elem_body<P, WANT_R, MOTION, EPB>(Pt, pp, time, dt, r_el, K_el, elist, blockIdx.x * EPB, nel, area_only, smem_raw);
 }
 
 // FP64 residual of the FP32 form: primal only, one thread per (element, area
@@ -1096,7 +1170,10 @@ struct OutRows {  // adds a point's rows into R[row]
   __device__ __forceinline__ void p(const Dual<double, Nil>& x) { addn(pp.dof_of[7], x.v); }
   __device__ __forceinline__ void l(const Dual<double, Nil>& x) { addn(pp.dof_of[6], x.v); }
 };
-constexpr int kResEPB = 16;  // elements per CTA: 144 threads
+// Elements per CTA: 63 threads, so that a patch of 32 x 32 elements spreads over
+// 147 SMs (an FP64 instruction holds its sub-partition for 64 cycles, so the
+// kernel's time is its longest warp chain): 98 -> MEASRES us against 16 per CTA.
+constexpr int kResEPB = 7;
 template <int MOTION>
 __device__ __forceinline__ void resid_body(const DevPatch& Pt, const PhysParams& pp, double time, double dt,
                                            double* __restrict__ r_el, int blk, unsigned char* smem_raw) {
@@ -1225,11 +1302,11 @@ __global__ void __launch_bounds__(kResEPB * 9) batch_resid_kernel(const AsmJob* 
   __syncthreads();
   resid_body<MOTION>(sP, spp, it.time, it.dt, J->r_el, off[0] + (int)blockIdx.x - off[k], smem_raw);
 }
-// Elements per CTA of the FP32 tangent kernel (one after the other): 2 or 4,
-// chosen per motion by the batch's autotuner (four share a CTA's set-up, two
-// spread small rounds over more SMs).
+// Elements per CTA of the FP32 tangent kernel: 2 or 4, chosen per motion by the
+// batch's autotuner (four share a CTA's set-up and phases 0 and 1, two spread
+// small rounds over more SMs).
 template <int MOTION, int EPB>
-__global__ void __launch_bounds__(Lay<MOTION>::threads, 2)
+__global__ void __launch_bounds__(Lay<MOTION>::threads, (Lay<MOTION>::template ctas<float>()))
     batch_tan_kernel(const AsmJob* __restrict__ jobs, const AsmItem* __restrict__ items, const int* __restrict__ off,
                      int m) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1242,38 +1319,35 @@ __global__ void __launch_bounds__(Lay<MOTION>::threads, 2)
   batch_copy(&sP, &J->P, (int)sizeof(DevPatch));
   batch_copy(&spp, &J->pp, (int)sizeof(PhysParams));
   __syncthreads();
-  const int e0 = (off[0] + (int)blockIdx.x - off[k]) * EPB;
-#pragma unroll 1
-  for (int e = e0; e < min(e0 + EPB, sP.numel); ++e) {
-    elem_one<float, false, MOTION>(sP, spp, it.time, it.dt, nullptr, J->K_el, e, e, 0, smem_raw);
-    __syncthreads();  // the next element overwrites the block just copied out
-  }
+  elem_body<float, false, MOTION, EPB>(sP, spp, it.time, it.dt, nullptr, J->K_el, nullptr,
+                                       (off[0] + (int)blockIdx.x - off[k]) * EPB, sP.numel, 0, smem_raw);
 }
 
 // ---- launchers -----------------------------------------------------------------------
 // The dynamic shared memory a kernel may ask for: the largest element (nq = 72)
 // with the most boundary points it can have (8 Neumann entries).
-template <class P, int MOTION>
+template <class P, int MOTION, int EPB>
 static size_t elem_smem(const PhysParams& pp) {
-  return elem_smem_values<P, MOTION>(pp.nq, pp.max_btask) * sizeof(P);
+  return elem_smem_values<P, MOTION, EPB>(pp.nq, pp.max_btask) * sizeof(P);
 }
-template <class P, int MOTION>
+template <class P, int MOTION, int EPB>
 static size_t elem_smem_cap() {
-  return elem_smem_values<P, MOTION>(72, 3 * kMaxNeu) * sizeof(P);
+  return elem_smem_values<P, MOTION, EPB>(72, 3 * kMaxNeu) * sizeof(P);
 }
 static size_t resid_smem(int nq) {
   return (size_t)kResEPB * (27 + 72) * 8 + (size_t)std::max(kResEPB * 9 * nq, kResEPB * 24 * 27) * 8;
 }
 
-template <class P, bool WANT_R, int MOTION>
+template <class P, bool WANT_R, int MOTION, int EPB>
 static cudaError_t launch_elem_t(const DevPatch& Pt, const PhysParams& pp, double time, double dt, double* r_el,
                                  P* K_el, cudaStream_t st, const int* elist, int nlist, int area_only) {
-  auto kern = elem_kernel<P, WANT_R, MOTION>;
+  auto kern = elem_kernel<P, WANT_R, MOTION, EPB>;
   cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)elem_smem_cap<P, MOTION>());
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)elem_smem_cap<P, MOTION, EPB>());
   if (e != cudaSuccess) return e;
-  const int blocks = elist ? nlist : Pt.numel;
-  kern<<<blocks, Lay<MOTION>::threads, elem_smem<P, MOTION>(pp), st>>>(Pt, pp, time, dt, r_el, K_el, elist, area_only);
+  const int nel = elist ? nlist : Pt.numel;
+  kern<<<(nel + EPB - 1) / EPB, Lay<MOTION>::threads, elem_smem<P, MOTION, EPB>(pp), st>>>(
+      Pt, pp, time, dt, r_el, K_el, elist, nel, area_only);
   return cudaGetLastError();
 }
 
@@ -1293,15 +1367,15 @@ cudaError_t launch_elem<double>(const DevPatch& Pt, const PhysParams& pp, double
                                 double* K_el, cudaStream_t st, const int* elist, int nlist, int area_only) {
   switch (pp.motion) {
     case MAFEM_STATIC:
-      return launch_elem_t<double, true, STATIC_>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
+      return launch_elem_t<double, true, STATIC_, 1>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
     case MAFEM_EUL:
-      return launch_elem_t<double, true, EUL_>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
+      return launch_elem_t<double, true, EUL_, 1>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
     case MAFEM_LAG:
-      return launch_elem_t<double, true, LAG_>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
+      return launch_elem_t<double, true, LAG_, 1>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
     case MAFEM_ALEV:
-      return launch_elem_t<double, true, ALEV_>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
+      return launch_elem_t<double, true, ALEV_, 1>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
     default:
-      return launch_elem_t<double, true, ALEVB_>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
+      return launch_elem_t<double, true, ALEVB_, 1>(Pt, pp, time, dt, r_el, K_el, st, elist, nlist, area_only);
   }
 }
 
@@ -1310,7 +1384,10 @@ template <int MOTION>
 static cudaError_t launch_elem_f(const DevPatch& Pt, const PhysParams& pp, double time, double dt, double* r_el,
                                  float* K_el, cudaStream_t st) {
   const cudaError_t e = launch_resid_t<MOTION>(Pt, pp, time, dt, r_el, st);
-  return e ? e : launch_elem_t<float, false, MOTION>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0);
+  if (e) return e;
+  // one element per CTA while all of them are resident at once (two CTAs on each of 152 SMs)
+  return Pt.numel <= 304 ? launch_elem_t<float, false, MOTION, 1>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0)
+                         : launch_elem_t<float, false, MOTION, 2>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0);
 }
 template <>
 cudaError_t launch_elem<float>(const DevPatch& Pt, const PhysParams& pp, double time, double dt, double* r_el,
@@ -1334,10 +1411,10 @@ static cudaError_t batch_setup_t() {
                                        (int)resid_smem(72));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(batch_tan_kernel<MOTION, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)elem_smem_cap<float, MOTION>());
+                             (int)elem_smem_cap<float, MOTION, 2>());
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(batch_tan_kernel<MOTION, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)elem_smem_cap<float, MOTION>());
+                             (int)elem_smem_cap<float, MOTION, 4>());
   return e;
 }
 cudaError_t batch_asm_setup() {
@@ -1365,9 +1442,12 @@ cudaError_t launch_batch_resid(int motion, const AsmJob* jobs, const AsmItem* it
 template <int MOTION>
 static void launch_batch_tan_m(int epb, const AsmJob* jobs, const AsmItem* items, const int* off, int m, int ctas,
                                const PhysParams& pp, cudaStream_t st) {
-  const size_t sm = elem_smem<float, MOTION>(pp);
-  if (epb == 2) batch_tan_kernel<MOTION, 2><<<ctas, Lay<MOTION>::threads, sm, st>>>(jobs, items, off, m);
-  else batch_tan_kernel<MOTION, 4><<<ctas, Lay<MOTION>::threads, sm, st>>>(jobs, items, off, m);
+  if (epb == 2)
+    batch_tan_kernel<MOTION, 2>
+        <<<ctas, Lay<MOTION>::threads, elem_smem<float, MOTION, 2>(pp), st>>>(jobs, items, off, m);
+  else
+    batch_tan_kernel<MOTION, 4>
+        <<<ctas, Lay<MOTION>::threads, elem_smem<float, MOTION, 4>(pp), st>>>(jobs, items, off, m);
 }
 cudaError_t launch_batch_tan(int epb, const AsmJob* jobs, const AsmItem* items, const int* off, int m, int ctas,
                              const PhysParams& pp, cudaStream_t st) {

@@ -91,6 +91,7 @@ struct DevPatch {
   const int* unk_node;                // [nmdf] node of unknown q (0-based)
   const int* unk_dof;                 // [nmdf] dof of unknown q (0-based)
   const int* node_unk;                // [numnp][ndf] unknown of (node, dof), -1 if Dirichlet
+  const int* node_first;              // [numnp + 1] first unknown of each node; null: not numbered node by node
   // state
   double* xms;                        // [3][numnp]
   double* cps;                        // [ndf][numnp]
@@ -118,7 +119,8 @@ template <class T>
 cudaError_t launch_elem(const DevPatch& P, const PhysParams& pp, double time, double dt, double* r_el, T* K_el,
                         cudaStream_t st, const int* elist = nullptr, int nlist = 0, int area_only = 0);
 template <class T>
-void launch_band_gather(const DevPatch& P, int ndf, int nq, const BandLayout& L, const T* K_el, T* ab,
+// kuf: super-diagonals the factorisation fills (gather_column)
+void launch_band_gather(const DevPatch& P, int ndf, int nq, const BandLayout& L, int kuf, const T* K_el, T* ab,
                         cudaStream_t st, T* ab2 = nullptr);
 void launch_resid_gather(const DevPatch& P, int ndf, int nq, const double* r_el, double* r, cudaStream_t st);
 void launch_predictor(const DevPatch& P, const PhysParams& pp, double dt, cudaStream_t st);
@@ -269,7 +271,7 @@ struct AsmJob {
   const int* dir_idx;     // [n_dir] inhomogeneous Dirichlet entries of cps (dof * numnp + node)
   const double* dir_val;  // [n_dir] their values
   int n_dir;
-  int pad;
+  int kuf;  // super-diagonals the factorisation fills
 };
 enum { kStartPredict = 1, kStartDirichlet = 2 };  // AsmItem::start
 struct AsmItem {  // one patch of a round
@@ -282,7 +284,7 @@ struct AsmOut {  // one patch's results of a round, read by the host
   double out[3];
   int info[4];
 };
-constexpr int kGatherCols = 4;  // band columns per CTA of the batched gather
+constexpr int kGatherCols = 8;  // band columns per CTA of the batched gather (a warp each)
 // CTAs per patch of each batched kernel
 int batch_resid_ctas(int numel);
 int batch_tan_ctas(int numel, int epb);  // epb: elements per CTA of the tangent kernel, 2 or 4
