@@ -599,18 +599,16 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
   if (precision != MAFEM_PLAIN_FP64 && h->use_blk && h->L.nb >= 32) {
     const int dyn = patch_solve_setup();
     cudaGetLastError();
-    if (dyn > 0 && patch_factor_smem(h->L.kl) <= (size_t)dyn && patch_refine_smem(n) <= (size_t)dyn) {
-      AL(h->d_inv, (size_t)h->blk.npan() * 2 * kBlkW * kBlkW);
+    if (dyn > 0 && patch_factor_smem() <= (size_t)dyn && patch_refine_smem(n, h->blk.npan()) <= (size_t)dyn) {
+      AL(h->d_inv, (size_t)h->blk.npan() * kBlkW * kBlkW);
       PatchJob& J = h->job;
       J.a21_rows = patch_a21_rows(h->L.kl);
-      AL(J.a21, (size_t)8 * 2 * J.a21_rows * 4);
+      AL(J.a21, (size_t)8 * 4 * 2 * J.a21_rows * 4);
       J.band = (float*)h->d_band;
       J.band0 = (const float*)h->d_band0;
       J.inv = h->d_inv;
       J.ps = h->blk.d_ps;
       J.blk_end = h->d_blk_end;
-      J.perm = h->d_perm;
-      J.rdiag = (float*)h->d_rdiag;
       J.info = h->d_info;
       J.stat = h->d_info + 2;
       J.rhs = h->d_r;
@@ -1311,8 +1309,7 @@ extern "C" int mafem_set_launch_ctas(mafem_handle* h, int32_t ctas) {
 
 // Order of a round's batched solves: the patches factored on four-CTA
 // clusters first, then those on two-CTA clusters, then the single-CTA ones,
-// each group largest first.  Returns the size of the first group in *n4 and of
-// the second in *n2.
+// each group largest first.  Returns the groups.
 // CTAs that factor the handle's patch in the batched FP32 form: the caller's
 // choice, else the autotuner's for this round, else by band width
 static int patch_ctas(const mafem_handle* h) {
@@ -1351,7 +1348,7 @@ static int patch_tune(mafem_handle* h, const PatchJob* d_jobs, int slot, int* d_
   CK(cudaMemcpyAsync(d_tmp, &slot, sizeof(int), cudaMemcpyHostToDevice, st));
   const int nrs[3] = {1, 2, 4};
   for (int k = 0; k < 3; ++k) {
-    const cudaError_t e = patch_time_factor(d_jobs, d_tmp, nrs[k], patch_factor_smem(h->L.kl), st, &ms[k]);
+    const cudaError_t e = patch_time_factor(d_jobs, d_tmp, nrs[k], patch_factor_smem(), st, &ms[k]);
     if (e != cudaSuccess) {
       h->err = std::string("factorisation autotuning: ") + cudaGetErrorString(e);
       return MAFEM_ERR_CUDA;
@@ -1459,18 +1456,21 @@ static int tan_epb(const mafem_handle* h) {
 static int tan_tune(mafem_handle* h, const AsmJob* d_ajobs, int slot, unsigned char* d_buf, unsigned char* h_buf,
                     cudaStream_t st);
 
-static void order_patch_jobs(std::vector<mafem_handle*>& hv, std::vector<int>& idx, int* n4, int* n2) {
+static PatchGroups order_patch_jobs(std::vector<mafem_handle*>& hv, std::vector<int>& idx) {
   auto nr = [&](int k) { return patch_ctas(hv[k]); };
   auto cost = [&](int k) { return (double)hv[k]->blk.npan() * hv[k]->L.kl * hv[k]->blk.kuf; };
   std::sort(idx.begin(), idx.end(), [&](int a, int b) {
     if (nr(a) != nr(b)) return nr(a) > nr(b);
     return cost(a) > cost(b);
   });
-  *n4 = *n2 = 0;
+  PatchGroups G;
   for (int k : idx) {
-    *n4 += nr(k) == 4 ? 1 : 0;
-    *n2 += nr(k) == 2 ? 1 : 0;
+    const int g = nr(k) == 4 ? 0 : nr(k) == 2 ? 1 : 2;
+    G.n4 += g == 0;
+    G.n2 += g == 1;
+    G.wide[g] |= patch_wide(hv[k]->L.kl, hv[k]->blk.kuf);
   }
+  return G;
 }
 
 // A batched round's host/device buffer: the items (patches of the round in
@@ -1704,8 +1704,8 @@ extern "C" int mafem_batch_create(mafem_handle* const* hs, int32_t n, int32_t ct
       b->slot.push_back((int)jobs.size());
       jobs.push_back(h->job);
       b->cost.push_back((double)h->blk.npan() * h->L.kl * h->blk.kuf);
-      b->smem_f = std::max(b->smem_f, patch_factor_smem(h->L.kl));
-      b->smem_r = std::max(b->smem_r, patch_refine_smem(h->L.n));
+      b->smem_f = std::max(b->smem_f, patch_factor_smem());
+      b->smem_r = std::max(b->smem_r, patch_refine_smem(h->L.n, h->blk.npan()));
     } else {
       b->slot.push_back(-1);
     }
@@ -1775,7 +1775,7 @@ extern "C" int mafem_batch_destroy(mafem_batch* b) {
 }
 
 // One batched Newton round of the FP32 patches hv[pj] (ordered for the
-// factorisation: the first n4 on four-CTA clusters, the next n2 on two; job
+// factorisation, in the groups G; job
 // index slot_of[i], step-start flags start[i] and Dirichlet scale dscale[i]
 // per handle) on R's streams: the Dirichlet scaling and the predictor of the
 // patches that start a time step, the FP64 residual and FP32 tangent kernels
@@ -1786,7 +1786,7 @@ extern "C" int mafem_batch_destroy(mafem_batch* b) {
 // of patches occurs and replayed from then on.  *launches: kernels per round.
 static cudaError_t run_round(RoundRunner& R, const PatchJob* d_jobs, const AsmJob* d_ajobs, size_t smem_f,
                              size_t smem_r, const std::vector<mafem_handle*>& hv, const std::vector<int>& slot_of,
-                             const std::vector<int>& pj, int n4, int n2, int max_sweeps, double tol,
+                             const std::vector<int>& pj, const PatchGroups& G, int max_sweeps, double tol,
                              const std::vector<int>& start, const std::vector<double>& dscale, int* launches) {
   const int m = (int)pj.size();
   if (m > R.cap) return cudaErrorInvalidValue;
@@ -1839,7 +1839,7 @@ static cudaError_t run_round(RoundRunner& R, const PatchJob* d_jobs, const AsmJo
     return reinterpret_cast<const int*>(dr + (t == kOffDir ? dir_off : RL.off[t])) + g0;
   };
   const int ng = (int)groups.size() - 1;
-  *launches = (any_dir ? 1 : 0) + (any_pred ? 1 : 0) + 2 * ng + 2 + patch_solve_launches(n4, n2, m) + 2;
+  *launches = (any_dir ? 1 : 0) + (any_pred ? 1 : 0) + 2 * ng + 2 + patch_solve_launches(G, m) + 2;
 
   auto enqueue = [&](bool capturing) -> cudaError_t {
     const unsigned fl = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
@@ -1871,7 +1871,7 @@ static cudaError_t run_round(RoundRunner& R, const PatchJob* d_jobs, const AsmJo
     }
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(R.rev[1], st, fl);
     if (e == cudaSuccess)
-      e = patch_solve(d_jobs, R.d_order, n4, n2, m, smem_f, smem_r, max_sweeps, tol, st, R.st2, R.efork, R.ejoin);
+      e = patch_solve(d_jobs, R.d_order, G, m, smem_f, smem_r, max_sweeps, tol, st, R.st2, R.efork, R.ejoin);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(R.rev[2], st, fl);
     if (e == cudaSuccess) {
       launch_batch_update(d_ajobs, d_items, d_off(4, 0), m, off[4][m], R.d_outs, st);
@@ -1887,7 +1887,7 @@ static cudaError_t run_round(RoundRunner& R, const PatchJob* d_jobs, const AsmJo
   if (!R.graph_on) return enqueue(false);
   // the graph's key: everything its nodes bake in (grids, copy sizes, kernel arguments)
   // (a job's shape too: a slot of a server may hold another patch later)
-  std::vector<int64_t> key{m, n4, n2, max_sweeps, (int64_t)smem_f, (int64_t)smem_r};
+  std::vector<int64_t> key{m, G.key(), max_sweeps, (int64_t)smem_f, (int64_t)smem_r};
   int64_t tb;
   std::memcpy(&tb, &tol, sizeof tb);
   key.push_back(tb);
@@ -1998,9 +1998,8 @@ extern "C" int mafem_batch_step(mafem_batch* b, const double* times, const doubl
     }
     bool round_ok = false;
     if (!pj.empty()) {
-      int n4 = 0, n2 = 0;
       choose_patch_ctas(b->hs, pj);
-      order_patch_jobs(b->hs, pj, &n4, &n2);
+      const PatchGroups G = order_patch_jobs(b->hs, pj);
       // one launch serves every patch: the strictest tolerance and the largest sweep cap among them
       b->max_sweeps = 1;
       b->tol = 1.0;
@@ -2010,7 +2009,7 @@ extern "C" int mafem_batch_step(mafem_batch* b, const double* times, const doubl
       }
       if (basm) {
         int nl = 0;
-        cudaError_t e = run_round(*b->rr, b->d_jobs, b->d_ajobs, b->smem_f, b->smem_r, b->hs, b->slot, pj, n4, n2,
+        cudaError_t e = run_round(*b->rr, b->d_jobs, b->d_ajobs, b->smem_f, b->smem_r, b->hs, b->slot, pj, G,
                                   b->max_sweeps, b->tol, start, dscale, &nl);
         if (e == cudaSuccess) e = cudaEventSynchronize(b->rr->rev[3]);
         for (int i : pj) start[i] = 0;
@@ -2033,7 +2032,7 @@ extern "C" int mafem_batch_step(mafem_batch* b, const double* times, const doubl
         cudaError_t e =
             cudaMemcpyAsync(b->d_order, b->h_order, pj.size() * sizeof(int), cudaMemcpyHostToDevice, b->bst);
         if (e == cudaSuccess)
-          e = patch_solve(b->d_jobs, b->d_order, n4, n2, (int)pj.size(), b->smem_f, b->smem_r, b->max_sweeps,
+          e = patch_solve(b->d_jobs, b->d_order, G, (int)pj.size(), b->smem_f, b->smem_r, b->max_sweeps,
                           b->tol, b->bst, b->bst2, b->efork, b->ejoin);
         if (e == cudaSuccess) e = cudaEventRecord(b->bev, b->bst);
         for (int i : pj) {
@@ -2043,7 +2042,7 @@ extern "C" int mafem_batch_step(mafem_batch* b, const double* times, const doubl
             st[i] = MAFEM_ERR_CUDA;
             continue;
           }
-          if (i == pj[0]) h->launches += patch_solve_launches(n4, n2, (int)pj.size());  // counted once
+          if (i == pj[0]) h->launches += patch_solve_launches(G, (int)pj.size());  // counted once
           const int rc = iter_enqueue_patch_end(h, b->bev);
           if (rc != MAFEM_OK) st[i] = rc;
         }
@@ -2304,7 +2303,7 @@ extern "C" int mafem_server_round(mafem_server* s, int32_t* n_active, int32_t* n
     q->h = h;
     q->bytes = h->bytes;
     s->used += h->bytes;
-    if (h->patch_ok && s->smem_dyn >= patch_factor_smem(h->L.kl) && s->smem_dyn >= patch_refine_smem(h->L.n) &&
+    if (h->patch_ok && s->smem_dyn >= patch_factor_smem() && s->smem_dyn >= patch_refine_smem(h->L.n, h->blk.npan()) &&
         !s->free_slots.empty()) {
       q->slot = s->free_slots.back();
       s->free_slots.pop_back();
@@ -2416,17 +2415,16 @@ extern "C" int mafem_server_round(mafem_server* s, int32_t* n_active, int32_t* n
       start[k] = q->start;
       dscale[k] = q->dscale;
       pj[k] = k;
-      smf = std::max(smf, patch_factor_smem(h->L.kl));
-      smr = std::max(smr, patch_refine_smem(h->L.n));
+      smf = std::max(smf, patch_factor_smem());
+      smr = std::max(smr, patch_refine_smem(h->L.n, h->blk.npan()));
       max_sw = std::max(max_sw, h->max_refine);
       tol = std::min(tol, h->refine_tol);
       if (q->start) cudaStreamWaitEvent(L.st, h->ev[5], 0);  // the handle's own work before the step
     }
-    int n4 = 0, n2 = 0;
     choose_patch_ctas(hv, pj);
-    order_patch_jobs(hv, pj, &n4, &n2);
+    const PatchGroups G = order_patch_jobs(hv, pj);
     int nl = 0;
-    cudaError_t e = run_round(L, s->d_jobs, s->d_ajobs, smf, smr, hv, slot_of, pj, n4, n2, max_sw, tol, start, dscale,
+    cudaError_t e = run_round(L, s->d_jobs, s->d_ajobs, smf, smr, hv, slot_of, pj, G, max_sw, tol, start, dscale,
                               &nl);
     for (ServerReq* q : rq) q->start = 0;
     if (e != cudaSuccess) {
@@ -2630,9 +2628,10 @@ extern "C" int mafem_trace_patch_solve(mafem_handle* h, double time, double dt, 
   const int dyn = patch_solve_setup();
   cudaEventRecord(e0, h->st);
   const int nr = patch_ctas(h);  // as a batch would run it
-  patch_solve_stage(d_job, d_ord, 1, nr, patch_factor_smem(h->L.kl), 0, 0, 0.0, h->st);
+  patch_solve_stage(d_job, d_ord, 1, nr, patch_factor_smem(), 0, false, 0, 0.0, h->st);
   cudaEventRecord(e1, h->st);
-  patch_solve_stage(d_job, d_ord, 1, 1, 0, patch_refine_smem(h->L.n), h->max_refine, h->refine_tol, h->st);
+  patch_solve_stage(d_job, d_ord, 1, 1, 0, patch_refine_smem(h->L.n, h->blk.npan()),
+                    patch_wide(h->L.kl, h->blk.kuf), h->max_refine, h->refine_tol, h->st);
   cudaEventRecord(e2, h->st);
   std::vector<long long> tr((size_t)ntr);
   CK(cudaMemcpyAsync(tr.data(), d_tr, tr.size() * sizeof(long long), cudaMemcpyDeviceToHost, h->st));

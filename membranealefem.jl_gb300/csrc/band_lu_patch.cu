@@ -1,30 +1,26 @@
 // band_lu_patch.cu -- many patches' FP32 linear solves in two launches.
 //
 // The batched FP32 form solves K Δu = -r for every patch of a batch with one
-// CTA per patch: `patch_factor_kernel` factors each patch's FP32 band with
-// node-block pivoting (the same factors as band_lu_blk.cu: L11\U11 with the
-// panel's rows permuted, U12 = L11^-1 P A12, raw A21, rdiag = 1/U(j,j),
-// perm_all[p * 32 + i]), and `patch_refine_kernel` runs the FP32 triangular
-// solves and FP64 iterative refinement x += LU^-1 (r - A0 x) until the last
-// correction is at most tol |x| -- the role of `K_gl \ r_gl` (FiniteElement.jl:38).
-// A single patch's LU is a chain of dependent panels; across a batch the
-// chains are independent, so one CTA per patch keeps every SM busy without
-// any inter-CTA synchronisation (the multi-CTA persistent kernel spends most
-// of its SM time waiting on the chain, which pays only for one patch alone).
+// CTA (or a small cluster) per patch: `patch_factor_kernel` factors each patch's
+// FP32 band and `patch_refine_kernel` runs the FP32 substitutions and FP64
+// iterative refinement x += K^-1 (r - A0 x) until the last correction is at most
+// tol |x| -- the role of `K_gl \ r_gl` (FiniteElement.jl:38).  A single patch's
+// LU is a chain of dependent panels; across a batch the chains are independent,
+// so one CTA per patch keeps every SM busy without any inter-CTA
+// synchronisation (the multi-CTA persistent kernel spends most of its SM time
+// waiting on the chain, which pays only for one patch alone).
 //
-// Per panel (columns [j0, j1), w <= 32 wide, R = w + kl rows) the CTA
-//   1. factors the w x w diagonal block (blk_panel_factor, warps 0..7),
-//   2. stages the panel columns (L11\U11 and A21) in shared memory and forms
-//      Li = L11^-1 and Ui = U11^-1 explicitly (one warp each, lane = column),
-//      Mi = Ui Li, and stores Li, Ui for the solves,
-//   3. for the kuf trailing columns, in chunks of 512: U12 = Li P A12 and
-//      Y = Mi P A12 (one thread per column, the column in registers, the
-//      inverses' rows as shared-memory broadcasts), then A22 -= A21 Y: each thread owns one
-//      row and 32 columns in registers, A21 from shared memory, Y as float4
-//      broadcasts, the band read and written once, coalesced along columns.
-// The explicit inverses turn the triangular solves of step 3 and of the
-// substitutions into small matrix products; the refinement absorbs their
-// rounding.
+// The factors are kept in block form.  Per panel (columns [j0, j1), w <= 32 wide,
+// whole node blocks) with A11 its diagonal block,
+//   Ai = A11^-1,  Y = Ai A12,  A22 -= A21 Y;
+// stored are Ai (job.inv), Y in place of A12 and the raw A21.  The
+// substitutions are then z = Ai b1, b2 -= A21 z forward and x1 = z - Y x2
+// backward: no triangle is ever solved, one 32 x 32 product per panel instead of
+// three (L11^-1, U11^-1 and their product), and Y serves the trailing update and
+// the back substitution alike.  Ai comes from one in-place Gauss-Jordan sweep
+// by a warp with the pivot of column k searched among the rows of k's node block
+// not yet used, the same pivots as a node-block pivoted LU; the refinement
+// absorbs the explicit inverse's rounding.
 
 #include <cuda_runtime.h>
 
@@ -36,35 +32,29 @@
 namespace mafem {
 
 constexpr int kPT = 512;   // threads per CTA of the factorisation (16 warps)
-constexpr int kRT = 768;   // threads per CTA of the refinement (24 warps)
+constexpr int kRT = 512;   // threads per CTA of the refinement (16 warps)
 constexpr int kNCH = 256;  // trailing columns per chunk at most (the MMA's N <= 256)
 constexpr int kMT = 128;   // rows of A22 per tensor-core tile (the MMA's M)
-constexpr int kIS = 36;    // shared-memory row stride of the 32 x 32 inverses (16-byte rows)
+constexpr int kIS = 36;    // shared-memory row stride of the 32 x 32 inverse (16-byte rows)
 // Y (the MMA's B operand, K-major core matrices): element (k, c) of a chunk at
-// float (k / 4) * 4 kNCH + 4 c + k % 4, hi and lo parts in two such arrays
-constexpr uint32_t kYPlane = 16u * kNCH;                // bytes between k-quads (the LBO of B)
-constexpr uint32_t kYBytes = 8u * kYPlane;              // one of Yh / Yl: 32 KB
+// float (k / 4) * kYQuad + 4 c + k % 4, hi and lo parts in two such arrays; the
+// k-quads are 16 bytes more than their size apart, so that a warp's 32 rows of
+// one column fall into 32 banks
+constexpr int kYQuad = 4 * kNCH + 4;
+constexpr uint32_t kYPlane = 4u * kYQuad;               // bytes between k-quads (the LBO of B)
+constexpr uint32_t kYBytes = 8u * kYPlane;              // one of Yh / Yl
 constexpr uint32_t kATile = 8u * kMT * 16u;             // one of A21h / A21l per M tile: 16 KB
 constexpr uint32_t kChunkBytes = 2 * kYBytes + 4 * kATile;  // Yh, Yl and two (A21h, A21l) tile buffers: 128 KB
+static_assert(kYBytes % 128 == 0, "the TMA tile buffers follow Y on a 128-byte boundary");
 constexpr uint32_t kTmemCols = 2 * kNCH;                // two FP32 accumulators of 128 x 256
-// A factorisation CTA asks for at least this much dynamic shared memory, so no
+// A factorisation CTA asks for more than half of an SM's shared memory, so no
 // two of them share an SM and its Tensor Memory (each allocates all 512 columns).
-constexpr size_t kExclusiveSmem = 116 * 1024;
+constexpr size_t kFactorSmem = kChunkBytes + sizeof(float) * (kBlkW * kIS + 16 * 4 * kBlkW);
+static_assert(kFactorSmem > 116 * 1024, "one factorisation CTA per SM");
 
-// panel column stride in shared memory: >= 32 + kl, == 8 mod 32 (conflict-free column staging)
-__host__ __device__ inline int patch_rp(int kl) { return ((kBlkW + kl + 23) & ~31) + 8; }
-__host__ __device__ inline size_t patch_region0(int kl) {
-  const size_t lp = sizeof(float) * (size_t)kBlkW * patch_rp(kl);
-  const size_t r = lp > kChunkBytes ? lp : kChunkBytes;
-  return (r + 1023) & ~(size_t)1023;
-}
-
-size_t patch_factor_smem(int kl) {
-  const size_t s = patch_region0(kl) + sizeof(float) * 3 * (size_t)kBlkW * kIS;
-  return s > kExclusiveSmem ? s : kExclusiveSmem;
-}
-// Rows of the split-A21 buffer per part (hi, lo): the most rows below a panel's
-// diagonal block (kl), rounded up to whole M tiles.
+size_t patch_factor_smem() { return kFactorSmem; }
+// Rows of the split-A21 buffer per part (hi, lo) and rank: the most rows below
+// a panel's diagonal block (kl), rounded up to whole M tiles.
 int patch_a21_rows(int kl) { return (kl + kMT - 1) / kMT * kMT; }
 
 // x = hi + lo with hi, lo TF32 (round to nearest): the 3xTF32 split
@@ -76,7 +66,6 @@ __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
   hi = __uint_as_float(h);
   lo = __uint_as_float(l);
 }
-size_t patch_refine_smem(int64_t n) { return sizeof(float) * (size_t)n; }
 
 __device__ __forceinline__ void stamp(long long* tr, int slot) {
   if (tr && threadIdx.x == 0) {
@@ -94,65 +83,142 @@ __device__ __forceinline__ void cluster_sync() {
 
 // Bounded wait on an mbarrier phase: after kMbarPolls polls the wait gives up
 // and records 1 in *err (the patch's wait-ran-out word); once that word is
-// set every later wait gives up at its first poll, so the kernel runs to its
-// end quickly, and the host reports the failure.
+// set every later wait gives up within 64 polls, so the kernel runs to its end
+// quickly, and the host reports the failure.
 constexpr int kMbarPolls = 1 << 20;
 __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t& ph, int* err) {
-  for (int it = 0; !mbar_try_wait(bar, ph); ++it)
-    if (it > kMbarPolls || *(volatile int*)err) {
+  for (int it = 0; !mbar_try_wait(bar, ph); ++it)  // (the word is in global memory: a look at it delays the next poll)
+    if (it > kMbarPolls || ((it & 63) == 63 && *(volatile int*)err)) {
       atomicExch(err, 1);
       break;
     }
   ph ^= 1u;
 }
 
+// Two FP32 FMAs in one instruction, each rounded as fmaf: (a, b) as 64-bit pairs.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rc, ra, rb, rc;\n\tmov.b64 {%0, %1}, rc;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
+// Inverse of the w x w block (row `lane` in S, zero beyond w) by one warp: a
+// Gauss-Jordan sweep in place.  Step k exchanges column k for the pivot row p_k,
+// picked by size among the rows of k's node block (they end at row bend of
+// position k) not yet used; rows are never moved.  Afterwards S of row p_k holds
+// row k of the inverse, its entry k' standing for the block's row p_k', and the
+// inverse goes to Ai[row][column] (stride kIS) and, transposed, to inv.  The
+// columns rotate through the registers, so that the pivot column is always S[0]
+// and the step is one small loop body (unrolled over k it is 70 KB of code,
+// which one warp fetches at 0.5 us a step).  The pivot row travels through shared
+// memory: one lane's 16-byte stores, then broadcast reads.
+// Returns the first step (1-based) that found no usable pivot, 0 if none.
+__device__ __forceinline__ int warp_inverse(float (&S)[32], int w, int bend, float* srow, int* sp, float* Ai,
+                                            float* inv) {
+  const int lane = threadIdx.x & 31;
+  unsigned used = 0u;
+  int pos = lane, bad = 0;
+  if (lane >= w) sp[lane] = lane;
+#pragma unroll 1
+  for (int k = 0; k < w; ++k) {
+    const int bk = __shfl_sync(kFull, bend, k);
+    const bool cand = lane < bk && !((used >> lane) & 1u);
+    const unsigned key = cand ? pkey(S[0]) : 0u;
+    const unsigned mx = __reduce_max_sync(kFull, key);
+    const int p = __ffs(__ballot_sync(kFull, cand && key == mx)) - 1;  // the candidates are never empty
+    if (mx == 0u && bad == 0) bad = k + 1;
+    const bool own = lane == p;
+    if (own) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        reinterpret_cast<float4*>(srow)[c] = make_float4(S[4 * c], S[4 * c + 1], S[4 * c + 2], S[4 * c + 3]);
+      pos = k;
+      sp[k] = p;
+    }
+    used |= 1u << p;
+    const float r = __frcp_rn(__shfl_sync(kFull, S[0], p));
+    const float f = S[0];
+    const float fr = f * r, m = own ? -r : -fr;
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float4 u = reinterpret_cast<const float4*>(srow)[c];
+      if (c) S[4 * c - 1] = fmaf(m, u.x, own ? 0.0f : S[4 * c]);
+      S[4 * c] = fmaf(m, u.y, own ? 0.0f : S[4 * c + 1]);
+      S[4 * c + 1] = fmaf(m, u.z, own ? 0.0f : S[4 * c + 2]);
+      S[4 * c + 2] = fmaf(m, u.w, own ? 0.0f : S[4 * c + 3]);
+    }
+    S[31] = own ? r : fr;
+    __syncwarp();  // the row buffer is free for the next step
+  }
+#pragma unroll
+  for (int c = 0; c < 32; ++c) {  // S[c] holds column (c + w) mod 32
+    const int col = sp[(c + w) & 31];
+    Ai[pos * kIS + col] = S[c];
+    if (inv) inv[col * kBlkW + pos] = S[c];
+  }
+  return bad;
+}
+
 // trace (J.trace, optional): per panel 6 globaltimer stamps -- [0] start,
-// [1] diagonal block factored, [2] panel staged, inverses formed and A21 split,
-// [3] U12 / Y of the first chunk, [4] its trailing update, [5] panel done
+// [1] diagonal block inverted, [2] A21 split too, [3] Y of the first chunk,
+// [4] its trailing update, [5] panel done
 //
-// NR = 2: a patch on a cluster of two CTAs (launched with cluster dims (2,1,1)).
-// Rank 0 factors the diagonal block; both ranks stage the panel, form the
-// inverses and split half of A21 each; rank r updates the trailing chunks
-// r, r + 2, ... .  A column moves from rank 1's chunks to rank 0's as the
-// panels advance, so every band read goes to L2 (ld.global.cg) and each panel
-// ends at a cluster barrier; the factored block is published by another after
-// the panel factorisation.  Both ranks run the same panel loop, so every
-// barrier is reached by all threads of both CTAs.
+// Per panel: warp 0 inverts the diagonal block while the other warps split A21
+// into TF32 hi / lo parts (it needs nothing from the inverse) and every warp has
+// its first A12 columns in flight; then, per chunk of up to 256 trailing columns,
+// Y = Ai A12 (a lane per row, four columns at a time, Ai's row in registers) and
+// A22 -= A21 Y.
 //
-// The trailing update A22 -= A21 Y runs on the fifth-generation tensor cores:
-// per 128-row tile of A22, 3 x 4 tcgen05.mma of kind::tf32 (the 3xTF32 split
+// NR > 1: a patch on a cluster of NR CTAs.  Every rank inverts the diagonal block
+// and splits A21 for itself (into its own part of the split buffer) and updates
+// the trailing chunks rank, rank + NR, ...: what a rank needs of the others'
+// work is the band itself, so a panel has one cluster barrier, at its end.  All
+// ranks run the same panel loop, so every barrier is reached by all threads of
+// all CTAs.  Band reads go to L2 (ld.global.cg): a column moves between the
+// ranks' chunks as the panels advance.
+//
+// The trailing update runs on the fifth-generation tensor cores: per 128-row
+// tile of A22, 3 x 4 tcgen05.mma of kind::tf32 (the 3xTF32 split
 // a b ~ al bh + ah bl + ah bh over K = 32 in steps of 8) accumulate A21 Y in
 // Tensor Memory; the A21 tiles come by TMA (a 3-D tensor map over the patch's
 // split-A21 buffer, written once per panel) into two shared-memory buffers, so
 // the copy of tile t + 2 and the MMAs of tile t + 1 run while all 16 warps read
-// tile t's accumulators back (tcgen05.ld) and write A22 - A21 Y to the band.
+// tile t's accumulators back (tcgen05.ld) and write A22 - A21 Y to the band.  What
+// bounds it is the band's round trip through L2: a warp has the next 16 columns'
+// loads in flight while it subtracts the current ones.
+// Measured on a GB300 against an LU with staged panels and per-rank hand-overs
+// (three small triangular products per panel, 64-bit indexing in every access; it
+// was bound by its instructions, 316 k per panel of 24 x 24 ALEVB): 16 x 16 ALEVB
+// on four CTAs 3.3 -> 1.4 ms, 24 x 24 on one 12.5 -> 8.1 ms, 32 x 32 on one 31.4
+// -> 20.9 ms, 48 x 48 on four 50.6 -> 28.5 ms.
 template <int NR>
 __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __restrict__ jobs,
                                                              const int* __restrict__ order) {
-  constexpr bool CG = NR > 1;
   const int rank = (int)(blockIdx.x % NR);
   const PatchJob& J = jobs[order[blockIdx.x / NR]];
   const BandLayout L = J.L;
   float* __restrict__ ab = J.band;
-  const int Rp = patch_rp(L.kl);
   extern __shared__ __align__(1024) unsigned char smem_fac[];
-  // region 0: the panel's columns while the panel is staged, then the chunk buffers
-  float* Lp = reinterpret_cast<float*>(smem_fac);  // [32][Rp]: A(j0 + r, j0 + c) at Lp[c * Rp + r]
-  float* Yh = reinterpret_cast<float*>(smem_fac);  // [8][kNCH][4]
+  float* Yh = reinterpret_cast<float*>(smem_fac);
   float* Yl = reinterpret_cast<float*>(smem_fac + kYBytes);
-  unsigned char* Abuf = smem_fac + 2 * kYBytes;  // [2][A21h tile | A21l tile]
-  float* Li = reinterpret_cast<float*>(smem_fac + patch_region0(L.kl));  // [32][kIS]
-  float* Ui = Li + kBlkW * kIS;
-  float* Mi = Ui + kBlkW * kIS;
-  __shared__ float s_l[2][32];
-  __shared__ int s_p[2];
+  unsigned char* Abuf = smem_fac + 2 * kYBytes;                       // [2][A21h tile | A21l tile]
+  float* Ai = reinterpret_cast<float*>(smem_fac + kChunkBytes);       // [32][kIS]
+  float* sA = Ai + kBlkW * kIS;                                       // [16 warps][4][32]: four columns of A12
+  __shared__ __align__(16) float srow[32];
   __shared__ int sp[32];
-  __shared__ float rd[32];
   __shared__ __align__(8) uint64_t bar_tma[2], bar_mma[2];
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t ldm = L.ldb - 1;  // A(i, j + 1) - A(i, j) in the band array
   const int nrp = J.a21_rows;     // rows per part of the split-A21 buffer
+  const int npan = J.npan, kuf = J.kuf;
+  const int* __restrict__ ps = J.ps;
+  float* a21 = J.a21 + (size_t)rank * 2 * nrp * 4;  // this rank's rows of every k-quad plane
+  const size_t plane = (size_t)4 * 2 * nrp;         // float4 per k-quad plane (four ranks)
   int* err = J.info + 1;
 
   if (tid == 0) {
@@ -171,148 +237,131 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
   tc::fence_after();
   const uint32_t tmem = s_tmem;
   uint32_t ph_tma[2] = {0u, 0u}, ph_mma[2] = {0u, 0u};  // phases (thread 0 uses ph_tma)
+  float* sAw = sA + warp * 4 * kBlkW;
 
-  for (int p = 0; p < J.npan; ++p) {
-    const int64_t j0 = J.ps[p], j1 = J.ps[p + 1];
+  int j1n = ps[1];
+  for (int p = 0; p < npan; ++p) {
+    const int64_t j0 = p ? (int64_t)ps[p] : 0, j1 = j1n;
     const int w = (int)(j1 - j0);
+    j1n = p + 1 < npan ? ps[p + 2] : 0;
     const int R = (int)min64b(L.n - j0, (int64_t)w + L.kl);
-    const int C = (int)(min64b(L.n, j1 + J.kuf) - j1);
-    int* perm = J.perm + (size_t)p * kBlkW;
+    const int C = (int)(min64b(L.n, j1 + kuf) - j1);
+    const int nr = R - w;
+    const int ntile = (nr + kMT - 1) / kMT;
+    // trailing columns [j1, j1 + C) in chunks of nch <= kNCH, balanced over the ranks
+    const int cpr = (C + NR * kNCH - 1) / (NR * kNCH);  // chunks per rank
+    const int nch = C > 0 ? ((C + NR * cpr - 1) / (NR * cpr) + 15) & ~15 : kNCH;
     long long* tr = J.trace ? J.trace + (size_t)p * 6 : nullptr;
     stamp(tr, 0);
 
-    // 1. the diagonal block
-    if (rank == 0 && warp < kPanelWarps)
-      blk_panel_factor<float, CG>(ab, L, j0, w, J.blk_end, perm, J.rdiag, J.info, s_l, s_p);
-    __syncthreads();
-    if (NR > 1) cluster_sync();
-    stamp(tr, 1);
-
-    // 2. panel columns (all copies in flight at once), then the inverses of
-    //    L11 and U11 by column, each lane's column in registers
-    for (int c = 0; c < w; ++c) {
-      const float* src = ab + bix(L, j0, j0 + c);
-      if (CG) {
-        for (int r = tid; r < R; r += kPT) Lp[c * Rp + r] = __ldcg(src + r);
-      } else {
-        for (int r = tid; r < R; r += kPT) cp_async(Lp + c * Rp + r, src + r);
-      }
-    }
-    if (tid < kBlkW) {
-      sp[tid] = tid < w ? ldx<CG>(perm + tid) : 0;
-      rd[tid] = tid < w ? ldx<CG>(J.rdiag + j0 + tid) : 0.0f;
-    }
-    if (!CG) cp_async_wait_all();
-    __syncthreads();
-    if (warp < 2) {
-      float x[32];
+    // this warp's columns of A12 in chunk cb: 4 (warp + 16 g) .. + 3, g < 4; a lane per row
+    float a12[4][4];
+    auto load_a12 = [&](int cb) {
+      const int nc = min(nch, C - cb);
+      const float* src = ab + bix(L, j0 + lane, j1 + cb);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) x[i] = i == lane ? 1.0f : 0.0f;
-      if (warp == 0) {  // L11 X = I (unit lower), forward by columns of L
-#pragma unroll
-        for (int k = 0; k < 32; ++k)
-          if (k < w) {
-            const float xk = x[k];
-#pragma unroll
-            for (int i = k + 1; i < 32; ++i)
-              if (i < w) x[i] = fmaf(-Lp[k * Rp + i], xk, x[i]);
-          }
-      } else {  // U11 X = I, backward by columns of U
-#pragma unroll
-        for (int k = 31; k >= 0; --k)
-          if (k < w) {
-            x[k] *= rd[k];
-            const float xk = x[k];
-#pragma unroll
-            for (int i = 0; i < k; ++i) x[i] = fmaf(-Lp[k * Rp + i], xk, x[i]);
-          }
-      }
-      float* X = warp == 0 ? Li : Ui;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) X[i * kIS + lane] = (lane < w && i < w) ? x[i] : 0.0f;
-    } else {
-      // A21 (rows w .. R-1 of the panel) split into TF32 hi / lo parts, written
-      // to the patch's split-A21 buffer as 8 k-quad planes [k/4][row][k%4]
-      // (hi rows 0 .. nrp-1, lo rows nrp .. 2 nrp-1), rows past the panel and
-      // columns k >= w zero; each rank of a cluster writes its share of the rows
-      const int nr = R - w;
-      const int nrt = (nr + kMT - 1) / kMT * kMT;
-      const int rlo = rank * (nrt / NR), rhi = rank + 1 == NR ? nrt : (rank + 1) * (nrt / NR);
-      for (int idx = tid - 64; idx < (rhi - rlo) * 8; idx += kPT - 64) {
-        const int r = rlo + idx % (rhi - rlo), kq = idx / (rhi - rlo);
-        float4 h, l;
-        float* hv = &h.x;
-        float* lv = &l.x;
+      for (int g = 0; g < 4; ++g)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int k = 4 * kq + e;
-          const float v = (r < nr && k < w) ? Lp[k * Rp + w + r] : 0.0f;
-          split_tf32(v, hv[e], lv[e]);
+          const int c = 4 * (warp + 16 * g) + e;
+          a12[g][e] = (c < nc && lane < w) ? __ldcg(src + (int64_t)c * ldm) : 0.0f;
         }
-        float4* plane = reinterpret_cast<float4*>(J.a21) + (size_t)kq * 2 * nrp;
-        plane[r] = h;
-        plane[nrp + r] = l;
+    };
+
+    // 1. the diagonal block's inverse; A21 split
+    if (warp == 0) {
+      float S[32];
+      const float* src = ab + bix(L, j0 + lane, j0);
+#pragma unroll
+      for (int c = 0; c < 32; ++c) S[c] = (lane < w && c < w) ? __ldcg(src + (int64_t)c * ldm) : 0.0f;
+      const int bend = lane < w ? (int)(J.blk_end[j0 + lane] - j0) : 0;
+      const int bad =
+          warp_inverse(S, w, bend, srow, sp, Ai, rank == 0 ? J.inv + (size_t)p * kBlkW * kBlkW : nullptr);
+      if (rank == 0 && lane == 0 && bad) atomicCAS(J.info, 0, (int)(j0 + bad));
+      load_a12(rank * nch);
+    } else {
+      load_a12(rank * nch);
+      // A21 (rows w .. R-1 of the panel) split into TF32 hi / lo parts, written to
+      // the rank's part of the split-A21 buffer as 8 k-quad planes [k/4][row][k%4]
+      // (hi rows 0 .. nrp-1, lo rows nrp .. 2 nrp-1), rows past the panel and
+      // columns k >= w zero
+      for (int task = warp - 1; task < ntile * (kMT / 4); task += kPT / 32 - 1) {  // a k-quad of 32 rows
+        const int kq = task & 7, r = (task >> 3) * 32 + lane;
+        const float* src = ab + bix(L, j0 + w + min(r, nr - 1), j0 + 4 * kq);
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = 4 * kq + e < w ? __ldcg(src + e * ldm) : 0.0f;
+        float4 h, l;
+        const bool in = r < nr;
+        split_tf32(in ? v[0] : 0.0f, h.x, l.x);
+        split_tf32(in ? v[1] : 0.0f, h.y, l.y);
+        split_tf32(in ? v[2] : 0.0f, h.z, l.z);
+        split_tf32(in ? v[3] : 0.0f, h.w, l.w);
+        float4* pl = reinterpret_cast<float4*>(a21) + kq * plane;
+        pl[r] = h;
+        pl[nrp + r] = l;
       }
-      fence_proxy_async_global();  // read by TMA (this CTA or, after the cluster barrier, the other)
+      fence_proxy_async_global();  // read by TMA
     }
+    stamp(tr, 1);
     __syncthreads();
-    float* inv = J.inv + (size_t)p * 2 * kBlkW * kBlkW;  // Li then Ui, 32 x 32, column-major
-    for (int idx = tid; idx < kBlkW * kBlkW; idx += kPT) {
-      const int i = idx >> 5, c = idx & 31;
-      float s = 0.0f;
-      for (int k = max(i, c); k < w; ++k) s = fmaf(Ui[i * kIS + k], Li[k * kIS + c], s);
-      Mi[i * kIS + c] = s;
-      if (rank == 0) {  // stored transposed: element (i, c) at c * 32 + i
-        inv[c * kBlkW + i] = Li[i * kIS + c];
-        inv[kBlkW * kBlkW + c * kBlkW + i] = Ui[i * kIS + c];
-      }
-    }
-    __syncthreads();
-    if (NR > 1) cluster_sync();  // both halves of the split A21 written (and Lp no longer read)
     stamp(tr, 2);
 
-    // 3. trailing columns [j1, j1 + C) in chunks of nch <= kNCH, balanced over the ranks
-    const int nr = R - w;
-    const int ntile = (nr + kMT - 1) / kMT;
-    const int cpr = (C + NR * kNCH - 1) / (NR * kNCH);  // chunks per rank
-    const int nch = C > 0 ? ((C + NR * cpr - 1) / (NR * cpr) + 15) & ~15 : kNCH;
     bool first = true;
     for (int cb = rank * nch; cb < C; cb += NR * nch) {
       const int nc = min(nch, C - cb);
       const int ncp = (nc + 15) & ~15;  // the MMA's N
-      // U12 = Li P A12 and Y = Mi P A12: one thread per column, the column in
-      // registers; Y goes to Yh / Yl split into TF32 parts (zero beyond nc)
-      for (int c = tid; c < ncp; c += kPT) {
-        const int64_t col = j1 + cb + c;
-        float* dst = ab + bix(L, j0, col);  // A(j0 + r, col) = dst[r]
-        float a[32];
+      auto tma_tile = [&](int t) {      // thread 0: tile t's A21h and A21l into buffer t & 1
+        const int b = t & 1, row = rank * 2 * nrp + t * kMT;
+        mbar_arrive_expect_tx(&bar_tma[b], 2 * kATile);
+        tc::tma_load_3d(Abuf + b * 2 * kATile, &J.a21_map, 0, row, 0, &bar_tma[b]);
+        tc::tma_load_3d(Abuf + b * 2 * kATile + kATile, &J.a21_map, 0, nrp + row, 0, &bar_tma[b]);
+      };
+      if (tid == 0 && ntile > 0) {
+        tma_tile(0);
+        if (ntile > 1) tma_tile(1);
+      }
+      // Y = Ai A12, split into TF32 parts for the MMA and written over A12
+      if (!first) load_a12(cb);
+      {
+        float ar[32];  // row `lane` of Ai
 #pragma unroll
-        for (int k = 0; k < 32; ++k) a[k] = (c < nc && k < w) ? ldx<CG>(dst + sp[k]) : 0.0f;
-#pragma unroll 2
-        for (int r = 0; r < 32; ++r) {
-          float u = 0.0f, y = 0.0f;
-          if (r < w) {  // block-uniform
-            const float4* l4 = reinterpret_cast<const float4*>(Li + r * kIS);
-            const float4* m4 = reinterpret_cast<const float4*>(Mi + r * kIS);
+        for (int k = 0; k < 8; ++k) {
+          const float4 q = reinterpret_cast<const float4*>(Ai + lane * kIS)[k];
+          ar[4 * k] = q.x, ar[4 * k + 1] = q.y, ar[4 * k + 2] = q.z, ar[4 * k + 3] = q.w;
+        }
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const float4 l = l4[k], m = m4[k];
-              u = fmaf(l.x, a[4 * k], u);
-              u = fmaf(l.y, a[4 * k + 1], u);
-              u = fmaf(l.z, a[4 * k + 2], u);
-              u = fmaf(l.w, a[4 * k + 3], u);
-              y = fmaf(m.x, a[4 * k], y);
-              y = fmaf(m.y, a[4 * k + 1], y);
-              y = fmaf(m.z, a[4 * k + 2], y);
-              y = fmaf(m.w, a[4 * k + 3], y);
+        for (int g = 0; g < 4; ++g) {
+          const int c = 4 * (warp + 16 * g);
+          if (c < ncp) {  // warp-uniform
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sAw[e * kBlkW + lane] = a12[g][e];
+            __syncwarp();
+            float y[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              float2 s0 = make_float2(0.0f, 0.0f), s1 = s0;
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const float4 q = reinterpret_cast<const float4*>(sAw + e * kBlkW)[k];
+                s0 = fma2(make_float2(ar[4 * k], ar[4 * k + 1]), make_float2(q.x, q.y), s0);
+                s1 = fma2(make_float2(ar[4 * k + 2], ar[4 * k + 3]), make_float2(q.z, q.w), s1);
+              }
+              y[e] = (s0.x + s0.y) + (s1.x + s1.y);
             }
-            if (c < nc) dst[r] = u;  // U12
+            __syncwarp();
+            float* dst = ab + bix(L, j0 + lane, j1 + cb + c);
+            const int o = (lane >> 2) * kYQuad + 4 * c + (lane & 3);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float v = (lane < w && c + e < nc) ? y[e] : 0.0f;  // rows k >= w of Y: zero
+              float yh, yl;
+              split_tf32(v, yh, yl);
+              Yh[o + 4 * e] = yh;
+              Yl[o + 4 * e] = yl;
+              if (lane < w && c + e < nc) dst[(int64_t)e * ldm] = y[e];
+            }
           }
-          float yh, yl;
-          split_tf32(y, yh, yl);  // rows r >= w: 0
-          const int o = (r >> 2) * (4 * kNCH) + 4 * c + (r & 3);
-          Yh[o] = yh;
-          Yl[o] = yl;
         }
       }
       fence_proxy_async_smem();  // Yh / Yl are read by the tensor cores
@@ -323,12 +372,6 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
       const uint32_t idesc = tc::idesc_tf32(kMT, ncp);
       const uint32_t yh = tc::saddr(Yh), yl = tc::saddr(Yl), a0 = tc::saddr(Abuf);
       const int ksteps = (w + 7) >> 3;
-      auto tma_tile = [&](int t) {  // thread 0: tile t's A21h and A21l into buffer t & 1
-        const int b = t & 1;
-        mbar_arrive_expect_tx(&bar_tma[b], 2 * kATile);
-        tc::tma_load_3d(Abuf + b * 2 * kATile, &J.a21_map, 0, t * kMT, 0, &bar_tma[b]);
-        tc::tma_load_3d(Abuf + b * 2 * kATile + kATile, &J.a21_map, 0, nrp + t * kMT, 0, &bar_tma[b]);
-      };
       auto mma_tile = [&](int t) {  // thread 0: tile t's products into accumulator t & 1
         const int b = t & 1;
         mbar_wait_bounded(&bar_tma[b], ph_tma[b], err);
@@ -345,16 +388,31 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
         }
         tc::commit(&bar_mma[b]);
       };
-      if (tid == 0 && ntile > 0) {
-        tma_tile(0);
-        if (ntile > 1) tma_tile(1);
-        mma_tile(0);
-      }
+      if (tid == 0 && ntile > 0) mma_tile(0);
       // epilogue roles: warp w reads lanes 32 (w % 4) .. + 31 (its rows) of
-      // column group w / 4 (a quarter of the chunk, in multiples of 8 columns)
+      // column group w / 4 (a quarter of the chunk, in multiples of 8 columns),
+      // 16 columns at a time
       const int q = warp & 3, grp = warp >> 2;
       const int cpg = ((ncp >> 2) + 7) & ~7;
-      const int cs = min(ncp, grp * cpg), ce = min(ncp, cs + cpg);
+      const int cs = min(ncp, grp * cpg), ce = min(ncp, cs + cpg), lim = min(ce, nc);
+      float vn[16];  // A22 of the next step
+      auto load_a22 = [&](int t, int c0) {
+        const float* pa = ab + bix(L, j0 + min(w + t * kMT + 32 * q + lane, R - 1), j1 + cb + c0);
+        if (c0 + 16 <= lim) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            vn[k] = __ldcg(pa);
+            pa += ldm;
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            vn[k] = c0 + k < lim ? __ldcg(pa) : 0.0f;
+            pa += ldm;
+          }
+        }
+      };
+      if (ntile > 0 && cs < lim) load_a22(0, cs);
       for (int t = 0; t < ntile; ++t) {
         const int b = t & 1;
         mbar_wait_bounded(&bar_mma[b], ph_mma[b], err);  // tile t's products are in Tensor Memory
@@ -365,19 +423,30 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
         tc::fence_after();
         const int row = w + t * kMT + 32 * q + lane;  // panel row of this thread
         const bool live = row < R;
-        float* pa = ab + bix(L, j0 + (live ? row : 0), j1 + cb);  // + c * ldm: A(j0 + row, j1 + cb + c)
+        float* pa = ab + bix(L, j0 + (live ? row : 0), j1 + cb + cs);
         const uint32_t dt = tmem + ((uint32_t)(32 * q) << 16) + b * kNCH;
-        for (int c0 = cs; c0 < ce; c0 += 16) {
-          float d0[8], d1[8];
+        for (int c0 = cs; c0 < lim; c0 += 16) {
+          float d0[8], d1[8], v[16];
           tc::ld8(dt + c0, d0);
           if (c0 + 8 < ce) tc::ld8(dt + c0 + 8, d1);
+#pragma unroll
+          for (int k = 0; k < 16; ++k) v[k] = vn[k];
+          if (c0 + 16 < lim) load_a22(t, c0 + 16);
+          else if (t + 1 < ntile) load_a22(t + 1, cs);
           tc::wait_ld();
-          float v[16];
+          if (live) {
+            if (c0 + 16 <= lim) {
 #pragma unroll
-          for (int k = 0; k < 16; ++k) v[k] = (live && c0 + k < ce && c0 + k < nc) ? ldx<CG>(pa + (int64_t)(c0 + k) * ldm) : 0.0f;
+              for (int k = 0; k < 16; ++k) {
+                *pa = v[k] - (k < 8 ? d0[k] : d1[k - 8]);
+                pa += ldm;
+              }
+            } else {
 #pragma unroll
-          for (int k = 0; k < 16; ++k)
-            if (live && c0 + k < ce && c0 + k < nc) pa[(int64_t)(c0 + k) * ldm] = v[k] - (k < 8 ? d0[k] : d1[k - 8]);
+              for (int k = 0; k < 16; ++k)
+                if (c0 + k < lim) pa[k * ldm] = v[k] - (k < 8 ? d0[k] : d1[k - 8]);
+            }
+          }
         }
         tc::fence_before();
         __syncthreads();  // accumulator b is read before the MMAs of tile t + 2 overwrite it
@@ -386,6 +455,7 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
       first = false;
     }
     if (NR > 1) cluster_sync();
+    else __syncthreads();
     stamp(tr, 5);
   }
   tc::fence_before();
@@ -415,170 +485,284 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 }
 
 constexpr int kTraceSweeps = 32;  // sweeps the refinement trace records
-constexpr int kFwdRows = 1;       // A21 rows per thread (warps 1..31) whose loads run ahead
-constexpr int kBwdCols = 24;      // U12 columns per warp whose loads run ahead
+constexpr int kRing = 4;          // panels whose critical blocks are staged ahead
+constexpr int kRowT = kRT - 32;   // rows (columns) the update warps hold per register set
+struct RefineSmem {
+  float ring[kRing][2][kBlkW * kBlkW];  // forward: A21's rows of the next panel, the next panel's Ai; backward: Y's columns
+  float zb[2][kBlkW];                   // z of the current panel, by parity
+  float bb[kBlkW];
+  float part[2][kRT / 32][kBlkW];       // backward: the update warps' sums, by parity
+  double red[kRT / 32];
+};
+size_t patch_refine_smem(int64_t n, int npan) {
+  return sizeof(RefineSmem) + sizeof(float) * (size_t)n + sizeof(int) * ((size_t)npan + 1);
+}
 
-// v <- (L U)^-1 v with the stored factors and inverses.  Every panel step
-// waits for one round trip at most: the next panel's inverses are copied into
-// a second shared buffer while the current panel is processed, and each
-// thread loads its next A21 rows (forward) or U12 columns (backward) into
-// registers as soon as it has used the current ones.
-// inv_s: 2 x (2 x 32 x 32) floats of shared memory, 16-byte aligned.
-// prof (trace mode, optional): thread 0 and thread 32 add the globaltimer
-// time of each phase -- [0..3] thread 0 forward: wait + barrier, warp-0 work,
-// barrier, row update; [4..7] thread 32 the same; [8..11] thread 0 backward:
-// partial sums + prefetch, wait + barrier, warp-0 work, barrier; [12..15] thread 32
 __device__ __forceinline__ long long gtime() {
   unsigned long long v;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v));
   return (long long)v;
 }
-__device__ void patch_lu_solve(const PatchJob& J, float* v, float* bz, float (*part)[33], float* inv_s,
-                               long long* prof) {
-  const bool pt = prof && (threadIdx.x == 0 || threadIdx.x == 32);
-  const int po = threadIdx.x == 32 ? 4 : 0;
-  long long tk = pt ? gtime() : 0;
-  auto lap = [&](int slot) {
-    if (pt) {
-      const long long t1 = gtime();
-      prof[slot] += t1 - tk;
-      tk = t1;
-    }
-  };
-  const BandLayout L = J.L;
+
+// sum_k m[k * 32 + lane] x[k]: a 32 x 32 block (column-major) times a vector, both in shared memory
+__device__ __forceinline__ float block_times(const float* m, const float* x) {
+  const int lane = threadIdx.x & 31;
+  float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float4 q = reinterpret_cast<const float4*>(x)[k];
+    s[0] = fmaf(m[(4 * k) * 32 + lane], q.x, s[0]);
+    s[1] = fmaf(m[(4 * k + 1) * 32 + lane], q.y, s[1]);
+    s[2] = fmaf(m[(4 * k + 2) * 32 + lane], q.z, s[2]);
+    s[3] = fmaf(m[(4 * k + 3) * 32 + lane], q.w, s[3]);
+  }
+  return (s[0] + s[1]) + (s[2] + s[3]);
+}
+
+// v <- K^-1 v with the block factors.  Warp 0 runs the chain: per panel of the
+// forward pass it finishes the next panel's rows (b1 = v - A21 z there), forms
+// z = Ai b1 and publishes it; the other 15 warps subtract A21 z from the rows
+// below (32 rows a warp), one step behind.  Backward: x1 = z - Y x2, the chain
+// with the columns of the panel solved last, the others with the columns beyond
+// (a run of columns per warp), one panel ahead of it.  One barrier per panel.  The
+// blocks of the chain come through a ring of cp.async copies kRing - 1 panels
+// ahead; the update warps hold their rows (columns) in registers, loaded ahead:
+// with RPT = 1 two panels ahead (bands up to 480 rows below the next panel), with
+// RPT = 2 two sets, one panel ahead; wider bands read the rest on the spot.  Bound:
+// the chain's two 32 x 32 products and the barrier, and the update warps'
+// instructions, one load per 32 entries.
+// Measured on a GB300, one forward and backward pass, against whole-CTA steps with
+// three small products and three barriers per panel: 16 x 16 ALEVB (70 panels) 666
+// -> 150 us, 32 x 32 3.13 -> 1.07 ms, 48 x 48 (RPT = 2) 10.7 -> 3.06 ms.
+// prof (trace mode, optional): [0] forward, [1] backward time of warp 0 in ns.
+__device__ __forceinline__ void solve_barrier() { bar_sync_n(1, kRT); }
+// dot product of 32 register values with 32 values in shared memory (16-byte aligned)
+__device__ __forceinline__ float dot32(const float (&x)[32], const float* z) {
+  float2 s0 = make_float2(0.0f, 0.0f), s1 = s0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float4 q = reinterpret_cast<const float4*>(z)[k];
+    s0 = fma2(make_float2(x[4 * k], x[4 * k + 1]), make_float2(q.x, q.y), s0);
+    s1 = fma2(make_float2(x[4 * k + 2], x[4 * k + 3]), make_float2(q.z, q.w), s1);
+  }
+  return (s0.x + s0.y) + (s1.x + s1.y);
+}
+// lambdas with register arrays: always inlined, so that the arrays stay in registers
+#define MAFEM_INLINE __attribute__((always_inline))
+template <int RPT>
+__device__ __forceinline__ void patch_solve_pass(const PatchJob& J, float* v, const int* ps, RefineSmem& S,
+                                                 long long* prof) {
+  constexpr int NB = 3 - RPT;          // panels in flight in registers
+  constexpr int kUW = kRT / 32 - 1;    // update warps
   const float* __restrict__ ab = J.band;
-  const int64_t ldm = L.ldb - 1;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int npan = J.npan;
-  constexpr int kInv = 2 * kBlkW * kBlkW;  // floats per panel: Li then Ui, column-major
-  auto inv_copy = [&](int p, int buf) {  // 512 threads x 16 bytes = one panel's Li and Ui
-    if (p >= 0 && p < npan && tid < kInv / 4)
-      cp_async16(inv_s + buf * kInv + tid * 4, J.inv + (size_t)p * kInv + tid * 4);
-    cp_async_commit();
-  };
-  // ---- forward: per panel y1 = Li P b1, z = Ui y1, b2 -= A21 z
-  const int rt = tid - 32;  // row slot of warps 1..15
-  float t[kFwdRows][32];
-  auto fwd_load = [&](int p) {  // this thread's A21 rows of panel p
-    if (rt < 0 || p >= npan) return;
-    const int64_t j0 = J.ps[p], j1 = J.ps[p + 1];
-    const int w = (int)(j1 - j0);
-    const int64_t rend = j0 + min64b(L.n - j0, (int64_t)w + L.kl);
-#pragma unroll
-    for (int q = 0; q < kFwdRows; ++q) {
-      const int64_t i = j1 + rt + (int64_t)q * (kRT - 32);
-      const float* a = ab + bix(L, i, j0);
-#pragma unroll
-      for (int k = 0; k < 32; ++k) t[q][k] = (i < rend && k < w) ? a[k * ldm] : 0.0f;
-    }
-  };
-  inv_copy(0, 0);
-  fwd_load(0);
-  int pnext = warp == 0 && lane < J.ps[1] - J.ps[0] ? J.perm[lane] : 0;  // panel 0's permutation
-  for (int p = 0; p < npan; ++p) {
-    const int64_t j0 = J.ps[p], j1 = J.ps[p + 1];
-    const int w = (int)(j1 - j0);
-    const int64_t rend = j0 + min64b(L.n - j0, (int64_t)w + L.kl);
-    inv_copy(p + 1, (p + 1) & 1);
-    cp_async_wait_group<1>();  // this panel's inverses (this thread's part)
-    __syncthreads();
-    lap(po + 0);
-    const float* Li = inv_s + (p & 1) * kInv;
-    const float* Ui = Li + kBlkW * kBlkW;
-    if (warp == 0) {
-      const int pm = pnext;
-      if (p + 1 < npan && lane < J.ps[p + 2] - j1) pnext = J.perm[(size_t)(p + 1) * kBlkW + lane];
-      const float b = lane < w ? v[j0 + pm] : 0.0f;
-      float y = 0.0f;
-#pragma unroll
-      for (int k = 0; k < 32; ++k) y = fmaf(Li[k * 32 + lane], __shfl_sync(kFull, b, k), y);
+  const float* __restrict__ invs = J.inv;
+  const int ldm = (int)J.L.ldb - 1, n = (int)J.L.n, off = (int)J.L.off;
+  const int lane = threadIdx.x & 31, cw = (int)(threadIdx.x >> 5) - 1;
+  const int npan = J.npan, kuf = J.kuf, kl = J.L.kl;
+  auto at = [&](int i, int j) MAFEM_INLINE { return ab + ((int64_t)j * ldm + off + i); };  // A(i, j)
+
+  if (cw < 0) {  // ---- warp 0: the chain
+    const long long t0 = prof ? gtime() : 0;
+    {
+      const int w = ps[1];
+      const float b = lane < w ? v[lane] : 0.0f;
       float z = 0.0f;
 #pragma unroll
-      for (int k = 0; k < 32; ++k) z = fmaf(Ui[k * 32 + lane], __shfl_sync(kFull, y, k), z);
-      if (lane < w) v[j0 + lane] = y;
-      bz[lane] = lane < w ? z : 0.0f;
+      for (int k = 0; k < 32; ++k) z = fmaf(__ldcg(invs + k * 32 + lane), __shfl_sync(kFull, b, k), z);
+      S.zb[0][lane] = lane < w ? z : 0.0f;
+      if (lane < w) v[lane] = z;
     }
-    lap(po + 1);
-    __syncthreads();
-    lap(po + 2);
-    if (rt >= 0) {
-#pragma unroll
-      for (int q = 0; q < kFwdRows; ++q) {
-        const int64_t i = j1 + rt + (int64_t)q * (kRT - 32);
-        if (i < rend) {
-          float sacc = 0.0f;
-#pragma unroll
-          for (int k = 0; k < 32; ++k) sacc = fmaf(t[q][k], bz[k], sacc);
-          v[i] -= sacc;
-        }
-      }
-      // rows beyond kFwdRows slots (very wide bands): loaded on the spot
-      for (int64_t i = j1 + rt + (int64_t)kFwdRows * (kRT - 32); i < rend; i += kRT - 32) {
-        const float* a = ab + bix(L, i, j0);
-        float sacc = 0.0f;
-        for (int k = 0; k < w; ++k) sacc = fmaf(a[k * ldm], bz[k], sacc);
-        v[i] -= sacc;
-      }
-      fwd_load(p + 1);
+    int j1 = ps[1];
+#pragma unroll 1
+    for (int p = 0; p + 1 < npan; ++p) {
+      const int j2 = ps[p + 2], wn = j2 - j1;
+      solve_barrier();  // ring slot p; the updates by panel p - 1
+      const float b = (lane < wn ? v[j1 + lane] : 0.0f) - block_times(S.ring[p % kRing][0], S.zb[p & 1]);
+      S.bb[lane] = lane < wn ? b : 0.0f;
+      __syncwarp();
+      const float z = block_times(S.ring[p % kRing][1], S.bb);
+      S.zb[(p + 1) & 1][lane] = lane < wn ? z : 0.0f;
+      if (lane < wn) v[j1 + lane] = z;
+      __syncwarp();
+      j1 = j2;
     }
-    lap(po + 3);
+    solve_barrier();
+    const long long t1 = prof ? gtime() : 0;
+    solve_barrier();  // the last panel's sums
+#pragma unroll 1
+    for (int p = npan - 1; p >= 0; --p) {
+      const int j0 = ps[p], w = ps[p + 1] - j0;
+      float s = p + 1 < npan ? block_times(S.ring[p % kRing][0], S.bb) : 0.0f;
+      float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int k = 0; k < kUW; ++k) a[k & 3] += S.part[p & 1][k][lane];
+      const float x = (lane < w ? v[j0 + lane] : 0.0f) - (s + ((a[0] + a[1]) + (a[2] + a[3])));
+      __syncwarp();  // bb is read before it is overwritten
+      S.bb[lane] = lane < w ? x : 0.0f;
+      if (lane < w) v[j0 + lane] = x;
+      solve_barrier();
+    }
+    if (prof && lane == 0) {
+      prof[0] += t1 - t0;
+      prof[1] += gtime() - t1;
+    }
+    return;
   }
-  cp_async_wait_group<0>();
-  __syncthreads();
-  tk = pt ? gtime() : 0;
-  // ---- backward: per panel x1 = Ui (y1 - U12 x2)
-  float u[kBwdCols];
-  auto bwd_load = [&](int p) {  // this lane's row of U12 in this warp's columns, panel p
-    if (p < 0) return;
-    const int64_t j0 = J.ps[p], j1 = J.ps[p + 1];
-    const int w = (int)(j1 - j0);
-    const int C = (int)(min64b(L.n, j1 + J.kuf) - j1);
-    const float* ur = ab + bix(L, j0 + lane, j1);  // U(j0 + lane, j1 + c) = ur[c * ldm]
+
+  // ---- the update warps
+  float t[2][32];
+  // ring slot p: A21 of panel p in panel p + 1's rows (a warp per column), Ai of panel p + 1
+  auto stage_fwd = [&](int p) MAFEM_INLINE {
+    if (p + 1 < npan) {
+      const int j0 = ps[p], j1 = ps[p + 1], w = j1 - j0, lim = min(ps[p + 2] - j1, kl);
+      float* T = S.ring[p % kRing][0];
+      for (int c = cw; c < kBlkW; c += kUW) {  // (columns c >= w meet zeros of z: they must be finite)
+        if (lane < lim && c < w) cp_async(T + c * 32 + lane, at(j1 + lane, j0 + c));
+        else T[c * 32 + lane] = 0.0f;
+      }
+      if (cw < 8)
+        cp_async16(S.ring[p % kRing][1] + 128 * cw + 4 * lane, invs + (size_t)(p + 1) * kBlkW * kBlkW + 128 * cw + 4 * lane);
+    }
+    cp_async_commit();
+  };
+  // this warp's 32 rows of panel p's A21 below panel p + 1: set q starts at row0 + 32 (cw + 15 q)
+  auto row0 = [&](int p) MAFEM_INLINE { return (p + 1 < npan ? ps[p + 2] : n) + 32 * cw; };
+  auto load_rows = [&](int p, float (&x)[32], int q) MAFEM_INLINE {
+    if (p >= npan) return;
+    const int j0 = ps[p], w = ps[p + 1] - j0, rend = min(n, ps[p + 1] + kl), i0 = row0(p) + 32 * kUW * q;
+    if (i0 >= rend) return;  // warp-uniform
+    const float* a = at(min(i0 + lane, rend - 1), j0);
+    if (w == 32) {
 #pragma unroll
-    for (int m = 0; m < kBwdCols; ++m) {
-      const int c = warp + m * (kRT / 32);
-      u[m] = (lane < w && c < C) ? ur[(int64_t)c * ldm] : 0.0f;
+      for (int k = 0; k < 32; ++k) {
+        x[k] = __ldcg(a);
+        a += ldm;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 32; ++k) {
+        x[k] = k < w ? __ldcg(a) : 0.0f;
+        a += ldm;
+      }
     }
   };
-  inv_copy(npan - 1, (npan - 1) & 1);
-  bwd_load(npan - 1);
-  for (int p = npan - 1; p >= 0; --p) {
-    const int64_t j0 = J.ps[p], j1 = J.ps[p + 1];
-    const int w = (int)(j1 - j0);
-    const int C = (int)(min64b(L.n, j1 + J.kuf) - j1);
-    inv_copy(p - 1, (p - 1) & 1);
-    float acc = 0.0f;
-#pragma unroll
-    for (int m = 0; m < kBwdCols; ++m) {
-      const int c = warp + m * (kRT / 32);
-      if (c < C) acc = fmaf(u[m], v[j1 + c], acc);
+  auto use_rows = [&](int p, const float (&x)[32], int q) MAFEM_INLINE {
+    const int rend = min(n, ps[p + 1] + kl), i0 = row0(p) + 32 * kUW * q;
+    if (i0 >= rend) return;
+    const float s = dot32(x, S.zb[p & 1]);
+    if (i0 + lane < rend) v[i0 + lane] -= s;
+  };
+  auto far_rows = [&](int p) MAFEM_INLINE {  // rows beyond the registers' reach
+    const int j0 = ps[p], w = ps[p + 1] - j0, rend = min(n, ps[p + 1] + kl);
+    for (int i = row0(p) + 32 * kUW * RPT + lane; i < rend; i += 32 * kUW) {
+      const float* a = at(i, j0);
+      float s = 0.0f;
+#pragma unroll 8
+      for (int k = 0; k < w; ++k) s = fmaf(__ldcg(a + (int64_t)k * ldm), S.zb[p & 1][k], s);
+      v[i] -= s;
     }
-    if (lane < w) {  // columns beyond kBwdCols slots (very wide bands): loaded on the spot
-      const float* ur = ab + bix(L, j0 + lane, j1);
-      for (int c = warp + kBwdCols * (kRT / 32); c < C; c += kRT / 32) acc = fmaf(ur[(int64_t)c * ldm], v[j1 + c], acc);
+  };
+  for (int p = 0; p < kRing - 1; ++p) stage_fwd(p);
+  load_rows(0, t[0], 0);
+  if constexpr (RPT == 1) load_rows(1, t[1], 0);
+  else load_rows(0, t[1], 1);
+  auto fwd_step = [&](int p, float (&x0)[32], float (&x1)[32]) MAFEM_INLINE {
+    cp_async_wait_group<kRing - 2>();  // ring slot p (this thread's part)
+    solve_barrier();                   // z of panel p; the updates by panel p - 1
+    stage_fwd(p + kRing - 1);
+    use_rows(p, x0, 0);
+    load_rows(p + NB, x0, 0);
+    if constexpr (RPT == 2) {
+      use_rows(p, x1, 1);
+      load_rows(p + NB, x1, 1);
+      far_rows(p);
     }
-    part[warp][lane] = acc;
-    bwd_load(p - 1);
-    lap(8 + po);
-    cp_async_wait_group<1>();  // this panel's inverses
-    __syncthreads();
-    lap(9 + po);
-    if (warp == 0) {
-      const float* Ui = inv_s + (p & 1) * kInv + kBlkW * kBlkW;
-      float sum = 0.0f;
-      for (int q = 0; q < kRT / 32; ++q) sum += part[q][lane];
-      const float tv = lane < w ? v[j0 + lane] - sum : 0.0f;
-      float x = 0.0f;
-#pragma unroll
-      for (int k = 0; k < 32; ++k) x = fmaf(Ui[k * 32 + lane], __shfl_sync(kFull, tv, k), x);
-      if (lane < w) v[j0 + lane] = x;
-    }
-    lap(10 + po);
-    __syncthreads();
-    lap(11 + po);
+  };
+#pragma unroll 1
+  for (int p = 0; p < npan; p += NB) {
+    fwd_step(p, t[0], t[1]);
+    if (NB == 2 && p + 1 < npan) fwd_step(p + 1, t[1], t[0]);
   }
   cp_async_wait_group<0>();
-  __syncthreads();
+  // backward.  Ring slot p: Y of panel p in panel p + 1's columns
+  auto stage_bwd = [&](int p) MAFEM_INLINE {
+    if (p >= 0 && p + 1 < npan) {
+      const int j0 = ps[p], j1 = ps[p + 1], w = j1 - j0, lim = min(ps[p + 2] - j1, kuf);
+      float* T = S.ring[p % kRing][0];
+      for (int c = cw; c < kBlkW; c += kUW) {
+        if (lane < w && c < lim) cp_async(T + c * 32 + lane, at(j0 + lane, j1 + c));
+        else T[c * 32 + lane] = 0.0f;
+      }
+    }
+    cp_async_commit();
+  };
+  // this warp's run of columns of panel p's Y beyond panel p + 1: `len` columns from first
+  struct Run {
+    int first, len;
+  };
+  auto run_of = [&](int p) MAFEM_INLINE {
+    const int c0 = p + 1 < npan ? ps[p + 2] : n, end = min(n, ps[p + 1] + kuf);
+    const int len = max(0, (end - c0 + kUW - 1) / kUW), first = c0 + cw * len;
+    return Run{first, max(0, min(len, end - first))};
+  };
+  auto load_cols = [&](int p, float (&x)[32], int q) MAFEM_INLINE {
+    if (p < 0) return;
+    const Run r = run_of(p);
+    const int j0 = ps[p], w = ps[p + 1] - j0;
+    const float* a = at(j0 + min(lane, w - 1), r.first + 32 * q);
+#pragma unroll
+    for (int m0 = 0; m0 < 32; m0 += 8) {
+      if (32 * q + m0 >= r.len) break;  // warp-uniform
+#pragma unroll
+      for (int m = m0; m < m0 + 8; ++m) {
+        x[m] = 32 * q + m < r.len ? __ldcg(a) : 0.0f;
+        a += ldm;
+      }
+    }
+  };
+  auto use_cols = [&](int p, const float (&x)[32], int q) MAFEM_INLINE {
+    const Run r = run_of(p);
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const float* vx = v + r.first + 32 * q;
+#pragma unroll
+    for (int m0 = 0; m0 < 32; m0 += 8) {
+      if (32 * q + m0 >= r.len) break;
+#pragma unroll
+      for (int m = m0; m < m0 + 8; ++m) s[m & 3] = fmaf(x[m], 32 * q + m < r.len ? vx[m] : 0.0f, s[m & 3]);
+    }
+    return (s[0] + s[1]) + (s[2] + s[3]);
+  };
+  auto far_cols = [&](int p) MAFEM_INLINE {
+    const Run r = run_of(p);
+    const int j0 = ps[p], w = ps[p + 1] - j0;
+    const float* a = at(j0 + min(lane, w - 1), r.first);
+    float s = 0.0f;
+#pragma unroll 8
+    for (int m = 32 * RPT; m < r.len; ++m) s = fmaf(__ldcg(a + (int64_t)m * ldm), v[r.first + m], s);
+    return s;
+  };
+  for (int k = 0; k < kRing - 1; ++k) stage_bwd(npan - 1 - k);
+  load_cols(npan - 1, t[0], 0);
+  if constexpr (RPT == 1) load_cols(npan - 2, t[1], 0);
+  else load_cols(npan - 1, t[1], 1);
+  // step p: the sums of panel p's far columns while warp 0 solves panel p + 1
+  auto bwd_step = [&](int p, float (&x0)[32], float (&x1)[32]) MAFEM_INLINE {
+    float s = use_cols(p, x0, 0);
+    if constexpr (RPT == 2) s += use_cols(p, x1, 1) + far_cols(p);
+    S.part[p & 1][cw][lane] = s;
+    load_cols(p - NB, x0, 0);
+    if constexpr (RPT == 2) load_cols(p - NB, x1, 1);
+    cp_async_wait_group<kRing - 2>();  // ring slot p
+    solve_barrier();
+    stage_bwd(p - (kRing - 1));
+  };
+#pragma unroll 1
+  for (int p = npan - 1; p >= 0; p -= NB) {
+    bwd_step(p, t[0], t[1]);
+    if (NB == 2 && p - 1 >= 0) bwd_step(p - 1, t[1], t[0]);
+  }
+  solve_barrier();  // x of panel 0
+  cp_async_wait_group<0>();
 }
 
 // One column run [j0, j1) of a warp's double-float row sums (see patch_residual).
@@ -689,20 +873,21 @@ __device__ double patch_residual(const PatchJob& J, const float2* xs, double* re
   return sqrt(block_sum(ss, red));
 }
 
+template <int RPT>
 __global__ void __launch_bounds__(kRT, 1) patch_refine_kernel(const PatchJob* __restrict__ jobs,
                                                              const int* __restrict__ order, int max_sweeps,
                                                              double tol) {
   const PatchJob& J = jobs[order[blockIdx.x]];
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* v = reinterpret_cast<float*>(smem_raw);  // [n]
-  __shared__ float bz[32];  // zero beyond the panel width
-  __shared__ float part[kRT / 32][33];
-  __shared__ __align__(16) float inv_s[2 * 2 * kBlkW * kBlkW];  // double-buffered panel inverses
-  __shared__ double red[kRT / 32];
+  RefineSmem& S = *reinterpret_cast<RefineSmem*>(smem_raw);
+  float* v = reinterpret_cast<float*>(smem_raw + sizeof(RefineSmem));  // [n]
+  int* ps = reinterpret_cast<int*>(v + J.L.n);                         // [npan + 1]
+  double* red = S.red;
   const int tid = threadIdx.x;
   const int64_t n = J.L.n;
   int* stat = J.stat;  // [0] status, [1] sweeps
   float2* xs = J.xs;   // x split into two floats
+  for (int k = tid; k <= J.npan; k += kRT) ps[k] = J.ps[k];
   if (J.info[1] != 0 || J.info[0] != 0) {  // a bounded wait ran out, or a node block had no usable pivot
     if (tid == 0) {
       stat[0] = J.info[1] != 0 ? MAFEM_ERR_CUDA : MAFEM_ZERO_PIVOT;
@@ -738,7 +923,8 @@ __global__ void __launch_bounds__(kRT, 1) patch_refine_kernel(const PatchJob* __
       const double sc = 1.0 / rn;
       for (int64_t i = tid; i < n; i += kRT) v[i] = (float)(J.res[i] * sc);
       __syncthreads();
-      patch_lu_solve(J, v, bz, part, inv_s, tr && k == 0 ? tr + 4 * kTraceSweeps : nullptr);
+      long long* prof = tr && k == 0 ? tr + 4 * kTraceSweeps : nullptr;
+      patch_solve_pass<RPT>(J, v, ps, S, prof);
       stamp(trk, 1);
       double dd = 0.0, xx = 0.0;
       for (int64_t i = tid; i < n; i += kRT) {
@@ -796,7 +982,7 @@ __global__ void __launch_bounds__(kRT, 1) patch_refine_kernel(const PatchJob* __
 int patch_chunk_cols() { return kNCH; }
 
 // The split-A21 buffer as a 3-D tensor (k % 4, row, k / 4) of FP32 with strides
-// 16 bytes (rows) and 2 a21_rows x 16 bytes (k-quad planes); one 4 x 128 x 8 box
+// 16 bytes (rows) and 8 a21_rows x 16 bytes (k-quad planes); one 4 x 128 x 8 box
 // is one M tile in the MMA's K-major core-matrix layout (k-quad planes 2 KB
 // apart, rows 16 bytes apart).
 bool patch_a21_map(PatchJob& J) {
@@ -812,8 +998,9 @@ bool patch_a21_map(PatchJob& J) {
       return false;
     encode = reinterpret_cast<EncodeFn>(fn);
   }
-  const cuuint64_t dims[3] = {4, (cuuint64_t)2 * J.a21_rows, 8};
-  const cuuint64_t strides[2] = {16, (cuuint64_t)2 * J.a21_rows * 16};
+  const cuuint64_t rows = (cuuint64_t)4 * 2 * J.a21_rows;  // four ranks x (hi, lo)
+  const cuuint64_t dims[3] = {4, rows, 8};
+  const cuuint64_t strides[2] = {16, rows * 16};
   const cuuint32_t box[3] = {4, (cuuint32_t)kMT, 8};
   const cuuint32_t estr[3] = {1, 1, 1};
   return encode(&J.a21_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, J.a21, dims, strides, box, estr,
@@ -825,11 +1012,12 @@ int patch_solve_setup() {
   int dev = 0, cap = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
-  const int dyn = cap - 20 * 1024;  // room for the kernels' static shared memory (refine: ~19 KB)
+  const int dyn = cap - 2 * 1024;  // room for the kernels' static shared memory
   if (cudaFuncSetAttribute(patch_factor_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
       cudaFuncSetAttribute(patch_factor_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
       cudaFuncSetAttribute(patch_factor_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
-      cudaFuncSetAttribute(patch_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
+      cudaFuncSetAttribute(patch_refine_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
+      cudaFuncSetAttribute(patch_refine_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
     return 0;
   return dyn;
 }
@@ -859,14 +1047,24 @@ static cudaError_t launch_factor(const PatchJob* d_jobs, const int* d_order, int
                  : cudaLaunchKernelEx(&cfg, patch_factor_kernel<2>, d_jobs, d_order);
 }
 
+// Whether a band needs the refinement's two register sets per thread: more rows
+// or columns beyond a panel than one set of the update warps holds.
+bool patch_wide(int kl, int kuf) { return kl > kRowT || kuf > kRowT; }
+static cudaError_t launch_refine(const PatchJob* d_jobs, const int* d_order, int njobs, bool wide, size_t smem,
+                                 int max_sweeps, double tol, cudaStream_t st) {
+  if (wide) patch_refine_kernel<2><<<njobs, kRT, smem, st>>>(d_jobs, d_order, max_sweeps, tol);
+  else patch_refine_kernel<1><<<njobs, kRT, smem, st>>>(d_jobs, d_order, max_sweeps, tol);
+  return cudaGetLastError();
+}
+
 cudaError_t patch_solve_stage(const PatchJob* d_jobs, const int* d_order, int njobs, int nr, size_t smem_factor,
-                              size_t smem_refine, int max_sweeps, double tol, cudaStream_t st) {
+                              size_t smem_refine, bool wide, int max_sweeps, double tol, cudaStream_t st) {
   if (njobs <= 0) return cudaSuccess;
   if (smem_factor) {
     const cudaError_t e = launch_factor(d_jobs, d_order, njobs, nr, smem_factor, st);
     if (e != cudaSuccess) return e;
   }
-  if (smem_refine) patch_refine_kernel<<<njobs, kRT, smem_refine, st>>>(d_jobs, d_order, max_sweeps, tol);
+  if (smem_refine) return launch_refine(d_jobs, d_order, njobs, wide, smem_refine, max_sweeps, tol, st);
   return cudaGetLastError();
 }
 
@@ -912,14 +1110,14 @@ cudaError_t patch_time_factor(const PatchJob* d_jobs, const int* d_order1, int n
   return e;
 }
 
-int patch_solve_launches(int n4, int n2, int njobs) {
-  const int groups = (n4 > 0) + (n2 > 0) + (njobs - n4 - n2 > 0);
+int patch_solve_launches(const PatchGroups& G, int njobs) {
+  const int groups = (G.n4 > 0) + (G.n2 > 0) + (njobs - G.n4 - G.n2 > 0);
   return groups + (groups > 1 ? 2 : 1);  // the factor launches and one refinement per stream
 }
 
-cudaError_t patch_solve(const PatchJob* d_jobs, const int* d_order, int n4, int n2, int njobs, size_t smem_factor,
-                        size_t smem_refine, int max_sweeps, double tol, cudaStream_t st, cudaStream_t st2,
-                        cudaEvent_t ev_fork, cudaEvent_t ev_join) {
+cudaError_t patch_solve(const PatchJob* d_jobs, const int* d_order, const PatchGroups& G, int njobs,
+                        size_t smem_factor, size_t smem_refine, int max_sweeps, double tol, cudaStream_t st,
+                        cudaStream_t st2, cudaEvent_t ev_fork, cudaEvent_t ev_join) {
   if (njobs <= 0) return cudaSuccess;
   cudaError_t e = cudaSuccess;
   // the groups in launch order: four-CTA clusters, two-CTA clusters, single
@@ -927,7 +1125,7 @@ cudaError_t patch_solve(const PatchJob* d_jobs, const int* d_order, int n4, int 
   // st2 beside it (their chains are the shorter ones).  Each stream refines its
   // own patches as soon as their factors are done, so the refinement of one
   // group overlaps the factorisations of the other.
-  const int cnt[3] = {n4, n2, njobs - n4 - n2}, nrs[3] = {4, 2, 1};
+  const int cnt[3] = {G.n4, G.n2, njobs - G.n4 - G.n2}, nrs[3] = {4, 2, 1};
   int first = 0;
   while (first < 3 && cnt[first] == 0) ++first;
   const bool fork = cnt[first] < njobs;
@@ -940,15 +1138,13 @@ cudaError_t patch_solve(const PatchJob* d_jobs, const int* d_order, int n4, int 
     if (cnt[g] == 0) continue;
     e = launch_factor(d_jobs, d_order + off, cnt[g], nrs[g], smem_factor, g == first ? st : st2);
     off += cnt[g];
-    if (g == first && e == cudaSuccess) {
-      patch_refine_kernel<<<cnt[g], kRT, smem_refine, st>>>(d_jobs, d_order, max_sweeps, tol);
-      e = cudaGetLastError();
-    }
+    if (g == first && e == cudaSuccess)
+      e = launch_refine(d_jobs, d_order, cnt[g], G.wide[g], smem_refine, max_sweeps, tol, st);
   }
   if (fork && e == cudaSuccess) {
-    patch_refine_kernel<<<njobs - cnt[first], kRT, smem_refine, st2>>>(d_jobs, d_order + cnt[first], max_sweeps,
-                                                                        tol);
-    e = cudaGetLastError();
+    bool wide = false;
+    for (int g = first + 1; g < 3; ++g) wide |= cnt[g] > 0 && G.wide[g];
+    e = launch_refine(d_jobs, d_order + cnt[first], njobs - cnt[first], wide, smem_refine, max_sweeps, tol, st2);
   }
   if (fork && e == cudaSuccess) e = cudaEventRecord(ev_join, st2);
   if (fork && e == cudaSuccess) e = cudaStreamWaitEvent(st, ev_join, 0);

@@ -1171,8 +1171,8 @@ struct OutRows {  // adds a point's rows into R[row]
   __device__ __forceinline__ void l(const Dual<double, Nil>& x) { addn(pp.dof_of[6], x.v); }
 };
 // Elements per CTA: 63 threads, so that a patch of 32 x 32 elements spreads over
-// 147 SMs (an FP64 instruction holds its sub-partition for 64 cycles, so the
-// kernel's time is its longest warp chain): 98 -> MEASRES us against 16 per CTA.
+// 147 SMs: an FP64 instruction holds its sub-partition for 64 cycles, so the
+// kernel's time is its longest warp chain (98 us with 16 per CTA on 64 SMs).
 constexpr int kResEPB = 7;
 template <int MOTION>
 __device__ __forceinline__ void resid_body(const DevPatch& Pt, const PhysParams& pp, double time, double dt,

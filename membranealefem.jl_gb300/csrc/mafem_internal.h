@@ -320,11 +320,9 @@ struct PatchJob {
   CUtensorMap a21_map;  // TMA view of a21: 3-D (k % 4, row, k / 4), box 4 x 128 x 8
   float* band;          // factored in place
   const float* band0;   // the unfactored band (refinement residual)
-  float* inv;           // [npan][2][32][32]: L11^-1, U11^-1 per panel, column-major
+  float* inv;           // [npan][32][32]: the inverse of each panel's diagonal block, column-major
   const int* ps;        // panel starts [npan + 1]
   const int* blk_end;   // [n]
-  int* perm;            // [npan][32]
-  float* rdiag;         // [n]
   int* info;            // [0] zero-pivot column, [2] status, [3] sweeps
   int* stat;            // = info + 2
   const double* rhs;    // [n]
@@ -334,7 +332,7 @@ struct PatchJob {
   BandLayout L;
   int kuf, npan;
   long long* trace;     // optional: 6 globaltimer stamps per panel (patch_factor_kernel)
-  float* a21;           // split A21 of the current panel: [8][2 a21_rows][4] floats (TF32 hi rows, then lo rows)
+  float* a21;           // split A21 of the current panel: [8][4 ranks][2 a21_rows][4] floats (TF32 hi rows, then lo rows)
   int a21_rows;         // rows per part, a multiple of 128 (patch_a21_rows)
   // the tangent's sparsity for the refinement residual: unknowns couple only
   // within 5 x 5 control points (biquadratic elements); null: walk the whole band
@@ -347,8 +345,8 @@ int patch_a21_rows(int kl);
 // Encodes J.a21_map over J.a21 (J.a21, J.a21_rows set); returns false if the
 // driver refuses the tensor map.
 bool patch_a21_map(PatchJob& J);
-size_t patch_factor_smem(int kl);
-size_t patch_refine_smem(int64_t n);
+size_t patch_factor_smem();
+size_t patch_refine_smem(int64_t n, int npan);
 // Sets the kernels' shared-memory limits; returns the dynamic bytes available (0: unusable).
 int patch_solve_setup();
 // Trailing columns per chunk of the factorisation (at most).
@@ -359,22 +357,31 @@ int patch_cluster_ctas(int kuf);
 // The factor kernel alone (smem_refine == 0; nr = CTAs per patch, 1, 2 or 4) or
 // the refine kernel alone (smem_factor == 0).
 cudaError_t patch_solve_stage(const PatchJob* d_jobs, const int* d_order, int njobs, int nr, size_t smem_factor,
-                              size_t smem_refine, int max_sweeps, double tol, cudaStream_t st);
+                              size_t smem_refine, bool wide, int max_sweeps, double tol, cudaStream_t st);
 // Time (ms, CUDA events) of factoring job d_order1[0] on a cluster of nr CTAs,
 // on a synthetic band of its shape written over the job's band (which the
 // next assembly rewrites); synchronises st.
 cudaError_t patch_time_factor(const PatchJob* d_jobs, const int* d_order1, int nr, size_t smem, cudaStream_t st,
                               float* ms);
+// Whether a patch's band is wide for the refinement kernel (two register sets per thread).
+bool patch_wide(int kl, int kuf);
+// The jobs of a round by cluster size: the first n4 on four CTAs, the next n2 on
+// two; wide[g]: group g (4, 2, 1 CTAs) holds a wide band.
+struct PatchGroups {
+  int n4 = 0, n2 = 0;
+  bool wide[3] = {false, false, false};
+  int64_t key() const { return n4 | ((int64_t)n2 << 24) | ((int64_t)wide[0] << 48) | ((int64_t)wide[1] << 49) | ((int64_t)wide[2] << 50); }
+};
 // kernel launches patch_solve makes for these group sizes
-int patch_solve_launches(int n4, int n2, int njobs);
-// Factor and solve the jobs d_order[0 .. njobs): the first n4 on four-CTA
-// clusters, the next n2 on two-CTA clusters, the rest one CTA each -- the first
+int patch_solve_launches(const PatchGroups& G, int njobs);
+// Factor and solve the jobs d_order[0 .. njobs): the first G.n4 on four-CTA
+// clusters, the next G.n2 on two-CTA clusters, the rest one CTA each -- the first
 // non-empty group on st, the others after one another on st2 (forked from and
 // joined to st with ev_fork / ev_join); each stream refines its own jobs after
 // their factorisations.
-cudaError_t patch_solve(const PatchJob* d_jobs, const int* d_order, int n4, int n2, int njobs, size_t smem_factor,
-                        size_t smem_refine, int max_sweeps, double tol, cudaStream_t st, cudaStream_t st2,
-                        cudaEvent_t ev_fork, cudaEvent_t ev_join);
+cudaError_t patch_solve(const PatchJob* d_jobs, const int* d_order, const PatchGroups& G, int njobs,
+                        size_t smem_factor, size_t smem_refine, int max_sweeps, double tol, cudaStream_t st,
+                        cudaStream_t st2, cudaEvent_t ev_fork, cudaEvent_t ev_join);
 }  // namespace mafem
 
 #include <condition_variable>
