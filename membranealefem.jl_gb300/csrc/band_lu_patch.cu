@@ -31,8 +31,12 @@
 
 namespace mafem {
 
+// lambdas with register arrays: always inlined, so that the arrays stay in registers
+#define MAFEM_INLINE __attribute__((always_inline))
+
 constexpr int kPT = 512;   // threads per CTA of the factorisation (16 warps)
 constexpr int kRT = 512;   // threads per CTA of the refinement (16 warps)
+constexpr int kEpi = 1;    // batches of 16 columns of A22 whose loads run ahead of the subtraction (2: +3 %, 3: +10 % time)
 constexpr int kNCH = 256;  // trailing columns per chunk at most (the MMA's N <= 256)
 constexpr int kMT = 128;   // rows of A22 per tensor-core tile (the MMA's M)
 constexpr int kIS = 36;    // shared-memory row stride of the 32 x 32 inverse (16-byte rows)
@@ -107,58 +111,54 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 
 // Inverse of the w x w block (row `lane` in S, zero beyond w) by one warp: a
 // Gauss-Jordan sweep in place.  Step k exchanges column k for the pivot row p_k,
-// picked by size among the rows of k's node block (they end at row bend of
-// position k) not yet used; rows are never moved.  Afterwards S of row p_k holds
-// row k of the inverse, its entry k' standing for the block's row p_k', and the
-// inverse goes to Ai[row][column] (stride kIS) and, transposed, to inv.  The
-// columns rotate through the registers, so that the pivot column is always S[0]
-// and the step is one small loop body (unrolled over k it is 70 KB of code,
-// which one warp fetches at 0.5 us a step).  The pivot row travels through shared
-// memory: one lane's 16-byte stores, then broadcast reads.
+// picked by size (to 17 bits) among the rows of k's node block -- they end at row
+// bend of position k -- not yet used; rows are never moved.  A row's scaling by
+// -1/pivot at its own step is kept apart (sc), since the later steps' multipliers
+// -S[k]/pivot do not see it: the step is 31 shuffles and 31 FMAs for every row
+// alike.  Afterwards sc S of row p_k is row k of the inverse, its entry k'
+// standing for the block's row p_k', and goes to Ai[row][column] (stride kIS)
+// and, transposed, to inv.  The columns rotate through the registers, so that the
+// pivot column is always S[0] and the step is one small loop body (unrolled over
+// k it is 70 KB of code, which one warp fetches at 0.5 us a step): 6.4 us for a
+// panel of 32 with the block's load, against 10.5 us for an eight-warp LU.
 // Returns the first step (1-based) that found no usable pivot, 0 if none.
-__device__ __forceinline__ int warp_inverse(float (&S)[32], int w, int bend, float* srow, int* sp, float* Ai,
-                                            float* inv) {
+__device__ __forceinline__ int warp_inverse(float (&S)[32], int w, int bend, int* sp, float* Ai, float* inv) {
   const int lane = threadIdx.x & 31;
-  unsigned used = 0u;
+  unsigned mine = lane < w ? 1u : 0u;  // this row can still be a pivot
   int pos = lane, bad = 0;
+  float sc = 1.0f;
   if (lane >= w) sp[lane] = lane;
+  int bk = __shfl_sync(kFull, bend, 0);
 #pragma unroll 1
   for (int k = 0; k < w; ++k) {
-    const int bk = __shfl_sync(kFull, bend, k);
-    const bool cand = lane < bk && !((used >> lane) & 1u);
-    const unsigned key = cand ? pkey(S[0]) : 0u;
-    const unsigned mx = __reduce_max_sync(kFull, key);
-    const int p = __ffs(__ballot_sync(kFull, cand && key == mx)) - 1;  // the candidates are never empty
-    if (mx == 0u && bad == 0) bad = k + 1;
+    const unsigned key = (mine && lane < bk) ? ((pkey(S[0]) & ~63u) | (63u - lane)) : 0u;
+    bk = __shfl_sync(kFull, bend, (k + 1) & 31);
+    const unsigned mx = __reduce_max_sync(kFull, key);  // the candidates are never empty
+    const int p = 63 - (int)(mx & 63u);
+    if (mx < 64u && bad == 0) bad = k + 1;
+    const float d = __shfl_sync(kFull, S[0], p);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = fmaf(r, fmaf(-d, r, 1.0f), r);  // one Newton step on the hardware's approximation
     const bool own = lane == p;
+    const float m = own ? 0.0f : -(S[0] * r);
     if (own) {
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        reinterpret_cast<float4*>(srow)[c] = make_float4(S[4 * c], S[4 * c + 1], S[4 * c + 2], S[4 * c + 3]);
       pos = k;
+      sc = -r;
+      mine = 0u;
       sp[k] = p;
     }
-    used |= 1u << p;
-    const float r = __frcp_rn(__shfl_sync(kFull, S[0], p));
-    const float f = S[0];
-    const float fr = f * r, m = own ? -r : -fr;
-    __syncwarp();
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const float4 u = reinterpret_cast<const float4*>(srow)[c];
-      if (c) S[4 * c - 1] = fmaf(m, u.x, own ? 0.0f : S[4 * c]);
-      S[4 * c] = fmaf(m, u.y, own ? 0.0f : S[4 * c + 1]);
-      S[4 * c + 1] = fmaf(m, u.z, own ? 0.0f : S[4 * c + 2]);
-      S[4 * c + 2] = fmaf(m, u.w, own ? 0.0f : S[4 * c + 3]);
-    }
-    S[31] = own ? r : fr;
-    __syncwarp();  // the row buffer is free for the next step
+    for (int c = 1; c < 32; ++c) S[c - 1] = fmaf(m, __shfl_sync(kFull, S[c], p), S[c]);
+    S[31] = own ? -1.0f : -m;
   }
+  __syncwarp();
 #pragma unroll
   for (int c = 0; c < 32; ++c) {  // S[c] holds column (c + w) mod 32
     const int col = sp[(c + w) & 31];
-    Ai[pos * kIS + col] = S[c];
-    if (inv) inv[col * kBlkW + pos] = S[c];
+    const float v = sc * S[c];
+    Ai[pos * kIS + col] = v;
+    if (inv) inv[col * kBlkW + pos] = v;
   }
   return bad;
 }
@@ -193,8 +193,8 @@ __device__ __forceinline__ int warp_inverse(float (&S)[32], int w, int bend, flo
 // Measured on a GB300 against an LU with staged panels and per-rank hand-overs
 // (three small triangular products per panel, 64-bit indexing in every access; it
 // was bound by its instructions, 316 k per panel of 24 x 24 ALEVB): 16 x 16 ALEVB
-// on four CTAs 3.3 -> 1.4 ms, 24 x 24 on one 12.5 -> 8.1 ms, 32 x 32 on one 31.4
-// -> 20.9 ms, 48 x 48 on four 50.6 -> 28.5 ms.
+// on four CTAs 3.3 -> 1.15 ms, 24 x 24 on one 12.5 -> 7.5 ms, 32 x 32 on one 31.4
+// -> 20.3 ms, 48 x 48 on four 50.6 -> 27.0 ms.
 template <int NR>
 __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __restrict__ jobs,
                                                              const int* __restrict__ order) {
@@ -208,7 +208,6 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
   unsigned char* Abuf = smem_fac + 2 * kYBytes;                       // [2][A21h tile | A21l tile]
   float* Ai = reinterpret_cast<float*>(smem_fac + kChunkBytes);       // [32][kIS]
   float* sA = Ai + kBlkW * kIS;                                       // [16 warps][4][32]: four columns of A12
-  __shared__ __align__(16) float srow[32];
   __shared__ int sp[32];
   __shared__ __align__(8) uint64_t bar_tma[2], bar_mma[2];
   __shared__ uint32_t s_tmem;
@@ -276,7 +275,7 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
       for (int c = 0; c < 32; ++c) S[c] = (lane < w && c < w) ? __ldcg(src + (int64_t)c * ldm) : 0.0f;
       const int bend = lane < w ? (int)(J.blk_end[j0 + lane] - j0) : 0;
       const int bad =
-          warp_inverse(S, w, bend, srow, sp, Ai, rank == 0 ? J.inv + (size_t)p * kBlkW * kBlkW : nullptr);
+          warp_inverse(S, w, bend, sp, Ai, rank == 0 ? J.inv + (size_t)p * kBlkW * kBlkW : nullptr);
       if (rank == 0 && lane == 0 && bad) atomicCAS(J.info, 0, (int)(j0 + bad));
       load_a12(rank * nch);
     } else {
@@ -395,25 +394,33 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
       const int q = warp & 3, grp = warp >> 2;
       const int cpg = ((ncp >> 2) + 7) & ~7;
       const int cs = min(ncp, grp * cpg), ce = min(ncp, cs + cpg), lim = min(ce, nc);
-      float vn[16];  // A22 of the next step
-      auto load_a22 = [&](int t, int c0) {
-        const float* pa = ab + bix(L, j0 + min(w + t * kMT + 32 * q + lane, R - 1), j1 + cb + c0);
-        if (c0 + 16 <= lim) {
+      // the steps of this warp: tile t, columns c .. c + 15 of its group; each
+      // buffer's loads are issued kEpi steps before their use
+      auto next = [&](int& t, int& c) MAFEM_INLINE {
+        c += 16;
+        if (c >= lim) {
+          c = cs;
+          ++t;
+        }
+      };
+      auto load_a22 = [&](float (&v)[16], int t, int c) MAFEM_INLINE {
+        if (t >= ntile) return;  // warp-uniform
+        const float* pa = ab + bix(L, j0 + min(w + t * kMT + 32 * q + lane, R - 1), j1 + cb + c);
+        if (c + 16 <= lim) {
 #pragma unroll
           for (int k = 0; k < 16; ++k) {
-            vn[k] = __ldcg(pa);
+            v[k] = __ldcg(pa);
             pa += ldm;
           }
         } else {
 #pragma unroll
           for (int k = 0; k < 16; ++k) {
-            vn[k] = c0 + k < lim ? __ldcg(pa) : 0.0f;
+            v[k] = c + k < lim ? __ldcg(pa) : 0.0f;
             pa += ldm;
           }
         }
       };
-      if (ntile > 0 && cs < lim) load_a22(0, cs);
-      for (int t = 0; t < ntile; ++t) {
+      auto tile_begin = [&](int t) MAFEM_INLINE {
         const int b = t & 1;
         mbar_wait_bounded(&bar_mma[b], ph_mma[b], err);  // tile t's products are in Tensor Memory
         if (tid == 0) {
@@ -421,35 +428,58 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
           if (t + 1 < ntile) mma_tile(t + 1);  // into the other accumulator, read back at t - 1
         }
         tc::fence_after();
-        const int row = w + t * kMT + 32 * q + lane;  // panel row of this thread
-        const bool live = row < R;
-        float* pa = ab + bix(L, j0 + (live ? row : 0), j1 + cb + cs);
-        const uint32_t dt = tmem + ((uint32_t)(32 * q) << 16) + b * kNCH;
-        for (int c0 = cs; c0 < lim; c0 += 16) {
-          float d0[8], d1[8], v[16];
-          tc::ld8(dt + c0, d0);
-          if (c0 + 8 < ce) tc::ld8(dt + c0 + 8, d1);
+      };
+      auto tile_end = [&]() MAFEM_INLINE {
+        tc::fence_before();
+        __syncthreads();  // the accumulator is read before the MMAs of tile t + 2 overwrite it
+      };
+      if (cs < lim) {
+        float va[kEpi][16];
+        int t = 0, c = cs, tl = 0, cl = cs;  // the step at hand, the next to load
 #pragma unroll
-          for (int k = 0; k < 16; ++k) v[k] = vn[k];
-          if (c0 + 16 < lim) load_a22(t, c0 + 16);
-          else if (t + 1 < ntile) load_a22(t + 1, cs);
-          tc::wait_ld();
-          if (live) {
-            if (c0 + 16 <= lim) {
+        for (int u = 0; u < kEpi; ++u) {
+          load_a22(va[u], tl, cl);
+          next(tl, cl);
+        }
+        while (t < ntile) {
 #pragma unroll
-              for (int k = 0; k < 16; ++k) {
-                *pa = v[k] - (k < 8 ? d0[k] : d1[k - 8]);
-                pa += ldm;
+          for (int u = 0; u < kEpi; ++u) {
+            if (t < ntile) {  // warp-uniform
+              if (c == cs) tile_begin(t);
+              const int row = w + t * kMT + 32 * q + lane;  // panel row of this thread
+              const uint32_t dt = tmem + ((uint32_t)(32 * q) << 16) + (t & 1) * kNCH;
+              float d0[8], d1[8];
+              tc::ld8(dt + c, d0);
+              if (c + 8 < ce) tc::ld8(dt + c + 8, d1);
+              tc::wait_ld();
+              if (row < R) {
+                float* pa = ab + bix(L, j0 + row, j1 + cb + c);  // A(j0 + row, j1 + cb + c), + ldm: the next column
+                if (c + 16 <= lim) {
+#pragma unroll
+                  for (int k = 0; k < 16; ++k) {
+                    *pa = va[u][k] - (k < 8 ? d0[k] : d1[k - 8]);
+                    pa += ldm;
+                  }
+                } else {
+#pragma unroll
+                  for (int k = 0; k < 16; ++k) {
+                    if (c + k < lim) *pa = va[u][k] - (k < 8 ? d0[k] : d1[k - 8]);
+                    pa += ldm;
+                  }
+                }
               }
-            } else {
-#pragma unroll
-              for (int k = 0; k < 16; ++k)
-                if (c0 + k < lim) pa[k * ldm] = v[k] - (k < 8 ? d0[k] : d1[k - 8]);
+              load_a22(va[u], tl, cl);
+              next(tl, cl);
+              if (c + 16 >= lim) tile_end();
+              next(t, c);
             }
           }
         }
-        tc::fence_before();
-        __syncthreads();  // accumulator b is read before the MMAs of tile t + 2 overwrite it
+      } else {  // no columns for this warp: the tiles' barriers only
+        for (int t = 0; t < ntile; ++t) {
+          tile_begin(t);
+          tile_end();
+        }
       }
       if (first) stamp(tr, 4);
       first = false;
@@ -547,8 +577,6 @@ __device__ __forceinline__ float dot32(const float (&x)[32], const float* z) {
   }
   return (s0.x + s0.y) + (s1.x + s1.y);
 }
-// lambdas with register arrays: always inlined, so that the arrays stay in registers
-#define MAFEM_INLINE __attribute__((always_inline))
 template <int RPT>
 __device__ __forceinline__ void patch_solve_pass(const PatchJob& J, float* v, const int* ps, RefineSmem& S,
                                                  long long* prof) {
@@ -768,35 +796,28 @@ __device__ __forceinline__ void patch_solve_pass(const PatchJob& J, float* v, co
 // One column run [j0, j1) of a warp's double-float row sums (see patch_residual).
 __device__ __forceinline__ void residual_run(const float* a, int64_t ldm, const float2* xs, int64_t j0, int64_t j1,
                                              float& sh, float& sl) {
-  int64_t j = j0;
-  for (; j + 8 <= j1; j += 8) {
-    float av[8];
-    float2 xv[8];
+  constexpr int kB = 16;  // columns whose loads are in flight together
+  for (int64_t j = j0; j < j1; j += kB) {
+    const int cnt = (int)min64b(kB, j1 - j);  // warp-uniform
+    float av[kB];
+    const float* p = a + j * ldm;
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {  // all loads in flight
-      av[m] = a[(j + m) * ldm];
-      xv[m] = xs[j + m];
+    for (int m = 0; m < kB; ++m) {
+      av[m] = m < cnt ? p[0] : 0.0f;
+      p += ldm;
     }
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
+    for (int m = 0; m < kB; ++m) {
+      if (m >= cnt) break;
+      const float2 xv = xs[j + m];
       // explicit roundings: a contraction of p into t would break TwoSum
-      const float p = __fmul_rn(av[m], xv[m].x);
-      const float e = fmaf(av[m], xv[m].y, fmaf(av[m], xv[m].x, -p));
+      const float p = __fmul_rn(av[m], xv.x);
+      const float e = fmaf(av[m], xv.y, fmaf(av[m], xv.x, -p));
       const float t = __fadd_rn(sh, p);
       const float z = __fsub_rn(t, sh);
       sl = __fadd_rn(sl, __fadd_rn(__fadd_rn(__fsub_rn(sh, __fsub_rn(t, z)), __fsub_rn(p, z)), e));
       sh = t;
     }
-  }
-  for (; j < j1; ++j) {
-    const float av = a[j * ldm];
-    const float2 xv = xs[j];
-    const float p = __fmul_rn(av, xv.x);
-    const float e = fmaf(av, xv.y, fmaf(av, xv.x, -p));
-    const float t = __fadd_rn(sh, p);
-    const float z = __fsub_rn(t, sh);
-    sl = __fadd_rn(sl, __fadd_rn(__fadd_rn(__fsub_rn(sh, __fsub_rn(t, z)), __fsub_rn(p, z)), e));
-    sh = t;
   }
 }
 
