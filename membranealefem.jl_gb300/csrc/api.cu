@@ -103,6 +103,7 @@ struct mafem_handle {
   // (band_lu.cu) is the fallback for a block without a usable pivot
   bool use_blk = false;
   bool last_blk = false;  // which factorisation the band currently holds
+  bool pinv_ready = false;  // d_pinv holds the inverses of its panels' triangles
   BlkPlan blk;
   int* d_blk_end = nullptr;
   int* d_flags = nullptr;  // per-panel completion flags of the cooperative back substitution
@@ -127,7 +128,7 @@ struct mafem_handle {
   // batched FP32 form (band_lu_patch.cu): the handle's job, usable when its band fits
   float* d_inv = nullptr;
   double* d_zbuf = nullptr;  // npan x 32: z = U11^-1 y1 per panel (cooperative forward substitution)
-  double* d_pinv = nullptr;  // npan x 2 x 32 x 32: L11^-1, U11^-1 per panel (cooperative substitutions)
+  double* d_pinv = nullptr;  // npan x 2 x 32 x 32: L11^-1, U11^-1 per panel (cooperative forward substitution)
   bool patch_ok = false;
   bool ss_patch = false;  // the iteration in progress ran through a batch's patch solve
   PatchJob job{};
@@ -745,10 +746,12 @@ static int assemble(mafem_handle* h, double time, double dt, bool both_bands = f
 // the fallback.
 // Launch the node-block factorisation (persistent kernel, or per-panel launches)
 // without waiting for it; `info` tells later whether a block had no usable pivot.
-// The panels' triangle inverses for the cooperative substitutions, stream-ordered
-// after a node-block factorisation.
-static void blk_after_factor(mafem_handle* h) {
-  if (!h->d_pinv) return;
+// The panels' triangle inverses for the cooperative forward substitution, formed
+// when a factorisation is first solved with again (a time step's right-hand side
+// rides along its factorisation and needs none; the kernel takes 50 us).
+static void blk_need_inverses(mafem_handle* h) {
+  if (h->pinv_ready) return;
+  h->pinv_ready = true;
   if (h->precision == MAFEM_PLAIN_FP64)
     blk_inverses<double, double>((const double*)h->d_band, h->L, h->blk, (const double*)h->d_rdiag, h->d_pinv, h->st);
   else
@@ -781,7 +784,7 @@ static int factor_enqueue(mafem_handle* h, double* x) {
                                                h->d_info, nullptr, h->st, h->st2, h->ev_pool.data(), nullptr);
     h->launches += nl;
   }
-  blk_after_factor(h);
+  h->pinv_ready = false;
   CK(cudaGetLastError());
   h->factored = true;
   h->last_blk = true;
@@ -858,15 +861,15 @@ template <class T>
 static void blk_back_solve(mafem_handle* h, double* y, const int* gate = nullptr) {
   if (h->bwd_grid > 0) {
     ++h->epoch;
-    if (blk_backward<double, T>((const T*)h->d_band, h->L, h->blk, h->d_pinv, y, h->d_flags, h->epoch,
-                                h->d_info + 1, h->bwd_grid, h->st, h->wait_test, gate) == 0) {
+    if (blk_backward<double, T>((const T*)h->d_band, h->L, h->blk, y, h->d_flags, h->epoch, h->d_info + 1,
+                                h->bwd_grid, h->st, h->wait_test, gate) == 0) {
       h->launches += 1;
       return;
     }
     cudaGetLastError();
     h->bwd_grid = 0;  // cooperative launch refused: use the single-CTA kernel from now on
   }
-  blk_backward_1cta<double, T>((const T*)h->d_band, h->L, h->blk, (const T*)h->d_rdiag, y, h->st);
+  blk_backward_1cta<double, T>((const T*)h->d_band, h->L, h->blk, y, h->st);
   h->launches += 1;
 }
 
@@ -875,6 +878,7 @@ static void blk_back_solve(mafem_handle* h, double* y, const int* gate = nullptr
 template <class T>
 static void blk_fwd_solve(mafem_handle* h, double* y, const int* gate = nullptr) {
   if (h->bwd_grid > 0) {
+    blk_need_inverses(h);
     ++h->epoch;
     if (blk_forward_coop<double, T>((const T*)h->d_band, h->L, h->blk, h->d_perm, h->d_pinv, y, h->d_zbuf,
                                     h->d_flags, h->epoch, h->d_info + 1, h->bwd_grid, h->st, h->wait_test,
@@ -2588,7 +2592,7 @@ extern "C" int mafem_trace_factor(mafem_handle* h, double time, double dt, int64
                       : blk_lu_factor_persist<float>((float*)h->d_band, h->L, h->blk, h->pers, h->fepoch, h->d_perm,
                                                      (float*)h->d_rdiag, h->d_info, nullptr, h->d_info + 1, h->st,
                                                      d_tr);
-  blk_after_factor(h);
+  h->pinv_ready = false;
   h->factored = true;
   h->last_blk = true;
   CK(cudaMemcpyAsync(out, d_tr, sizeof(long long) * 12 * npan, cudaMemcpyDeviceToHost, h->st));
@@ -2941,7 +2945,7 @@ extern "C" int mafem_profile_factor(mafem_handle* h, double time, double dt, maf
     else
       blk_lu_factor<float>((float*)h->d_band, h->L, h->blk, h->d_perm, (float*)h->d_rdiag, h->d_info, nullptr, h->st,
                            nullptr, nullptr, ev.data());
-    blk_after_factor(h);
+    h->pinv_ready = false;
   } else if (fp64) {
     h->band_dirty = true;
     band_lu_factor<double>((double*)h->d_band, h->L, h->d_ipiv, h->d_perm, h->rmax, h->d_info, h->d_x,

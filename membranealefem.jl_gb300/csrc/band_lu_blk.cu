@@ -13,13 +13,17 @@
 //   * the pivot search is one warp reduction over <= 8 rows;
 //   * rows below a panel never take part in its pivot steps, so their
 //     multipliers L21 = A21 U11^-1 are never formed: the trailing update and
-//     the forward substitution apply L21 u = A21 (U11^-1 u) with the raw A21.
+//     the forward substitution apply L21 u = A21 (U11^-1 u) with the raw A21;
+//   * the solved columns Y = A11^-1 A12 are kept in place of U12 = U11 Y: the
+//     forward substitution then leaves z = A11^-1 b1, the back substitution is
+//     x1 = z - Y x2, and no triangle is solved on its chain of panels.
 // A zero or non-finite pivot sets `info`; the caller then falls back to the
 // full partial-pivoting factorisation (band_lu.cu).
 //
 // After panel p (columns [j0, j1), w = j1 - j0 <= 32) the band holds, in the
 // panel's columns, L11 (unit, strict lower) and U11 in rows [j0, j1) and the
-// untouched A21 in rows [j1, j0 + R), R = w + kl; rdiag[j] = 1 / U(j, j);
+// untouched A21 in rows [j1, j0 + R), R = w + kl, and Y in rows [j0, j1) of the
+// columns right of it; rdiag[j] = 1 / U(j, j);
 // perm_all[p * kBlkW + i] = the panel row moved to position i.
 
 #include <cuda_runtime.h>
@@ -49,7 +53,7 @@ __global__ void __launch_bounds__(32 * kPanelWarps) blk_panel_kernel(T* __restri
 // of warps (warps q and q + 4 share a sub-partition's FP64 pipe, so one warp's
 // issue stalls overlap the other's work).  Per column segment
 // s = A(j0 .. j0+R-1, c), rows [0, w) permuted:
-//   u = L11^-1 s[0:w]   (kept as U12),   y = U11^-1 u,   s[w:R] -= A21 y.
+//   u = L11^-1 s[0:w],   y = U11^-1 u   (kept as Y),   s[w:R] -= A21 y.
 // Warp q stages the column and runs the two triangular solves, then releases
 // warp q + 4 (named barrier 1 + q); the two split the 32-row chunks of the
 // A21 y update (NCH chunks each per pass).  Before warp q overwrites the
@@ -97,7 +101,6 @@ __global__ void __launch_bounds__(256) blk_apply_kernel(T* __restrict__ ab, Band
         const T xk = __shfl_sync(kFull, x, k);
         if (lane > k && lane < w) x -= Lp[k * R + lane] * xk;
       }
-      if (lane < w) dst[lane] = x;  // U12
       T v = x;
       for (int k = w - 1; k >= 0; --k) {
         T yk = lane == k ? v * rd[k] : T(0);
@@ -105,6 +108,7 @@ __global__ void __launch_bounds__(256) blk_apply_kernel(T* __restrict__ ab, Band
         if (lane == k) v = yk;
         if (lane < k) v -= Lp[k * R + lane] * yk;
       }
+      if (lane < w) dst[lane] = v;  // Y
       yw[lane] = v;
       bar_arrive_n(1 + slot, 64);
     } else {
@@ -161,7 +165,6 @@ __global__ void __launch_bounds__(128) blk_apply_col_kernel(T* __restrict__ ab, 
       const T xk = __shfl_sync(kFull, x, k);
       if (lane > k && lane < w) x -= T11[k][lane] * xk;
     }
-    if (lane < w) s[lane] = x;
     T v = x;
     for (int k = w - 1; k >= 0; --k) {
       T yk = lane == k ? v * rd[k] : T(0);
@@ -169,6 +172,7 @@ __global__ void __launch_bounds__(128) blk_apply_col_kernel(T* __restrict__ ab, 
       if (lane == k) v = yk;
       if (lane < k) v -= T11[k][lane] * yk;
     }
+    if (lane < w) s[lane] = v;
     y[lane] = lane < w ? v : T(0);
   }
   __syncthreads();
@@ -241,7 +245,6 @@ __global__ void __launch_bounds__(1024) blk_forward_kernel(const T* __restrict__
         const V xk = __shfl_sync(kFull, x, k);
         if (tid > k && tid < w) x -= Ls[k][tid] * xk;
       }
-      if (tid < w) s[tid] = x;
       V v = x;
       for (int k = w - 1; k >= 0; --k) {
         V yk = tid == k ? v * rd[k] : V(0);
@@ -249,6 +252,7 @@ __global__ void __launch_bounds__(1024) blk_forward_kernel(const T* __restrict__
         if (tid == k) v = yk;
         if (tid < k) v -= Ls[k][tid] * yk;
       }
+      if (tid < w) s[tid] = v;
       y[tid] = tid < w ? v : V(0);
     }
     __syncthreads();
@@ -265,25 +269,18 @@ __global__ void __launch_bounds__(1024) blk_forward_kernel(const T* __restrict__
   }
 }
 
-// Back substitution U x = y, one CTA, panels in reverse; U has kuf
-// super-diagonals and its diagonal reciprocals are in rdiag.
+// Back substitution x1 = z - Y x2, one CTA, panels in reverse; Y has kuf
+// super-diagonals.
 template <class T, class V>
 __global__ void __launch_bounds__(1024) blk_backward_kernel(const T* __restrict__ ab, BandLayout L, int kuf,
-                                                            const int* __restrict__ ps, int npan,
-                                                            const T* __restrict__ rdiag, V* __restrict__ y) {
+                                                            const int* __restrict__ ps, int npan, V* __restrict__ y) {
   __shared__ V part[32][33];
-  __shared__ V Us[32][33];
-  __shared__ V xs[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   for (int pnl = npan - 1; pnl >= 0; --pnl) {
     const int64_t j0 = ps[pnl];
     const int w = ps[pnl + 1] - ps[pnl];
     const int64_t j1 = j0 + w;
     const int64_t jend = min64b(L.n, j1 + kuf);
-    for (int k = tid; k < w * w; k += blockDim.x) {
-      const int c = k / w, i = k - c * w;
-      Us[c][i] = i < c ? V(ab[bix(L, j0 + i, j0 + c)]) : (i == c ? V(rdiag[j0 + c]) : V(0));
-    }
     V acc = V(0);
     if (lane < w) {
       int64_t c = j1 + warp;
@@ -304,24 +301,15 @@ __global__ void __launch_bounds__(1024) blk_backward_kernel(const T* __restrict_
     if (warp == 0) {
       V sum = V(0);
       for (int k = 0; k < nw; ++k) sum += part[k][lane];
-      V v = lane < w ? y[j0 + lane] - sum : V(0);
-      for (int k = w - 1; k >= 0; --k) {
-        V xk = lane == k ? v * Us[k][k] : V(0);  // Us[k][k] holds 1 / U(k, k)
-        xk = __shfl_sync(kFull, xk, k);
-        if (lane == k) v = xk;
-        if (lane < k) v -= Us[k][lane] * xk;
-      }
-      if (lane < w) xs[lane] = v;
+      if (lane < w) y[j0 + lane] -= sum;
     }
-    __syncthreads();
-    if (tid < w) y[j0 + tid] = xs[tid];
     __syncthreads();
   }
 }
 
 // ---------------------------------------------------------------------------
 // Explicit inverses of every panel's diagonal triangles for the cooperative
-// substitutions: Li = L11^-1 (unit lower) and Ui = U11^-1 (upper, 1 / U(k, k)
+// forward substitution: Li = L11^-1 (unit lower) and Ui = U11^-1 (upper, 1 / U(k, k)
 // from rdiag), 32 x 32 each with element (i, k) at k * 32 + i, zero outside
 // the panel's w x w block; inv[p] = Li then Ui.  One warp per panel (four per
 // CTA), lane c
@@ -372,9 +360,9 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
 
 // ---------------------------------------------------------------------------
 // Back substitution on many SMs: one cooperative launch, panel q handled by
-// CTA (npan - 1 - q) mod gridDim.x.  A CTA accumulates U(q rows, c) x(c) over
+// CTA (npan - 1 - q) mod gridDim.x.  A CTA accumulates Y(q rows, c) x(c) over
 // the columns of the panels above it as their flags appear (most are done
-// long before it needs them), then solves its U11 triangle and publishes
+// long before it needs them), subtracts the sum from z and publishes
 // x(q) with a release store of the flag.  Flags hold the epoch of the solve
 // that set them, so they never need clearing.  Waits are bounded: after
 // wt.limit polls (kSpinLimit by default) the kernel records MAFEM status in
@@ -384,12 +372,10 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
 // and every CTA returns.
 template <class T, class V>
 __global__ void __launch_bounds__(256) blk_backward_coop_kernel(const T* __restrict__ ab, BandLayout L, int kuf,
-                                                                const int* __restrict__ ps, int npan,
-                                                                const V* __restrict__ inv, V* y, int* flags,
+                                                                const int* __restrict__ ps, int npan, V* y, int* flags,
                                                                 int epoch, int* err, WaitTest wt,
                                                                 const int* gate) {
   __shared__ V part[8][33];
-  __shared__ V Uis[32 * 32];  // U11^-1 of the panel, element (i, k) at k * 32 + i
   __shared__ int s_ok;
   if (gate && *gate) return;  // every CTA reads the same word: all return (refinement already stopped)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -397,8 +383,6 @@ __global__ void __launch_bounds__(256) blk_backward_coop_kernel(const T* __restr
     const int64_t j0 = ps[q], j1 = ps[q + 1];
     const int w = (int)(j1 - j0);
     const int64_t jend = min64b(L.n, j1 + kuf);
-    const V* Ui = inv + (size_t)q * 2 * kBlkW * kBlkW + kBlkW * kBlkW;
-    for (int k = tid; k < kBlkW * kBlkW; k += 256) Uis[k] = __ldcg(Ui + k);
     int pl = q + 1;  // last panel with columns in [j1, jend)
     while (pl + 1 < npan && ps[pl + 1] < jend) ++pl;
     V acc = V(0);
@@ -413,12 +397,7 @@ __global__ void __launch_bounds__(256) blk_backward_coop_kernel(const T* __restr
     if (warp == 0) {
       const V sum = ((part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane])) +
                     ((part[4][lane] + part[5][lane]) + (part[6][lane] + part[7][lane]));  // tree: 3 dependent adds
-      // x1 = U11^-1 (y1 - U12 x2): one dot product per lane, the shuffles independent
-      const V v = lane < w ? __ldcg(y + j0 + lane) - sum : V(0);
-      V x = V(0);
-#pragma unroll
-      for (int k = 0; k < 32; ++k) x = fma(Uis[k * 32 + lane], __shfl_sync(kFull, v, k), x);
-      if (lane < w) __stcg(y + j0 + lane, x);
+      if (lane < w) __stcg(y + j0 + lane, __ldcg(y + j0 + lane) - sum);  // x1 = z - Y x2
       __threadfence();
       __syncwarp();
       if (lane == 0 && npan - 1 - q != wt.withhold) st_release(flags + q, epoch);
@@ -433,7 +412,7 @@ __global__ void __launch_bounds__(256) blk_backward_coop_kernel(const T* __restr
 // the contributions A21(q) z(q) of the earlier panels q whose rows reach them
 // (rows of panel q end at ps[q + 1] + kl), each as soon as q's flag appears,
 // then applies the panel's interchanges and triangles like blk_forward_kernel:
-// y1 = L11^-1 P b1 replaces b1 in place, z = U11^-1 y1 goes to zbuf[p] with a
+// z = U11^-1 L11^-1 P b1 replaces b1 in place and goes to zbuf[p] with a
 // release store of the flag.  A panel waits only for lower-numbered panels,
 // which CTAs take in increasing order, so the chain always progresses; waits
 // are bounded (kSpinLimit polls, then *err and every CTA returns).
@@ -483,7 +462,7 @@ __global__ void __launch_bounds__(256) blk_forward_coop_kernel(const T* __restri
 #pragma unroll
       for (int k = 0; k < 32; ++k) v = fma(Is[kBlkW * kBlkW + k * 32 + lane], __shfl_sync(kFull, y1, k), v);
       if (lane < w) {
-        __stcg(b + j0 + lane, y1);
+        __stcg(b + j0 + lane, v);
         __stcg(zbuf + (size_t)p * kBlkW + lane, v);
       }
       __threadfence();
@@ -638,21 +617,21 @@ void blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, const T* r
   blk_inverses_kernel<T, V><<<(B.npan() + 3) / 4, 128, 0, st>>>(ab, L, B.d_ps, B.npan(), rdiag, inv);
 }
 template <class V, class T>
-int blk_backward(const T* ab, const BandLayout& L, const BlkPlan& B, const V* inv, V* y, int* flags, int epoch,
-                 int* err, int grid, cudaStream_t st, WaitTest wt, const int* gate) {
+int blk_backward(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, int* flags, int epoch, int* err, int grid,
+                 cudaStream_t st, WaitTest wt, const int* gate) {
   const int npan = B.npan();
   int kuf = B.kuf;
   const int* ps = B.d_ps;
-  void* args[] = {(void*)&ab,    (void*)&L,     (void*)&kuf, (void*)&ps, (void*)&npan, (void*)&inv,
-                  (void*)&y,     (void*)&flags, (void*)&epoch, (void*)&err, (void*)&wt,  (void*)&gate};
+  void* args[] = {(void*)&ab,    (void*)&L,     (void*)&kuf, (void*)&ps, (void*)&npan, (void*)&y,
+                  (void*)&flags, (void*)&epoch, (void*)&err, (void*)&wt, (void*)&gate};
   const cudaError_t e = cudaLaunchCooperativeKernel((const void*)blk_backward_coop_kernel<T, V>,
                                                     dim3(std::min(grid, npan)), dim3(256), args, 0, st);
   return e == cudaSuccess ? 0 : -1;
 }
 // single-CTA back substitution (used when a cooperative launch is not possible)
 template <class V, class T>
-void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, const T* rdiag, V* y, cudaStream_t st) {
-  blk_backward_kernel<T, V><<<1, 1024, 0, st>>>(ab, L, B.kuf, B.d_ps, B.npan(), rdiag, y);
+void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, cudaStream_t st) {
+  blk_backward_kernel<T, V><<<1, 1024, 0, st>>>(ab, L, B.kuf, B.d_ps, B.npan(), y);
 }
 // cooperative forward substitution; returns 0, or -1 if the launch was refused
 template <class V, class T>
@@ -691,13 +670,13 @@ template void blk_inverses<double, double>(const double*, const BandLayout&, con
                                            cudaStream_t);
 template void blk_inverses<double, float>(const float*, const BandLayout&, const BlkPlan&, const float*, double*,
                                           cudaStream_t);
-template int blk_backward<double, double>(const double*, const BandLayout&, const BlkPlan&, const double*, double*,
-                                          int*, int, int*, int, cudaStream_t, WaitTest, const int*);
-template int blk_backward<double, float>(const float*, const BandLayout&, const BlkPlan&, const double*, double*, int*,
-                                         int, int*, int, cudaStream_t, WaitTest, const int*);
-template void blk_backward_1cta<double, double>(const double*, const BandLayout&, const BlkPlan&, const double*,
-                                                double*, cudaStream_t);
-template void blk_backward_1cta<double, float>(const float*, const BandLayout&, const BlkPlan&, const float*, double*,
+template int blk_backward<double, double>(const double*, const BandLayout&, const BlkPlan&, double*, int*, int, int*,
+                                          int, cudaStream_t, WaitTest, const int*);
+template int blk_backward<double, float>(const float*, const BandLayout&, const BlkPlan&, double*, int*, int, int*,
+                                         int, cudaStream_t, WaitTest, const int*);
+template void blk_backward_1cta<double, double>(const double*, const BandLayout&, const BlkPlan&, double*,
+                                                cudaStream_t);
+template void blk_backward_1cta<double, float>(const float*, const BandLayout&, const BlkPlan&, double*,
                                                cudaStream_t);
 template int blk_backward_grid<double, double>();
 template int blk_backward_grid<double, float>();

@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
         issue_cols(b0, nb, false);
         if (!wait_bar(&s_bar[0], ph0)) return;
       }
-      // triangular solves, one warp per column: u = L11^-1 P s[0:w] (kept as U12), y = U11^-1 u
+      // triangular solves, one warp per column: u = L11^-1 P s[0:w], y = U11^-1 u (kept as Y in place of A12)
       if (warp < 4) {
         T v = T(0);
         if (warp < nb) {
@@ -291,7 +291,6 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
               if (lane > k) x = fma(-Tr[k], xk, x);
             }
           }
-          if (lane < w) dst[lane] = x;  // U12: not read again by this kernel
           // y = U11^-1 u with this lane's U row pre-scaled by 1/U(lane, lane)
           // (unit diagonal): each step is one shuffle and one FMA
           const T rl = lane < w ? rd[lane] : T(0);
@@ -306,6 +305,7 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
               if (lane < k) v = fma(-Tr[k], yk, v);
             }
           }
+          if (lane < w) dst[lane] = v;  // Y (the right-hand side: z); not read again by this kernel
         }
         Y[warp * 32 + lane] = (warp < nb && lane < w) ? v : T(0);
       }

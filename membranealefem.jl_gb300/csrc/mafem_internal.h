@@ -190,7 +190,7 @@ int blk_lu_factor(T* ab, const BandLayout& L, const BlkPlan& B, int* perm_all, T
 template <class V, class T>
 void blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, const int* perm_all, const T* rdiag, V* b,
                  cudaStream_t st);
-// Back substitution U x = y in place on many SMs (one cooperative launch of
+// Back substitution x1 = z - Y x2 in place on many SMs (one cooperative launch of
 // `grid` CTAs, grid <= blk_backward_grid()).  flags: npan ints, epoch: a value
 // they do not hold yet (incremented per call); err: nonzero after a bounded
 // wait ran out.  Returns -1 if the launch failed.
@@ -202,12 +202,12 @@ struct WaitTest {
   int withhold = -1;
 };
 // Explicit inverses of the stored panels' L11 and U11 (inv: npan x 2 x 32 x
-// 32 in V) for the cooperative substitutions; run after each factorisation.
+// 32 in V) for the cooperative forward substitution.
 template <class V, class T>
 void blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, const T* rdiag, V* inv, cudaStream_t st);
 template <class V, class T>
-int blk_backward(const T* ab, const BandLayout& L, const BlkPlan& B, const V* inv, V* y, int* flags, int epoch,
-                 int* err, int grid, cudaStream_t st, WaitTest wt = WaitTest(), const int* gate = nullptr);
+int blk_backward(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, int* flags, int epoch, int* err, int grid,
+                 cudaStream_t st, WaitTest wt = WaitTest(), const int* gate = nullptr);
 template <class V, class T>
 int blk_backward_grid();
 // Forward substitution (P, L11, A21 of the stored panels) on `grid` CTAs of one
@@ -243,7 +243,7 @@ template <class T>
 int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, const BlkPersist& S, int epoch, int* perm_all,
                           T* rdiag, int* info, T* rhs, int* err, cudaStream_t st, long long* trace = nullptr);
 template <class V, class T>
-void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, const T* rdiag, V* y, cudaStream_t st);
+void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, cudaStream_t st);
 }  // namespace mafem
 
 namespace mafem {
