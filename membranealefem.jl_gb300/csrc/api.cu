@@ -102,6 +102,7 @@ struct mafem_handle {
   // node-block pivoting (band_lu_blk.cu): the default; full partial pivoting
   // (band_lu.cu) is the fallback for a block without a usable pivot
   bool use_blk = false;
+  bool last_two = false;  // node-block factors: of the elimination from both ends
   bool last_blk = false;  // which factorisation the band currently holds
   bool pinv_ready = false;  // d_pinv holds the inverses of its panels' triangles
   BlkPlan blk;
@@ -122,7 +123,6 @@ struct mafem_handle {
   int lu_path = MAFEM_LU_AUTO;
   int patch_nr = 0;  // CTAs per cluster of the batched FP32 factor (0: chosen per round)
   int round_nr = 0;  // the cluster size the autotuner chose for this round (0: by band width)
-  int fepoch = 0;          // epoch of the last persistent factorisation
   void* d_rdiag = nullptr;
   int64_t fallbacks = 0;
   // batched FP32 form (band_lu_patch.cu): the handle's job, usable when its band fits
@@ -523,10 +523,40 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
       UP(h->blk.d_ps, h->blk.ps);
       h->blk.d_blk_end = h->d_blk_end;
       h->use_blk = true;
-      AL(h->d_flags, (size_t)h->blk.npan());
-      AL(h->d_zbuf, (size_t)h->blk.npan() * kBlkW);
-      AL(h->d_pinv, (size_t)h->blk.npan() * 2 * kBlkW * kBlkW);
-      cudaMemset(h->d_flags, 0, (size_t)h->blk.npan() * sizeof(int));
+      BlkChain& one = h->blk.one;
+      one.org = h->L.off;
+      one.sj = h->L.ldb - 1;
+      one.ps = h->blk.d_ps;
+      one.npan = h->blk.npan();
+      one.n = (int)n;
+      one.blk_end = h->d_blk_end;
+      std::vector<int> ps0, ps1, blk_end1;
+      if (precision == MAFEM_PLAIN_FP64 && blk_two_plan(blk_end, h->L, h->blk, ps0, ps1, blk_end1)) {
+        h->blk.has_two = true;
+        BlkChain &a = h->blk.two[0], &b = h->blk.two[1];
+        int *d_ps0 = nullptr, *d_ps1 = nullptr, *d_end1 = nullptr;
+        UP(d_ps0, ps0);
+        UP(d_ps1, ps1);
+        UP(d_end1, blk_end1);
+        a = b = one;
+        a.ps = d_ps0;
+        a.npan = (int)ps0.size() - 1;
+        a.n = h->blk.mid;
+        b.org = (n - 1) * h->L.ldb + h->L.off;  // entry (n - 1, n - 1)
+        b.si = -1;
+        b.sj = -one.sj;
+        b.vorg = n - 1;
+        b.ps = d_ps1;
+        b.npan = (int)ps1.size() - 1;
+        b.blk_end = d_end1;
+        b.pbase = a.npan;
+        b.rbase = h->blk.mid;
+      }
+      const size_t npx = (size_t)h->blk.npan_max();
+      AL(h->d_flags, npx);
+      AL(h->d_zbuf, npx * kBlkW);
+      AL(h->d_pinv, npx * 2 * kBlkW * kBlkW);
+      cudaMemset(h->d_flags, 0, npx * sizeof(int));
       h->bwd_grid = precision == MAFEM_PLAIN_FP64 ? blk_backward_grid<double, double>() : blk_backward_grid<double, float>();
       h->bwd_max = h->bwd_grid;
       cudaGetLastError();
@@ -534,7 +564,9 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
                                                    : blk_persist_setup<float>(h->L, h->blk, h->pers);
       cudaGetLastError();
       if (pg > 0) {
-        const size_t np = (size_t)h->blk.npan();
+        const size_t np = (size_t)h->blk.npan() + (size_t)h->blk.two[0].npan + (size_t)h->blk.two[1].npan;
+        AL(h->pers.d_bdone, 1);
+        cudaMemset(h->pers.d_bdone, 0, sizeof(int));
         AL(h->pers.d_pdone, np);
         AL(h->pers.d_critcnt, np);
         AL(h->pers.d_a21cnt, np);
@@ -563,7 +595,7 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
   AL(h->d_part, 2048);
   AL(h->d_out, 16);
   AL(h->d_ipiv, n);
-  AL(h->d_perm, std::max((size_t)h->npan * h->rmax, (size_t)h->blk.npan() * kBlkW));
+  AL(h->d_perm, std::max((size_t)h->npan * h->rmax, (size_t)h->blk.npan_max() * kBlkW));
   AL(h->d_rstate, 4);
   AL(h->d_info, 4);  // [0] zero-pivot column (1-based), [1] nonzero: a bounded device wait ran out
   cudaMemset(h->d_info, 0, 4 * sizeof(int));
@@ -707,6 +739,7 @@ static int band_clear(mafem_handle* h, cudaStream_t st) {
 // super-diagonals the next factorisation fills: full partial pivoting fills the
 // top kl rows of the band, which band_clear empties
 static int fill_diagonals(const mafem_handle* h) { return h->use_blk ? h->blk.kuf : (int)h->L.ku; }
+static int fill_rows(const mafem_handle* h) { return h->use_blk && h->blk.has_two ? h->blk.kuf + kBlkW : h->L.kl; }
 
 // element kernel + gathers: r -> d_r, K -> d_band
 static int assemble(mafem_handle* h, double time, double dt, bool both_bands = false) {
@@ -719,7 +752,7 @@ static int assemble(mafem_handle* h, double time, double dt, bool both_bands = f
       h->err = std::string("element kernel: ") + cudaGetErrorString(e);
       return MAFEM_ERR_CUDA;
     }
-    launch_band_gather<double>(h->P, h->ndf, h->nq, h->L, fill_diagonals(h), (const double*)h->d_Kel,
+    launch_band_gather<double>(h->P, h->ndf, h->nq, h->L, fill_diagonals(h), fill_rows(h), (const double*)h->d_Kel,
                                (double*)h->d_band, h->st);
     h->launches += 2;
   } else {
@@ -728,7 +761,7 @@ static int assemble(mafem_handle* h, double time, double dt, bool both_bands = f
       h->err = std::string("element kernel: ") + cudaGetErrorString(e);
       return MAFEM_ERR_CUDA;
     }
-    launch_band_gather<float>(h->P, h->ndf, h->nq, h->L, fill_diagonals(h), (const float*)h->d_Kel,
+    launch_band_gather<float>(h->P, h->ndf, h->nq, h->L, fill_diagonals(h), fill_rows(h), (const float*)h->d_Kel,
                               (float*)h->d_band, h->st, both_bands ? (float*)h->d_band0 : nullptr);
     h->launches += 2;
   }
@@ -752,11 +785,11 @@ static int assemble(mafem_handle* h, double time, double dt, bool both_bands = f
 static void blk_need_inverses(mafem_handle* h) {
   if (h->pinv_ready) return;
   h->pinv_ready = true;
-  if (h->precision == MAFEM_PLAIN_FP64)
-    blk_inverses<double, double>((const double*)h->d_band, h->L, h->blk, (const double*)h->d_rdiag, h->d_pinv, h->st);
-  else
-    blk_inverses<double, float>((const float*)h->d_band, h->L, h->blk, (const float*)h->d_rdiag, h->d_pinv, h->st);
-  h->launches += 1;
+  h->launches += h->precision == MAFEM_PLAIN_FP64
+                     ? blk_inverses<double, double>((const double*)h->d_band, h->blk, h->last_two,
+                                                    (const double*)h->d_rdiag, h->d_pinv, h->st)
+                     : blk_inverses<double, float>((const float*)h->d_band, h->blk, h->last_two,
+                                                   (const float*)h->d_rdiag, h->d_pinv, h->st);
 }
 
 static int factor_enqueue(mafem_handle* h, double* x) {
@@ -764,11 +797,13 @@ static int factor_enqueue(mafem_handle* h, double* x) {
   CK(cudaMemsetAsync(h->d_info, 0, sizeof(int), h->st));
   bool launched = false;
   if (h->pers.grid > 0 && h->lu_path == MAFEM_LU_AUTO) {
-    ++h->fepoch;
-    const int nl = fp64 ? blk_lu_factor_persist<double>((double*)h->d_band, h->L, h->blk, h->pers, h->fepoch, h->d_perm,
+    // from both ends where the grid allows (blk_two_plan)
+    const bool two = fp64 && x && h->pers.min_two > 0 && h->pers.grid >= h->pers.min_two && h->bwd_grid > 0;
+    const int nl = fp64 ? blk_lu_factor_persist<double>((double*)h->d_band, h->L, h->blk, h->pers, two, h->d_perm,
                                                         (double*)h->d_rdiag, h->d_info, x, h->d_info + 1, h->st)
-                        : blk_lu_factor_persist<float>((float*)h->d_band, h->L, h->blk, h->pers, h->fepoch, h->d_perm,
+                        : blk_lu_factor_persist<float>((float*)h->d_band, h->L, h->blk, h->pers, two, h->d_perm,
                                                        (float*)h->d_rdiag, h->d_info, nullptr, h->d_info + 1, h->st);
+    h->last_two = two && nl > 0;
     if (nl < 0) {
       cudaGetLastError();
       h->pers.grid = 0;  // cooperative launch refused: per-panel launches from now on
@@ -778,6 +813,7 @@ static int factor_enqueue(mafem_handle* h, double* x) {
     }
   }
   if (!launched) {
+    h->last_two = false;
     const int nl = fp64 ? blk_lu_factor<double>((double*)h->d_band, h->L, h->blk, h->d_perm, (double*)h->d_rdiag,
                                                 h->d_info, x, h->st, h->st2, h->ev_pool.data(), nullptr)
                         : blk_lu_factor<float>((float*)h->d_band, h->L, h->blk, h->d_perm, (float*)h->d_rdiag,
@@ -822,7 +858,7 @@ static int factor(mafem_handle* h, double* x, const double* rhs0) {
       CK(cudaMemcpyAsync(h->d_band, h->host_band, (size_t)h->L.ldb * n * sizeof(double), cudaMemcpyHostToDevice,
                          h->st));
     else if (fp64)
-      launch_band_gather<double>(h->P, h->ndf, h->nq, h->L, fill_diagonals(h), (const double*)h->d_Kel,
+      launch_band_gather<double>(h->P, h->ndf, h->nq, h->L, fill_diagonals(h), fill_rows(h), (const double*)h->d_Kel,
                                  (double*)h->d_band, h->st);
     else
       CK(cudaMemcpyAsync(h->d_band, h->d_band0, (size_t)h->L.ldb * n * sizeof(float), cudaMemcpyDeviceToDevice,
@@ -860,10 +896,10 @@ static int factor(mafem_handle* h, double* x, const double* rhs0) {
 template <class T>
 static void blk_back_solve(mafem_handle* h, double* y, const int* gate = nullptr) {
   if (h->bwd_grid > 0) {
-    ++h->epoch;
-    if (blk_backward<double, T>((const T*)h->d_band, h->L, h->blk, y, h->d_flags, h->epoch, h->d_info + 1,
-                                h->bwd_grid, h->st, h->wait_test, gate) == 0) {
-      h->launches += 1;
+    const int nl = blk_backward<double, T>((const T*)h->d_band, h->blk, h->last_two, y, h->d_flags, h->epoch,
+                                           h->d_info + 1, h->bwd_grid, h->st, h->wait_test, gate);
+    if (nl > 0 || h->last_two) {  // the factors of the two chains are for the cooperative kernel alone:
+      h->launches += std::max(nl, 0);  // a refused launch stays as the CUDA error that the caller reports
       return;
     }
     cudaGetLastError();
@@ -879,11 +915,11 @@ template <class T>
 static void blk_fwd_solve(mafem_handle* h, double* y, const int* gate = nullptr) {
   if (h->bwd_grid > 0) {
     blk_need_inverses(h);
-    ++h->epoch;
-    if (blk_forward_coop<double, T>((const T*)h->d_band, h->L, h->blk, h->d_perm, h->d_pinv, y, h->d_zbuf,
-                                    h->d_flags, h->epoch, h->d_info + 1, h->bwd_grid, h->st, h->wait_test,
-                                    gate) == 0) {
-      h->launches += 1;
+    const int nl = blk_forward_coop<double, T>((const T*)h->d_band, h->L, h->blk, h->last_two, h->d_perm, h->d_pinv, y,
+                                               h->d_zbuf, h->d_flags, h->epoch, h->d_info + 1, h->bwd_grid, h->st,
+                                               h->wait_test, gate);
+    if (nl > 0 || h->last_two) {
+      h->launches += std::max(nl, 0);
       return;
     }
     cudaGetLastError();
@@ -2584,17 +2620,17 @@ extern "C" int mafem_trace_factor(mafem_handle* h, double time, double dt, int64
   if (rc) return rc;
   CK(cudaMemcpyAsync(h->d_x, h->d_r, h->nmdf * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
   CK(cudaMemsetAsync(h->d_info, 0, sizeof(int), h->st));
-  ++h->fepoch;
   const bool fp64 = h->precision == MAFEM_PLAIN_FP64;
-  const int nl = fp64 ? blk_lu_factor_persist<double>((double*)h->d_band, h->L, h->blk, h->pers, h->fepoch, h->d_perm,
+  const int nl = fp64 ? blk_lu_factor_persist<double>((double*)h->d_band, h->L, h->blk, h->pers, false, h->d_perm,
                                                       (double*)h->d_rdiag, h->d_info, h->d_x, h->d_info + 1, h->st,
                                                       d_tr)
-                      : blk_lu_factor_persist<float>((float*)h->d_band, h->L, h->blk, h->pers, h->fepoch, h->d_perm,
+                      : blk_lu_factor_persist<float>((float*)h->d_band, h->L, h->blk, h->pers, false, h->d_perm,
                                                      (float*)h->d_rdiag, h->d_info, nullptr, h->d_info + 1, h->st,
                                                      d_tr);
   h->pinv_ready = false;
   h->factored = true;
   h->last_blk = true;
+  h->last_two = false;
   CK(cudaMemcpyAsync(out, d_tr, sizeof(long long) * 12 * npan, cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
   cudaFree(d_tr);
@@ -2957,6 +2993,7 @@ extern "C" int mafem_profile_factor(mafem_handle* h, double time, double dt, maf
   }
   h->factored = true;
   h->last_blk = h->use_blk;
+  h->last_two = false;
   CK(cudaStreamSynchronize(h->st));
   float ms = 0;
   cudaEventElapsedTime(&ms, a0, a1);

@@ -24,9 +24,10 @@ __host__ __device__ __forceinline__ int64_t min64(int64_t a, int64_t b) { return
 __host__ __device__ __forceinline__ int64_t max64(int64_t a, int64_t b) { return a > b ? a : b; }
 
 // Band column j, by one warp.  Written are the rows the factorisation may have
-// changed since the last gather -- j - kuf - kBlkW .. j + kl: the fill of
-// node-block pivoting (kuf super-diagonals; a panel's interchanges reach at most
-// kBlkW rows further, where it stores zeros) -- first as zeros in 16-byte
+// changed since the last gather -- j - kuf - kBlkW .. j + klf: the fill of
+// node-block pivoting (kuf super-diagonals and kBlkW rows beyond for Y; klf: kl,
+// or as far below the diagonal for an elimination from both ends, the rows beyond
+// the column's last being the first ones of the next) -- first as zeros in 16-byte
 // stores, then the column's element stencil: the unknowns of 5 x 5 control
 // points, one run of rows per row of the control-point grid, a lane per row
 // adding its <= 3 x 3 element contributions (consecutive rows read consecutive
@@ -39,7 +40,7 @@ __host__ __device__ __forceinline__ int64_t max64(int64_t a, int64_t b) { return
 // band (58 MB, 0.5 TB/s); every patch of a 256-patch round (14 GB written that way)
 // takes 2.8 ms here.
 template <class T>
-__device__ __forceinline__ void gather_column(const DevPatch& P, int ndf, int nq, const BandLayout& L, int kuf,
+__device__ __forceinline__ void gather_column(const DevPatch& P, int ndf, int nq, const BandLayout& L, int kuf, int klf,
                                               const T* __restrict__ K_el, T* __restrict__ ab, T* __restrict__ ab2,
                                               int64_t j) {
   constexpr int E = 16 / (int)sizeof(T);
@@ -47,9 +48,10 @@ __device__ __forceinline__ void gather_column(const DevPatch& P, int ndf, int nq
   const int NJ = P.unk_node[j], dj = P.unk_dof[j], W = P.num1np;
   const int s2J = NJ / W, s1J = NJ - s2J * W;
   {
-    const int s0 = max((int)L.off - kuf - kBlkW, 0) / E, s1 = (int)(L.off + L.kl) / E;
+    const int V = (int)L.ldb / E;
+    const int s0 = max((int)L.off - kuf - kBlkW, 0) / E, s1 = (int)(L.off + klf) / E;
     float4* col = reinterpret_cast<float4*>(ab + j * L.ldb);
-    for (int v = s0 + lane; v <= s1; v += 32) col[v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int v = s0 + lane; v <= s1; v += 32) col[v < V ? v : v - V] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
   __syncwarp();  // a row's zero before its value
   T* col = ab + j * L.ldb + L.off - j;  // + i: row i
@@ -92,10 +94,11 @@ __device__ __forceinline__ void gather_column(const DevPatch& P, int ndf, int nq
 constexpr int kGatherWarps = 8;  // columns per CTA
 template <class T>
 __global__ void __launch_bounds__(32 * kGatherWarps)
-    band_gather_kernel(DevPatch P, int ndf, int nq, BandLayout L, int kuf, const T* __restrict__ K_el,
+    band_gather_kernel(DevPatch P, int ndf, int nq, BandLayout L, int kuf, int klf,
+                       const T* __restrict__ K_el,
                        T* __restrict__ ab, T* __restrict__ ab2) {
   const int64_t j = blockIdx.x * (int64_t)kGatherWarps + (threadIdx.x >> 5);
-  if (j < L.n) gather_column<T>(P, ndf, nq, L, kuf, K_el, ab, ab2, j);
+  if (j < L.n) gather_column<T>(P, ndf, nq, L, kuf, klf, K_el, ab, ab2, j);
 }
 
 // r[i] = Σ_e r_el[e][(a, di)] over the elements containing node(i) (FiniteElement.jl:131)
@@ -300,7 +303,7 @@ __global__ void __launch_bounds__(32 * kGatherCols) batch_gather_kernel(const As
   const int k = batch_item(off, m, &s_k);
   const AsmJob& J = jobs[items[k].job];
   const int64_t j = (int64_t)(off[0] + (int)blockIdx.x - off[k]) * kGatherCols + (threadIdx.x >> 5);
-  if (j < J.L.n) gather_column<float>(J.P, J.pp.ndf, J.pp.nq, J.L, J.kuf, J.K_el, J.band, J.band0, j);
+  if (j < J.L.n) gather_column<float>(J.P, J.pp.ndf, J.pp.nq, J.L, J.kuf, J.L.kl, J.K_el, J.band, J.band0, j);
 }
 
 // The residual, 256 unknowns per CTA; the patch's first CTA also zeroes its
@@ -413,10 +416,10 @@ void launch_batch_dirichlet(const AsmJob* jobs, const AsmItem* items, const int*
   if (ctas > 0) batch_dirichlet_kernel<<<ctas, 256, 0, st>>>(jobs, items, off, m);
 }
 template <class T>
-void launch_band_gather(const DevPatch& P, int ndf, int nq, const BandLayout& L, int kuf, const T* K_el, T* ab,
-                        cudaStream_t st, T* ab2) {
+void launch_band_gather(const DevPatch& P, int ndf, int nq, const BandLayout& L, int kuf, int klf, const T* K_el,
+                        T* ab, cudaStream_t st, T* ab2) {
   const unsigned grid = (unsigned)((L.n + kGatherWarps - 1) / kGatherWarps);
-  band_gather_kernel<T><<<grid, 32 * kGatherWarps, 0, st>>>(P, ndf, nq, L, kuf, K_el, ab, ab2);
+  band_gather_kernel<T><<<grid, 32 * kGatherWarps, 0, st>>>(P, ndf, nq, L, kuf, klf, K_el, ab, ab2);
 }
 void launch_resid_gather(const DevPatch& P, int ndf, int nq, const double* r_el, double* r, cudaStream_t st) {
   const int blocks = (int)min64(1024, (P.nmdf + 255) / 256);
@@ -526,9 +529,9 @@ void launch_axpy(int64_t n, const double* dx, double* x, cudaStream_t st) {
   axpy_kernel<<<blocks, 256, 0, st>>>(n, dx, x);
 }
 
-template void launch_band_gather<double>(const DevPatch&, int, int, const BandLayout&, int, const double*, double*,
+template void launch_band_gather<double>(const DevPatch&, int, int, const BandLayout&, int, int, const double*, double*,
                                          cudaStream_t, double*);
-template void launch_band_gather<float>(const DevPatch&, int, int, const BandLayout&, int, const float*, float*,
+template void launch_band_gather<float>(const DevPatch&, int, int, const BandLayout&, int, int, const float*, float*,
                                         cudaStream_t, float*);
 template void launch_band_residual<double>(const double*, const BandLayout&, const double*, const double*, double*,
                                            double*, double*, cudaStream_t, const int*);

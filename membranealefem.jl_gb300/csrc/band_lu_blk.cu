@@ -45,7 +45,8 @@ __global__ void __launch_bounds__(32 * kPanelWarps) blk_panel_kernel(T* __restri
                                                                      int* __restrict__ info) {
   __shared__ T s_l[2][32];
   __shared__ int s_p[2];
-  blk_panel_factor<T, false>(ab, L, j0, w, blk_end, perm, rdiag, info, s_l, s_p);
+  blk_panel_factor<T, false>(ab + bix(L, j0, j0), 1, L.ldb - 1, (int)j0, w, (int)j0 + 1, 1, blk_end + j0, perm,
+                             rdiag + j0, info, s_l, s_p);
 }
 
 // ---------------------------------------------------------------------------
@@ -318,19 +319,19 @@ __global__ void __launch_bounds__(1024) blk_backward_kernel(const T* __restrict_
 // is two 32-term dot products per lane with independent shuffles instead of
 // two 32-step dependent chains.
 template <class T, class V>
-__global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__ ab, BandLayout L,
-                                                           const int* __restrict__ ps, int npan,
-                                                           const T* __restrict__ rdiag, V* __restrict__ inv) {
-  __shared__ V S[4][32][33];  // per warp: S[c][i] = A(j0 + i, j0 + c) of its panel
+__global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__ ab, BlkChain c,
+                                                           const T* __restrict__ rdiag_all, V* __restrict__ inv) {
+  __shared__ V S[4][32][33];  // per warp: S[k][i] = A(j0 + i, j0 + k) of its panel
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int p = blockIdx.x * 4 + warp;
-  if (p >= npan) return;  // warp-uniform; only warp-level synchronisation below
-  const int64_t j0 = ps[p];
-  const int w = (int)(ps[p + 1] - j0);
-  for (int c = 0; c < 32; ++c) S[warp][c][lane] = (c < w && lane < w) ? V(ab[bix(L, j0 + lane, j0 + c)]) : V(0);
+  if (p >= c.npan) return;  // warp-uniform; only warp-level synchronisation below
+  const int j0 = c.ps[p], w = c.ps[p + 1] - j0;
+  const T* blk = ab + c.org + j0 * c.si + j0 * c.sj;
+  const T* rdiag = rdiag_all + c.rbase;
+  for (int k = 0; k < 32; ++k) S[warp][k][lane] = (k < w && lane < w) ? V(blk[lane * c.si + k * c.sj]) : V(0);
   const V rd = lane < w ? V(rdiag[j0 + lane]) : V(0);
   __syncwarp();
-  V* Li = inv + (size_t)p * 2 * kBlkW * kBlkW;
+  V* Li = inv + (size_t)(c.pbase + p) * 2 * kBlkW * kBlkW;
   V* Ui = Li + kBlkW * kBlkW;
   V x[32];
   // column `lane` of L11^-1: L11 x = e_lane, forward
@@ -370,37 +371,56 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
 // wt.withhold = k >= 0 (failure-detection tests only): the flag of panel
 // npan - 1 - k is never published, so the CTAs that need it run out of polls
 // and every CTA returns.
+//
+// A launch covers panels [p0, p1) of one chain, or of two chains side by side
+// (CTAs below `split` the first): the columns right of panel p1 - 1 belong to
+// panels solved by an earlier launch.
+struct BlkSpan {
+  BlkChain c;
+  int p0, p1;
+};
 template <class T, class V>
-__global__ void __launch_bounds__(256) blk_backward_coop_kernel(const T* __restrict__ ab, BandLayout L, int kuf,
-                                                                const int* __restrict__ ps, int npan, V* y, int* flags,
-                                                                int epoch, int* err, WaitTest wt,
-                                                                const int* gate) {
+__global__ void __launch_bounds__(256) blk_backward_coop_kernel(const T* __restrict__ ab, int kuf, BlkSpan s0, BlkSpan s1,
+                                                                int split, V* yv, int* flags_all, int epoch, int* err,
+                                                                WaitTest wt, const int* gate) {
   __shared__ V part[8][33];
   __shared__ int s_ok;
   if (gate && *gate) return;  // every CTA reads the same word: all return (refinement already stopped)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int q = npan - 1 - (int)blockIdx.x; q >= 0; q -= gridDim.x) {
-    const int64_t j0 = ps[q], j1 = ps[q + 1];
-    const int w = (int)(j1 - j0);
-    const int64_t jend = min64b(L.n, j1 + kuf);
-    int pl = q + 1;  // last panel with columns in [j1, jend)
-    while (pl + 1 < npan && ps[pl + 1] < jend) ++pl;
+  const bool second = (int)blockIdx.x >= split;
+  const BlkSpan& S = second ? s1 : s0;
+  const int me = (int)blockIdx.x - (second ? split : 0), G = second ? (int)gridDim.x - split : split;
+  const int* __restrict__ ps = S.c.ps;
+  const int64_t si = S.c.si, sj = S.c.sj;
+  const T* a0 = ab + S.c.org;
+  V* y = yv + S.c.vorg;  // element i at y[i si]
+  int* flags = flags_all + S.c.pbase;
+  for (int q = S.p1 - 1 - me; q >= S.p0; q -= G) {
+    const int j0 = ps[q], j1 = ps[q + 1];
+    const int w = j1 - j0;
+    const int jend = min(S.c.n, j1 + kuf);
+    const T* arow = a0 + (j0 + lane) * si;
     V acc = V(0);
-    for (int p = (j1 < jend) ? pl : q; p > q; --p) {
+    if (lane < w)  // columns solved before this launch
+      for (int c = max(j1, ps[S.p1]) + warp; c < jend; c += 8) acc += V(arow[c * sj]) * __ldcg(y + c * si);
+    int pl = q + 1;  // last panel of the launch with columns in [j1, jend)
+    while (pl + 1 < S.p1 && ps[pl + 1] < jend) ++pl;
+    for (int p = (j1 < jend && q + 1 < S.p1) ? pl : q; p > q; --p) {
       if (!wait_flag(flags, p, epoch, err, &s_ok, wt.limit)) return;
-      const int64_t cb = ps[p], ce = min64b(ps[p + 1], jend);
+      const int cb = ps[p], ce = min(ps[p + 1], jend);
       if (lane < w)
-        for (int64_t c = cb + warp; c < ce; c += 8) acc += V(ab[bix(L, j0 + lane, c)]) * __ldcg(y + c);
+        for (int c = cb + warp; c < ce; c += 8) acc += V(arow[c * sj]) * __ldcg(y + c * si);
     }
     part[warp][lane] = acc;
     __syncthreads();
     if (warp == 0) {
       const V sum = ((part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane])) +
                     ((part[4][lane] + part[5][lane]) + (part[6][lane] + part[7][lane]));  // tree: 3 dependent adds
-      if (lane < w) __stcg(y + j0 + lane, __ldcg(y + j0 + lane) - sum);  // x1 = z - Y x2
+      V* yj = y + (j0 + lane) * si;
+      if (lane < w) __stcg(yj, __ldcg(yj) - sum);  // x1 = z - Y x2
       __threadfence();
       __syncwarp();
-      if (lane == 0 && npan - 1 - q != wt.withhold) st_release(flags + q, epoch);
+      if (lane == 0 && (second || S.c.npan - 1 - q != wt.withhold)) st_release(flags + q, epoch);
     }
     __syncthreads();
   }
@@ -416,12 +436,13 @@ __global__ void __launch_bounds__(256) blk_backward_coop_kernel(const T* __restr
 // release store of the flag.  A panel waits only for lower-numbered panels,
 // which CTAs take in increasing order, so the chain always progresses; waits
 // are bounded (kSpinLimit polls, then *err and every CTA returns).
+// A launch covers panels [p0, p1) of one or two chains like the back substitution's;
+// the panels before p0 were done by an earlier launch.
 template <class T, class V>
-__global__ void __launch_bounds__(256) blk_forward_coop_kernel(const T* __restrict__ ab, BandLayout L,
-                                                               const int* __restrict__ ps, int npan,
-                                                               const int* __restrict__ perm_all,
-                                                               const V* __restrict__ inv, V* b, V* zbuf,
-                                                               int* flags, int epoch, int* err, WaitTest wt,
+__global__ void __launch_bounds__(256) blk_forward_coop_kernel(const T* __restrict__ ab, int kl, BlkSpan s0, BlkSpan s1,
+                                                               int split, const int* __restrict__ perm_all,
+                                                               const V* __restrict__ inv_all, V* bv, V* zbuf_all,
+                                                               int* flags_all, int epoch, int* err, WaitTest wt,
                                                                const int* gate) {
   __shared__ V part[8][33];
   __shared__ V Is[2 * 32 * 32];  // L11^-1 then U11^-1 of the panel, element (i, k) at k * 32 + i
@@ -429,22 +450,32 @@ __global__ void __launch_bounds__(256) blk_forward_coop_kernel(const T* __restri
   __shared__ int s_ok;
   if (gate && *gate) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int p = blockIdx.x; p < npan; p += gridDim.x) {
-    const int64_t j0 = ps[p], j1 = ps[p + 1];
-    const int w = (int)(j1 - j0);
-    const V* Ip = inv + (size_t)p * 2 * kBlkW * kBlkW;
+  const bool second = (int)blockIdx.x >= split;
+  const BlkSpan& S = second ? s1 : s0;
+  const int me = (int)blockIdx.x - (second ? split : 0), G = second ? (int)gridDim.x - split : split;
+  const int* __restrict__ ps = S.c.ps;
+  const int64_t si = S.c.si, sj = S.c.sj;
+  const T* a0 = ab + S.c.org;
+  V* b = bv + S.c.vorg;  // element i at b[i si]
+  V* zbuf = zbuf_all + (size_t)S.c.pbase * kBlkW;
+  int* flags = flags_all + S.c.pbase;
+  for (int p = S.p0 + me; p < S.p1; p += G) {
+    const int j0 = ps[p], j1 = ps[p + 1];
+    const int w = j1 - j0;
+    const V* Ip = inv_all + (size_t)(S.c.pbase + p) * 2 * kBlkW * kBlkW;
     for (int k = tid; k < 2 * kBlkW * kBlkW; k += 256) Is[k] = __ldcg(Ip + k);
     int pf = p;  // earliest panel whose rows reach j0
-    while (pf > 0 && ps[pf] + L.kl > j0) --pf;
+    while (pf > 0 && ps[pf] + kl > j0) --pf;
+    const T* arow = a0 + (j0 + lane) * si;
     V acc = V(0);
     for (int q = pf; q < p; ++q) {
-      if (!wait_flag(flags, q, epoch, err, &s_ok, wt.limit)) return;
-      const int64_t q0 = ps[q];
+      if (q >= S.p0 && !wait_flag(flags, q, epoch, err, &s_ok, wt.limit)) return;
+      const int q0 = ps[q];
       const int wq = ps[q + 1] - ps[q];
       if (lane < w)
         for (int k = warp; k < wq; k += 8)
-          if (j0 + lane - (q0 + k) <= L.kl)  // inside panel q's band rows
-            acc += V(ab[bix(L, j0 + lane, q0 + k)]) * __ldcg(zbuf + (size_t)q * kBlkW + k);
+          if (j0 + lane - (q0 + k) <= kl)  // inside panel q's band rows
+            acc += V(arow[(q0 + k) * sj]) * __ldcg(zbuf + (size_t)q * kBlkW + k);
     }
     part[warp][lane] = acc;
     __syncthreads();
@@ -452,8 +483,8 @@ __global__ void __launch_bounds__(256) blk_forward_coop_kernel(const T* __restri
       accs[lane] = ((part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane])) +
                    ((part[4][lane] + part[5][lane]) + (part[6][lane] + part[7][lane]));
       __syncwarp();
-      const int pr = lane < w ? perm_all[(size_t)p * kBlkW + lane] : 0;
-      const V x = lane < w ? __ldcg(b + j0 + pr) - accs[pr] : V(0);
+      const int pr = lane < w ? perm_all[(size_t)(S.c.pbase + p) * kBlkW + lane] : 0;
+      const V x = lane < w ? __ldcg(b + (j0 + pr) * si) - accs[pr] : V(0);
       // y1 = L11^-1 P b1, z = U11^-1 y1: dot products with independent shuffles
       V y1 = V(0);
 #pragma unroll
@@ -462,7 +493,7 @@ __global__ void __launch_bounds__(256) blk_forward_coop_kernel(const T* __restri
 #pragma unroll
       for (int k = 0; k < 32; ++k) v = fma(Is[kBlkW * kBlkW + k * 32 + lane], __shfl_sync(kFull, y1, k), v);
       if (lane < w) {
-        __stcg(b + j0 + lane, v);
+        __stcg(b + (j0 + lane) * si, v);
         __stcg(zbuf + (size_t)p * kBlkW + lane, v);
       }
       __threadfence();
@@ -471,6 +502,21 @@ __global__ void __launch_bounds__(256) blk_forward_coop_kernel(const T* __restri
     }
     __syncthreads();
   }
+}
+// The backward chain's contributions to the rows [lo, mid) above it, before the
+// forward chain goes on through them: b[i] -= sum_j A(i, j) z(j) over the columns
+// j >= mid that reach row i (physical numbering; z stands in b).  A warp per row.
+template <class T, class V>
+__global__ void __launch_bounds__(256) blk_forward_mid_kernel(const T* __restrict__ ab, BandLayout L, int mid, int lo,
+                                                              V* __restrict__ b, const int* __restrict__ gate) {
+  if (gate && *gate) return;
+  const int i = lo + blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (i >= mid) return;
+  const int jend = (int)min64b(L.n, (int64_t)i + L.ku + 1);
+  V s = V(0);
+  for (int j = mid + lane; j < jend; j += 32) s += V(ab[bix(L, i, j)]) * b[j];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+  if (lane == 0) b[i] -= s;
 }
 
 // ---------------------------------------------------------------------------
@@ -505,6 +551,39 @@ bool blk_plan(const std::vector<int>& blk_end, int wmax, int ku, BlkPlan& out) {
   }
   out.kuf = ku + out.ndfp;
   return true;
+}
+
+// The backward chain takes the unknowns [mid, n), whole pivot blocks, so many that
+// 2 kuf unknowns are left between the chains when the forward chain has done as
+// many: until then a panel of the forward chain (it reaches kuf unknowns beyond
+// itself) and one of the backward chain never touch the same entries.  pm: the
+// forward chain's first panel that may.  The chain of dependent panels is then
+// n / 2 + kuf unknowns long instead of n; bands shorter than 10/3 kuf keep the one
+// chain (LAG 8 x 8 at 3.6 kuf, six panels instead of eight and a meeting of all
+// CTAs: 0.24 -> 0.19 ms; below, the meeting costs what the shorter chain saves).
+bool blk_two_plan(const std::vector<int>& blk_end, const BandLayout& L, BlkPlan& out, std::vector<int>& ps0,
+                  std::vector<int>& ps1, std::vector<int>& blk_end1) {
+  const int n = (int)blk_end.size(), kuf = out.kuf, kl = L.kl;
+  // the backward chain's fill takes rows up to kuf + kBlkW below the diagonal of a
+  // band column; those beyond ldb are the first rows of the next one, unused there
+  if (kl != L.ku || L.ldb <= 2 * ((int64_t)kuf + kBlkW) || 3 * (int64_t)n < 10 * (int64_t)kuf) return false;
+  const int want = (n - 2 * kuf) / 2;  // unknowns of the backward chain
+  int mid = n;
+  std::vector<int> first(n);  // first unknown of each unknown's block
+  for (int q = 0; q < n; ++q) first[q] = q > 0 && blk_end[q - 1] > q ? first[q - 1] : q;
+  while (mid > 0 && n - first[mid - 1] <= want) mid = first[mid - 1];
+  if (n - mid < 2 * kBlkW || mid < 2 * kBlkW) return false;
+  BlkPlan a, b;
+  std::vector<int> e0(blk_end.begin(), blk_end.begin() + mid);
+  blk_end1.resize(n - mid);
+  for (int j = 0; j < n - mid; ++j) blk_end1[j] = n - first[n - 1 - j];  // reversed: the block ends where it began
+  if (!blk_plan(e0, out.wmax, kl, a) || !blk_plan(blk_end1, out.wmax, kl, b)) return false;
+  ps0 = a.ps;
+  ps1 = b.ps;
+  out.mid = mid;
+  out.pm = 0;
+  while (out.pm < a.npan() && ps0[out.pm + 1] + kuf <= mid - kuf) ++out.pm;
+  return out.pm > 0;  // their panels are no wider than out.wmax
 }
 
 template <class T>
@@ -613,38 +692,67 @@ void blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, const int* 
   blk_forward_kernel<T, V><<<1, 1024, sm, st>>>(ab, L, B.d_ps, B.npan(), perm_all, rdiag, b);
 }
 template <class V, class T>
-void blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, const T* rdiag, V* inv, cudaStream_t st) {
-  blk_inverses_kernel<T, V><<<(B.npan() + 3) / 4, 128, 0, st>>>(ab, L, B.d_ps, B.npan(), rdiag, inv);
+int blk_inverses(const T* ab, const BlkPlan& B, bool two, const T* rdiag, V* inv, cudaStream_t st) {
+  for (int k = 0; k < (two ? 2 : 1); ++k) {
+    const BlkChain& c = two ? B.two[k] : B.one;
+    blk_inverses_kernel<T, V><<<(c.npan + 3) / 4, 128, 0, st>>>(ab, c, rdiag, inv);
+  }
+  return two ? 2 : 1;
+}
+// One cooperative launch over spans a and (optionally) b, its CTAs shared out by their panels.
+template <class F>
+static int coop_spans(F&& launch, const BlkSpan& a, const BlkSpan* b, int grid) {
+  const int na = a.p1 - a.p0, nb = b ? b->p1 - b->p0 : 0;
+  if (na + nb <= 0) return 0;
+  if (nb > 0 && grid < 2) {  // one after the other
+    const int ra = coop_spans(launch, a, nullptr, grid), rb = coop_spans(launch, *b, nullptr, grid);
+    return ra < 0 || rb < 0 ? -1 : ra + rb;
+  }
+  const int ga = std::min(na, nb > 0 ? grid / 2 : grid), gb = std::min(nb, grid - ga);
+  return launch(a, b ? *b : a, ga, ga + gb) == cudaSuccess ? 1 : -1;
 }
 template <class V, class T>
-int blk_backward(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, int* flags, int epoch, int* err, int grid,
+int blk_backward(const T* ab, const BlkPlan& B, bool two, V* y, int* flags, int& epoch, int* err, int grid,
                  cudaStream_t st, WaitTest wt, const int* gate) {
-  const int npan = B.npan();
   int kuf = B.kuf;
-  const int* ps = B.d_ps;
-  void* args[] = {(void*)&ab,    (void*)&L,     (void*)&kuf, (void*)&ps, (void*)&npan, (void*)&y,
-                  (void*)&flags, (void*)&epoch, (void*)&err, (void*)&wt, (void*)&gate};
-  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)blk_backward_coop_kernel<T, V>,
-                                                    dim3(std::min(grid, npan)), dim3(256), args, 0, st);
-  return e == cudaSuccess ? 0 : -1;
+  auto launch = [&](BlkSpan a, BlkSpan b, int split, int ctas) {
+    ++epoch;
+    void* args[] = {(void*)&ab, (void*)&kuf,   (void*)&a,   (void*)&b,  (void*)&split, (void*)&y, (void*)&flags,
+                    (void*)&epoch, (void*)&err, (void*)&wt, (void*)&gate};
+    return cudaLaunchCooperativeKernel((const void*)blk_backward_coop_kernel<T, V>, dim3(ctas), dim3(256), args, 0, st);
+  };
+  if (!two) return coop_spans(launch, BlkSpan{B.one, 0, B.one.npan}, nullptr, grid);
+  // the unknowns between the chains, then both chains side by side
+  const int r1 = coop_spans(launch, BlkSpan{B.two[0], B.pm, B.two[0].npan}, nullptr, grid);
+  if (r1 < 0) return r1;
+  const BlkSpan b1{B.two[1], 0, B.two[1].npan};
+  const int r2 = coop_spans(launch, BlkSpan{B.two[0], 0, B.pm}, &b1, grid);
+  return r2 < 0 ? r2 : r1 + r2;
 }
 // single-CTA back substitution (used when a cooperative launch is not possible)
 template <class V, class T>
 void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, cudaStream_t st) {
   blk_backward_kernel<T, V><<<1, 1024, 0, st>>>(ab, L, B.kuf, B.d_ps, B.npan(), y);
 }
-// cooperative forward substitution; returns 0, or -1 if the launch was refused
 template <class V, class T>
-int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, const int* perm_all, const V* inv, V* b,
-                     V* zbuf, int* flags, int epoch, int* err, int grid, cudaStream_t st, WaitTest wt,
+int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const V* inv,
+                     V* b, V* zbuf, int* flags, int& epoch, int* err, int grid, cudaStream_t st, WaitTest wt,
                      const int* gate) {
-  const int npan = B.npan();
-  const int* ps = B.d_ps;
-  void* args[] = {(void*)&ab,    (void*)&L,    (void*)&ps,    (void*)&npan,  (void*)&perm_all, (void*)&inv,
-                  (void*)&b,     (void*)&zbuf, (void*)&flags, (void*)&epoch, (void*)&err, (void*)&wt, (void*)&gate};
-  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)blk_forward_coop_kernel<T, V>,
-                                                    dim3(std::min(grid, npan)), dim3(256), args, 0, st);
-  return e == cudaSuccess ? 0 : -1;
+  int kl = L.kl;
+  auto launch = [&](BlkSpan s0, BlkSpan s1, int split, int ctas) {
+    ++epoch;
+    void* args[] = {(void*)&ab, (void*)&kl,   (void*)&s0,    (void*)&s1,    (void*)&split, (void*)&perm_all, (void*)&inv,
+                    (void*)&b,  (void*)&zbuf, (void*)&flags, (void*)&epoch, (void*)&err,   (void*)&wt,       (void*)&gate};
+    return cudaLaunchCooperativeKernel((const void*)blk_forward_coop_kernel<T, V>, dim3(ctas), dim3(256), args, 0, st);
+  };
+  if (!two) return coop_spans(launch, BlkSpan{B.one, 0, B.one.npan}, nullptr, grid);
+  const BlkSpan s1{B.two[1], 0, B.two[1].npan};
+  const int r1 = coop_spans(launch, BlkSpan{B.two[0], 0, B.pm}, &s1, grid);
+  if (r1 < 0) return r1;
+  const int lo = std::max(0, B.mid - L.kl);
+  blk_forward_mid_kernel<T, V><<<(B.mid - lo + 7) / 8, 256, 0, st>>>(ab, L, B.mid, lo, b, gate);
+  const int r2 = coop_spans(launch, BlkSpan{B.two[0], B.pm, B.two[0].npan}, nullptr, grid);
+  return r2 < 0 ? r2 : r1 + 1 + r2;
 }
 // CTAs of the cooperative back substitution that can be resident at once
 template <class V, class T>
@@ -666,25 +774,23 @@ template void blk_forward<double, double>(const double*, const BandLayout&, cons
                                           double*, cudaStream_t);
 template void blk_forward<double, float>(const float*, const BandLayout&, const BlkPlan&, const int*, const float*,
                                          double*, cudaStream_t);
-template void blk_inverses<double, double>(const double*, const BandLayout&, const BlkPlan&, const double*, double*,
-                                           cudaStream_t);
-template void blk_inverses<double, float>(const float*, const BandLayout&, const BlkPlan&, const float*, double*,
-                                          cudaStream_t);
-template int blk_backward<double, double>(const double*, const BandLayout&, const BlkPlan&, double*, int*, int, int*,
-                                          int, cudaStream_t, WaitTest, const int*);
-template int blk_backward<double, float>(const float*, const BandLayout&, const BlkPlan&, double*, int*, int, int*,
-                                         int, cudaStream_t, WaitTest, const int*);
+template int blk_inverses<double, double>(const double*, const BlkPlan&, bool, const double*, double*, cudaStream_t);
+template int blk_inverses<double, float>(const float*, const BlkPlan&, bool, const float*, double*, cudaStream_t);
+template int blk_backward<double, double>(const double*, const BlkPlan&, bool, double*, int*, int&, int*, int,
+                                          cudaStream_t, WaitTest, const int*);
+template int blk_backward<double, float>(const float*, const BlkPlan&, bool, double*, int*, int&, int*, int,
+                                         cudaStream_t, WaitTest, const int*);
 template void blk_backward_1cta<double, double>(const double*, const BandLayout&, const BlkPlan&, double*,
                                                 cudaStream_t);
 template void blk_backward_1cta<double, float>(const float*, const BandLayout&, const BlkPlan&, double*,
                                                cudaStream_t);
 template int blk_backward_grid<double, double>();
 template int blk_backward_grid<double, float>();
-template int blk_forward_coop<double, double>(const double*, const BandLayout&, const BlkPlan&, const int*,
-                                              const double*, double*, double*, int*, int, int*, int, cudaStream_t,
+template int blk_forward_coop<double, double>(const double*, const BandLayout&, const BlkPlan&, bool, const int*,
+                                              const double*, double*, double*, int*, int&, int*, int, cudaStream_t,
                                               WaitTest, const int*);
-template int blk_forward_coop<double, float>(const float*, const BandLayout&, const BlkPlan&, const int*,
-                                             const double*, double*, double*, int*, int, int*, int, cudaStream_t,
+template int blk_forward_coop<double, float>(const float*, const BandLayout&, const BlkPlan&, bool, const int*,
+                                             const double*, double*, double*, int*, int&, int*, int, cudaStream_t,
                                              WaitTest, const int*);
 
 }  // namespace mafem

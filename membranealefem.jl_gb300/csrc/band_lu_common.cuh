@@ -150,9 +150,10 @@ __device__ __forceinline__ bool wait_flag(const int* flags, int p, int epoch, in
 // pivot among the block's rows not yet eliminated, form the multipliers,
 // publish them (shared memory + named-barrier arrive) and record the pivot.
 // Returns the column's final value for this lane: the multiplier below the
-// pivot, the U entry (or the pivot itself) otherwise.
+// pivot, the U entry (or the pivot itself) otherwise.  rdiag: the panel's;
+// col1: 1 + column k's number in the matrix, for info.
 template <class T>
-__device__ __forceinline__ T blk_pivot_step(int k, T col, int w, int lane, int bend, unsigned E, int64_t j0,
+__device__ __forceinline__ T blk_pivot_step(int k, T col, int w, int lane, int bend, unsigned E, int col1,
                                             T (*s_l)[32], int* s_p, int* perm, T* rdiag, int* info, int& op,
                                             T& ol, int nthreads) {
   const int bk = __shfl_sync(kFull, bend, k);  // the block of position k ends at row bk
@@ -171,8 +172,8 @@ __device__ __forceinline__ T blk_pivot_step(int k, T col, int w, int lane, int b
   bar_arrive_n(1 + (k & 1), nthreads);
   if (lane == 0) {
     perm[k] = p;
-    rdiag[j0 + k] = fma(r0, t, r0);
-    if (mx == 0u) atomicCAS(info, 0, (int)(j0 + k + 1));
+    rdiag[k] = fma(r0, t, r0);
+    if (mx == 0u) atomicCAS(info, 0, col1);
   }
   op = p;
   ol = l;
@@ -197,27 +198,30 @@ __device__ __forceinline__ T blk_pivot_step(int k, T col, int w, int lane, int b
 // CG: read the block with L2-only loads (it was written by other CTAs of the
 // same kernel).  NW warps (4: one per sub-partition, so the pivot chain's FP64
 // operations never queue behind a partner warp's).  Uses named barriers 1 and
-// 2 and must be called by exactly the CTA's warps 0 .. NW-1.
+// 2 and must be called by exactly the CTA's warps 0 .. NW-1.  Element (r, c) of
+// the block is at blk[r si + c sj]; blk_end, rdiag: of the panel's first column j0;
+// matrix column of its column c: col1 - 1 + cinc c (for info).
 template <class T, bool CG, int NW = kPanelWarps>
-__device__ __forceinline__ void blk_panel_factor(T* __restrict__ ab, const BandLayout& L, int64_t j0, int w,
+__device__ __forceinline__ void blk_panel_factor(T* __restrict__ blk, int64_t si, int64_t sj, int j0, int w,
+                                                 int col1, int cinc,
                                                  const int* __restrict__ blk_end, int* __restrict__ perm,
                                                  T* __restrict__ rdiag, int* __restrict__ info, T (*s_l)[32],
                                                  int* s_p) {
   const int tid = threadIdx.x, lane = tid & 31, q = tid >> 5;
-  const int bend = lane < w ? (int)(blk_end[j0 + lane] - j0) : 0;
+  const int bend = lane < w ? blk_end[lane] - j0 : 0;
   constexpr int NCOL = 32 / NW;
   T v[NCOL];
 #pragma unroll
   for (int m = 0; m < NCOL; ++m) {
     const int c = q + NW * m;
-    v[m] = (c < w && lane < w) ? ldx<CG>(ab + bix(L, j0 + lane, j0 + c)) : T(0);
+    v[m] = (c < w && lane < w) ? ldx<CG>(blk + lane * si + c * sj) : T(0);
   }
   unsigned E = 0u;  // eliminated rows
   int mypos = 0;
   int op = 0;
   T ol = T(0);  // the step this warp published last: pivot row, multiplier of this lane's row
 
-  if (q == 0) v[0] = blk_pivot_step(0, v[0], w, lane, bend, E, j0, s_l, s_p, perm, rdiag, info, op, ol, 32 * NW);
+  if (q == 0) v[0] = blk_pivot_step(0, v[0], w, lane, bend, E, col1, s_l, s_p, perm, rdiag, info, op, ol, 32 * NW);
   for (int k = 0; k < w; ++k) {
     int p;
     T l;
@@ -237,61 +241,17 @@ __device__ __forceinline__ void blk_panel_factor(T* __restrict__ ab, const BandL
       if (c > k && c < w) {  // warp-uniform
         const T u = __shfl_sync(kFull, v[m], p);
         v[m] = fma(-l, u, v[m]);  // l == 0 on eliminated rows
-        if (c == k + 1) v[m] = blk_pivot_step(k + 1, v[m], w, lane, bend, E, j0, s_l, s_p, perm, rdiag, info, op, ol, 32 * NW);
+        if (c == k + 1)
+          v[m] = blk_pivot_step(k + 1, v[m], w, lane, bend, E, col1 + cinc * (k + 1), s_l, s_p, perm, rdiag, info, op, ol,
+                                32 * NW);
       }
     }
   }
 #pragma unroll
   for (int m = 0; m < NCOL; ++m) {
     const int c = q + NW * m;
-    if (c < w && lane < w) ab[bix(L, j0 + mypos, j0 + c)] = v[m];
+    if (c < w && lane < w) blk[mypos * si + c * sj] = v[m];
   }
-}
-
-
-// Variant of blk_panel_factor with the block in shared memory (P[c][r],
-// 32 x 33): a warp visits its columns with a run-time index, so the pivot
-// step is one call site instead of one per register slot (smaller code, no
-// per-slot branches); the column of the next pivot is still updated first.
-template <class T, bool CG, int NW = kPanelWarps>
-__device__ __forceinline__ void blk_panel_factor_smem(T* __restrict__ ab, const BandLayout& L, int64_t j0, int w,
-                                                      const int* __restrict__ blk_end, int* __restrict__ perm,
-                                                      T* __restrict__ rdiag, int* __restrict__ info, T (*s_l)[32],
-                                                      int* s_p, T (*P)[33]) {
-  const int tid = threadIdx.x, lane = tid & 31, q = tid >> 5;
-  const int bend = lane < w ? (int)(blk_end[j0 + lane] - j0) : 0;
-  for (int c = q; c < w; c += NW) P[c][lane] = lane < w ? ldx<CG>(ab + bix(L, j0 + lane, j0 + c)) : T(0);
-  __syncwarp();
-  unsigned E = 0u;
-  int mypos = 0, op = 0;
-  T ol = T(0);
-  if (q == 0) P[0][lane] = blk_pivot_step(0, P[0][lane], w, lane, bend, E, j0, s_l, s_p, perm, rdiag, info, op, ol,
-                                          32 * NW);
-  for (int k = 0; k < w; ++k) {
-    int p;
-    T l;
-    if (q == k % NW) {
-      p = op;
-      l = ol;
-    } else {
-      bar_sync_n(1 + (k & 1), 32 * NW);
-      p = s_p[k & 1];
-      l = s_l[k & 1][lane];
-    }
-    E |= 1u << p;
-    if (lane == p) mypos = k;
-    // my columns > k, the next pivot's first
-    for (int c = k + 1 + (((q - (k + 1)) % NW) + NW) % NW; c < w; c += NW) {
-      const T u = P[c][p];
-      T v = fma(-l, u, P[c][lane]);  // l == 0 on eliminated rows
-      if (c == k + 1) v = blk_pivot_step(k + 1, v, w, lane, bend, E, j0, s_l, s_p, perm, rdiag, info, op, ol, 32 * NW);
-      __syncwarp();
-      P[c][lane] = v;
-      __syncwarp();
-    }
-  }
-  for (int c = q; c < w; c += NW)
-    if (lane < w) ab[bix(L, j0 + mypos, j0 + c)] = P[c][lane];
 }
 
 }  // namespace mafem

@@ -25,13 +25,26 @@
 // epoch that set it, critcnt[t] / a21cnt[t] reach epoch * w(t).  All waits
 // are bounded (kSpinLimit polls) and abort every CTA through *err.
 //
-// L1 coherence.  Bulk copies into shared memory use cp.async (L1-allocating)
-// only for data that no other SM writes after this SM may have cached it: a
-// column's segments (written only by its owner) and the rows below a panel's
-// diagonal block (written only by the owners of the panel's columns).  The
-// diagonal block itself is rewritten by the factorising CTA after the column
-// owners last touched it, so it -- like the pivot data and the flags -- is
-// read with L2-only loads (__ldcg / ld.acquire).
+// From both ends (FP64 with a right-hand side; blk_two_plan).  A panel takes ~24 us of
+// dependent steps however narrow the band is, so the number of panels in a row is
+// what bounds narrow bands, and a band's last unknowns can be eliminated beside its
+// first ones: two chains, each on half of the CTAs with its own factorising CTA,
+// meet in the middle.  The second numbers rows and columns from the last unknown,
+// so it is the same code on descending addresses (its fill and Y lie below the
+// diagonal).  Up to panel pm of the first one the two touch different entries; there
+// all CTAs meet (*bdone) and share the columns of what is left, 2 kuf unknowns.
+// The chain of dependent panels is n / 2 + kuf unknowns long instead of n.  Factor
+// and back substitution, ms per Newton iteration, one chain -> two:
+//   ALEVB 17 x 17 (n 2410, kuf 310)     1.88 + 0.24 -> 1.18 + 0.16
+//   ALEVB 32 x 32 (n 8410, kuf 550)     7.37 + 0.69 -> 6.10 + 0.44
+//   ALEVB 64 x 64 (n 33242, kuf 1062)   98.9 + 5.1  -> 83.4 + 3.4
+// The last two are bound by the FP64 units (1.25 TFLOP/s: 4.0 and 60 ms for the
+// 2 n kl kuf operations): there the gain is that one chain's hand-overs hide behind
+// the other's updates.  A worker has twice the columns while the chains run beside
+// each other (kMaxCols, and eight staged at once where shared memory allows).
+//
+// L1 coherence.  Band entries written by other SMs are read by TMA or with L2-only
+// loads (__ldcg), as are the pivot data; flags with ld.acquire.
 
 #include "band_lu_common.cuh"
 
@@ -42,10 +55,12 @@ namespace {
 template <class T>
 struct PersistArgs {
   T* ab;
-  BandLayout L;
-  const int* ps;
-  int npan, kuf, rmax, wmax;  // rmax = wmax + kl: rows of a staged panel column
-  const int* blk_end;
+  BlkChain c[2];              // TWO: c[0] forward on CTAs [0, split), c[1] backward on the others
+  int split;
+  int n, off, kl, kuf;
+  int rmax, wmax, nslot;      // rmax = wmax + kl: rows of a staged panel column
+  int pm, bdone_target;       // nobody starts on panel pm of c[0] before *bdone reaches the target
+  int* bdone;
   int* perm_all;
   T* rdiag;
   int* info;
@@ -58,7 +73,7 @@ struct PersistArgs {
   long long* trace;  // optional: kTraceSlots device-clock stamps per panel (diagnostics)
 };
 constexpr int kTraceSlots = 12;
-constexpr int kMaxCols = 8;  // columns a worker handles per panel (more: the grid is too small)
+constexpr int kMaxCols = 16;  // columns a worker handles per panel (more: the grid is too small)
 __device__ __forceinline__ void stamp(long long* trace, int t, int slot) {
   if (trace && threadIdx.x == 0) {
     long long v;
@@ -87,62 +102,71 @@ __device__ __forceinline__ bool wait_geq(const int* p, int target, int* err, int
 
 }  // namespace
 
-template <class T>
-__global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<T> a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+enum Role { kWorker, kRhs, kFactor };
+// Panels [p0, p1) of one chain by one CTA: worker `me` of GW, the CTA of the
+// right-hand side or the factorising one.  REV: the chain that eliminates from the
+// last unknown; rows and columns are numbered in the chain's order, so row i of a
+// column (and of its copy in shared memory) lies at a descending address.  false
+// after a wait ran out.
+template <class T, bool REV, bool TWO>
+__device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const BlkChain& C, int p0, int p1, int me, int GW,
+                                               Role role, unsigned char* smem_raw, uint64_t* s_bar, uint32_t& ph0,
+                                               uint32_t& ph1) {
+  constexpr int SG = REV ? -1 : 1;  // address step from a row to the next
   __shared__ T s_l[2][32];
   __shared__ int s_p[2];
   __shared__ int s_ok;
-  __shared__ int64_t s_col[kMaxCols];  // this panel's columns (-1: the right-hand side)
-  __shared__ T s_part[4][32];          // partial sums of the critical rows
-  const BandLayout& L = a.L;
-  // CTA G-1 factorises; with a right-hand side CTA G-2 carries it alone (its
-  // extra column would otherwise make one worker late every few panels);
-  // CTAs 0 .. GW-1 own the columns.
-  const int G = gridDim.x, me = blockIdx.x, GW = G - 1 - (a.rhs ? 1 : 0);
-  const bool rhs_cta = a.rhs != nullptr && me == G - 2;
+  __shared__ int s_col[kMaxCols];  // this panel's columns (-1: the right-hand side)
+  __shared__ T s_part[4][32];      // partial sums of the critical rows
+  const int* __restrict__ ps = C.ps;
+  const int npan = C.npan;
+  const int64_t sj = C.sj;
+  T* const ab = a.ab + C.org;                             // element (i, j) at ab[i SG + j sj]
+  T* const rhs = a.rhs ? a.rhs + C.vorg : nullptr;        // element i at rhs[i SG]
+  int* const pdone = a.pdone + C.pbase;
+  int* const critcnt = a.critcnt + C.pbase;
+  int* const a21cnt = a.a21cnt + C.pbase;
+  int* const perm_all = a.perm_all + (size_t)C.pbase * kBlkW;
+  T* const rdiag = a.rdiag + C.rbase;
+  const bool rhs_cta = role == kRhs;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-  if (me == G - 1) {  // the factorising CTA
-    for (int t = 0; t < a.npan; ++t) {
-      const int wt = a.ps[t + 1] - a.ps[t];
+  if (role == kFactor) {
+    for (int t = p0; t < p1; ++t) {
+      const int j0 = ps[t], wt = ps[t + 1] - j0;
       stamp(a.trace, t, 0);
-      if (t > 0 && !wait_geq(a.critcnt + t, a.epoch * wt, a.err, &s_ok)) return;
+      if (t > 0 && !wait_geq(critcnt + t, a.epoch * wt, a.err, &s_ok)) return false;
       stamp(a.trace, t, 1);
-      blk_panel_factor<T, true>(a.ab, L, a.ps[t], wt, a.blk_end, a.perm_all + (size_t)t * kBlkW, a.rdiag, a.info,
-                                s_l, s_p);
+      blk_panel_factor<T, true>(ab + j0 * SG + j0 * sj, SG, sj, j0, wt, REV ? a.n - j0 : j0 + 1, SG, C.blk_end + j0,
+                                perm_all + (size_t)t * kBlkW, rdiag + j0, a.info, s_l, s_p);
       fence_proxy_async_global();  // the factors are read by TMA on other SMs
       __threadfence();
       __syncthreads();
-      if (tid == 0) st_release(a.pdone + t, a.epoch);
+      if (tid == 0) st_release(pdone + t, a.epoch);
       stamp(a.trace, t, 2);
     }
-    return;
+    return true;
   }
 
   // Shared memory.  Column slots of LDp elements: the panel's w columns (Lp)
-  // and four column segments (S).  A segment starting at global element index
+  // and nslot column segments (S).  A segment starting at global element index
   // g is placed at slot offset g mod E (E elements = 16 bytes), so that its
   // 16-byte-aligned global elements land 16-byte-aligned in shared memory and
   // the bulk of it can be one TMA copy (cp.async.bulk); the at most E - 1
   // elements before and after the aligned bulk are loaded directly.
   constexpr int E = 16 / (int)sizeof(T);
   const int LDp = (a.rmax + 2 * E - 1) / E * E;
-  T* Lp = reinterpret_cast<T*>(smem_raw);             // [kBlkW][LDp] (+64: chunk reads past R)
-  T* S = Lp + (size_t)a.wmax * LDp + 64;              // [4][LDp] column segments
-  T* Y = S + (size_t)4 * LDp;                         // [4][32]
-  T* rd = Y + 128;                                    // [32]
+  T* Lp = reinterpret_cast<T*>(smem_raw) + (TWO ? 64 : 0);  // [kBlkW][LDp] (64 around it: chunk reads past R)
+  T* S = Lp + (size_t)a.wmax * LDp + 64;              // [nslot][LDp] column segments
+  T* Y = S + (size_t)a.nslot * LDp;                   // [nslot][32]
+  T* rd = Y + a.nslot * 32;                           // [32]
   int* sp = reinterpret_cast<int*>(rd + 32);          // [32]
-  __shared__ __align__(8) uint64_t s_bar[2];          // TMA completion: [0] tops, [1] the panel's A21
-  __shared__ int s_sb[4];                             // S slot offsets
-  if (tid == 0) {
-    mbar_init(&s_bar[0], 1);
-    mbar_init(&s_bar[1], 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
-  uint32_t ph0 = 0, ph1 = 0;
-  auto lpa = [&](int k) -> T* { return Lp + (size_t)k * LDp + ((L.off - k) & (E - 1)); };  // panel column k, row 0
+  __shared__ int s_sb[8];                             // row 0 of the segments, from S
+  int R = 0;  // rows of the current panel's columns
+  // panel column k, row 0 (row r: SG r further)
+  auto lpa = [&](int k) -> T* {
+    return REV ? Lp + k * LDp + ((a.off + k - R + 1) & (E - 1)) + R - 1 : Lp + k * LDp + ((a.off - k) & (E - 1));
+  };
   // Copy of n elements src[0..n) -> dst[0..n) (same address phase mod 16 bytes): mode 0 returns the bytes
   // of the aligned bulk, mode 1 issues it as one TMA copy on `bar`, mode 2 loads the unaligned head and
   // tail (at most E - 1 elements each) directly -- after every TMA copy is in flight.
@@ -178,23 +202,23 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
     return __syncthreads_and(ok) != 0;
   };
 
-  for (int p = 0; p < a.npan; ++p) {
-    const int64_t j0 = a.ps[p], j1 = a.ps[p + 1];
-    const int w = (int)(j1 - j0);
-    const int R = (int)min64b(L.n - j0, (int64_t)w + L.kl);
-    const int64_t jend = min64b(L.n, j1 + a.kuf);
-    const int64_t jn = p + 1 < a.npan ? a.ps[p + 2] : j1;  // panel p + 1 = columns [j1, jn)
-    const int64_t cend = jend > jn ? jend : jn;
+  for (int p = p0; p < p1; ++p) {
+    const int j0 = ps[p], j1 = ps[p + 1];
+    const int w = j1 - j0;
+    R = min(C.n - j0, w + a.kl);
+    const int jend = min(C.n, j1 + a.kuf);
+    const int jn = p + 1 < npan ? ps[p + 2] : j1;  // panel p + 1 = columns [j1, jn)
+    const int cend = max(jend, jn);
     const bool is_rhs = rhs_cta;
-    const int64_t cfirst = rhs_cta ? cend : j1 + (((me - j1) % GW) + GW) % GW;
+    const int cfirst = rhs_cta ? cend : j1 + (((me - j1) % GW) + GW) % GW;
     if (cfirst >= cend && !is_rhs) continue;
-    const bool tr_owner = p + 1 < a.npan && me == j1 % GW;
+    const bool tr_owner = !TWO && p + 1 < npan && me == j1 % GW;
     if (tr_owner) stamp(a.trace, p + 1, 3);
     if (p > 0) {
-      if (!wait_geq(a.pdone + p, a.epoch, a.err, &s_ok)) return;
-      if (!wait_geq(a.a21cnt + p, a.epoch * w, a.err, &s_ok)) return;
-    } else if (!wait_geq(a.pdone, a.epoch, a.err, &s_ok)) {
-      return;
+      if (!wait_geq(pdone + p, a.epoch, a.err, &s_ok)) return false;
+      if (!wait_geq(a21cnt + p, a.epoch * w, a.err, &s_ok)) return false;
+    } else if (!wait_geq(pdone, a.epoch, a.err, &s_ok)) {
+      return false;
     }
     if (tr_owner) stamp(a.trace, p + 1, 4);
     const int nch = (R - w + 31) / 32;  // 32-row chunks below the diagonal block
@@ -203,9 +227,9 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
     const int ncol = nown + (is_rhs ? 1 : 0);
     if (ncol > kMaxCols || (nown > 1 && cfirst + GW < jn)) {  // grid too small (the host setup rules this out)
       if (tid == 0) atomicCAS(a.err, 0, 2);
-      return;
+      return false;
     }
-    if (tid < nown) s_col[tid] = cfirst + (int64_t)tid * GW;
+    if (tid < nown) s_col[tid] = cfirst + tid * GW;
     if (tid == 0 && is_rhs) s_col[nown] = -1;
     fence_proxy_async_smem();  // earlier reads / writes of the buffers before the TMA writes below
     __syncthreads();
@@ -219,24 +243,30 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
       T* sd = nullptr;
       const T* ss = nullptr;
       if (lane < nb) {
-        const int64_t c = s_col[b0 + lane];
-        ss = c < 0 ? a.rhs + j0 : a.ab + bix(L, j0, c);
+        const int c = s_col[b0 + lane];
+        ss = c < 0 ? rhs + j0 * SG : ab + j0 * SG + c * sj;
+        if (REV) ss -= R - 1;  // the segment's lowest address
         const int off = (int)(((uintptr_t)ss / sizeof(T)) & (E - 1));
-        s_sb[lane] = lane * LDp + off;
+        s_sb[lane] = lane * LDp + off + (REV ? R - 1 : 0);
         sd = S + lane * LDp + off;
       }
       const bool pc = with_panel && lane < w;
-      const T* pd_src = pc ? a.ab + bix(L, j0, j0 + lane) : nullptr;
+      const T* pd_src = pc ? ab + j0 * SG + (j0 + lane) * sj : nullptr;
       // rows [0, P1) of panel column `lane` (diagonal block + chunk 0, the rows the
       // next factorisation's update reads) on s_bar[0], rows [P1, R) on s_bar[1];
-      // P1 = first 16-byte-aligned row at or after w + 32
+      // P1 = first row at or after w + 32 that 16-byte-aligned copies can start at
+      // (REV: that they can end before)
       const int br = min(R, w + 32);
-      const int P1 = min(R, br + (int)((-(L.off - lane + br)) & (E - 1)));
+      const int P1 = min(R, br + (REV ? (a.off + lane + 1 - br) & (E - 1) : (-(a.off - lane + br)) & (E - 1)));
+      T* const pt = REV ? lpa(lane) - (P1 - 1) : lpa(lane);            // rows [0, P1)
+      const T* const pt_src = REV ? pd_src - (P1 - 1) : pd_src;
+      T* const pb = REV ? lpa(lane) - (R - 1) : lpa(lane) + P1;        // rows [P1, R)
+      const T* const pb_src = REV ? pd_src - (R - 1) : pd_src + P1;
       uint32_t b0b = 0, b1b = 0;
       if (lane < nb) b0b += seg_copy(sd, ss, R, &s_bar[0], 0);
       if (pc) {
-        b0b += seg_copy(lpa(lane), pd_src, P1, &s_bar[0], 0);
-        if (R > P1) b1b += seg_copy(lpa(lane) + P1, pd_src + P1, R - P1, &s_bar[1], 0);
+        b0b += seg_copy(pt, pt_src, P1, &s_bar[0], 0);
+        if (R > P1) b1b += seg_copy(pb, pb_src, R - P1, &s_bar[1], 0);
       }
       for (int o = 16; o > 0; o >>= 1) {
         b0b += __shfl_xor_sync(kFull, b0b, o);
@@ -250,40 +280,40 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
       for (int mode = 1; mode <= 2; ++mode) {
         if (lane < nb) seg_copy(sd, ss, R, &s_bar[0], mode);
         if (pc) {
-          seg_copy(lpa(lane), pd_src, P1, &s_bar[0], mode);
-          if (R > P1) seg_copy(lpa(lane) + P1, pd_src + P1, R - P1, &s_bar[1], mode);
+          seg_copy(pt, pt_src, P1, &s_bar[0], mode);
+          if (R > P1) seg_copy(pb, pb_src, R - P1, &s_bar[1], mode);
         }
       }
     };
-    issue_cols(0, min(4, ncol), true);
+    issue_cols(0, min(a.nslot, ncol), true);
     if (tid >= 32 && tid < 32 + w) {
-      rd[tid - 32] = __ldcg(a.rdiag + j0 + tid - 32);
-      sp[tid - 32] = __ldcg(a.perm_all + (size_t)p * kBlkW + tid - 32);
+      rd[tid - 32] = __ldcg(rdiag + j0 + tid - 32);
+      sp[tid - 32] = __ldcg(perm_all + (size_t)p * kBlkW + tid - 32);
     }
-    if (!wait_bar(&s_bar[0], ph0)) return;  // tops + diagonal block
+    if (!wait_bar(&s_bar[0], ph0)) return false;  // tops + diagonal block
     if (tr_owner) stamp(a.trace, p + 1, 5);
 
-    for (int b0 = 0; b0 < ncol; b0 += 4) {
-      const int nb = min(4, ncol - b0);
+    for (int b0 = 0; b0 < ncol; b0 += a.nslot) {
+      const int nb = min(a.nslot, ncol - b0);
       if (b0 > 0) {  // later batches (small grids only)
         fence_proxy_async_smem();
         __syncthreads();
         issue_cols(b0, nb, false);
-        if (!wait_bar(&s_bar[0], ph0)) return;
+        if (!wait_bar(&s_bar[0], ph0)) return false;
       }
       // triangular solves, one warp per column: u = L11^-1 P s[0:w], y = U11^-1 u (kept as Y in place of A12)
-      if (warp < 4) {
+      if (warp < a.nslot) {
         T v = T(0);
         if (warp < nb) {
-          const int64_t c = s_col[b0 + warp];
+          const int c = s_col[b0 + warp];
           const T* s = S + s_sb[warp];
-          T* dst = c < 0 ? a.rhs + j0 : a.ab + bix(L, j0, c);
+          T* dst = c < 0 ? rhs + j0 * SG : ab + j0 * SG + c * sj;
           // this lane's row of the diagonal block in registers (no shared-memory
           // load on the dependency chains): L(lane, k) for k < lane, U(lane, k) for k > lane
           T Tr[32];
 #pragma unroll
-          for (int k = 0; k < 32; ++k) Tr[k] = (k < w && lane < w) ? lpa(k)[lane] : T(0);
-          T x = lane < w ? s[sp[lane]] : T(0);  // row `lane` of the permuted top
+          for (int k = 0; k < 32; ++k) Tr[k] = (k < w && lane < w) ? lpa(k)[lane * SG] : T(0);
+          T x = lane < w ? s[sp[lane] * SG] : T(0);  // row `lane` of the permuted top
 #pragma unroll
           for (int k = 0; k < 32; ++k) {
             if (k < w) {
@@ -305,7 +335,7 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
               if (lane < k) v = fma(-Tr[k], yk, v);
             }
           }
-          if (lane < w) dst[lane] = v;  // Y (the right-hand side: z); not read again by this kernel
+          if (lane < w) dst[lane * SG] = v;  // Y (the right-hand side: z); not read again by this kernel
         }
         Y[warp * 32 + lane] = (warp < nb && lane < w) ? v : T(0);
       }
@@ -319,12 +349,12 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
           const int r = w + 32 * ci + lane;
           const T* s = S + s_sb[qq];
           const T* yq = Y + qq * 32;
-          T acc = s[min(r, R - 1)];
-          for (int k = 0; k < w; ++k) acc = fma(-lpa(k)[r], yq[k], acc);
+          T acc = s[min(r, R - 1) * SG];
+          for (int k = 0; k < w; ++k) acc = fma(-lpa(k)[r * SG], yq[k], acc);
           if (r < R) {
-            const int64_t c = s_col[b0 + qq];
-            T* dst = c < 0 ? a.rhs + j0 : a.ab + bix(L, j0, c);
-            dst[r] = acc;
+            const int c = s_col[b0 + qq];
+            T* dst = c < 0 ? rhs + j0 * SG : ab + j0 * SG + c * sj;
+            dst[r * SG] = acc;
           }
         }
         fence_proxy_async_global();  // these rows are read by TMA later
@@ -337,32 +367,85 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
           const int r = w + lane;
           if (warp < 4) {
             T part = T(0);
-            for (int k = 8 * warp; k < min(w, 8 * warp + 8); ++k) part = fma(-lpa(k)[r], Y[k], part);
+            for (int k = 8 * warp; k < min(w, 8 * warp + 8); ++k) part = fma(-lpa(k)[r * SG], Y[k], part);
             s_part[warp][lane] = part;
           }
           __syncthreads();
           if (warp == 0 && r < R) {
-            T* dst = a.ab + bix(L, j0, s_col[0]);
-            dst[r] = S[s_sb[0] + min(r, R - 1)] +
+            T* dst = ab + j0 * SG + s_col[0] * sj;
+            dst[r * SG] = S[s_sb[0] + min(r, R - 1) * SG] +
                      ((s_part[0][lane] + s_part[1][lane]) + (s_part[2][lane] + s_part[3][lane]));
           }
           __threadfence();  // read by the factorising CTA with L2-only loads (and rewritten by it before any TMA read)
           __syncthreads();
         }
-        if (tid == 0) atomicAdd(a.critcnt + p + 1, 1);
+        if (tid == 0) atomicAdd(critcnt + p + 1, 1);
         if (tr_owner) stamp(a.trace, p + 1, 7);
-        if (!wait_bar(&s_bar[1], ph1)) return;  // the rest of A21
+        if (!wait_bar(&s_bar[1], ph1)) return false;  // the rest of A21
         if (reach) {
           rows(0, 1, min(1, nch), nch);
           __threadfence();
           __syncthreads();
         }
-        if (tid == 0) atomicAdd(a.a21cnt + p + 1, 1);
+        if (tid == 0) atomicAdd(a21cnt + p + 1, 1);
         if (tr_owner) stamp(a.trace, p + 1, 8);
         q0 = 1;
       }
-      if (b0 == 0 && q0 == 0 && !wait_bar(&s_bar[1], ph1)) return;  // the rest of A21
+      if (b0 == 0 && q0 == 0 && !wait_bar(&s_bar[1], ph1)) return false;  // the rest of A21
       if (q0 < nb) rows(q0, nb, 0, nch);
+    }
+  }
+  return true;
+}
+
+// With a right-hand side the last CTA but one of a chain carries it alone (its extra
+// column would otherwise make one worker late every few panels); the last factorises.
+template <class T, bool TWO>
+__global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t s_bar[2];  // TMA completion: [0] tops, [1] the panel's A21
+  const int G = (int)gridDim.x;
+  int me = blockIdx.x;
+  if (threadIdx.x == 0) {
+    mbar_init(&s_bar[0], 1);
+    mbar_init(&s_bar[1], 1);
+    mbar_init_fence();
+  }
+  __syncthreads();
+  uint32_t ph0 = 0, ph1 = 0;
+  if constexpr (!TWO) {
+    const int GW = G - 1 - (a.rhs ? 1 : 0);
+    persist_panels<T, false, false>(a, a.c[0], 0, a.c[0].npan, me, GW,
+                                    me == G - 1 ? kFactor : a.rhs && me == G - 2 ? kRhs : kWorker, smem_raw, s_bar, ph0,
+                                    ph1);
+  } else {
+    __shared__ int s_ok;
+    // first each chain on its own CTAs, the forward one up to panel pm, then the rest on all of them
+    const bool rev = me >= a.split;
+    const int G0 = rev ? G - a.split : a.split;
+    if (rev) me -= a.split;
+    Role role = me == G0 - 1 ? kFactor : me == G0 - 2 ? kRhs : kWorker;
+    if (rev) {
+      if (!persist_panels<T, true, true>(a, a.c[1], 0, a.c[1].npan, me, G0 - 2, role, smem_raw, s_bar, ph0, ph1)) return;
+    }
+#pragma unroll 1
+    for (int half = rev || role == kFactor ? 1 : 0; half < 2; ++half) {
+      if (half == 1 && (rev || role != kFactor)) {
+        // the columns change hands, and each side reads what the other one updated
+        fence_proxy_async_global();
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) atomicAdd(a.bdone, 1);
+        if (!wait_geq(a.bdone, a.bdone_target, a.err, &s_ok)) return;
+        if (rev) {
+          role = kWorker;
+          me += a.split - 2;
+        }
+      }
+      const int p0 = half == 1 && role != kFactor ? a.pm : 0, p1 = half == 0 ? a.pm : a.c[0].npan;
+      if (!persist_panels<T, false, true>(a, a.c[0], p0, p1, me, half == 0 ? a.split - 2 : G - 2, role, smem_raw, s_bar,
+                                          ph0, ph1))
+        return;
     }
   }
 }
@@ -370,75 +453,105 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
 // ---------------------------------------------------------------------------
 // host side
 template <class T>
-static size_t persist_smem(const BandLayout& L, int wmax) {
+static size_t persist_smem(const BandLayout& L, int wmax, int nslot, bool two) {
   constexpr int E = 16 / (int)sizeof(T);
   const size_t rmax = (size_t)wmax + L.kl;
   const size_t ldp = (rmax + 2 * E - 1) / E * E;
-  return ((size_t)wmax * ldp + 64 + 4 * ldp + 128 + 32) * sizeof(T) + 32 * sizeof(int);
+  return ((two ? 64 : 0) + (size_t)wmax * ldp + 64 + nslot * (ldp + 32) + 32) * sizeof(T) + 32 * sizeof(int);
+}
+
+template <class T, bool TWO>
+static bool persist_fits(size_t sm) {
+  int per = 0;
+  return cudaFuncSetAttribute(blk_factor_persist_kernel<T, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) ==
+             cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, blk_factor_persist_kernel<T, TWO>, 256, sm) ==
+             cudaSuccess &&
+         per >= 1;
 }
 
 template <class T>
 int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
-  int dev = 0, sms = 0, cap = 0, per = 0;
+  int dev = 0, sms = 0, cap = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   int coop = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  const size_t sm = persist_smem<T>(L, B.wmax);
-  if (!coop || sm + 12 * 1024 > (size_t)cap || B.wmax > kBlkW) return 0;  // + static shared memory
-  if (cudaFuncSetAttribute(blk_factor_persist_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
-      cudaSuccess)
-    return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, blk_factor_persist_kernel<T>, 256, sm) != cudaSuccess ||
-      per < 1)
-    return 0;
-  // workers need at most kMaxCols columns each per panel (columns c of the
+  S.smem = persist_smem<T>(L, B.wmax, 4, false);
+  if (!coop || S.smem + 12 * 1024 > (size_t)cap || B.wmax > kBlkW) return 0;  // + static shared memory
+  if (!persist_fits<T, false>(S.smem)) return 0;
+  // workers need at most kMinCols columns each per panel (columns c of the
   // trailing range, owned by c mod (G - 1), plus the right-hand side)
+  constexpr int kMinCols = 8;
   S.grid = sms;
-  // workers: <= kMaxCols columns each per panel, and at least one per column of
+  // workers: <= kMinCols columns each per panel, and at least one per column of
   // the widest panel (a worker owns at most one column of the next panel);
   // + the right-hand-side CTA + the factorising CTA
-  S.min_grid = std::max((int)((B.kuf + B.wmax + 1 + kMaxCols - 1) / kMaxCols), B.wmax) + 2;
+  S.min_grid = std::max((int)((B.kuf + B.wmax + 1 + kMinCols - 1) / kMinCols), B.wmax) + 2;
   if (S.grid < S.min_grid) return S.grid = 0;
   S.max_grid = S.grid;
-  S.smem = sm;
+  // two chains: each on half of the CTAs, a worker with up to kMaxCols columns per panel
+  S.min_two = 0;
+  if constexpr (sizeof(T) == 8) {
+    for (int nslot : {8, 4}) {
+      if (!B.has_two) break;
+      S.nslot2 = nslot;
+      S.smem2 = persist_smem<T>(L, B.wmax, nslot, true);
+      if (S.smem2 + 12 * 1024 <= (size_t)cap && persist_fits<T, true>(S.smem2)) {
+        S.min_two = 2 * (std::max((int)((B.kuf + B.wmax + 1 + kMaxCols - 1) / kMaxCols), B.wmax) + 2);
+        break;
+      }
+    }
+    cudaGetLastError();
+  }
   return S.grid;
 }
 
 template <class T>
-int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, const BlkPersist& S, int epoch, int* perm_all,
+int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersist& S, bool two, int* perm_all,
                           T* rdiag, int* info, T* rhs, int* err, cudaStream_t st, long long* trace) {
   PersistArgs<T> a;
   a.ab = ab;
-  a.L = L;
-  a.ps = B.d_ps;
-  a.npan = B.npan();
+  a.c[0] = two ? B.two[0] : B.one;
+  a.c[1] = B.two[1];
+  const int after = two ? B.npan() : 0;  // the two chains' flags stand after the one chain's
+  a.split = two ? (S.grid + 1) / 2 : S.grid;
+  a.n = (int)L.n;
+  a.off = (int)L.off;
+  a.kl = L.kl;
   a.kuf = B.kuf;
   a.rmax = B.wmax + (int)L.kl;
   a.wmax = B.wmax;
-  a.blk_end = B.d_blk_end;
+  a.nslot = two ? S.nslot2 : 4;
+  a.pm = B.pm;
+  a.bdone = S.d_bdone;
+  a.bdone_target = S.bdone + S.grid - 1;  // all CTAs but the forward chain's factorising one
   a.perm_all = perm_all;
   a.rdiag = rdiag;
   a.info = info;
   a.rhs = rhs;
-  a.pdone = S.d_pdone;
-  a.critcnt = S.d_critcnt;
-  a.a21cnt = S.d_a21cnt;
-  a.epoch = epoch;
+  a.pdone = S.d_pdone + after;
+  a.critcnt = S.d_critcnt + after;
+  a.a21cnt = S.d_a21cnt + after;
+  a.epoch = S.epoch[two] + 1;
   a.err = err;
-  a.trace = trace;
+  a.trace = two ? nullptr : trace;
   void* args[] = {(void*)&a};
-  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)blk_factor_persist_kernel<T>, dim3(S.grid),
-                                                    dim3(256), args, S.smem, st);
-  return e == cudaSuccess ? 1 : -1;
+  const void* fn = (const void*)blk_factor_persist_kernel<T, false>;
+  if constexpr (sizeof(T) == 8)
+    if (two) fn = (const void*)blk_factor_persist_kernel<T, true>;
+  if (cudaLaunchCooperativeKernel(fn, dim3(S.grid), dim3(256), args, two ? S.smem2 : S.smem, st) != cudaSuccess) return -1;
+  S.epoch[two] = a.epoch;
+  if (two) S.bdone = a.bdone_target;
+  return 1;
 }
 
 template int blk_persist_setup<double>(const BandLayout&, const BlkPlan&, BlkPersist&);
 template int blk_persist_setup<float>(const BandLayout&, const BlkPlan&, BlkPersist&);
-template int blk_lu_factor_persist<double>(double*, const BandLayout&, const BlkPlan&, const BlkPersist&, int, int*,
-                                           double*, int*, double*, int*, cudaStream_t, long long*);
-template int blk_lu_factor_persist<float>(float*, const BandLayout&, const BlkPlan&, const BlkPersist&, int, int*,
-                                          float*, int*, float*, int*, cudaStream_t, long long*);
+template int blk_lu_factor_persist<double>(double*, const BandLayout&, const BlkPlan&, BlkPersist&, bool, int*, double*,
+                                           int*, double*, int*, cudaStream_t, long long*);
+template int blk_lu_factor_persist<float>(float*, const BandLayout&, const BlkPlan&, BlkPersist&, bool, int*, float*,
+                                          int*, float*, int*, cudaStream_t, long long*);
 
 }  // namespace mafem

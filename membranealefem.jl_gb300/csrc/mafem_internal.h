@@ -1,6 +1,7 @@
 // mafem_internal.h -- internal types shared by the library's translation units.
 #pragma once
 
+#include <algorithm>
 #include <array>
 #include <cstdint>
 #include <string>
@@ -119,8 +120,8 @@ template <class T>
 cudaError_t launch_elem(const DevPatch& P, const PhysParams& pp, double time, double dt, double* r_el, T* K_el,
                         cudaStream_t st, const int* elist = nullptr, int nlist = 0, int area_only = 0);
 template <class T>
-// kuf: super-diagonals the factorisation fills (gather_column)
-void launch_band_gather(const DevPatch& P, int ndf, int nq, const BandLayout& L, int kuf, const T* K_el, T* ab,
+// kuf: super-diagonals the factorisation fills, klf: rows below the diagonal it does (gather_column)
+void launch_band_gather(const DevPatch& P, int ndf, int nq, const BandLayout& L, int kuf, int klf, const T* K_el, T* ab,
                         cudaStream_t st, T* ab2 = nullptr);
 void launch_resid_gather(const DevPatch& P, int ndf, int nq, const double* r_el, double* r, cudaStream_t st);
 void launch_predictor(const DevPatch& P, const PhysParams& pp, double dt, cudaStream_t st);
@@ -170,6 +171,19 @@ void band_backward(const T* ab, const BandLayout& L, V* y, cudaStream_t st);
 // node-block pivoted banded LU (band_lu_blk.cu).  Panels are runs of whole
 // pivot blocks (the unknowns of one control point), at most wmax <= 32 wide.
 constexpr int kBlkW = 32;  // widest panel; also the stride of the per-panel permutations
+// One elimination order over (part of) the unknowns: its numbering of the band's
+// rows and columns, and its panels.  The forward chain numbers them as the band
+// does; the backward chain from the last unknown down.
+struct BlkChain {
+  int64_t org = 0, si = 1, sj = 0;  // element (i, j) at band[org + i si + j sj]
+  int64_t vorg = 0;                 // element i of a vector at v[vorg + i si]
+  const int* ps = nullptr;          // device panel starts [npan + 1]
+  int npan = 0;
+  int n = 0;                        // its rows and columns: those at or beyond are never touched
+  const int* blk_end = nullptr;     // per unknown: one past the last unknown of its pivot block
+  int pbase = 0;                    // its first panel in the arrays kept per panel (permutations, flags, z, inverses)
+  int rbase = 0;                    // its first unknown in rdiag
+};
 struct BlkPlan {
   int ndfp = 0;          // largest block size - 1
   int wmax = 0;          // widest panel
@@ -177,8 +191,20 @@ struct BlkPlan {
   std::vector<int> ps;   // panel starts; ps.back() == n
   int* d_ps = nullptr;   // device copy of ps
   const int* d_blk_end = nullptr;  // per unknown: one past the last unknown of its block
+  BlkChain one;          // the whole band as one forward chain
+  // The same as two chains (blk_two_plan): two[0] eliminates the unknowns from the
+  // first, two[1] from the last up to unknown mid, beside it; two[0] then goes on
+  // through the rest up to mid, from its panel pm on, once two[1] is done.
+  bool has_two = false;
+  BlkChain two[2];
+  int mid = 0, pm = 0;
   int npan() const { return (int)ps.size() - 1; }
+  int npan_max() const { return has_two ? std::max(npan(), two[0].npan + two[1].npan) : npan(); }
 };
+// Host part of the two-chain plan: panel starts of both chains and the backward
+// chain's block ends (out.mid, out.pm set); false if the band is too short for it.
+bool blk_two_plan(const std::vector<int>& blk_end, const BandLayout& L, BlkPlan& out, std::vector<int>& ps0,
+                  std::vector<int>& ps1, std::vector<int>& blk_end1);
 // Host: panel starts for blocks `blk_end` (false if a block is wider than wmax).
 bool blk_plan(const std::vector<int>& blk_end, int wmax, int ku, BlkPlan& out);
 // Widest panel (<= kBlkW, <= L.nb) whose kernels fit the device's shared memory; 0 if none.
@@ -190,10 +216,11 @@ int blk_lu_factor(T* ab, const BandLayout& L, const BlkPlan& B, int* perm_all, T
 template <class V, class T>
 void blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, const int* perm_all, const T* rdiag, V* b,
                  cudaStream_t st);
-// Back substitution x1 = z - Y x2 in place on many SMs (one cooperative launch of
-// `grid` CTAs, grid <= blk_backward_grid()).  flags: npan ints, epoch: a value
-// they do not hold yet (incremented per call); err: nonzero after a bounded
-// wait ran out.  Returns -1 if the launch failed.
+// Back substitution x1 = z - Y x2 in place on many SMs (cooperative launches of
+// at most `grid` CTAs, grid <= blk_backward_grid()).  flags: npan_max ints; epoch: a
+// value they do not hold yet is taken per launch; err: nonzero after a bounded
+// wait ran out.  two: the factors of the two-chain elimination.  Returns the
+// kernels launched, or -1 if a launch failed.
 // Failure-detection test hook of the cooperative substitutions: limit = polls
 // before a wait gives up (<= 0: the default), withhold = k: the back
 // substitution never publishes the flag of panel npan - 1 - k (-1: none).
@@ -204,26 +231,32 @@ struct WaitTest {
 // Explicit inverses of the stored panels' L11 and U11 (inv: npan x 2 x 32 x
 // 32 in V) for the cooperative forward substitution.
 template <class V, class T>
-void blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, const T* rdiag, V* inv, cudaStream_t st);
+int blk_inverses(const T* ab, const BlkPlan& B, bool two, const T* rdiag, V* inv, cudaStream_t st);
 template <class V, class T>
-int blk_backward(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, int* flags, int epoch, int* err, int grid,
+int blk_backward(const T* ab, const BlkPlan& B, bool two, V* y, int* flags, int& epoch, int* err, int grid,
                  cudaStream_t st, WaitTest wt = WaitTest(), const int* gate = nullptr);
 template <class V, class T>
 int blk_backward_grid();
-// Forward substitution (P, L11, A21 of the stored panels) on `grid` CTAs of one
-// cooperative launch, in place on b; zbuf: npan x 32 scratch; flags/epoch as
-// for blk_backward.  Returns 0, or -1 if the cooperative launch was refused.
+// Forward substitution (P, L11, A21 of the stored panels) on at most `grid` CTAs of
+// cooperative launches, in place on b; zbuf: npan_max x 32 scratch; flags / epoch / two
+// as for blk_backward.  Returns the kernels launched, or -1 if a launch was refused.
 template <class V, class T>
-int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, const int* perm_all, const V* inv, V* b,
-                     V* zbuf, int* flags, int epoch, int* err, int grid, cudaStream_t st, WaitTest wt = WaitTest(),
-                     const int* gate = nullptr);
+int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const V* inv,
+                     V* b, V* zbuf, int* flags, int& epoch, int* err, int grid, cudaStream_t st,
+                     WaitTest wt = WaitTest(), const int* gate = nullptr);
 // Persistent cooperative factorisation (band_lu_persist.cu): launch shape and
-// per-panel flags.  Flags are zeroed once; epochs make them reusable.
+// per-panel flags.  Flags are zeroed once; epochs make them reusable.  The arrays
+// hold the one chain's npan panels, then the two chains'.
 struct BlkPersist {
   int grid = 0;            // CTAs of the launch: min_grid <= grid <= max_grid
   int min_grid = 0;        // fewest CTAs that give every worker <= kMaxCols columns per panel
   int max_grid = 0;        // the device's SM count
-  size_t smem = 0;
+  int min_two = 0;         // fewest CTAs of the two-chain form (0: not available)
+  int nslot2 = 0;          // two chains: columns a worker stages at once
+  size_t smem = 0, smem2 = 0;  // shared memory as one chain, as two
+  int epoch[2] = {0, 0};   // factorisations so far: as one chain, as two
+  int bdone = 0;           // *d_bdone once the last two-chain factorisation is done
+  int* d_bdone = nullptr;  // counts the CTAs that are done with what the two chains do apart
   int* d_pdone = nullptr;
   int* d_critcnt = nullptr;
   int* d_a21cnt = nullptr;
@@ -240,7 +273,8 @@ template <class T>
 // solved, [7] the rows t reads are written, [8] the rest of the rows,
 // [9] its column copies are issued, [10] the A21 copies are issued, [11] the
 // diagonal block is in shared memory.
-int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, const BlkPersist& S, int epoch, int* perm_all,
+// two: eliminate from both ends (needs B.has_two, a right-hand side and grid >= min_two).
+int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersist& S, bool two, int* perm_all,
                           T* rdiag, int* info, T* rhs, int* err, cudaStream_t st, long long* trace = nullptr);
 template <class V, class T>
 void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, cudaStream_t st);
