@@ -531,7 +531,7 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
       one.n = (int)n;
       one.blk_end = h->d_blk_end;
       std::vector<int> ps0, ps1, blk_end1;
-      if (precision == MAFEM_PLAIN_FP64 && blk_two_plan(blk_end, h->L, h->blk, ps0, ps1, blk_end1)) {
+      if (blk_two_plan(blk_end, h->L, h->blk, ps0, ps1, blk_end1)) {
         h->blk.has_two = true;
         BlkChain &a = h->blk.two[0], &b = h->blk.two[1];
         int *d_ps0 = nullptr, *d_ps1 = nullptr, *d_end1 = nullptr;
@@ -798,7 +798,7 @@ static int factor_enqueue(mafem_handle* h, double* x) {
   bool launched = false;
   if (h->pers.grid > 0 && h->lu_path == MAFEM_LU_AUTO) {
     // from both ends where the grid allows (blk_two_plan)
-    const bool two = fp64 && x && h->pers.min_two > 0 && h->pers.grid >= h->pers.min_two && h->bwd_grid > 0;
+    const bool two = (x || !fp64) && h->pers.min_two > 0 && h->pers.grid >= h->pers.min_two && h->bwd_grid > 0;
     const int nl = fp64 ? blk_lu_factor_persist<double>((double*)h->d_band, h->L, h->blk, h->pers, two, h->d_perm,
                                                         (double*)h->d_rdiag, h->d_info, x, h->d_info + 1, h->st)
                         : blk_lu_factor_persist<float>((float*)h->d_band, h->L, h->blk, h->pers, two, h->d_perm,
@@ -1611,6 +1611,7 @@ static AsmJob asm_job(const mafem_handle* h) {
   a.dir_val = h->d_dir_val;
   a.n_dir = h->n_dir;
   a.kuf = h->blk.kuf;
+  a.klf = fill_rows(h);
   return a;
 }
 

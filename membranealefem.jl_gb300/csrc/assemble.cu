@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(32 * kGatherCols) batch_gather_kernel(const As
   const int k = batch_item(off, m, &s_k);
   const AsmJob& J = jobs[items[k].job];
   const int64_t j = (int64_t)(off[0] + (int)blockIdx.x - off[k]) * kGatherCols + (threadIdx.x >> 5);
-  if (j < J.L.n) gather_column<float>(J.P, J.pp.ndf, J.pp.nq, J.L, J.kuf, J.L.kl, J.K_el, J.band, J.band0, j);
+  if (j < J.L.n) gather_column<float>(J.P, J.pp.ndf, J.pp.nq, J.L, J.kuf, J.klf, J.K_el, J.band, J.band0, j);
 }
 
 // The residual, 256 unknowns per CTA; the patch's first CTA also zeroes its

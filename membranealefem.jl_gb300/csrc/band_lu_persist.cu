@@ -423,10 +423,11 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
     // first each chain on its own CTAs, the forward one up to panel pm, then the rest on all of them
     const bool rev = me >= a.split;
     const int G0 = rev ? G - a.split : a.split;
+    const int nx = a.rhs ? 2 : 1;  // CTAs of a chain that own no columns
     if (rev) me -= a.split;
-    Role role = me == G0 - 1 ? kFactor : me == G0 - 2 ? kRhs : kWorker;
+    Role role = me == G0 - 1 ? kFactor : a.rhs && me == G0 - 2 ? kRhs : kWorker;
     if (rev) {
-      if (!persist_panels<T, true, true>(a, a.c[1], 0, a.c[1].npan, me, G0 - 2, role, smem_raw, s_bar, ph0, ph1)) return;
+      if (!persist_panels<T, true, true>(a, a.c[1], 0, a.c[1].npan, me, G0 - nx, role, smem_raw, s_bar, ph0, ph1)) return;
     }
 #pragma unroll 1
     for (int half = rev || role == kFactor ? 1 : 0; half < 2; ++half) {
@@ -439,11 +440,11 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
         if (!wait_geq(a.bdone, a.bdone_target, a.err, &s_ok)) return;
         if (rev) {
           role = kWorker;
-          me += a.split - 2;
+          me += a.split - nx;
         }
       }
       const int p0 = half == 1 && role != kFactor ? a.pm : 0, p1 = half == 0 ? a.pm : a.c[0].npan;
-      if (!persist_panels<T, false, true>(a, a.c[0], p0, p1, me, half == 0 ? a.split - 2 : G - 2, role, smem_raw, s_bar,
+      if (!persist_panels<T, false, true>(a, a.c[0], p0, p1, me, half == 0 ? a.split - nx : G - nx, role, smem_raw, s_bar,
                                           ph0, ph1))
         return;
     }
@@ -493,18 +494,16 @@ int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
   S.max_grid = S.grid;
   // two chains: each on half of the CTAs, a worker with up to kMaxCols columns per panel
   S.min_two = 0;
-  if constexpr (sizeof(T) == 8) {
-    for (int nslot : {8, 4}) {
-      if (!B.has_two) break;
-      S.nslot2 = nslot;
-      S.smem2 = persist_smem<T>(L, B.wmax, nslot, true);
-      if (S.smem2 + 12 * 1024 <= (size_t)cap && persist_fits<T, true>(S.smem2)) {
-        S.min_two = 2 * (std::max((int)((B.kuf + B.wmax + 1 + kMaxCols - 1) / kMaxCols), B.wmax) + 2);
-        break;
-      }
+  for (int nslot : {8, 4}) {
+    if (!B.has_two) break;
+    S.nslot2 = nslot;
+    S.smem2 = persist_smem<T>(L, B.wmax, nslot, true);
+    if (S.smem2 + 12 * 1024 <= (size_t)cap && persist_fits<T, true>(S.smem2)) {
+      S.min_two = 2 * (std::max((int)((B.kuf + B.wmax + 1 + kMaxCols - 1) / kMaxCols), B.wmax) + 2);
+      break;
     }
-    cudaGetLastError();
   }
+  cudaGetLastError();
   return S.grid;
 }
 
@@ -538,9 +537,7 @@ int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersi
   a.err = err;
   a.trace = two ? nullptr : trace;
   void* args[] = {(void*)&a};
-  const void* fn = (const void*)blk_factor_persist_kernel<T, false>;
-  if constexpr (sizeof(T) == 8)
-    if (two) fn = (const void*)blk_factor_persist_kernel<T, true>;
+  const void* fn = two ? (const void*)blk_factor_persist_kernel<T, true> : (const void*)blk_factor_persist_kernel<T, false>;
   if (cudaLaunchCooperativeKernel(fn, dim3(S.grid), dim3(256), args, two ? S.smem2 : S.smem, st) != cudaSuccess) return -1;
   S.epoch[two] = a.epoch;
   if (two) S.bdone = a.bdone_target;

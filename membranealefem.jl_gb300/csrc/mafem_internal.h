@@ -305,7 +305,7 @@ struct AsmJob {
   const int* dir_idx;     // [n_dir] inhomogeneous Dirichlet entries of cps (dof * numnp + node)
   const double* dir_val;  // [n_dir] their values
   int n_dir;
-  int kuf;  // super-diagonals the factorisation fills
+  int kuf, klf;  // super-diagonals the factorisation fills, rows below the diagonal (the handle's own solver)
 };
 enum { kStartPredict = 1, kStartDirichlet = 2 };  // AsmItem::start
 struct AsmItem {  // one patch of a round

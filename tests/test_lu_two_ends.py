@@ -61,3 +61,21 @@ def test_both_solves_match_the_matrix(motion, scenario, n1, n2):
         x = s.solve_band(ab0, r)
         assert backward_error(K, -x, r) < tol
         assert np.array_equal(s.calc_r_K(xms, cps, 0.01, 0.01)[1], ab0)
+
+
+@pytest.mark.parametrize("motion,scenario,n1,n2", [c for c in CASES if c[2] < 68])
+def test_fp32_factors_refine_to_the_stopping_rule(motion, scenario, n1, n2):
+    """FP32 factors of both orders: the refinement in FP64 ends by its stopping
+    rule |r - K x| <= 1e-10 |r| (2-norm) on the FP32 tangent."""
+    p, _ = params_pair(motion, scenario, n1, n2, bend_mf=0.5, bend_tm=2.0)
+    mesh = M.Mesh(p)
+    n, kl = mesh.nmdf, mesh.half_bw
+    xms, cps = state(p, mesh, seed=6, amp=1e-2, vel_amp=0.02)
+    with M.Solver(mesh, p, M.FP32_REFINE) as s:
+        s.set_refinement(60, 1e-10)
+        for ctas in (0, 1):
+            s.set_launch_ctas(ctas)
+            r, ab = s.calc_r_K(xms, cps, 0.01, 0.01)
+            K = O.band_to_csr(ab, kl, kl, n)
+            for b in (r, -2.0 * r):  # the second with the stored factors
+                assert np.linalg.norm(K @ s.solve(b) + b) <= 1e-10 * np.linalg.norm(b) * (1 + 1e-3)
