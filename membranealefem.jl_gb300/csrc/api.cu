@@ -107,7 +107,7 @@ struct mafem_handle {
   bool pinv_ready = false;  // d_pinv holds the inverses of its panels' triangles
   BlkPlan blk;
   int* d_blk_end = nullptr;
-  int* d_flags = nullptr;  // per-panel completion flags of the cooperative back substitution
+  SolveWord* d_xch = nullptr;  // what the panels of the cooperative substitutions hand on: npan_max x 32
   int epoch = 0;           // value the flags are set to by the next back substitution
   int bwd_grid = 0;        // CTAs of the cooperative back substitution (0: single-CTA kernel)
   BlkPersist pers;         // persistent cooperative factorisation (grid 0: per-panel launches)
@@ -127,8 +127,7 @@ struct mafem_handle {
   int64_t fallbacks = 0;
   // batched FP32 form (band_lu_patch.cu): the handle's job, usable when its band fits
   float* d_inv = nullptr;
-  double* d_zbuf = nullptr;  // npan x 32: z = U11^-1 y1 per panel (cooperative forward substitution)
-  double* d_pinv = nullptr;  // npan x 2 x 32 x 32: L11^-1, U11^-1 per panel (cooperative forward substitution)
+  double* d_pinv = nullptr;  // npan_max x 2 x 32 x 32 (blk_inverses)
   bool patch_ok = false;
   bool ss_patch = false;  // the iteration in progress ran through a batch's patch solve
   PatchJob job{};
@@ -553,11 +552,10 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
         b.rbase = h->blk.mid;
       }
       const size_t npx = (size_t)h->blk.npan_max();
-      AL(h->d_flags, npx);
-      AL(h->d_zbuf, npx * kBlkW);
+      AL(h->d_xch, npx * kBlkW);
       AL(h->d_pinv, npx * 2 * kBlkW * kBlkW);
-      cudaMemset(h->d_flags, 0, npx * sizeof(int));
-      h->bwd_grid = precision == MAFEM_PLAIN_FP64 ? blk_backward_grid<double, double>() : blk_backward_grid<double, float>();
+      cudaMemset(h->d_xch, 0, npx * kBlkW * sizeof(SolveWord));
+      h->bwd_grid = precision == MAFEM_PLAIN_FP64 ? blk_backward_grid<double>() : blk_backward_grid<float>();
       h->bwd_max = h->bwd_grid;
       cudaGetLastError();
       const int pg = precision == MAFEM_PLAIN_FP64 ? blk_persist_setup<double>(h->L, h->blk, h->pers)
@@ -786,10 +784,10 @@ static void blk_need_inverses(mafem_handle* h) {
   if (h->pinv_ready) return;
   h->pinv_ready = true;
   h->launches += h->precision == MAFEM_PLAIN_FP64
-                     ? blk_inverses<double, double>((const double*)h->d_band, h->blk, h->last_two,
-                                                    (const double*)h->d_rdiag, h->d_pinv, h->st)
-                     : blk_inverses<double, float>((const float*)h->d_band, h->blk, h->last_two,
-                                                   (const float*)h->d_rdiag, h->d_pinv, h->st);
+                     ? blk_inverses<double, double>((const double*)h->d_band, h->L, h->blk, h->last_two,
+                                                    h->d_perm, (const double*)h->d_rdiag, h->d_pinv, h->st)
+                     : blk_inverses<double, float>((const float*)h->d_band, h->L, h->blk, h->last_two,
+                                                   h->d_perm, (const float*)h->d_rdiag, h->d_pinv, h->st);
 }
 
 static int factor_enqueue(mafem_handle* h, double* x) {
@@ -896,7 +894,7 @@ static int factor(mafem_handle* h, double* x, const double* rhs0) {
 template <class T>
 static void blk_back_solve(mafem_handle* h, double* y, const int* gate = nullptr) {
   if (h->bwd_grid > 0) {
-    const int nl = blk_backward<double, T>((const T*)h->d_band, h->blk, h->last_two, y, h->d_flags, h->epoch,
+    const int nl = blk_backward<T>((const T*)h->d_band, h->blk, h->last_two, y, h->d_xch, h->epoch,
                                            h->d_info + 1, h->bwd_grid, h->st, h->wait_test, gate);
     if (nl > 0 || h->last_two) {  // the factors of the two chains are for the cooperative kernel alone:
       h->launches += std::max(nl, 0);  // a refused launch stays as the CUDA error that the caller reports
@@ -915,8 +913,8 @@ template <class T>
 static void blk_fwd_solve(mafem_handle* h, double* y, const int* gate = nullptr) {
   if (h->bwd_grid > 0) {
     blk_need_inverses(h);
-    const int nl = blk_forward_coop<double, T>((const T*)h->d_band, h->L, h->blk, h->last_two, h->d_perm, h->d_pinv, y,
-                                               h->d_zbuf, h->d_flags, h->epoch, h->d_info + 1, h->bwd_grid, h->st,
+    const int nl = blk_forward_coop<T>((const T*)h->d_band, h->L, h->blk, h->last_two, h->d_pinv, y, h->d_xch, h->epoch,
+                                       h->d_info + 1, h->bwd_grid, h->st,
                                                h->wait_test, gate);
     if (nl > 0 || h->last_two) {
       h->launches += std::max(nl, 0);

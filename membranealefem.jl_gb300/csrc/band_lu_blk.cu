@@ -309,19 +309,17 @@ __global__ void __launch_bounds__(1024) blk_backward_kernel(const T* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// Explicit inverses of every panel's diagonal triangles for the cooperative
-// forward substitution: Li = L11^-1 (unit lower) and Ui = U11^-1 (upper, 1 / U(k, k)
-// from rdiag), 32 x 32 each with element (i, k) at k * 32 + i, zero outside
-// the panel's w x w block; inv[p] = Li then Ui.  One warp per panel (four per
-// CTA), lane c
-// forming column c of both by substitution.  With them the step of a
-// substitution that lies on its critical path -- the panel's two triangles --
-// is two 32-term dot products per lane with independent shuffles instead of
-// two 32-step dependent chains.
+// Two 32 x 32 matrices per panel for the cooperative forward substitution:
+// Ai = U11^-1 L11^-1 P, and W = Ai A(p, p - 1), the panel's rows of the panel before
+// it, so that of z(p) = Ai (b - sum over q < p of A(p, q) z(q)) everything but
+// W z(p - 1) can be formed before z(p - 1) is there.  Element (i, k) at k * 32 + i,
+// zero outside the panel's rows and columns; inv[p] = Ai then W.  One warp per panel
+// (four per CTA), lane c forming column c of both.
 template <class T, class V>
-__global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__ ab, BlkChain c,
+__global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__ ab, BlkChain c, int kl,
+                                                           const int* __restrict__ perm_all,
                                                            const T* __restrict__ rdiag_all, V* __restrict__ inv) {
-  __shared__ V S[4][32][33];  // per warp: S[k][i] = A(j0 + i, j0 + k) of its panel
+  __shared__ V S[4][32][33];  // per warp: S[k][i] = A(j0 + i, j0 + k) of its panel, then Ai
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int p = blockIdx.x * 4 + warp;
   if (p >= c.npan) return;  // warp-uniform; only warp-level synchronisation below
@@ -330,13 +328,14 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
   const T* rdiag = rdiag_all + c.rbase;
   for (int k = 0; k < 32; ++k) S[warp][k][lane] = (k < w && lane < w) ? V(blk[lane * c.si + k * c.sj]) : V(0);
   const V rd = lane < w ? V(rdiag[j0 + lane]) : V(0);
+  const int pr = lane < w ? perm_all[(size_t)(c.pbase + p) * kBlkW + lane] : -1;
   __syncwarp();
-  V* Li = inv + (size_t)(c.pbase + p) * 2 * kBlkW * kBlkW;
-  V* Ui = Li + kBlkW * kBlkW;
+  V* Ai = inv + (size_t)(c.pbase + p) * 2 * kBlkW * kBlkW;
+  V* W = Ai + kBlkW * kBlkW;
+  // column `lane`: L11 y = P e_lane forward, U11 x = y backward
   V x[32];
-  // column `lane` of L11^-1: L11 x = e_lane, forward
 #pragma unroll
-  for (int i = 0; i < 32; ++i) x[i] = i == lane ? V(1) : V(0);
+  for (int i = 0; i < 32; ++i) x[i] = __shfl_sync(kFull, pr, i) == lane ? V(1) : V(0);
 #pragma unroll
   for (int k = 0; k < 32; ++k) {
     const V xk = x[k];
@@ -344,163 +343,230 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
     for (int i = k + 1; i < 32; ++i) x[i] = fma(-S[warp][k][i], xk, x[i]);
   }
 #pragma unroll
-  for (int i = 0; i < 32; ++i) Li[lane * 32 + i] = (lane < w && i < w) ? x[i] : V(0);
-  // column `lane` of U11^-1: U11 x = e_lane, backward
-#pragma unroll
-  for (int i = 0; i < 32; ++i) x[i] = i == lane ? V(1) : V(0);
-#pragma unroll
   for (int k = 31; k >= 0; --k) {
     const V xk = x[k] * __shfl_sync(kFull, rd, k);
     x[k] = xk;
 #pragma unroll
     for (int i = 0; i < k; ++i) x[i] = fma(-S[warp][k][i], xk, x[i]);
   }
+  __syncwarp();
 #pragma unroll
-  for (int i = 0; i < 32; ++i) Ui[lane * 32 + i] = (lane < w && i < w) ? x[i] : V(0);
+  for (int i = 0; i < 32; ++i) {
+    const V v = (lane < w && i < w) ? x[i] : V(0);
+    Ai[lane * 32 + i] = v;
+    S[warp][lane][i] = v;
+  }
+  __syncwarp();
+  const int q0 = p > 0 ? c.ps[p - 1] : j0;  // column q0 + lane of the panel before
+  const T* col = ab + c.org + j0 * c.si + (q0 + lane) * c.sj;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) x[i] = V(0);
+  for (int m = 0; m < w; ++m) {
+    const V am = q0 + lane < j0 && j0 + m - (q0 + lane) <= kl ? V(col[m * c.si]) : V(0);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) x[i] = fma(S[warp][m][i], am, x[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 32; ++i) W[lane * 32 + i] = x[i];
 }
 
 // ---------------------------------------------------------------------------
-// Back substitution on many SMs: one cooperative launch, panel q handled by
-// CTA (npan - 1 - q) mod gridDim.x.  A CTA accumulates Y(q rows, c) x(c) over
-// the columns of the panels above it as their flags appear (most are done
-// long before it needs them), subtracts the sum from z and publishes
-// x(q) with a release store of the flag.  Flags hold the epoch of the solve
-// that set them, so they never need clearing.  Waits are bounded: after
-// wt.limit polls (kSpinLimit by default) the kernel records MAFEM status in
-// *err and every CTA returns (no GPU hang; the host reports the error).
-// wt.withhold = k >= 0 (failure-detection tests only): the flag of panel
-// npan - 1 - k is never published, so the CTAs that need it run out of polls
-// and every CTA returns.
-//
-// A launch covers panels [p0, p1) of one chain, or of two chains side by side
-// (CTAs below `split` the first): the columns right of panel p1 - 1 belong to
-// panels solved by an earlier launch.
+// Substitutions on many SMs: one cooperative launch, panel by panel over its CTAs
+// of four warps (one per sub-partition).  A panel's solution is handed on as
+// 16-byte words of a value and a tag, written and read whole: whoever needs it polls
+// the words themselves, so a panel's step on the chain is one store, one load, eight
+// multiply-adds per lane and two shuffles -- no fence, no flag, no barrier.  (With a
+// flag per panel, a fence before it and a barrier after it: 2.9 us per panel back,
+// about 8 us forward.)  A lane holds one of its warp's 8 rows and every fourth
+// column; the matrix entries of the next panel are loaded before the poll.  Tags are
+// the launch's epoch, so they never need clearing.  Waits are bounded: after wt.limit
+// polls (kSpinLimit by default) the kernel sets *err and every CTA returns (no GPU
+// hang; the host reports the error).  wt.withhold = k >= 0 (failure-detection tests
+// only): the back substitution's panel npan - 1 - k is never published, so the CTAs
+// that need it run out of polls.
+__device__ __forceinline__ void publish(SolveWord* p, double v, int tag) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p),
+               "l"(__double_as_longlong(v)), "l"((long long)tag)
+               : "memory");
+}
+__device__ __forceinline__ double peek(const SolveWord* p, long long& tag) {
+  long long v;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(v), "=l"(tag)
+               : "l"(p)
+               : "memory");
+  return __longlong_as_double(v);
+}
+// This lane's entries cg, cg + 4, ... < nc of a panel's words X, once all of the warp's
+// carry the tag (tag 0: from an earlier launch, at once).  false, for the whole warp,
+// when the polls ran out or another warp has set *err.
+__device__ __forceinline__ bool fetch(const SolveWord* X, int cg, int nc, int tag, bool far, double (&y)[8], int* err,
+                                      int limit) {
+  const int lim = limit > 0 ? limit : kSpinLimit;
+  for (int it = 0;; ++it) {
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      long long t = tag;
+      y[i] = cg + 4 * i < nc ? peek(X + cg + 4 * i, t) : 0.0;
+      ok &= t == tag;
+    }
+    if (tag == 0 || __all_sync(kFull, ok)) return true;
+    if (it > lim || ((it & 31) == 31 && __any_sync(kFull, *(volatile int*)err != 0))) {
+      if ((threadIdx.x & 31) == 0) atomicCAS(err, 0, 1);
+      return false;
+    }
+    __nanosleep(far ? 200 : 20);
+  }
+}
+
+// A launch covers panels [p0, p1) of one chain, or of two chains side by side (CTAs
+// below `split` the first): the columns right of panel p1 - 1 (backward) or the panels
+// before p0 (forward) belong to an earlier launch.
 struct BlkSpan {
   BlkChain c;
   int p0, p1;
 };
-template <class T, class V>
-__global__ void __launch_bounds__(256) blk_backward_coop_kernel(const T* __restrict__ ab, int kuf, BlkSpan s0, BlkSpan s1,
-                                                                int split, V* yv, int* flags_all, int epoch, int* err,
-                                                                WaitTest wt, const int* gate) {
-  __shared__ V part[8][33];
-  __shared__ int s_ok;
+constexpr int kSolveThreads = 128;
+
+// Back substitution x1 = z - Y x2.
+template <class T>
+__global__ void __launch_bounds__(kSolveThreads)
+    blk_backward_coop_kernel(const T* __restrict__ ab, int kuf, BlkSpan s0, BlkSpan s1, int split, double* yv,
+                             SolveWord* xch, int epoch, int* err, WaitTest wt, const int* gate) {
   if (gate && *gate) return;  // every CTA reads the same word: all return (refinement already stopped)
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int lane = threadIdx.x & 31, row = 8 * (threadIdx.x >> 5) + (lane & 7), cg = lane >> 3;
   const bool second = (int)blockIdx.x >= split;
   const BlkSpan& S = second ? s1 : s0;
   const int me = (int)blockIdx.x - (second ? split : 0), G = second ? (int)gridDim.x - split : split;
   const int* __restrict__ ps = S.c.ps;
   const int64_t si = S.c.si, sj = S.c.sj;
-  const T* a0 = ab + S.c.org;
-  V* y = yv + S.c.vorg;  // element i at y[i si]
-  int* flags = flags_all + S.c.pbase;
+  double* y = yv + S.c.vorg;  // element i at y[i si]
+  SolveWord* X = xch + (size_t)S.c.pbase * kBlkW;
   for (int q = S.p1 - 1 - me; q >= S.p0; q -= G) {
     const int j0 = ps[q], j1 = ps[q + 1];
     const int w = j1 - j0;
     const int jend = min(S.c.n, j1 + kuf);
-    const T* arow = a0 + (j0 + lane) * si;
-    V acc = V(0);
-    if (lane < w)  // columns solved before this launch
-      for (int c = max(j1, ps[S.p1]) + warp; c < jend; c += 8) acc += V(arow[c * sj]) * __ldcg(y + c * si);
-    int pl = q + 1;  // last panel of the launch with columns in [j1, jend)
-    while (pl + 1 < S.p1 && ps[pl + 1] < jend) ++pl;
-    for (int p = (j1 < jend && q + 1 < S.p1) ? pl : q; p > q; --p) {
-      if (!wait_flag(flags, p, epoch, err, &s_ok, wt.limit)) return;
-      const int cb = ps[p], ce = min(ps[p + 1], jend);
-      if (lane < w)
-        for (int c = cb + warp; c < ce; c += 8) acc += V(arow[c * sj]) * __ldcg(y + c * si);
+    const int r = j0 + min(row, w - 1);
+    const T* arow = ab + S.c.org + r * si;
+    const double z = y[r * si];
+    double acc[2] = {0.0, 0.0};
+    for (int c0 = max(j1, ps[S.p1]) + cg; c0 < jend; c0 += 32) {  // columns solved before this launch
+      T av[8];
+      double xv[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int c = c0 + 4 * i;
+        av[i] = c < jend ? arow[c * sj] : T(0);
+        xv[i] = c < jend ? y[c * si] : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i & 1] = fma((double)av[i], xv[i], acc[i & 1]);
     }
-    part[warp][lane] = acc;
-    __syncthreads();
-    if (warp == 0) {
-      const V sum = ((part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane])) +
-                    ((part[4][lane] + part[5][lane]) + (part[6][lane] + part[7][lane]));  // tree: 3 dependent adds
-      V* yj = y + (j0 + lane) * si;
-      if (lane < w) __stcg(yj, __ldcg(yj) - sum);  // x1 = z - Y x2
-      __threadfence();
-      __syncwarp();
-      if (lane == 0 && (second || S.c.npan - 1 - q != wt.withhold)) st_release(flags + q, epoch);
+    int p = q;  // last panel of the launch with columns in [j1, jend)
+    while (p + 1 < S.p1 && ps[p + 1] < jend) ++p;
+    T an[8];
+    auto load = [&](int pp) {
+      const int cb = ps[pp], ce = min(ps[pp + 1], jend);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) an[i] = cb + cg + 4 * i < ce ? arow[(cb + cg + 4 * i) * sj] : T(0);
+    };
+    if (p > q) load(p);
+    for (; p > q; --p) {
+      double av[8], xv[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) av[i] = (double)an[i];
+      if (p - 1 > q) load(p - 1);
+      if (!fetch(X + (size_t)p * kBlkW, cg, min(ps[p + 1], jend) - ps[p], epoch, p > q + 2, xv, err, wt.limit)) return;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i & 1] = fma(av[i], xv[i], acc[i & 1]);
     }
-    __syncthreads();
+    double s = acc[0] + acc[1];
+    s += __shfl_xor_sync(kFull, s, 8);
+    s += __shfl_xor_sync(kFull, s, 16);
+    if (cg == 0 && row < w) {
+      const double x = z - s;
+      if (second || S.c.npan - 1 - q != wt.withhold) publish(X + (size_t)q * kBlkW + row, x, epoch);
+      y[r * si] = x;
+    }
   }
 }
 
-// ---------------------------------------------------------------------------
-// Forward substitution on many SMs: one cooperative launch, panel p handled by
-// CTA p mod gridDim.x in increasing order.  For its panel's rows a CTA gathers
-// the contributions A21(q) z(q) of the earlier panels q whose rows reach them
-// (rows of panel q end at ps[q + 1] + kl), each as soon as q's flag appears,
-// then applies the panel's interchanges and triangles like blk_forward_kernel:
-// z = U11^-1 L11^-1 P b1 replaces b1 in place and goes to zbuf[p] with a
-// release store of the flag.  A panel waits only for lower-numbered panels,
-// which CTAs take in increasing order, so the chain always progresses; waits
-// are bounded (kSpinLimit polls, then *err and every CTA returns).
-// A launch covers panels [p0, p1) of one or two chains like the back substitution's;
-// the panels before p0 were done by an earlier launch.
-template <class T, class V>
-__global__ void __launch_bounds__(256) blk_forward_coop_kernel(const T* __restrict__ ab, int kl, BlkSpan s0, BlkSpan s1,
-                                                               int split, const int* __restrict__ perm_all,
-                                                               const V* __restrict__ inv_all, V* bv, V* zbuf_all,
-                                                               int* flags_all, int epoch, int* err, WaitTest wt,
-                                                               const int* gate) {
-  __shared__ V part[8][33];
-  __shared__ V Is[2 * 32 * 32];  // L11^-1 then U11^-1 of the panel, element (i, k) at k * 32 + i
-  __shared__ V accs[32];
-  __shared__ int s_ok;
+// Forward substitution z(p) = Ai(p) (b(p) - sum over q < p of A(p, q) z(q)), each panel's
+// contributions pulled from the panels before it; the last of them by W (above).
+template <class T>
+__global__ void __launch_bounds__(kSolveThreads)
+    blk_forward_coop_kernel(const T* __restrict__ ab, int kl, BlkSpan s0, BlkSpan s1, int split,
+                            const double* __restrict__ inv_all, double* bv, SolveWord* xch, int epoch, int* err,
+                            WaitTest wt, const int* gate) {
+  __shared__ double xs[2][32];
   if (gate && *gate) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int lane = threadIdx.x & 31, row = 8 * (threadIdx.x >> 5) + (lane & 7), cg = lane >> 3;
   const bool second = (int)blockIdx.x >= split;
   const BlkSpan& S = second ? s1 : s0;
   const int me = (int)blockIdx.x - (second ? split : 0), G = second ? (int)gridDim.x - split : split;
   const int* __restrict__ ps = S.c.ps;
   const int64_t si = S.c.si, sj = S.c.sj;
-  const T* a0 = ab + S.c.org;
-  V* b = bv + S.c.vorg;  // element i at b[i si]
-  V* zbuf = zbuf_all + (size_t)S.c.pbase * kBlkW;
-  int* flags = flags_all + S.c.pbase;
-  for (int p = S.p0 + me; p < S.p1; p += G) {
-    const int j0 = ps[p], j1 = ps[p + 1];
-    const int w = j1 - j0;
-    const V* Ip = inv_all + (size_t)(S.c.pbase + p) * 2 * kBlkW * kBlkW;
-    for (int k = tid; k < 2 * kBlkW * kBlkW; k += 256) Is[k] = __ldcg(Ip + k);
-    int pf = p;  // earliest panel whose rows reach j0
-    while (pf > 0 && ps[pf] + kl > j0) --pf;
-    const T* arow = a0 + (j0 + lane) * si;
-    V acc = V(0);
-    for (int q = pf; q < p; ++q) {
-      if (q >= S.p0 && !wait_flag(flags, q, epoch, err, &s_ok, wt.limit)) return;
-      const int q0 = ps[q];
-      const int wq = ps[q + 1] - ps[q];
-      if (lane < w)
-        for (int k = warp; k < wq; k += 8)
-          if (j0 + lane - (q0 + k) <= kl)  // inside panel q's band rows
-            acc += V(arow[(q0 + k) * sj]) * __ldcg(zbuf + (size_t)q * kBlkW + k);
+  double* b = bv + S.c.vorg;  // element i at b[i si]
+  SolveWord* X = xch + (size_t)S.c.pbase * kBlkW;
+  int par = 0;
+  bool ok = true;
+  for (int p = S.p0 + me; p < S.p1; p += G, par ^= 1) {
+    const int j0 = ps[p];
+    const int w = ps[p + 1] - j0;
+    const int r = j0 + min(row, w - 1);
+    const T* arow = ab + S.c.org + r * si;
+    const double br = row < w ? b[r * si] : 0.0;
+    const double* Ip = inv_all + (size_t)(S.c.pbase + p) * 2 * kBlkW * kBlkW;
+    double Ai[8], W[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      Ai[i] = Ip[(cg + 4 * i) * 32 + row];
+      W[i] = Ip[kBlkW * kBlkW + (cg + 4 * i) * 32 + row];
     }
-    part[warp][lane] = acc;
-    __syncthreads();
-    if (warp == 0) {
-      accs[lane] = ((part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane])) +
-                   ((part[4][lane] + part[5][lane]) + (part[6][lane] + part[7][lane]));
-      __syncwarp();
-      const int pr = lane < w ? perm_all[(size_t)(S.c.pbase + p) * kBlkW + lane] : 0;
-      const V x = lane < w ? __ldcg(b + (j0 + pr) * si) - accs[pr] : V(0);
-      // y1 = L11^-1 P b1, z = U11^-1 y1: dot products with independent shuffles
-      V y1 = V(0);
+    int q = p;  // earliest panel whose rows reach j0
+    while (q > 0 && ps[q] + kl > j0) --q;
+    double acc[2] = {0.0, 0.0};
+    T an[8];
+    auto load = [&](int qq) {
+      const int cb = ps[qq], ce = ps[qq + 1];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) y1 = fma(Is[k * 32 + lane], __shfl_sync(kFull, x, k), y1);
-      V v = V(0);
-#pragma unroll
-      for (int k = 0; k < 32; ++k) v = fma(Is[kBlkW * kBlkW + k * 32 + lane], __shfl_sync(kFull, y1, k), v);
-      if (lane < w) {
-        __stcg(b + (j0 + lane) * si, v);
-        __stcg(zbuf + (size_t)p * kBlkW + lane, v);
+      for (int i = 0; i < 8; ++i) {
+        const int c = cb + cg + 4 * i;
+        an[i] = c < ce && r - c <= kl ? arow[c * sj] : T(0);  // inside that panel's band rows
       }
-      __threadfence();
-      __syncwarp();
-      if (lane == 0) st_release(flags + p, epoch);
+    };
+    if (q < p - 1) load(q);
+    for (; ok && q < p - 1; ++q) {
+      double av[8], zv[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) av[i] = (double)an[i];
+      if (q + 1 < p - 1) load(q + 1);
+      ok = fetch(X + (size_t)q * kBlkW, cg, ps[q + 1] - ps[q], q >= S.p0 ? epoch : 0, q < p - 3, zv, err, wt.limit);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i & 1] = fma(av[i], zv[i], acc[i & 1]);
     }
-    __syncthreads();
+    double s = acc[0] + acc[1];
+    s += __shfl_xor_sync(kFull, s, 8);
+    s += __shfl_xor_sync(kFull, s, 16);
+    if (cg == 0) xs[par][row] = br - (row < w ? s : 0.0);
+    if (!__syncthreads_and(ok)) return;
+    double u[2] = {0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) u[i & 1] = fma(Ai[i], xs[par][cg + 4 * i], u[i & 1]);
+    if (p > 0) {
+      double zv[8];
+      ok = fetch(X + (size_t)(p - 1) * kBlkW, cg, j0 - ps[p - 1], p - 1 >= S.p0 ? epoch : 0, false, zv, err, wt.limit);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) u[i & 1] = fma(-W[i], zv[i], u[i & 1]);
+    }
+    double z = u[0] + u[1];
+    z += __shfl_xor_sync(kFull, z, 8);
+    z += __shfl_xor_sync(kFull, z, 16);
+    if (cg == 0 && row < w && ok) {
+      publish(X + (size_t)p * kBlkW + row, z, epoch);
+      b[r * si] = z;
+    }
   }
 }
 // The backward chain's contributions to the rows [lo, mid) above it, before the
@@ -692,10 +758,11 @@ void blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, const int* 
   blk_forward_kernel<T, V><<<1, 1024, sm, st>>>(ab, L, B.d_ps, B.npan(), perm_all, rdiag, b);
 }
 template <class V, class T>
-int blk_inverses(const T* ab, const BlkPlan& B, bool two, const T* rdiag, V* inv, cudaStream_t st) {
+int blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
+                 V* inv, cudaStream_t st) {
   for (int k = 0; k < (two ? 2 : 1); ++k) {
     const BlkChain& c = two ? B.two[k] : B.one;
-    blk_inverses_kernel<T, V><<<(c.npan + 3) / 4, 128, 0, st>>>(ab, c, rdiag, inv);
+    blk_inverses_kernel<T, V><<<(c.npan + 3) / 4, 128, 0, st>>>(ab, c, L.kl, perm_all, rdiag, inv);
   }
   return two ? 2 : 1;
 }
@@ -711,15 +778,16 @@ static int coop_spans(F&& launch, const BlkSpan& a, const BlkSpan* b, int grid) 
   const int ga = std::min(na, nb > 0 ? grid / 2 : grid), gb = std::min(nb, grid - ga);
   return launch(a, b ? *b : a, ga, ga + gb) == cudaSuccess ? 1 : -1;
 }
-template <class V, class T>
-int blk_backward(const T* ab, const BlkPlan& B, bool two, V* y, int* flags, int& epoch, int* err, int grid,
+template <class T>
+int blk_backward(const T* ab, const BlkPlan& B, bool two, double* y, SolveWord* xch, int& epoch, int* err, int grid,
                  cudaStream_t st, WaitTest wt, const int* gate) {
   int kuf = B.kuf;
   auto launch = [&](BlkSpan a, BlkSpan b, int split, int ctas) {
     ++epoch;
-    void* args[] = {(void*)&ab, (void*)&kuf,   (void*)&a,   (void*)&b,  (void*)&split, (void*)&y, (void*)&flags,
+    void* args[] = {(void*)&ab,    (void*)&kuf, (void*)&a,  (void*)&b,   (void*)&split, (void*)&y, (void*)&xch,
                     (void*)&epoch, (void*)&err, (void*)&wt, (void*)&gate};
-    return cudaLaunchCooperativeKernel((const void*)blk_backward_coop_kernel<T, V>, dim3(ctas), dim3(256), args, 0, st);
+    return cudaLaunchCooperativeKernel((const void*)blk_backward_coop_kernel<T>, dim3(ctas), dim3(kSolveThreads), args, 0,
+                                       st);
   };
   if (!two) return coop_spans(launch, BlkSpan{B.one, 0, B.one.npan}, nullptr, grid);
   // the unknowns between the chains, then both chains side by side
@@ -734,34 +802,35 @@ template <class V, class T>
 void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, cudaStream_t st) {
   blk_backward_kernel<T, V><<<1, 1024, 0, st>>>(ab, L, B.kuf, B.d_ps, B.npan(), y);
 }
-template <class V, class T>
-int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const V* inv,
-                     V* b, V* zbuf, int* flags, int& epoch, int* err, int grid, cudaStream_t st, WaitTest wt,
-                     const int* gate) {
+template <class T>
+int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const double* inv, double* b,
+                     SolveWord* xch, int& epoch, int* err, int grid, cudaStream_t st, WaitTest wt, const int* gate) {
   int kl = L.kl;
   auto launch = [&](BlkSpan s0, BlkSpan s1, int split, int ctas) {
     ++epoch;
-    void* args[] = {(void*)&ab, (void*)&kl,   (void*)&s0,    (void*)&s1,    (void*)&split, (void*)&perm_all, (void*)&inv,
-                    (void*)&b,  (void*)&zbuf, (void*)&flags, (void*)&epoch, (void*)&err,   (void*)&wt,       (void*)&gate};
-    return cudaLaunchCooperativeKernel((const void*)blk_forward_coop_kernel<T, V>, dim3(ctas), dim3(256), args, 0, st);
+    void* args[] = {(void*)&ab, (void*)&kl,  (void*)&s0,    (void*)&s1,  (void*)&split, (void*)&inv,
+                    (void*)&b,  (void*)&xch, (void*)&epoch, (void*)&err, (void*)&wt,    (void*)&gate};
+    return cudaLaunchCooperativeKernel((const void*)blk_forward_coop_kernel<T>, dim3(ctas), dim3(kSolveThreads), args, 0,
+                                       st);
   };
   if (!two) return coop_spans(launch, BlkSpan{B.one, 0, B.one.npan}, nullptr, grid);
   const BlkSpan s1{B.two[1], 0, B.two[1].npan};
   const int r1 = coop_spans(launch, BlkSpan{B.two[0], 0, B.pm}, &s1, grid);
   if (r1 < 0) return r1;
   const int lo = std::max(0, B.mid - L.kl);
-  blk_forward_mid_kernel<T, V><<<(B.mid - lo + 7) / 8, 256, 0, st>>>(ab, L, B.mid, lo, b, gate);
+  blk_forward_mid_kernel<T, double><<<(B.mid - lo + 7) / 8, 256, 0, st>>>(ab, L, B.mid, lo, b, gate);
   const int r2 = coop_spans(launch, BlkSpan{B.two[0], B.pm, B.two[0].npan}, nullptr, grid);
   return r2 < 0 ? r2 : r1 + 1 + r2;
 }
 // CTAs of the cooperative back substitution that can be resident at once
-template <class V, class T>
+template <class T>
 int blk_backward_grid() {
-  int dev = 0, sms = 0, per = 0;
+  int dev = 0, sms = 0, back = 0, forw = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, blk_backward_coop_kernel<T, V>, 256, 0);
-  return std::max(0, sms * std::min(per, 1));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&back, blk_backward_coop_kernel<T>, kSolveThreads, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&forw, blk_forward_coop_kernel<T>, kSolveThreads, 0);
+  return std::max(0, sms * std::min(std::min(back, forw), 1));
 }
 
 template int blk_lu_setup<double>(const BandLayout&);
@@ -774,23 +843,23 @@ template void blk_forward<double, double>(const double*, const BandLayout&, cons
                                           double*, cudaStream_t);
 template void blk_forward<double, float>(const float*, const BandLayout&, const BlkPlan&, const int*, const float*,
                                          double*, cudaStream_t);
-template int blk_inverses<double, double>(const double*, const BlkPlan&, bool, const double*, double*, cudaStream_t);
-template int blk_inverses<double, float>(const float*, const BlkPlan&, bool, const float*, double*, cudaStream_t);
-template int blk_backward<double, double>(const double*, const BlkPlan&, bool, double*, int*, int&, int*, int,
-                                          cudaStream_t, WaitTest, const int*);
-template int blk_backward<double, float>(const float*, const BlkPlan&, bool, double*, int*, int&, int*, int,
-                                         cudaStream_t, WaitTest, const int*);
+template int blk_inverses<double, double>(const double*, const BandLayout&, const BlkPlan&, bool, const int*,
+                                          const double*, double*, cudaStream_t);
+template int blk_inverses<double, float>(const float*, const BandLayout&, const BlkPlan&, bool, const int*, const float*,
+                                         double*, cudaStream_t);
+template int blk_backward<double>(const double*, const BlkPlan&, bool, double*, SolveWord*, int&, int*, int, cudaStream_t,
+                                  WaitTest, const int*);
+template int blk_backward<float>(const float*, const BlkPlan&, bool, double*, SolveWord*, int&, int*, int, cudaStream_t,
+                                 WaitTest, const int*);
 template void blk_backward_1cta<double, double>(const double*, const BandLayout&, const BlkPlan&, double*,
                                                 cudaStream_t);
 template void blk_backward_1cta<double, float>(const float*, const BandLayout&, const BlkPlan&, double*,
                                                cudaStream_t);
-template int blk_backward_grid<double, double>();
-template int blk_backward_grid<double, float>();
-template int blk_forward_coop<double, double>(const double*, const BandLayout&, const BlkPlan&, bool, const int*,
-                                              const double*, double*, double*, int*, int&, int*, int, cudaStream_t,
-                                              WaitTest, const int*);
-template int blk_forward_coop<double, float>(const float*, const BandLayout&, const BlkPlan&, bool, const int*,
-                                             const double*, double*, double*, int*, int&, int*, int, cudaStream_t,
-                                             WaitTest, const int*);
+template int blk_backward_grid<double>();
+template int blk_backward_grid<float>();
+template int blk_forward_coop<double>(const double*, const BandLayout&, const BlkPlan&, bool, const double*, double*,
+                                      SolveWord*, int&, int*, int, cudaStream_t, WaitTest, const int*);
+template int blk_forward_coop<float>(const float*, const BandLayout&, const BlkPlan&, bool, const double*, double*,
+                                     SolveWord*, int&, int*, int, cudaStream_t, WaitTest, const int*);
 
 }  // namespace mafem

@@ -216,11 +216,15 @@ int blk_lu_factor(T* ab, const BandLayout& L, const BlkPlan& B, int* perm_all, T
 template <class V, class T>
 void blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, const int* perm_all, const T* rdiag, V* b,
                  cudaStream_t st);
-// Back substitution x1 = z - Y x2 in place on many SMs (cooperative launches of
-// at most `grid` CTAs, grid <= blk_backward_grid()).  flags: npan_max ints; epoch: a
-// value they do not hold yet is taken per launch; err: nonzero after a bounded
+// Back substitution x1 = z - Y x2 in place on many SMs (cooperative launches of at
+// most `grid` CTAs, grid <= blk_backward_grid()).  xch: npan_max x 32 words; epoch: a
+// value that no word's tag holds yet is taken per launch; err: nonzero after a bounded
 // wait ran out.  two: the factors of the two-chain elimination.  Returns the
 // kernels launched, or -1 if a launch failed.
+struct alignas(16) SolveWord {
+  double v;
+  long long tag;
+};
 // Failure-detection test hook of the cooperative substitutions: limit = polls
 // before a wait gives up (<= 0: the default), withhold = k: the back
 // substitution never publishes the flag of panel npan - 1 - k (-1: none).
@@ -228,22 +232,22 @@ struct WaitTest {
   int limit = 0;
   int withhold = -1;
 };
-// Explicit inverses of the stored panels' L11 and U11 (inv: npan x 2 x 32 x
-// 32 in V) for the cooperative forward substitution.
+// Per panel the inverse of its diagonal block and its product with the rows of the
+// panel before (inv: npan_max x 2 x 32 x 32) for the cooperative forward substitution.
 template <class V, class T>
-int blk_inverses(const T* ab, const BlkPlan& B, bool two, const T* rdiag, V* inv, cudaStream_t st);
-template <class V, class T>
-int blk_backward(const T* ab, const BlkPlan& B, bool two, V* y, int* flags, int& epoch, int* err, int grid,
+int blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
+                 V* inv, cudaStream_t st);
+template <class T>
+int blk_backward(const T* ab, const BlkPlan& B, bool two, double* y, SolveWord* xch, int& epoch, int* err, int grid,
                  cudaStream_t st, WaitTest wt = WaitTest(), const int* gate = nullptr);
-template <class V, class T>
+template <class T>
 int blk_backward_grid();
-// Forward substitution (P, L11, A21 of the stored panels) on at most `grid` CTAs of
-// cooperative launches, in place on b; zbuf: npan_max x 32 scratch; flags / epoch / two
-// as for blk_backward.  Returns the kernels launched, or -1 if a launch was refused.
-template <class V, class T>
-int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const V* inv,
-                     V* b, V* zbuf, int* flags, int& epoch, int* err, int grid, cudaStream_t st,
-                     WaitTest wt = WaitTest(), const int* gate = nullptr);
+// Forward substitution (P, L11, A21 of the stored panels), in place on b; the rest as for
+// blk_backward.  Returns the kernels launched, or -1 if a launch was refused.
+template <class T>
+int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const double* inv, double* b,
+                     SolveWord* xch, int& epoch, int* err, int grid, cudaStream_t st, WaitTest wt = WaitTest(),
+                     const int* gate = nullptr);
 // Persistent cooperative factorisation (band_lu_persist.cu): launch shape and
 // per-panel flags.  Flags are zeroed once; epochs make them reusable.  The arrays
 // hold the one chain's npan panels, then the two chains'.
