@@ -590,7 +590,7 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
   AL(h->d_x, n);
   AL(h->d_res, n);
   AL(h->d_dx, n);
-  AL(h->d_part, 2048);
+  AL(h->d_part, 4096);  // partial sums: of an update (2 x 1024), of a residual (2048)
   AL(h->d_out, 16);
   AL(h->d_ipiv, n);
   AL(h->d_perm, std::max((size_t)h->npan * h->rmax, (size_t)h->blk.npan_max() * kBlkW));
@@ -954,10 +954,10 @@ static int check_info(mafem_handle* h) {
 static void refine_begin(mafem_handle* h, const double* rhs_dev) {
   const int64_t n = h->nmdf;
   cudaMemsetAsync(h->d_x, 0, n * sizeof(double), h->st);
-  launch_band_residual<float>((const float*)h->d_band0, h->L, h->d_x, rhs_dev, h->d_res, h->d_part, h->d_out + 4,
+  launch_band_residual<float>((const float*)h->d_band0, h->L, nullptr, rhs_dev, h->d_res, h->d_part + 2048,
                               h->st);  // res = rhs, |rhs|
-  launch_refine_init(h->d_out + 4, h->d_rstate, h->d_out + 12, h->st);
-  h->launches += 3;
+  launch_refine_init(n, h->d_part + 2048, h->d_rstate, h->d_out + 12, h->st);
+  h->launches += 2;
 }
 static void refine_sweeps(mafem_handle* h, const double* rhs_dev, int count) {
   const int64_t n = h->nmdf;
@@ -972,11 +972,11 @@ static void refine_sweeps(mafem_handle* h, const double* rhs_dev, int count) {
       band_backward<float, double>((const float*)h->d_band, h->L, h->d_dx, h->st);
       h->launches += 2;
     }
-    launch_axpy_norms(n, h->d_dx, h->d_x, h->d_part, h->d_out + 8, h->st, gate);
-    launch_band_residual<float>((const float*)h->d_band0, h->L, h->d_x, rhs_dev, h->d_res, h->d_part, h->d_out + 3,
-                                h->st, gate);
-    launch_refine_check(h->d_out + 3, h->d_out + 8, gate, h->d_out + 12, h->refine_tol, h->max_refine, h->st);
-    h->launches += 6;
+    launch_axpy_partials(n, h->d_dx, h->d_x, h->d_part, h->st, gate);
+    launch_band_residual<float>((const float*)h->d_band0, h->L, h->d_x, rhs_dev, h->d_res, h->d_part + 2048, h->st,
+                                gate);
+    launch_refine_check(n, h->d_part + 2048, h->d_part, gate, h->d_out + 12, h->refine_tol, h->max_refine, h->st);
+    h->launches += 4;
   }
 }
 

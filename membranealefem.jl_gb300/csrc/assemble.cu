@@ -194,49 +194,64 @@ __global__ void newton_norm_kernel(const double* __restrict__ part, int nblk, in
 }
 
 // Refinement residual res = r - A0 x in FP64 arithmetic, A0 = the unfactored
-// band (any storage type).  A warp owns 32 consecutive rows and walks the
-// columns of its band window, so every load of A0 is a coalesced 32-row
-// column segment.
+// band (any storage type); x null: res = r.  A CTA owns 32 consecutive rows (a
+// lane each, so every load of A0 is a coalesced 32-row column segment) and shares
+// out the columns of their band window over its warps, eight in flight per lane.
+// Bound: the conversions and multiply-adds, each ~64 cycles of a sub-partition's
+// FP64 pipe (29 us for the 32 x 32 ALEVB band).  A warp per 32 rows left most of the
+// chip idle and each load exposed: 570 us.
+constexpr int kResWarps = 8;
 template <class T>
-__global__ void band_residual_kernel(const T* __restrict__ a0, BandLayout L, const double* __restrict__ x,
-                                     const double* __restrict__ r, double* __restrict__ res,
-                                     double* __restrict__ part, const int* __restrict__ gate) {
-  __shared__ double s_p[32];
+__global__ void __launch_bounds__(32 * kResWarps)
+    band_residual_kernel(const T* __restrict__ a0, BandLayout L, const double* __restrict__ x,
+                         const double* __restrict__ r, double* __restrict__ res, double* __restrict__ part,
+                         const int* __restrict__ gate) {
+  __shared__ double s_p[kResWarps][33];
   if (gate && *gate) return;  // the refinement has already stopped
-  const int lane = threadIdx.x & 31;
-  const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = (int)L.n;
   double nrm = 0.0;
-  for (int64_t wi = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); wi * 32 < L.n; wi += nwarps) {
-    const int64_t i0 = wi * 32, i = i0 + lane;
-    const int64_t jlo = max64(0, i0 - L.kl), jhi = min64(L.n - 1, i0 + 31 + L.ku);
-    double acc = 0.0;
-    for (int64_t j = jlo; j <= jhi; ++j) {
-      const double xj = x[j];
-      if (i < L.n && i - j >= -L.ku && i - j <= L.kl) acc += (double)a0[j * L.ldb + L.off + i - j] * xj;
+  for (int i0 = blockIdx.x * 32; i0 < n; i0 += gridDim.x * 32) {
+    const int i = i0 + lane;
+    const int jlo = max(0, i0 - L.kl), jhi = x ? min(n - 1, i0 + 31 + L.ku) : -1;
+    const T* row = a0 + L.off + i;  // + j (ldb - 1): column j
+    double acc[2] = {0.0, 0.0};
+    for (int j0 = jlo + warp; j0 <= jhi; j0 += 8 * kResWarps) {
+      T av[8];
+      double xv[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int j = j0 + kResWarps * k;
+        const bool in = j <= jhi && i < n && i - j >= -L.ku && i - j <= L.kl;
+        av[k] = in ? row[j * (L.ldb - 1)] : T(0);
+        xv[k] = in ? x[j] : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[k & 1] = fma((double)av[k], xv[k], acc[k & 1]);
     }
-    if (i < L.n) {
-      const double v = r[i] - acc;
+    s_p[warp][lane] = acc[0] + acc[1];
+    __syncthreads();
+    if (warp == 0 && i < n) {
+      double a = 0.0;
+#pragma unroll
+      for (int k = 0; k < kResWarps; ++k) a += s_p[k][lane];
+      const double v = r[i] - a;
       res[i] = v;
-      nrm += v * v;
+      nrm = fma(v, v, nrm);
     }
+    __syncthreads();
   }
-  for (int o = 16; o > 0; o >>= 1) nrm += __shfl_down_sync(0xffffffffu, nrm, o);
-  if (lane == 0) s_p[threadIdx.x >> 5] = nrm;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) a += s_p[k];
-    part[blockIdx.x] = a;
+  if (warp == 0) {
+    for (int o = 16; o > 0; o >>= 1) nrm += __shfl_down_sync(0xffffffffu, nrm, o);
+    if (lane == 0) part[blockIdx.x] = nrm;
   }
 }
-__global__ void sqrt_sum_kernel(const double* __restrict__ part, int n, double* __restrict__ out,
-                                const int* __restrict__ gate) {
-  if (gate && *gate) return;
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double a = 0;
-    for (int k = 0; k < n; ++k) a += part[k];
-    *out = sqrt(a);
-  }
+// sum of p[0], p[stride], ... over n block partial sums by one warp, in a fixed order
+__device__ __forceinline__ double sum_partials(const double* __restrict__ p, int n, int stride) {
+  double a = 0.0;
+  for (int k = threadIdx.x & 31; k < n; k += 32) a += p[k * stride];
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
 }
 __global__ void axpy_kernel(int64_t n, const double* __restrict__ dx, double* __restrict__ x) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -275,16 +290,12 @@ __global__ void axpy_norms_kernel(int64_t n, const double* __restrict__ dx, doub
     part[2 * blockIdx.x + 1] = b;
   }
 }
-// out[0] = |dx|, out[1] = |x| from the block partial sums, in a fixed order
+// out[0] = |dx|, out[1] = |x| from the block partial sums
 __global__ void sqrt_pair_kernel(const double* __restrict__ part, int nblk, double* __restrict__ out,
                                  const int* __restrict__ gate) {
   if (gate && *gate) return;
+  const double a = sum_partials(part, nblk, 2), b = sum_partials(part + 1, nblk, 2);
   if (threadIdx.x == 0) {
-    double a = 0.0, b = 0.0;
-    for (int k = 0; k < nblk; ++k) {
-      a += part[2 * k];
-      b += part[2 * k + 1];
-    }
     out[0] = sqrt(a);
     out[1] = sqrt(b);
   }
@@ -445,27 +456,28 @@ void launch_newton_update(const DevPatch& P, const PhysParams& pp, double dt, co
   newton_update_kernel<<<blocks, 256, 0, st>>>(P, pp, dt, x, r, part, skip, skip2, skip3);
   newton_norm_kernel<<<1, 32, 0, st>>>(part, blocks, P.nmdf, out);
 }
-int band_residual_blocks(int64_t n) { return (int)min64(304, (n + 255) / 256); }
+static int residual_blocks(int64_t n) { return (int)min64(2048, (n + 31) / 32); }
+static int norm_blocks(int64_t n) { return (int)min64(1024, (n + 255) / 256); }
 template <class T>
 void launch_band_residual(const T* a0, const BandLayout& L, const double* x, const double* r, double* res,
-                          double* part, double* out, cudaStream_t st, const int* gate) {
-  const int blocks = band_residual_blocks(L.n);
-  band_residual_kernel<T><<<blocks, 256, 0, st>>>(a0, L, x, r, res, part, gate);
-  sqrt_sum_kernel<<<1, 32, 0, st>>>(part, blocks, out, gate);
+                          double* part, cudaStream_t st, const int* gate) {
+  band_residual_kernel<T><<<residual_blocks(L.n), 32 * kResWarps, 0, st>>>(a0, L, x, r, res, part, gate);
 }
-void launch_axpy_norms(int64_t n, const double* dx, double* x, double* part, double* out, cudaStream_t st,
-                       const int* gate) {
-  const int blocks = (int)min64(1024, (n + 255) / 256);  // part holds 2048 doubles
-  axpy_norms_kernel<<<blocks, 256, 0, st>>>(n, dx, x, part, gate);
-  sqrt_pair_kernel<<<1, 32, 0, st>>>(part, blocks, out, gate);
+void launch_axpy_partials(int64_t n, const double* dx, double* x, double* part, cudaStream_t st, const int* gate) {
+  axpy_norms_kernel<<<norm_blocks(n), 256, 0, st>>>(n, dx, x, part, gate);
+}
+void launch_axpy_norms(int64_t n, const double* dx, double* x, double* part, double* out, cudaStream_t st) {
+  launch_axpy_partials(n, dx, x, part, st, nullptr);
+  sqrt_pair_kernel<<<1, 32, 0, st>>>(part, norm_blocks(n), out, nullptr);
 }
 
 // ---- device-side stopping test of one handle's iterative refinement ----------------
 // st[0] done, st[1] sweeps, st[2] status; nrm[0] |r0|, nrm[1] the previous
-// residual norm.  rn: the residual norm after the sweep (band_residual's out).
-__global__ void refine_init_kernel(const double* __restrict__ r0, int* __restrict__ st, double* __restrict__ nrm) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    const double v = *r0;
+// residual norm.  part: the partial sums of the residual's squares (launch_band_residual).
+__global__ void refine_init_kernel(const double* __restrict__ part, int nblk, int* __restrict__ st,
+                                   double* __restrict__ nrm) {
+  const double v = sqrt(sum_partials(part, nblk, 1));
+  if (threadIdx.x == 0) {
     nrm[0] = v;
     nrm[1] = v;
     st[1] = 0;
@@ -482,10 +494,14 @@ __global__ void refine_init_kernel(const double* __restrict__ r0, int* __restric
 // or max_sweeps (MAFEM_REFINE_STALLED, or MAFEM_OK when the last correction is
 // at most 1e-8 |x|: the residual has reached its rounding floor, which in a
 // late Newton iteration, where |r0| is itself tiny, lies above tol |r0|).
-__global__ void refine_check_kernel(const double* __restrict__ rn, const double* __restrict__ dxn, int* __restrict__ st,
-                                    double* __restrict__ nrm, double tol, int max_sweeps) {
-  if (threadIdx.x != 0 || blockIdx.x != 0 || st[0]) return;
-  const double r = *rn, d = dxn[0], xv = dxn[1];
+// dxpart: the partial sums of launch_axpy_partials.
+__global__ void refine_check_kernel(const double* __restrict__ part, int nblk, const double* __restrict__ dxpart,
+                                    int ndx, int* __restrict__ st, double* __restrict__ nrm, double tol,
+                                    int max_sweeps) {
+  if (st[0]) return;
+  const double r = sqrt(sum_partials(part, nblk, 1)), d = sqrt(sum_partials(dxpart, ndx, 2)),
+               xv = sqrt(sum_partials(dxpart + 1, ndx, 2));
+  if (threadIdx.x != 0) return;
   // (refine_init_kernel clears st[0..2]; st[3] is written by refine_seal_kernel)
   const int k = st[1] + 1;
   st[1] = k;
@@ -508,12 +524,12 @@ __global__ void copy_gated_kernel(int64_t n, const double* __restrict__ src, dou
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     dst[i] = src[i];
 }
-void launch_refine_init(const double* r0, int* st, double* nrm, cudaStream_t s) {
-  refine_init_kernel<<<1, 32, 0, s>>>(r0, st, nrm);
+void launch_refine_init(int64_t n, const double* part, int* st, double* nrm, cudaStream_t s) {
+  refine_init_kernel<<<1, 32, 0, s>>>(part, residual_blocks(n), st, nrm);
 }
-void launch_refine_check(const double* rn, const double* dxn, int* st, double* nrm, double tol, int max_sweeps,
-                         cudaStream_t s) {
-  refine_check_kernel<<<1, 32, 0, s>>>(rn, dxn, st, nrm, tol, max_sweeps);
+void launch_refine_check(int64_t n, const double* part, const double* dxpart, int* st, double* nrm, double tol,
+                         int max_sweeps, cudaStream_t s) {
+  refine_check_kernel<<<1, 32, 0, s>>>(part, residual_blocks(n), dxpart, norm_blocks(n), st, nrm, tol, max_sweeps);
 }
 // st[3] = 1 unless the refinement has stopped with MAFEM_OK (the Newton update's skip word)
 __global__ void refine_seal_kernel(int* __restrict__ st) {
@@ -534,8 +550,8 @@ template void launch_band_gather<double>(const DevPatch&, int, int, const BandLa
 template void launch_band_gather<float>(const DevPatch&, int, int, const BandLayout&, int, int, const float*, float*,
                                         cudaStream_t, float*);
 template void launch_band_residual<double>(const double*, const BandLayout&, const double*, const double*, double*,
-                                           double*, double*, cudaStream_t, const int*);
+                                           double*, cudaStream_t, const int*);
 template void launch_band_residual<float>(const float*, const BandLayout&, const double*, const double*, double*,
-                                          double*, double*, cudaStream_t, const int*);
+                                          double*, cudaStream_t, const int*);
 
 }  // namespace mafem

@@ -316,12 +316,15 @@ __global__ void __launch_bounds__(1024) blk_backward_kernel(const T* __restrict_
 // zero outside the panel's rows and columns; inv[p] = Ai then W.  One warp per panel
 // (four per CTA), lane c forming column c of both.
 template <class T, class V>
-__global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__ ab, BlkChain c, int kl,
+__global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__ ab, BlkChain c0, BlkChain c1, int split,
+                                                           int kl,
                                                            const int* __restrict__ perm_all,
                                                            const T* __restrict__ rdiag_all, V* __restrict__ inv) {
   __shared__ V S[4][32][33];  // per warp: S[k][i] = A(j0 + i, j0 + k) of its panel, then Ai
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p = blockIdx.x * 4 + warp;
+  const bool second = (int)blockIdx.x >= split;
+  const BlkChain& c = second ? c1 : c0;
+  const int p = ((int)blockIdx.x - (second ? split : 0)) * 4 + warp;
   if (p >= c.npan) return;  // warp-uniform; only warp-level synchronisation below
   const int j0 = c.ps[p], w = c.ps[p + 1] - j0;
   const T* blk = ab + c.org + j0 * c.si + j0 * c.sj;
@@ -760,11 +763,10 @@ void blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, const int* 
 template <class V, class T>
 int blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
                  V* inv, cudaStream_t st) {
-  for (int k = 0; k < (two ? 2 : 1); ++k) {
-    const BlkChain& c = two ? B.two[k] : B.one;
-    blk_inverses_kernel<T, V><<<(c.npan + 3) / 4, 128, 0, st>>>(ab, c, L.kl, perm_all, rdiag, inv);
-  }
-  return two ? 2 : 1;
+  const BlkChain &c0 = two ? B.two[0] : B.one, &c1 = B.two[1];
+  const int b0 = (c0.npan + 3) / 4, b1 = two ? (c1.npan + 3) / 4 : 0;
+  blk_inverses_kernel<T, V><<<b0 + b1, 128, 0, st>>>(ab, c0, c1, b0, L.kl, perm_all, rdiag, inv);
+  return 1;
 }
 // One cooperative launch over spans a and (optionally) b, its CTAs shared out by their panels.
 template <class F>

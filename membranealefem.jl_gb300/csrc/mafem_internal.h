@@ -131,20 +131,21 @@ int newton_update_blocks(int64_t nmdf);
 void launch_newton_update(const DevPatch& P, const PhysParams& pp, double dt, const double* x, const double* r,
                           double* part, double* out, cudaStream_t st, const int* skip = nullptr,
                           const int* skip2 = nullptr, const int* skip3 = nullptr);
-int band_residual_blocks(int64_t n);
+// res = r - A0 x (x null: r); part[2048]: partial sums of its squares.
 template <class T>
 void launch_band_residual(const T* a0, const BandLayout& L, const double* x, const double* r, double* res,
-                          double* part, double* out, cudaStream_t st, const int* gate = nullptr);
+                          double* part, cudaStream_t st, const int* gate = nullptr);
 void launch_axpy(int64_t n, const double* dx, double* x, cudaStream_t st);
-// x += dx; out[0] = |dx|, out[1] = |x| (part: 2048 doubles of scratch)
-void launch_axpy_norms(int64_t n, const double* dx, double* x, double* part, double* out, cudaStream_t st,
-                       const int* gate = nullptr);
+// x += dx, with partial sums of the squares of both in part[2048]; or with out[0] = |dx|, out[1] = |x|.
+void launch_axpy_partials(int64_t n, const double* dx, double* x, double* part, cudaStream_t st,
+                          const int* gate = nullptr);
+void launch_axpy_norms(int64_t n, const double* dx, double* x, double* part, double* out, cudaStream_t st);
 // Device-side stopping test of a handle's iterative refinement (assemble.cu):
 // st = {done, sweeps, status}, nrm = {|r0|, previous |r|}; kernels given
 // gate = st do nothing once done is set.
-void launch_refine_init(const double* r0, int* st, double* nrm, cudaStream_t s);
-void launch_refine_check(const double* rn, const double* dxn, int* st, double* nrm, double tol, int max_sweeps,
-                         cudaStream_t s);
+void launch_refine_init(int64_t n, const double* part, int* st, double* nrm, cudaStream_t s);
+void launch_refine_check(int64_t n, const double* part, const double* dxpart, int* st, double* nrm, double tol,
+                         int max_sweeps, cudaStream_t s);
 void launch_copy_gated(int64_t n, const double* src, double* dst, const int* gate, cudaStream_t s);
 // st[3] = 1 unless the refinement has stopped with MAFEM_OK.
 void launch_refine_seal(int* st, cudaStream_t s);
