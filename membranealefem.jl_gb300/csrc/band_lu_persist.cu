@@ -110,8 +110,7 @@ enum Role { kWorker, kRhs, kFactor };
 // after a wait ran out.
 template <class T, bool REV, bool TWO>
 __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const BlkChain& C, int p0, int p1, int me, int GW,
-                                               Role role, unsigned char* smem_raw, uint64_t* s_bar, uint32_t& ph0,
-                                               uint32_t& ph1) {
+                                               Role role, unsigned char* smem_raw, uint64_t* s_bar, uint32_t& ph) {
   constexpr int SG = REV ? -1 : 1;  // address step from a row to the next
   __shared__ T s_l[2][32];
   __shared__ int s_p[2];
@@ -159,8 +158,6 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
   T* Lp = reinterpret_cast<T*>(smem_raw) + (TWO ? 64 : 0);  // [kBlkW][LDp] (64 around it: chunk reads past R)
   T* S = Lp + (size_t)a.wmax * LDp + 64;              // [nslot][LDp] column segments
   T* Y = S + (size_t)a.nslot * LDp;                   // [nslot][32]
-  T* rd = Y + a.nslot * 32;                           // [32]
-  int* sp = reinterpret_cast<int*>(rd + 32);          // [32]
   __shared__ int s_sb[8];                             // row 0 of the segments, from S
   int R = 0;  // rows of the current panel's columns
   // panel column k, row 0 (row r: SG r further)
@@ -214,13 +211,7 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
     if (cfirst >= cend && !is_rhs) continue;
     const bool tr_owner = !TWO && p + 1 < npan && me == j1 % GW;
     if (tr_owner) stamp(a.trace, p + 1, 3);
-    if (p > 0) {
-      if (!wait_geq(pdone + p, a.epoch, a.err, &s_ok)) return false;
-      if (!wait_geq(a21cnt + p, a.epoch * w, a.err, &s_ok)) return false;
-    } else if (!wait_geq(pdone, a.epoch, a.err, &s_ok)) {
-      return false;
-    }
-    if (tr_owner) stamp(a.trace, p + 1, 4);
+    if (p > 0 && !wait_geq(a21cnt + p, a.epoch * w, a.err, &s_ok)) return false;
     const int nch = (R - w + 31) / 32;  // 32-row chunks below the diagonal block
     // columns of this panel: the one of panel p + 1 first, then the others, then the right-hand side
     const int nown = cfirst < cend ? (int)((cend - 1 - cfirst) / GW) + 1 : 0;
@@ -233,10 +224,9 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
     if (tid == 0 && is_rhs) s_col[nown] = -1;
     fence_proxy_async_smem();  // earlier reads / writes of the buffers before the TMA writes below
     __syncthreads();
-    // Warp 0 issues the copies: lane l the diagonal block rows [0, w) of panel
-    // column l and the segment of this CTA's column l (both on s_bar[0]), and
-    // rows [w, R) of panel column l (on s_bar[1]).  So the triangular solves
-    // start as soon as the small copies land, while the panel's A21 streams in.
+    // Warp 0 issues the copies, while the panel's diagonal block is still being
+    // factorised: lane l the rows below it (A21) of panel column l and the segment of
+    // this CTA's column l.
     auto issue_cols = [&](int b0, int nb, bool with_panel) {
       if (warp != 0) return;
       fence_proxy_async_global();  // data written by ordinary stores (here or, before a flag, elsewhere)
@@ -250,48 +240,27 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
         s_sb[lane] = lane * LDp + off + (REV ? R - 1 : 0);
         sd = S + lane * LDp + off;
       }
-      const bool pc = with_panel && lane < w;
-      const T* pd_src = pc ? ab + j0 * SG + (j0 + lane) * sj : nullptr;
-      // rows [0, P1) of panel column `lane` (diagonal block + chunk 0, the rows the
-      // next factorisation's update reads) on s_bar[0], rows [P1, R) on s_bar[1];
-      // P1 = first row at or after w + 32 that 16-byte-aligned copies can start at
-      // (REV: that they can end before)
-      const int br = min(R, w + 32);
-      const int P1 = min(R, br + (REV ? (a.off + lane + 1 - br) & (E - 1) : (-(a.off - lane + br)) & (E - 1)));
-      T* const pt = REV ? lpa(lane) - (P1 - 1) : lpa(lane);            // rows [0, P1)
-      const T* const pt_src = REV ? pd_src - (P1 - 1) : pd_src;
-      T* const pb = REV ? lpa(lane) - (R - 1) : lpa(lane) + P1;        // rows [P1, R)
-      const T* const pb_src = REV ? pd_src - (R - 1) : pd_src + P1;
-      uint32_t b0b = 0, b1b = 0;
-      if (lane < nb) b0b += seg_copy(sd, ss, R, &s_bar[0], 0);
-      if (pc) {
-        b0b += seg_copy(pt, pt_src, P1, &s_bar[0], 0);
-        if (R > P1) b1b += seg_copy(pb, pb_src, R - P1, &s_bar[1], 0);
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        b0b += __shfl_xor_sync(kFull, b0b, o);
-        b1b += __shfl_xor_sync(kFull, b1b, o);
-      }
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&s_bar[0], b0b);
-        if (with_panel) mbar_arrive_expect_tx(&s_bar[1], b1b);
-      }
+      const bool pc = with_panel && lane < w && R > w;
+      const int lo = REV ? 1 - R : w;  // rows [w, R), from the lowest address
+      T* const pd = lpa(lane) + lo;
+      const T* const pd_src = ab + j0 * SG + (j0 + lane) * sj + lo;
+      uint32_t bytes = 0;
+      if (lane < nb) bytes += seg_copy(sd, ss, R, s_bar, 0);
+      if (pc) bytes += seg_copy(pd, pd_src, R - w, s_bar, 0);
+      for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(kFull, bytes, o);
+      if (lane == 0) mbar_arrive_expect_tx(s_bar, bytes);
       __syncwarp();
       for (int mode = 1; mode <= 2; ++mode) {
-        if (lane < nb) seg_copy(sd, ss, R, &s_bar[0], mode);
-        if (pc) {
-          seg_copy(pt, pt_src, P1, &s_bar[0], mode);
-          if (R > P1) seg_copy(pb, pb_src, R - P1, &s_bar[1], mode);
-        }
+        if (lane < nb) seg_copy(sd, ss, R, s_bar, mode);
+        if (pc) seg_copy(pd, pd_src, R - w, s_bar, mode);
       }
     };
     issue_cols(0, min(a.nslot, ncol), true);
-    if (tid >= 32 && tid < 32 + w) {
-      rd[tid - 32] = __ldcg(rdiag + j0 + tid - 32);
-      sp[tid - 32] = __ldcg(perm_all + (size_t)p * kBlkW + tid - 32);
+    if (!wait_geq(pdone + p, a.epoch, a.err, &s_ok)) {
+      wait_bar(s_bar, ph);  // no copy in flight when the CTA ends
+      return false;
     }
-    if (!wait_bar(&s_bar[0], ph0)) return false;  // tops + diagonal block
-    if (tr_owner) stamp(a.trace, p + 1, 5);
+    if (tr_owner) stamp(a.trace, p + 1, 4);
 
     for (int b0 = 0; b0 < ncol; b0 += a.nslot) {
       const int nb = min(a.nslot, ncol - b0);
@@ -299,8 +268,22 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
         fence_proxy_async_smem();
         __syncthreads();
         issue_cols(b0, nb, false);
-        if (!wait_bar(&s_bar[0], ph0)) return false;
       }
+      // this lane's row of the diagonal block in registers (nothing to load on the
+      // dependency chains): L(lane, k) for k < lane, U(lane, k) for k > lane
+      T Tr[32], rl = T(0);
+      int pr = 0;
+      if (warp < nb) {
+        const T* row = ab + (j0 + min(lane, w - 1)) * SG + j0 * sj;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) Tr[k] = (k < w && lane < w) ? __ldcg(row + k * sj) : T(0);
+        if (lane < w) {
+          rl = __ldcg(rdiag + j0 + lane);
+          pr = __ldcg(perm_all + (size_t)p * kBlkW + lane);
+        }
+      }
+      if (!wait_bar(s_bar, ph)) return false;
+      if (tr_owner && b0 == 0) stamp(a.trace, p + 1, 5);
       // triangular solves, one warp per column: u = L11^-1 P s[0:w], y = U11^-1 u (kept as Y in place of A12)
       if (warp < a.nslot) {
         T v = T(0);
@@ -308,12 +291,7 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
           const int c = s_col[b0 + warp];
           const T* s = S + s_sb[warp];
           T* dst = c < 0 ? rhs + j0 * SG : ab + j0 * SG + c * sj;
-          // this lane's row of the diagonal block in registers (no shared-memory
-          // load on the dependency chains): L(lane, k) for k < lane, U(lane, k) for k > lane
-          T Tr[32];
-#pragma unroll
-          for (int k = 0; k < 32; ++k) Tr[k] = (k < w && lane < w) ? lpa(k)[lane * SG] : T(0);
-          T x = lane < w ? s[sp[lane] * SG] : T(0);  // row `lane` of the permuted top
+          T x = lane < w ? s[pr * SG] : T(0);  // row `lane` of the permuted top
 #pragma unroll
           for (int k = 0; k < 32; ++k) {
             if (k < w) {
@@ -323,7 +301,6 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
           }
           // y = U11^-1 u with this lane's U row pre-scaled by 1/U(lane, lane)
           // (unit diagonal): each step is one shuffle and one FMA
-          const T rl = lane < w ? rd[lane] : T(0);
 #pragma unroll
           for (int k = 0; k < 32; ++k)
             if (k > lane) Tr[k] *= rl;
@@ -381,7 +358,6 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
         }
         if (tid == 0) atomicAdd(critcnt + p + 1, 1);
         if (tr_owner) stamp(a.trace, p + 1, 7);
-        if (!wait_bar(&s_bar[1], ph1)) return false;  // the rest of A21
         if (reach) {
           rows(0, 1, min(1, nch), nch);
           __threadfence();
@@ -391,7 +367,6 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
         if (tr_owner) stamp(a.trace, p + 1, 8);
         q0 = 1;
       }
-      if (b0 == 0 && q0 == 0 && !wait_bar(&s_bar[1], ph1)) return false;  // the rest of A21
       if (q0 < nb) rows(q0, nb, 0, nch);
     }
   }
@@ -403,21 +378,20 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
 template <class T, bool TWO>
 __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t s_bar[2];  // TMA completion: [0] tops, [1] the panel's A21
+  __shared__ __align__(8) uint64_t s_bar;  // completion of the TMA copies
   const int G = (int)gridDim.x;
   int me = blockIdx.x;
   if (threadIdx.x == 0) {
-    mbar_init(&s_bar[0], 1);
-    mbar_init(&s_bar[1], 1);
+    mbar_init(&s_bar, 1);
     mbar_init_fence();
   }
   __syncthreads();
-  uint32_t ph0 = 0, ph1 = 0;
+  uint32_t ph = 0;
   if constexpr (!TWO) {
     const int GW = G - 1 - (a.rhs ? 1 : 0);
     persist_panels<T, false, false>(a, a.c[0], 0, a.c[0].npan, me, GW,
-                                    me == G - 1 ? kFactor : a.rhs && me == G - 2 ? kRhs : kWorker, smem_raw, s_bar, ph0,
-                                    ph1);
+                                    me == G - 1 ? kFactor : a.rhs && me == G - 2 ? kRhs : kWorker, smem_raw, &s_bar,
+                                    ph);
   } else {
     __shared__ int s_ok;
     // first each chain on its own CTAs, the forward one up to panel pm, then the rest on all of them
@@ -427,7 +401,7 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
     if (rev) me -= a.split;
     Role role = me == G0 - 1 ? kFactor : a.rhs && me == G0 - 2 ? kRhs : kWorker;
     if (rev) {
-      if (!persist_panels<T, true, true>(a, a.c[1], 0, a.c[1].npan, me, G0 - nx, role, smem_raw, s_bar, ph0, ph1)) return;
+      if (!persist_panels<T, true, true>(a, a.c[1], 0, a.c[1].npan, me, G0 - nx, role, smem_raw, &s_bar, ph)) return;
     }
 #pragma unroll 1
     for (int half = rev || role == kFactor ? 1 : 0; half < 2; ++half) {
@@ -444,8 +418,8 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
         }
       }
       const int p0 = half == 1 && role != kFactor ? a.pm : 0, p1 = half == 0 ? a.pm : a.c[0].npan;
-      if (!persist_panels<T, false, true>(a, a.c[0], p0, p1, me, half == 0 ? a.split - nx : G - nx, role, smem_raw, s_bar,
-                                          ph0, ph1))
+      if (!persist_panels<T, false, true>(a, a.c[0], p0, p1, me, half == 0 ? a.split - nx : G - nx, role, smem_raw, &s_bar,
+                                          ph))
         return;
     }
   }
@@ -458,7 +432,7 @@ static size_t persist_smem(const BandLayout& L, int wmax, int nslot, bool two) {
   constexpr int E = 16 / (int)sizeof(T);
   const size_t rmax = (size_t)wmax + L.kl;
   const size_t ldp = (rmax + 2 * E - 1) / E * E;
-  return ((two ? 64 : 0) + (size_t)wmax * ldp + 64 + nslot * (ldp + 32) + 32) * sizeof(T) + 32 * sizeof(int);
+  return ((two ? 64 : 0) + (size_t)wmax * ldp + 64 + nslot * (ldp + 32)) * sizeof(T);
 }
 
 template <class T, bool TWO>
