@@ -38,15 +38,15 @@ __device__ __forceinline__ unsigned pkey(float v) {
 // every f64<->f32 conversion) occupies a sub-partition's FP64 pipe for ~64
 // cycles, so this takes three pipe slots where a divide takes a long sequence.
 // Pivots are normal numbers here (pkey rejects the rest), which the ftz form
-// requires.
+// requires.  FP32 likewise, with the one correction it needs.
 __device__ __forceinline__ void recip2(double d, double& r0, double& t) {
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(d));
   const double e = fma(-d, r0, 1.0);
   t = fma(e, e, e);
 }
 __device__ __forceinline__ void recip2(float d, float& r0, float& t) {
-  r0 = __frcp_rn(d);
-  t = 0.0f;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r0) : "f"(d));
+  t = fmaf(-d, r0, 1.0f);
 }
 template <class T>
 __device__ __forceinline__ T mul_recip(T x, T r0, T t) {
@@ -157,19 +157,14 @@ __device__ __forceinline__ T blk_pivot_step(int k, T col, int w, int lane, int b
                                             T (*s_l)[32], int* s_p, int* perm, T* rdiag, int* info, int& op,
                                             T& ol, int nthreads) {
   T r0, t;
-  if constexpr (sizeof(T) == 8) recip2(col, r0, t);  // every lane's own, beside the search (its pivot step: 0.46 -> 0.42 us)
+  recip2(col, r0, t);  // every lane's own, beside the search
   const int bk = __shfl_sync(kFull, bend, k);  // the block of position k ends at row bk
-  const bool cand = lane < bk && !((E >> lane) & 1u);
-  const unsigned key = cand ? pkey(col) : 0u;
+  // key and lane in one word: the largest key (to its top 27 bits), then the first such row
+  const unsigned key = (lane < bk && !((E >> lane) & 1u)) ? (pkey(col) & ~31u) | (31u - lane) : 0u;
   const unsigned mx = __reduce_max_sync(kFull, key);
-  const unsigned bal = __ballot_sync(kFull, cand && key == mx);
-  const int p = __ffs(bal) - 1;  // the candidates are never empty
-  if constexpr (sizeof(T) == 8) {
-    r0 = __shfl_sync(kFull, r0, p);
-    t = __shfl_sync(kFull, t, p);
-  } else {
-    recip2(__shfl_sync(kFull, col, p), r0, t);
-  }
+  const int p = 31 - (int)(mx & 31u);  // the candidates are never empty
+  r0 = __shfl_sync(kFull, r0, p);
+  t = __shfl_sync(kFull, t, p);
   const bool act = lane < w && lane != p && !((E >> lane) & 1u);
   const T l = act ? mul_recip(col, r0, t) : T(0);
   s_l[k & 1][lane] = l;
@@ -178,7 +173,7 @@ __device__ __forceinline__ T blk_pivot_step(int k, T col, int w, int lane, int b
   if (lane == 0) {
     perm[k] = p;
     rdiag[k] = fma(r0, t, r0);
-    if (mx == 0u) atomicCAS(info, 0, col1);
+    if (mx < 32u) atomicCAS(info, 0, col1);
   }
   op = p;
   ol = l;

@@ -87,7 +87,7 @@ __device__ __forceinline__ bool wait_geq(const int* p, int target, int* err, int
   if (threadIdx.x == 0) {
     int ok = 1;
     for (int it = 0; ld_acquire(p) < target; ++it) {
-      if (it > kSpinLimit || *(volatile int*)err) {
+      if (it > kSpinLimit || ((it & 31) == 31 && *(volatile int*)err)) {  // (a look at it delays the next poll)
         atomicCAS(err, 0, 1);
         ok = 0;
         break;
@@ -138,8 +138,6 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
       stamp(a.trace, t, 1);
       blk_panel_factor<T, true>(ab + j0 * SG + j0 * sj, SG, sj, j0, wt, REV ? a.n - j0 : j0 + 1, SG, C.blk_end + j0,
                                 perm_all + (size_t)t * kBlkW, rdiag + j0, a.info, s_l, s_p);
-      fence_proxy_async_global();  // the factors are read by TMA on other SMs
-      __threadfence();
       __syncthreads();
       if (tid == 0) st_release(pdone + t, a.epoch);
       stamp(a.trace, t, 2);
