@@ -645,6 +645,7 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
       J.rhs = h->d_r;
       J.x = h->d_x;
       J.res = h->d_res;
+      J.rs = h->d_part + 2048;  // unused by this form
       J.xs = reinterpret_cast<float2*>(h->d_dx);  // d_dx: n doubles, unused by this form
       J.L = h->L;
       J.kuf = h->blk.kuf;
@@ -1878,7 +1879,7 @@ static cudaError_t run_round(RoundRunner& R, const PatchJob* d_jobs, const AsmJo
     return reinterpret_cast<const int*>(dr + (t == kOffDir ? dir_off : RL.off[t])) + g0;
   };
   const int ng = (int)groups.size() - 1;
-  *launches = (any_dir ? 1 : 0) + (any_pred ? 1 : 0) + 2 * ng + 2 + patch_solve_launches(G, m) + 2;
+  *launches = (any_dir ? 1 : 0) + (any_pred ? 1 : 0) + 2 * ng + 2 + patch_solve_launches(G, m, max_sweeps) + 2;
 
   auto enqueue = [&](bool capturing) -> cudaError_t {
     const unsigned fl = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
@@ -2081,7 +2082,7 @@ extern "C" int mafem_batch_step(mafem_batch* b, const double* times, const doubl
             st[i] = MAFEM_ERR_CUDA;
             continue;
           }
-          if (i == pj[0]) h->launches += patch_solve_launches(G, (int)pj.size());  // counted once
+          if (i == pj[0]) h->launches += patch_solve_launches(G, (int)pj.size(), b->max_sweeps);  // counted once
           const int rc = iter_enqueue_patch_end(h, b->bev);
           if (rc != MAFEM_OK) st[i] = rc;
         }

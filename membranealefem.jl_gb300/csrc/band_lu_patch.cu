@@ -563,7 +563,9 @@ __device__ __forceinline__ float block_times(const float* m, const float* x) {
 // instructions, one load per 32 entries.
 // Measured on a GB300, one forward and backward pass, against whole-CTA steps with
 // three small products and three barriers per panel: 16 x 16 ALEVB (70 panels) 666
-// -> 150 us, 32 x 32 3.13 -> 1.07 ms, 48 x 48 (RPT = 2) 10.7 -> 3.06 ms.
+// -> 150 us, 32 x 32 3.13 -> 1.07 ms, 48 x 48 (RPT = 2) 10.7 -> 3.06 ms; 116 us,
+// 0.83 and 2.37 ms in a kernel without the residual, whose registers had made this
+// pass spill.
 // prof (trace mode, optional): [0] forward, [1] backward time of warp 0 in ns.
 __device__ __forceinline__ void solve_barrier() { bar_sync_n(1, kRT); }
 // dot product of 32 register values with 32 values in shared memory (16-byte aligned)
@@ -796,7 +798,7 @@ __device__ __forceinline__ void patch_solve_pass(const PatchJob& J, float* v, co
 // One column run [j0, j1) of a warp's double-float row sums (see patch_residual).
 __device__ __forceinline__ void residual_run(const float* a, int64_t ldm, const float2* xs, int64_t j0, int64_t j1,
                                              float& sh, float& sl) {
-  constexpr int kB = 16;  // columns whose loads are in flight together
+  constexpr int kB = 16;  // columns whose loads, of A0 and of x, are in flight together
   for (int64_t j = j0; j < j1; j += kB) {
     const int cnt = (int)min64b(kB, j1 - j);  // warp-uniform
     float av[kB];
@@ -837,16 +839,16 @@ __device__ __forceinline__ void residual_run(const float* a, int64_t ldm, const 
 // them: at most two runs per grid row.  The columns skipped hold stored
 // zeros, whose products leave the pair unchanged: the sums equal a walk of
 // the whole band window.
-__device__ double patch_residual(const PatchJob& J, const float2* xs, double* red) {
+__device__ __forceinline__ double residual_rows(const PatchJob& J, const float2* xs, int w0, int nw) {
   const BandLayout L = J.L;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int64_t ldm = L.ldb - 1;
   double ss = 0.0;
   // With nb >= 32 every (i, j) of the band window [rb - ku, rb + 32 + kl) lies
   // inside the band's storage, where the entries outside the band are stored
   // zeros, so A0(i, j) = a[j * ldm + lane] with a at row rb of column 0 needs
   // no guard but i < n; the runs are clipped to that window.
-  for (int64_t rb = (int64_t)warp * 32; rb < L.n; rb += kRT) {
+  for (int64_t rb = (int64_t)w0 * 32; rb < L.n; rb += (int64_t)nw * 32) {
     const int64_t i = rb + lane;
     const bool live = i < L.n;
     const int64_t jlo = rb - L.ku > 0 ? rb - L.ku : 0;
@@ -891,12 +893,44 @@ __device__ double patch_residual(const PatchJob& J, const float2* xs, double* re
       ss = fma(r, r, ss);
     }
   }
-  return sqrt(block_sum(ss, red));
+  return ss;
+}
+__device__ double patch_residual(const PatchJob& J, const float2* xs, double* red) {
+  return sqrt(block_sum(residual_rows(J, xs, threadIdx.x >> 5, kRT / 32), red));
+}
+// The residual after a sweep on kResC CTAs per patch: partial sums of its squares to J.rs + 8.
+constexpr int kResC = 8, kResT = 256;
+__global__ void __launch_bounds__(kResT) patch_residual_kernel(const PatchJob* __restrict__ jobs,
+                                                              const int* __restrict__ order) {
+  const PatchJob& J = jobs[order[blockIdx.x / kResC]];
+  const int c = blockIdx.x % kResC;
+  if (J.rs[4] != 0.0) return;  // this patch's refinement has ended
+  __shared__ double red[kResT / 32];
+  double ss = residual_rows(J, J.xs, c * (kResT / 32) + (threadIdx.x >> 5), kResC * kResT / 32);
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(kFull, ss, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int q = 0; q < kResT / 32; ++q) t += red[q];
+    J.rs[8 + c] = t;
+  }
 }
 
-template <int RPT>
+
+// The refinement.  The first kSplit sweeps are launches of their own (MONO = false),
+// each followed by patch_residual_kernel, which has several CTAs per patch where a
+// sweep can have but one; this kernel with MONO = true then ends the patches that
+// need more.  Measured on a GB300, the residual of one patch and the whole
+// refinement (two sweeps; three at 48 x 48), against sweeps and residuals in one
+// CTA: 16 x 16 ALEVB 157 -> 51 and 485 -> 342 us, 32 x 32 706 -> 171 us and 2.96 ->
+// 1.96 ms, 48 x 48 1740 -> 383 us and 8.8 -> 5.4 ms.  What a sweep hands on stands in J.rs: [0] |r0|, [1] the last
+// correction's norm, [2] and [3] the norms of the current one and of x, [4] nonzero
+// once the patch is done, [8 ..] the residual's partial sums.
+constexpr int kSplit = 3;
+template <int RPT, bool MONO>
 __global__ void __launch_bounds__(kRT, 1) patch_refine_kernel(const PatchJob* __restrict__ jobs,
-                                                             const int* __restrict__ order, int max_sweeps,
+                                                             const int* __restrict__ order, int k0, int max_sweeps,
                                                              double tol) {
   const PatchJob& J = jobs[order[blockIdx.x]];
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -908,95 +942,129 @@ __global__ void __launch_bounds__(kRT, 1) patch_refine_kernel(const PatchJob* __
   const int64_t n = J.L.n;
   int* stat = J.stat;  // [0] status, [1] sweeps
   float2* xs = J.xs;   // x split into two floats
-  for (int k = tid; k <= J.npan; k += kRT) ps[k] = J.ps[k];
-  if (J.info[1] != 0 || J.info[0] != 0) {  // a bounded wait ran out, or a node block had no usable pivot
+  auto end = [&](int status, int sweeps) MAFEM_INLINE {  // by every thread, none of which reads J.rs[4] again
     if (tid == 0) {
-      stat[0] = J.info[1] != 0 ? MAFEM_ERR_CUDA : MAFEM_ZERO_PIVOT;
-      stat[1] = 0;
+      stat[0] = status;
+      stat[1] = sweeps;
+      J.rs[4] = 1.0;
     }
+  };
+  double r0, rn, prev_dn;
+  if (k0 == 0) {
+    if (J.info[1] != 0 || J.info[0] != 0) {  // a bounded wait ran out, or a node block had no usable pivot
+      end(J.info[1] != 0 ? MAFEM_ERR_CUDA : MAFEM_ZERO_PIVOT, 0);
+      return;
+    }
+    double ss = 0.0;
+    for (int64_t i = tid; i < n; i += kRT) {
+      const double r = J.rhs[i];
+      J.res[i] = r;
+      J.x[i] = 0.0;
+      ss = fma(r, r, ss);
+    }
+    r0 = rn = sqrt(block_sum(ss, red));
+    prev_dn = INFINITY;
+    if (tid == 0) {
+      J.rs[0] = r0;
+      J.rs[4] = 0.0;
+    }
+    if (!(r0 > 0.0)) {
+      end(MAFEM_OK, 0);
+      return;
+    }
+  } else if (J.rs[4] != 0.0) {
     return;
   }
-  double ss = 0.0;
-  for (int64_t i = tid; i < n; i += kRT) {
-    const double r = J.rhs[i];
-    J.res[i] = r;
-    J.x[i] = 0.0;
-    ss = fma(r, r, ss);
-  }
-  const double r0 = sqrt(block_sum(ss, red));
+  for (int k = J.npan - tid; k >= 0; k -= kRT) ps[k] = J.ps[k];
   // trace: per sweep 4 stamps after J.trace's 6 per panel -- [0] sweep start,
   // [1] substitutions done, [2] x updated and norms formed, [3] residual done
   long long* tr = J.trace ? J.trace + (size_t)J.npan * 6 : nullptr;
-  // Stop when the error left in x is small against x.  After sweep k that
-  // error is about the next correction, rho |d_k| with rho = |d_k| / |d_k-1|
-  // the sweeps' contraction: stop once rho |d_k| <= tol |x| while the sweeps
-  // contract (rho <= 1/2), or once |d_k| <= tol |x| itself.  A bound on the
-  // forward error of x whatever the conditioning, where a residual test would
-  // accept a large error in x on an ill-conditioned tangent; the residual
-  // after the final sweep is never needed.
-  int status = MAFEM_OK, sweeps = 0;
-  double rn = r0, prev_dn = INFINITY;
-  if (r0 > 0.0) {
-    status = MAFEM_REFINE_STALLED;
-    for (int k = 0; k < max_sweeps; ++k) {
-      long long* trk = tr && k < kTraceSweeps ? tr + 4 * k : nullptr;
-      stamp(trk, 0);
-      const double sc = 1.0 / rn;
-      for (int64_t i = tid; i < n; i += kRT) v[i] = (float)(J.res[i] * sc);
-      __syncthreads();
-      long long* prof = tr && k == 0 ? tr + 4 * kTraceSweeps : nullptr;
-      patch_solve_pass<RPT>(J, v, ps, S, prof);
-      stamp(trk, 1);
-      double dd = 0.0, xx = 0.0;
-      for (int64_t i = tid; i < n; i += kRT) {
-        const double d = rn * (double)v[i];
-        const double x = J.x[i] + d;
-        J.x[i] = x;
-        const float xh = (float)x;
-        xs[i] = make_float2(xh, (float)(x - (double)xh));
-        dd = fma(d, d, dd);
-        xx = fma(x, x, xx);
+  // After sweep k (counted from 0) and its residual rn: a residual at FP64 level
+  // (<= min(tol, 1e-10) |r0|) ends the solve: on large, stiff tangents the relative
+  // correction has a rounding floor (about 1e-9 on the 64 x 64 patch) that a tight
+  // tol would never reach.  So does the end of the contraction: at the rounding
+  // floor (the correction a small part of x) the solution is as accurate as the
+  // factors allow, and is accepted.
+  auto after_residual = [&](int k, double dn, double xn) -> bool {
+    if (tr && tid == 0 && k < kTraceSweeps) {  // trace: the residual after each sweep, relative to |r0|
+      stamp(tr + 4 * k, 3);
+      tr[4 * kTraceSweeps + 16 + k] = __double_as_longlong(rn / r0);
+    }
+    if (!isfinite(rn)) {
+      end(MAFEM_NAN_DETECTED, k + 1);
+    } else if (rn <= fmin(tol, 1e-10) * r0) {
+      end(MAFEM_OK, k + 1);
+    } else if (k >= 3 && dn > 0.5 * prev_dn) {
+      end(dn <= 1e-8 * xn ? MAFEM_OK : MAFEM_REFINE_STALLED, k + 1);
+    } else {
+      return true;
+    }
+    return false;
+  };
+  if (k0 > 0) {
+    r0 = J.rs[0];
+    prev_dn = J.rs[1];
+    const double dn = J.rs[2], xn = J.rs[3];
+    double ss = 0.0;
+    for (int q = 0; q < kResC; ++q) ss += J.rs[8 + q];
+    rn = sqrt(ss);
+    __syncthreads();  // J.rs is read
+    if (!after_residual(k0 - 1, dn, xn)) return;
+    prev_dn = dn;
+  }
+  for (int k = k0;; ++k) {
+    if (k >= max_sweeps) {
+      end(MAFEM_REFINE_STALLED, k);
+      return;
+    }
+    long long* trk = tr && k < kTraceSweeps ? tr + 4 * k : nullptr;
+    stamp(trk, 0);
+    const double sc = 1.0 / rn;
+    for (int64_t i = tid; i < n; i += kRT) v[i] = (float)(J.res[i] * sc);
+    __syncthreads();
+    patch_solve_pass<RPT>(J, v, ps, S, tr && k == 0 ? tr + 4 * kTraceSweeps : nullptr);
+    stamp(trk, 1);
+    double dd = 0.0, xx = 0.0;
+    for (int64_t i = tid; i < n; i += kRT) {
+      const double d = rn * (double)v[i];
+      const double x = J.x[i] + d;
+      J.x[i] = x;
+      const float xh = (float)x;
+      xs[i] = make_float2(xh, (float)(x - (double)xh));
+      dd = fma(d, d, dd);
+      xx = fma(x, x, xx);
+    }
+    const double dn = sqrt(block_sum(dd, red));
+    const double xn = sqrt(block_sum(xx, red));
+    stamp(trk, 2);
+    if (!isfinite(dn) || !isfinite(xn)) {
+      end(MAFEM_NAN_DETECTED, k + 1);
+      return;
+    }
+    // Stop when the error left in x is small against x.  After sweep k that
+    // error is about the next correction, rho |d_k| with rho = |d_k| / |d_k-1|
+    // the sweeps' contraction: stop once rho |d_k| <= tol |x| while the sweeps
+    // contract (rho <= 1/2), or once |d_k| <= tol |x| itself.  A bound on the
+    // forward error of x whatever the conditioning, where a residual test would
+    // accept a large error in x on an ill-conditioned tangent; the residual
+    // after the final sweep is never needed.
+    const double rho = dn / prev_dn;  // 0 after the first sweep (prev_dn infinite)
+    if (dn <= tol * xn || (k >= 1 && rho <= 0.5 && rho * dn <= tol * xn)) {
+      end(MAFEM_OK, k + 1);
+      return;
+    }
+    if constexpr (!MONO) {
+      if (tid == 0) {
+        J.rs[1] = prev_dn;
+        J.rs[2] = dn;
+        J.rs[3] = xn;
       }
-      const double dn = sqrt(block_sum(dd, red));
-      const double xn = sqrt(block_sum(xx, red));
-      stamp(trk, 2);
-      sweeps = k + 1;
-      if (!isfinite(dn) || !isfinite(xn)) {
-        status = MAFEM_NAN_DETECTED;
-        break;
-      }
-      const double rho = dn / prev_dn;  // 0 after the first sweep (prev_dn infinite)
-      if (dn <= tol * xn || (k >= 1 && rho <= 0.5 && rho * dn <= tol * xn)) {
-        status = MAFEM_OK;
-        break;
-      }
+      return;
+    } else {
       rn = patch_residual(J, xs, red);  // block_sum orders the x / xs writes before it
-      stamp(trk, 3);
-      if (tr && tid == 0 && k < kTraceSweeps)  // trace: the residual after each sweep, relative to |r0|
-        tr[4 * kTraceSweeps + 16 + k] = __double_as_longlong(rn / r0);
-      if (!isfinite(rn)) {
-        status = MAFEM_NAN_DETECTED;
-        break;
-      }
-      // A residual at FP64 level (<= min(tol, 1e-10) |r0|) also ends the solve:
-      // on large, stiff tangents the relative correction has a rounding floor
-      // (about 1e-9 on the 64 x 64 patch) that a tight tol would never reach.
-      if (rn <= fmin(tol, 1e-10) * r0) {
-        status = MAFEM_OK;
-        break;
-      }
-      if (k >= 3 && dn > 0.5 * prev_dn) {  // no longer contracting
-        // at the rounding floor (the correction a small part of x) the
-        // solution is as accurate as the factors allow: accept it
-        if (dn <= 1e-8 * xn) status = MAFEM_OK;
-        break;
-      }
+      if (!after_residual(k, dn, xn)) return;
       prev_dn = dn;
     }
-  }
-  if (tid == 0) {
-    stat[0] = status;
-    stat[1] = sweeps;
   }
 }
 
@@ -1037,8 +1105,10 @@ int patch_solve_setup() {
   if (cudaFuncSetAttribute(patch_factor_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
       cudaFuncSetAttribute(patch_factor_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
       cudaFuncSetAttribute(patch_factor_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
-      cudaFuncSetAttribute(patch_refine_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
-      cudaFuncSetAttribute(patch_refine_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
+      cudaFuncSetAttribute(patch_refine_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
+      cudaFuncSetAttribute(patch_refine_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
+      cudaFuncSetAttribute(patch_refine_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
+      cudaFuncSetAttribute(patch_refine_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
     return 0;
   return dyn;
 }
@@ -1072,9 +1142,16 @@ static cudaError_t launch_factor(const PatchJob* d_jobs, const int* d_order, int
 // or columns beyond a panel than one set of the update warps holds.
 bool patch_wide(int kl, int kuf) { return kl > kRowT || kuf > kRowT; }
 static cudaError_t launch_refine(const PatchJob* d_jobs, const int* d_order, int njobs, bool wide, size_t smem,
-                                 int max_sweeps, double tol, cudaStream_t st) {
-  if (wide) patch_refine_kernel<2><<<njobs, kRT, smem, st>>>(d_jobs, d_order, max_sweeps, tol);
-  else patch_refine_kernel<1><<<njobs, kRT, smem, st>>>(d_jobs, d_order, max_sweeps, tol);
+                                 int max_sweeps, double tol, cudaStream_t st, bool apart = true) {
+  auto sweeps = [&](auto kern, int k0) { kern<<<njobs, kRT, smem, st>>>(d_jobs, d_order, k0, max_sweeps, tol); };
+  const int split = apart ? std::min(kSplit, max_sweeps) : 0;
+  for (int k = 0; k < split; ++k) {
+    if (wide) sweeps(patch_refine_kernel<2, false>, k);
+    else sweeps(patch_refine_kernel<1, false>, k);
+    patch_residual_kernel<<<njobs * kResC, kResT, 0, st>>>(d_jobs, d_order);
+  }
+  if (wide) sweeps(patch_refine_kernel<2, true>, split);
+  else sweeps(patch_refine_kernel<1, true>, split);
   return cudaGetLastError();
 }
 
@@ -1131,9 +1208,10 @@ cudaError_t patch_time_factor(const PatchJob* d_jobs, const int* d_order1, int n
   return e;
 }
 
-int patch_solve_launches(const PatchGroups& G, int njobs) {
+int patch_solve_launches(const PatchGroups& G, int njobs, int max_sweeps) {
   const int groups = (G.n4 > 0) + (G.n2 > 0) + (njobs - G.n4 - G.n2 > 0);
-  return groups + (groups > 1 ? 2 : 1);  // the factor launches and one refinement per stream
+  // the factor launches, and the refinement of each stream (launch_refine)
+  return groups + 1 + 2 * std::min(kSplit, max_sweeps) + (groups > 1 ? 1 : 0);
 }
 
 cudaError_t patch_solve(const PatchJob* d_jobs, const int* d_order, const PatchGroups& G, int njobs,
@@ -1145,7 +1223,8 @@ cudaError_t patch_solve(const PatchJob* d_jobs, const int* d_order, const PatchG
   // CTAs; the first non-empty group on st, the others one after the other on
   // st2 beside it (their chains are the shorter ones).  Each stream refines its
   // own patches as soon as their factors are done, so the refinement of one
-  // group overlaps the factorisations of the other.
+  // group overlaps the factorisations of the other.  The first group's sweeps and
+  // residuals are launches apart (it ends the round); beside it one kernel will do.
   const int cnt[3] = {G.n4, G.n2, njobs - G.n4 - G.n2}, nrs[3] = {4, 2, 1};
   int first = 0;
   while (first < 3 && cnt[first] == 0) ++first;
@@ -1165,7 +1244,7 @@ cudaError_t patch_solve(const PatchJob* d_jobs, const int* d_order, const PatchG
   if (fork && e == cudaSuccess) {
     bool wide = false;
     for (int g = first + 1; g < 3; ++g) wide |= cnt[g] > 0 && G.wide[g];
-    e = launch_refine(d_jobs, d_order + cnt[first], njobs - cnt[first], wide, smem_refine, max_sweeps, tol, st2);
+    e = launch_refine(d_jobs, d_order + cnt[first], njobs - cnt[first], wide, smem_refine, max_sweeps, tol, st2, false);
   }
   if (fork && e == cudaSuccess) e = cudaEventRecord(ev_join, st2);
   if (fork && e == cudaSuccess) e = cudaStreamWaitEvent(st, ev_join, 0);

@@ -368,6 +368,7 @@ struct PatchJob {
   double* x;            // [n] solution
   double* res;          // [n] FP64 residual (workspace)
   float2* xs;           // [n] x as two floats (workspace)
+  double* rs;           // [16] the refinement's state between its launches (patch_refine_kernel)
   BandLayout L;
   int kuf, npan;
   long long* trace;     // optional: 6 globaltimer stamps per panel (patch_factor_kernel)
@@ -412,7 +413,7 @@ struct PatchGroups {
   int64_t key() const { return n4 | ((int64_t)n2 << 24) | ((int64_t)wide[0] << 48) | ((int64_t)wide[1] << 49) | ((int64_t)wide[2] << 50); }
 };
 // kernel launches patch_solve makes for these group sizes
-int patch_solve_launches(const PatchGroups& G, int njobs);
+int patch_solve_launches(const PatchGroups& G, int njobs, int max_sweeps);
 // Factor and solve the jobs d_order[0 .. njobs): the first G.n4 on four-CTA
 // clusters, the next G.n2 on two-CTA clusters, the rest one CTA each -- the first
 // non-empty group on st, the others after one another on st2 (forked from and
