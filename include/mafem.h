@@ -341,19 +341,19 @@ int mafem_server_get_stats(const mafem_server* s, mafem_server_stats* out);
 /* ---- diagnostics --------------------------------------------------------------- */
 
 /* Assemble the resident state at (time, dt), factor once with the persistent
- * node-block LU and copy its per-panel clock stamps (12 int64 per panel) to
+ * node-block LU as one chain of panels and copy its per-panel clock stamps (12 int64 per panel) to
  * out[0 .. 12 npan).  cap >= 12 npan.  Returns npan, or MAFEM_ERR_UNSUPPORTED if
  * the handle does not use that factorisation. */
 int mafem_trace_factor(mafem_handle* h, double time, double dt, int64_t* out, int64_t cap);
 
 /* FP32 form: assemble the resident state and run the batched one-CTA solve on
  * this handle alone, its factorisation traced -- 6 globaltimer stamps (ns) per
- * panel in out[6p .. 6p+5] (start, diagonal block factored, panel staged and
- * inverses formed, first chunk's U12/Y, its trailing update, panel done), then
+ * panel in out[6p .. 6p+5] (start, diagonal block inverted, A21 split, first
+ * chunk's Y, its trailing update, panel done), then
  * the factor and refine kernels' event times in ns, then 4 stamps per
  * refinement sweep for up to 32 sweeps (start, substitutions done, x updated,
  * residual done; 0 where not reached), then 16 phase sums (ns) of the first
- * sweep's substitutions (see patch_lu_solve), then the relative residual
+ * sweep's substitutions (patch_solve_pass), then the relative residual
  * |r - A0 x| / |r| after each sweep (up to 32, as double bit patterns), then
  * the refinement's status and sweep count.  cap >= 6 npan + 182.
  * Returns npan, or MAFEM_ERR_UNSUPPORTED if the handle cannot use that solve. */

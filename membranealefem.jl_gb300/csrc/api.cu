@@ -645,7 +645,7 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
       J.rhs = h->d_r;
       J.x = h->d_x;
       J.res = h->d_res;
-      J.rs = h->d_part + 2048;  // unused by this form
+      J.rs = h->d_part + 2048;  // free while a batched solve runs
       J.xs = reinterpret_cast<float2*>(h->d_dx);  // d_dx: n doubles, unused by this form
       J.L = h->L;
       J.kuf = h->blk.kuf;

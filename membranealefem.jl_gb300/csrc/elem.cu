@@ -39,7 +39,7 @@
 // and 9 x ~700 in phase 3, against 72 x 9 dual residual evaluations of ~2400
 // (FP64) when every element dof is a direction of its own.
 // Measured on a GB300, against one dual residual evaluation per dof: assembly
-// with its gathers (mafem_calc_r_K) in FP64 3.16 -> 0.92 ms on 32 x 32 ALEVB,
+// with its gathers (mafem_calc_r_K) in FP64 3.16 -> 0.78 ms on 32 x 32 ALEVB,
 // 0.58 -> 0.09 ms on 8 x 8 LAG; the FP32 tangent of 32 x 32 ALEVB alone
 // 171 -> 72 us.
 //

@@ -274,11 +274,9 @@ template <class T>
 // trace (optional, device): 12 globaltimer stamps per panel t -- [0] the
 // factorising CTA starts waiting for t's columns, [1] they are ready, [2] t is
 // published; for the owner of t's first column: [3] it starts step t - 1,
-// [4] its waits are over, [5] panel t - 1 is staged, [6] its columns are
-// solved, [7] the rows t reads are written, [8] the rest of the rows,
-// [9] its column copies are issued, [10] the A21 copies are issued, [11] the
-// diagonal block is in shared memory.
-// two: eliminate from both ends (needs B.has_two, a right-hand side and grid >= min_two).
+// [4] panel t - 1 is published, [5] the copies issued before are there, [6] its
+// columns are solved, [7] the rows t reads are written, [8] the rest of the rows.
+// One chain only.  two: eliminate from both ends (needs B.has_two and grid >= min_two).
 int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersist& S, bool two, int* perm_all,
                           T* rdiag, int* info, T* rhs, int* err, cudaStream_t st, long long* trace = nullptr);
 template <class V, class T>
