@@ -66,6 +66,15 @@ enum mafem_lu_path {
   MAFEM_LU_FULL = 2    /* full partial pivoting (LAPACK gbtrf's pivot rule) */
 };
 
+/* How a handle's own solver factored its band last (mafem_lu_form). */
+enum mafem_lu_form_kind {
+  MAFEM_FORM_NONE = 0,      /* not yet */
+  MAFEM_FORM_FULL = 1,      /* full partial pivoting */
+  MAFEM_FORM_PANELS = 2,    /* node-block pivoting, per-panel launches */
+  MAFEM_FORM_ONE_CHAIN = 3, /* node-block pivoting, one persistent launch, from the first unknown to the last */
+  MAFEM_FORM_BOTH_ENDS = 4  /* the same from both ends: two chains of panels that meet in the middle */
+};
+
 /* Params (src/input/Params.jl:36-55), field for field. */
 typedef struct mafem_params {
   int32_t motion, scenario, num1el, num2el;
@@ -410,6 +419,20 @@ int mafem_set_refinement(mafem_handle* h, int32_t max_sweeps, double tol);
  * MAFEM_ERR_UNSUPPORTED if the handle cannot run that path (e.g. the node-block
  * forms when the band is too wide for their shared-memory panels). */
 int mafem_set_lu_path(mafem_handle* h, int32_t path);
+
+/* Form (enum mafem_lu_form_kind) of the last factorisation by the handle's own
+ * solver; the batched FP32 solve leaves it as it is. */
+int mafem_lu_form(const mafem_handle* h);
+/* Host only: the plan of the elimination from both ends for a mesh, with panels
+ * of at most `width` unknowns (1 .. 32; a handle takes the widest whose kernels fit
+ * the device).  Returns 1 and out = {kuf, mid, pm, np0, np1, the np0 + 1 panel
+ * starts of the forward chain, the np1 + 1 of the backward chain}: the forward
+ * chain eliminates the unknowns [0, mid) in order, the backward chain unknowns
+ * n - 1 down to mid (its panel starts count from the last unknown), and the chains
+ * meet before the forward chain's panel pm; a panel [j0, j1) reaches the rows
+ * below j1 + kl and the columns below j1 + kuf.  0: the band is eliminated as one
+ * chain.  cap: entries of out (2 nmdf + 7 always suffice). */
+int mafem_two_chain_plan(const mafem_mesh_desc* d, int32_t precision, int32_t width, int64_t* out, int64_t cap);
 
 /* Batched FP32 form: the CTAs (one thread-block cluster) that factor this
  * handle's patch -- 1, 2 or 4; 0 (the default) chooses by band width: one CTA

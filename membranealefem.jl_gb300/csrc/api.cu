@@ -103,6 +103,7 @@ struct mafem_handle {
   // (band_lu.cu) is the fallback for a block without a usable pivot
   bool use_blk = false;
   bool last_two = false;  // node-block factors: of the elimination from both ends
+  int lu_form = MAFEM_FORM_NONE;  // form of the last factorisation (mafem_lu_form)
   bool last_blk = false;  // which factorisation the band currently holds
   bool pinv_ready = false;  // d_pinv holds the inverses of its panels' triangles
   BlkPlan blk;
@@ -267,6 +268,20 @@ static int validate(const mafem_mesh_desc* d, const mafem_params* p, std::string
   return MAFEM_OK;
 }
 
+// Per unknown: one past the last unknown of its pivot block, the unknowns of one
+// node (consecutive in the ID numbering).
+static std::vector<int> pivot_blocks(const std::vector<int>& unk_node) {
+  const int64_t n = (int64_t)unk_node.size();
+  std::vector<int> blk_end(n);
+  for (int64_t q = 0; q < n;) {
+    int64_t e = q;
+    while (e < n && unk_node[e] == unk_node[q]) ++e;
+    for (int64_t k = q; k < e; ++k) blk_end[k] = (int)e;
+    q = e;
+  }
+  return blk_end;
+}
+
 static int64_t footprint(const mafem_mesh_desc* d, int precision, int64_t kl) {
   const int nb = choose_nb((int)kl, precision);
   BandLayout L = make_band_layout(d->nmdf, (int)kl, (int)kl, nb ? nb : 8);
@@ -286,6 +301,34 @@ extern "C" int64_t mafem_mesh_half_bandwidth(const mafem_mesh_desc* d) { return 
 extern "C" int64_t mafem_footprint_bytes(const mafem_mesh_desc* d, int32_t precision) {
   if (!d || !d->IX || !d->ID) return -1;
   return footprint(d, precision, half_bandwidth(*d));
+}
+
+extern "C" int mafem_two_chain_plan(const mafem_mesh_desc* d, int32_t precision, int32_t width, int64_t* out,
+                                    int64_t cap) {
+  if (!d || !d->IX || !d->ID || d->nmdf < 1 || width < 1 || width > kBlkW || !out) return MAFEM_ERR_ARG;
+  const int64_t n = d->nmdf;
+  const int kl = (int)half_bandwidth(*d), nb = choose_nb(kl, precision);
+  if (!nb || width > nb) return MAFEM_ERR_UNSUPPORTED;
+  const BandLayout L = make_band_layout(n, kl, kl, nb);
+  std::vector<int> unk_node(n, -1);
+  for (int64_t k = 0; k < d->ndf * d->numnp; ++k) {
+    if (d->ID[k] < 0 || d->ID[k] > n) return MAFEM_ERR_ARG;
+    if (d->ID[k] > 0) unk_node[d->ID[k] - 1] = (int)(k / d->ndf);
+  }
+  const std::vector<int> blk_end = pivot_blocks(unk_node);
+  BlkPlan B;
+  std::vector<int> ps0, ps1, blk_end1;
+  if (!blk_plan(blk_end, width, kl, B)) return MAFEM_ERR_UNSUPPORTED;
+  if (!blk_two_plan(blk_end, L, B, ps0, ps1, blk_end1)) return 0;
+  if (cap < 5 + (int64_t)(ps0.size() + ps1.size())) return MAFEM_ERR_ARG;
+  *out++ = B.kuf;
+  *out++ = B.mid;
+  *out++ = B.pm;
+  *out++ = (int64_t)ps0.size() - 1;
+  *out++ = (int64_t)ps1.size() - 1;
+  for (int v : ps0) *out++ = v;
+  for (int v : ps1) *out++ = v;
+  return 1;
 }
 
 extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, const mafem_args* a,
@@ -504,16 +547,9 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
     for (int v = 0; v < numnp; ++v) nf[(size_t)v + 1] += nf[v];
     if (mono) UP(d_nf, nf);
   }
-  // pivot blocks: the unknowns of one node (consecutive in the ID numbering)
-  std::vector<int> blk_end(n);
+  const std::vector<int> blk_end = pivot_blocks(unk_node);
   int maxblk = 1;
-  for (int64_t q = 0; q < n;) {
-    int64_t e = q;
-    while (e < n && unk_node[e] == unk_node[q]) ++e;
-    for (int64_t k = q; k < e; ++k) blk_end[k] = (int)e;
-    maxblk = std::max(maxblk, (int)(e - q));
-    q = e;
-  }
+  for (int64_t q = 0; q < n; q = blk_end[q]) maxblk = std::max(maxblk, blk_end[q] - (int)q);
   UP(h->d_blk_end, blk_end);
   {
     const int wmax = precision == MAFEM_PLAIN_FP64 ? blk_lu_setup<double>(h->L) : blk_lu_setup<float>(h->L);
@@ -803,6 +839,7 @@ static int factor_enqueue(mafem_handle* h, double* x) {
                         : blk_lu_factor_persist<float>((float*)h->d_band, h->L, h->blk, h->pers, two, h->d_perm,
                                                        (float*)h->d_rdiag, h->d_info, nullptr, h->d_info + 1, h->st);
     h->last_two = two && nl > 0;
+    h->lu_form = two ? MAFEM_FORM_BOTH_ENDS : MAFEM_FORM_ONE_CHAIN;
     if (nl < 0) {
       cudaGetLastError();
       h->pers.grid = 0;  // cooperative launch refused: per-panel launches from now on
@@ -813,6 +850,7 @@ static int factor_enqueue(mafem_handle* h, double* x) {
   }
   if (!launched) {
     h->last_two = false;
+    h->lu_form = MAFEM_FORM_PANELS;
     const int nl = fp64 ? blk_lu_factor<double>((double*)h->d_band, h->L, h->blk, h->d_perm, (double*)h->d_rdiag,
                                                 h->d_info, x, h->st, h->st2, h->ev_pool.data(), nullptr)
                         : blk_lu_factor<float>((float*)h->d_band, h->L, h->blk, h->d_perm, (float*)h->d_rdiag,
@@ -879,6 +917,7 @@ static int factor(mafem_handle* h, double* x, const double* rhs0) {
   h->launches += nl;
   h->factored = true;
   h->last_blk = false;
+  h->lu_form = MAFEM_FORM_FULL;
   // full partial pivoting found no usable pivot either: the matrix is singular
   // (or not finite); report it before any solve uses the factors
   int zp = 0;
@@ -1337,6 +1376,8 @@ extern "C" int mafem_time_step(mafem_handle* h, double time, double dt, mafem_st
   step_stats(h, stats);
   return rc == kIterDone ? MAFEM_OK : rc;
 }
+
+extern "C" int mafem_lu_form(const mafem_handle* h) { return h ? h->lu_form : MAFEM_ERR_ARG; }
 
 extern "C" int mafem_set_launch_ctas(mafem_handle* h, int32_t ctas) {
   if (!h || ctas < 0) return MAFEM_ERR_ARG;
@@ -2631,6 +2672,7 @@ extern "C" int mafem_trace_factor(mafem_handle* h, double time, double dt, int64
   h->factored = true;
   h->last_blk = true;
   h->last_two = false;
+  h->lu_form = MAFEM_FORM_ONE_CHAIN;
   CK(cudaMemcpyAsync(out, d_tr, sizeof(long long) * 12 * npan, cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
   cudaFree(d_tr);
@@ -2994,6 +3036,7 @@ extern "C" int mafem_profile_factor(mafem_handle* h, double time, double dt, maf
   h->factored = true;
   h->last_blk = h->use_blk;
   h->last_two = false;
+  h->lu_form = h->use_blk ? MAFEM_FORM_PANELS : MAFEM_FORM_FULL;
   CK(cudaStreamSynchronize(h->st));
   float ms = 0;
   cudaEventElapsedTime(&ms, a0, a1);

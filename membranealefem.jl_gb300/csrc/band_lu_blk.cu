@@ -625,11 +625,16 @@ bool blk_plan(const std::vector<int>& blk_end, int wmax, int ku, BlkPlan& out) {
 // The backward chain takes the unknowns [mid, n), whole pivot blocks, so many that
 // 2 kuf unknowns are left between the chains when the forward chain has done as
 // many: until then a panel of the forward chain (it reaches kuf unknowns beyond
-// itself) and one of the backward chain never touch the same entries.  pm: the
-// forward chain's first panel that may.  The chain of dependent panels is then
-// n / 2 + kuf unknowns long instead of n; bands shorter than 10/3 kuf keep the one
-// chain (LAG 8 x 8 at 3.6 kuf, six panels instead of eight and a meeting of all
-// CTAs: 0.24 -> 0.19 ms; below, the meeting costs what the shorter chain saves).
+// itself) and one of the backward chain (it reaches down to mid - kuf) never touch
+// the same entries.  pm: the forward chain's panel at which they meet; the panels
+// before it reach no further than mid - kuf.  Panel pm's own block ends there too:
+// the forward chain's factorising CTA does not wait at the meeting and may factorise
+// panel pm before it, once the panels before pm have updated its columns.  (In a band
+// with kuf < 32 a panel can be wider than its reach, so that this asks for more.)
+// The chain of dependent panels is then n / 2 + kuf unknowns long instead of n; bands
+// shorter than 10/3 kuf keep the one chain (LAG 8 x 8 at 3.6 kuf, six panels instead
+// of eight and a meeting of all CTAs: 0.24 -> 0.19 ms; below, the meeting costs what
+// the shorter chain saves).
 bool blk_two_plan(const std::vector<int>& blk_end, const BandLayout& L, BlkPlan& out, std::vector<int>& ps0,
                   std::vector<int>& ps1, std::vector<int>& blk_end1) {
   const int n = (int)blk_end.size(), kuf = out.kuf, kl = L.kl;
@@ -652,6 +657,7 @@ bool blk_two_plan(const std::vector<int>& blk_end, const BandLayout& L, BlkPlan&
   out.mid = mid;
   out.pm = 0;
   while (out.pm < a.npan() && ps0[out.pm + 1] + kuf <= mid - kuf) ++out.pm;
+  while (out.pm > 0 && ps0[out.pm + 1] > mid - kuf) --out.pm;
   return out.pm > 0;  // their panels are no wider than out.wmax
 }
 

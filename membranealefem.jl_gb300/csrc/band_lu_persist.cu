@@ -59,7 +59,8 @@ struct PersistArgs {
   int split;
   int n, off, kl, kuf;
   int rmax, wmax, nslot;      // rmax = wmax + kl: rows of a staged panel column
-  int pm, bdone_target;       // nobody starts on panel pm of c[0] before *bdone reaches the target
+  int pm, bdone_target;       // panel pm of c[0] and later ones: after *bdone has reached the target, but for
+                              // the factorising CTA (pm's block lies clear of c[1], blk_two_plan)
   int* bdone;
   int* perm_all;
   T* rdiag;
@@ -392,7 +393,9 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
                                     ph);
   } else {
     __shared__ int s_ok;
-    // first each chain on its own CTAs, the forward one up to panel pm, then the rest on all of them
+    // first each chain on its own CTAs, the forward one up to panel pm, then the rest on all of them; the
+    // forward chain's factorising CTA goes on without the meeting: of its panels pm alone can come before
+    // it (later ones wait for columns that are updated after it), and pm's block is out of c[1]'s reach
     const bool rev = me >= a.split;
     const int G0 = rev ? G - a.split : a.split;
     const int nx = a.rhs ? 2 : 1;  // CTAs of a chain that own no columns

@@ -40,6 +40,7 @@ BOTTOM, RIGHT, TOP, LEFT = 1, 2, 3, 4
 SHEAR, STRETCH, MOMENT = 1, 2, 3
 PLAIN_FP64, FP32_REFINE = 0, 1
 LU_AUTO, LU_PANELS, LU_FULL = 0, 1, 2  # mafem_set_lu_path
+FORM_NONE, FORM_FULL, FORM_PANELS, FORM_ONE_CHAIN, FORM_BOTH_ENDS = 0, 1, 2, 3, 4  # mafem_lu_form
 
 OK = 0
 NEWTON_NOT_CONVERGED, ZERO_PIVOT, NAN_DETECTED, REFINE_STALLED = 1, 2, 3, 4
@@ -174,6 +175,8 @@ def lib():
         L.mafem_launch_count.argtypes = [vp]
         L.mafem_launch_count.restype = C.c_int64
         L.mafem_set_lu_path.argtypes = [vp, C.c_int32]
+        L.mafem_lu_form.argtypes = [vp]
+        L.mafem_two_chain_plan.argtypes = [C.POINTER(MeshDesc), C.c_int32, C.c_int32, _P64, C.c_int64]
         L.mafem_set_patch_ctas.argtypes = [vp, C.c_int32]
         L.mafem_autotune_patch.argtypes = [vp]
         L.mafem_set_refinement.argtypes = [vp, C.c_int32, C.c_double]
@@ -391,6 +394,19 @@ def footprint_bytes(mesh: Mesh, precision: int = PLAIN_FP64) -> int:
     return int(lib().mafem_footprint_bytes(C.byref(mesh.desc), precision))
 
 
+def two_chain_plan(mesh: Mesh, precision: int = PLAIN_FP64, width: int = 32):
+    """mafem_two_chain_plan (host only): (kuf, mid, pm, forward panel starts, backward
+    panel starts), or None for a band that is eliminated as one chain."""
+    out = np.zeros(2 * mesh.nmdf + 7, dtype=np.int64)
+    rc = lib().mafem_two_chain_plan(C.byref(mesh.desc), precision, width, out.ctypes.data_as(_P64), out.size)
+    if rc < 0:
+        raise MafemError(rc, "no elimination plan for this mesh and panel width")
+    if rc == 0:
+        return None
+    kuf, mid, pm, np0, np1 = (int(v) for v in out[:5])
+    return kuf, mid, pm, out[5:6 + np0], out[6 + np0:7 + np0 + np1]
+
+
 class Solver:
     """Device-resident state of one patch: the replacement of ``calc_r_K`` + ``\\``
     and of ``time_step!`` (src/analysis/FiniteElement.jl:11-200)."""
@@ -529,6 +545,10 @@ class Solver:
     def set_lu_path(self, path: int) -> None:
         """Select the banded LU: LU_AUTO (default), LU_PANELS or LU_FULL."""
         _raise(lib().mafem_set_lu_path(self.h, path), self.h)
+
+    def lu_form(self) -> int:
+        """How this handle's own solver factored its band last (FORM_*)."""
+        return int(lib().mafem_lu_form(self.h))
 
     def set_patch_ctas(self, ctas: int) -> None:
         """Batched FP32 form: CTAs (1, 2 or 4) of the cluster that factors this
