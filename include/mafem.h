@@ -404,6 +404,15 @@ int mafem_set_dirichlet_scale(mafem_handle* h, double scale);
  * and the next call (after mafem_set_wait_test(h, 0, -1)) runs normally. */
 int mafem_set_wait_test(mafem_handle* h, int32_t limit_polls, int32_t withhold_panel);
 
+/* Test hook of the persistent factorisation's counters (no reference counterpart):
+ * set them as after `count` factorisations -- they are kept modulo 2^32 -- with the
+ * meeting of the two chains `missing` arrivals short, as after a factorisation that
+ * gave up, and let its waits give up after limit_polls polls (0: the default, 2^22).
+ * A factorisation whose wait runs out leaves the state unchanged and returns
+ * MAFEM_ERR_CUDA.
+ * MAFEM_ERR_UNSUPPORTED for a handle without that factorisation. */
+int mafem_set_lu_count(mafem_handle* h, uint32_t count, uint32_t missing, int32_t limit_polls);
+
 /* FP32 form: FP64 iterative refinement of each linear solve stops at tol
  * (default 1e-10) or fails after max_sweeps sweeps (default 30) or when it stops
  * converging (MAFEM_REFINE_STALLED).  A handle stepped on its own stops when

@@ -109,7 +109,7 @@ struct mafem_handle {
   BlkPlan blk;
   int* d_blk_end = nullptr;
   SolveWord* d_xch = nullptr;  // what the panels of the cooperative substitutions hand on: npan_max x 32
-  int epoch = 0;           // value the flags are set to by the next back substitution
+  int64_t epoch = 0;       // tag of the last cooperative substitution launch
   int bwd_grid = 0;        // CTAs of the cooperative back substitution (0: single-CTA kernel)
   BlkPersist pers;         // persistent cooperative factorisation (grid 0: per-panel launches)
   std::vector<int> h_ix;   // IX, 0-based [element][9] (pull-force neighbourhood)
@@ -568,6 +568,8 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
       std::vector<int> ps0, ps1, blk_end1;
       if (blk_two_plan(blk_end, h->L, h->blk, ps0, ps1, blk_end1)) {
         h->blk.has_two = true;
+        h->blk.ps0 = ps0;
+        h->blk.ps1 = ps1;
         BlkChain &a = h->blk.two[0], &b = h->blk.two[1];
         int *d_ps0 = nullptr, *d_ps1 = nullptr, *d_end1 = nullptr;
         UP(d_ps0, ps0);
@@ -807,11 +809,6 @@ static int assemble(mafem_handle* h, double time, double dt, bool both_bands = f
   return MAFEM_OK;
 }
 
-// Factorise the assembled band: node-block pivoting first; if a node block has
-// no usable pivot, re-gather the band from the element blocks and factor it
-// with full partial pivoting.  `x` (may be null) is the right-hand side that
-// rides along the factorisation (forward substitution); `rhs0` restores it for
-// the fallback.
 // Launch the node-block factorisation (persistent kernel, or per-panel launches)
 // without waiting for it; `info` tells later whether a block had no usable pivot.
 // The panels' triangle inverses for the cooperative forward substitution, formed
@@ -2894,6 +2891,14 @@ extern "C" int mafem_set_dirichlet_scale(mafem_handle* h, double scale) {
   launch_dirichlet_scale(h->P.cps, h->d_dir_idx, h->d_dir_val, h->n_dir, scale, h->st);
   h->launches += h->n_dir > 0 ? 1 : 0;
   CK(cudaGetLastError());
+  return MAFEM_OK;
+}
+
+extern "C" int mafem_set_lu_count(mafem_handle* h, uint32_t count, uint32_t missing, int32_t limit_polls) {
+  if (!h || limit_polls < 0) return MAFEM_ERR_ARG;
+  if (h->pers.max_grid <= 0) return MAFEM_ERR_UNSUPPORTED;
+  h->pers.limit = limit_polls;
+  CK(blk_persist_count(h->blk, h->pers, count, missing, h->st));
   return MAFEM_OK;
 }
 

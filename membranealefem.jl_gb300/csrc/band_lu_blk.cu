@@ -387,9 +387,9 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
 // hang; the host reports the error).  wt.withhold = k >= 0 (failure-detection tests
 // only): the back substitution's panel npan - 1 - k is never published, so the CTAs
 // that need it run out of polls.
-__device__ __forceinline__ void publish(SolveWord* p, double v, int tag) {
+__device__ __forceinline__ void publish(SolveWord* p, double v, long long tag) {
   asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p),
-               "l"(__double_as_longlong(v)), "l"((long long)tag)
+               "l"(__double_as_longlong(v)), "l"(tag)
                : "memory");
 }
 __device__ __forceinline__ double peek(const SolveWord* p, long long& tag) {
@@ -403,7 +403,7 @@ __device__ __forceinline__ double peek(const SolveWord* p, long long& tag) {
 // This lane's entries cg, cg + 4, ... < nc of a panel's words X, once all of the warp's
 // carry the tag (tag 0: from an earlier launch, at once).  false, for the whole warp,
 // when the polls ran out or another warp has set *err.
-__device__ __forceinline__ bool fetch(const SolveWord* X, int cg, int nc, int tag, bool far, double (&y)[8], int* err,
+__device__ __forceinline__ bool fetch(const SolveWord* X, int cg, int nc, long long tag, bool far, double (&y)[8], int* err,
                                       int limit) {
   const int lim = limit > 0 ? limit : kSpinLimit;
   for (int it = 0;; ++it) {
@@ -436,7 +436,7 @@ constexpr int kSolveThreads = 128;
 template <class T>
 __global__ void __launch_bounds__(kSolveThreads)
     blk_backward_coop_kernel(const T* __restrict__ ab, int kuf, BlkSpan s0, BlkSpan s1, int split, double* yv,
-                             SolveWord* xch, int epoch, int* err, WaitTest wt, const int* gate) {
+                             SolveWord* xch, long long epoch, int* err, WaitTest wt, const int* gate) {
   if (gate && *gate) return;  // every CTA reads the same word: all return (refinement already stopped)
   const int lane = threadIdx.x & 31, row = 8 * (threadIdx.x >> 5) + (lane & 7), cg = lane >> 3;
   const bool second = (int)blockIdx.x >= split;
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(kSolveThreads)
 template <class T>
 __global__ void __launch_bounds__(kSolveThreads)
     blk_forward_coop_kernel(const T* __restrict__ ab, int kl, BlkSpan s0, BlkSpan s1, int split,
-                            const double* __restrict__ inv_all, double* bv, SolveWord* xch, int epoch, int* err,
+                            const double* __restrict__ inv_all, double* bv, SolveWord* xch, long long epoch, int* err,
                             WaitTest wt, const int* gate) {
   __shared__ double xs[2][32];
   if (gate && *gate) return;
@@ -787,7 +787,7 @@ static int coop_spans(F&& launch, const BlkSpan& a, const BlkSpan* b, int grid) 
   return launch(a, b ? *b : a, ga, ga + gb) == cudaSuccess ? 1 : -1;
 }
 template <class T>
-int blk_backward(const T* ab, const BlkPlan& B, bool two, double* y, SolveWord* xch, int& epoch, int* err, int grid,
+int blk_backward(const T* ab, const BlkPlan& B, bool two, double* y, SolveWord* xch, int64_t& epoch, int* err, int grid,
                  cudaStream_t st, WaitTest wt, const int* gate) {
   int kuf = B.kuf;
   auto launch = [&](BlkSpan a, BlkSpan b, int split, int ctas) {
@@ -812,7 +812,7 @@ void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, V* y,
 }
 template <class T>
 int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const double* inv, double* b,
-                     SolveWord* xch, int& epoch, int* err, int grid, cudaStream_t st, WaitTest wt, const int* gate) {
+                     SolveWord* xch, int64_t& epoch, int* err, int grid, cudaStream_t st, WaitTest wt, const int* gate) {
   int kl = L.kl;
   auto launch = [&](BlkSpan s0, BlkSpan s1, int split, int ctas) {
     ++epoch;
@@ -855,9 +855,9 @@ template int blk_inverses<double, double>(const double*, const BandLayout&, cons
                                           const double*, double*, cudaStream_t);
 template int blk_inverses<double, float>(const float*, const BandLayout&, const BlkPlan&, bool, const int*, const float*,
                                          double*, cudaStream_t);
-template int blk_backward<double>(const double*, const BlkPlan&, bool, double*, SolveWord*, int&, int*, int, cudaStream_t,
+template int blk_backward<double>(const double*, const BlkPlan&, bool, double*, SolveWord*, int64_t&, int*, int, cudaStream_t,
                                   WaitTest, const int*);
-template int blk_backward<float>(const float*, const BlkPlan&, bool, double*, SolveWord*, int&, int*, int, cudaStream_t,
+template int blk_backward<float>(const float*, const BlkPlan&, bool, double*, SolveWord*, int64_t&, int*, int, cudaStream_t,
                                  WaitTest, const int*);
 template void blk_backward_1cta<double, double>(const double*, const BandLayout&, const BlkPlan&, double*,
                                                 cudaStream_t);
@@ -866,8 +866,8 @@ template void blk_backward_1cta<double, float>(const float*, const BandLayout&, 
 template int blk_backward_grid<double>();
 template int blk_backward_grid<float>();
 template int blk_forward_coop<double>(const double*, const BandLayout&, const BlkPlan&, bool, const double*, double*,
-                                      SolveWord*, int&, int*, int, cudaStream_t, WaitTest, const int*);
+                                      SolveWord*, int64_t&, int*, int, cudaStream_t, WaitTest, const int*);
 template int blk_forward_coop<float>(const float*, const BandLayout&, const BlkPlan&, bool, const double*, double*,
-                                     SolveWord*, int&, int*, int, cudaStream_t, WaitTest, const int*);
+                                     SolveWord*, int64_t&, int*, int, cudaStream_t, WaitTest, const int*);
 
 }  // namespace mafem

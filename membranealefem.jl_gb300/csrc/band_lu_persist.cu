@@ -21,9 +21,10 @@
 // panel is: stage, one triangular solve, 32 rows of one column, the panel
 // factorisation, and two flag hand-overs -- no kernel launches.
 //
-// Flags and counters are monotone across factorisations: pdone[t] holds the
-// epoch that set it, critcnt[t] / a21cnt[t] reach epoch * w(t).  All waits
-// are bounded (kSpinLimit polls) and abort every CTA through *err.
+// Flags and counters go on across factorisations: pdone[t] holds the epoch that set
+// it, critcnt[t] / a21cnt[t] reach epoch * w(t), modulo 2^32; a wait compares
+// differences, so they may wrap.  All waits are bounded (kSpinLimit polls) and abort
+// every CTA through *err.
 //
 // From both ends (FP64 with a right-hand side; blk_two_plan).  A panel takes ~24 us of
 // dependent steps however narrow the band is, so the number of panels in a row is
@@ -59,7 +60,8 @@ struct PersistArgs {
   int split;
   int n, off, kl, kuf;
   int rmax, wmax, nslot;      // rmax = wmax + kl: rows of a staged panel column
-  int pm, bdone_target;       // panel pm of c[0] and later ones: after *bdone has reached the target, but for
+  int pm;
+  unsigned bdone_target;      // panel pm of c[0] and later ones: after *bdone has reached the target, but for
                               // the factorising CTA (pm's block lies clear of c[1], blk_two_plan)
   int* bdone;
   int* perm_all;
@@ -69,8 +71,9 @@ struct PersistArgs {
   int* pdone;
   int* critcnt;
   int* a21cnt;
-  int epoch;
+  unsigned epoch;
   int* err;
+  int limit;        // polls before a wait gives up
   long long* trace;  // optional: kTraceSlots device-clock stamps per panel (diagnostics)
 };
 constexpr int kTraceSlots = 12;
@@ -83,12 +86,12 @@ __device__ __forceinline__ void stamp(long long* trace, int t, int slot) {
   }
 }
 
-// thread 0 waits until *p >= target; false (uniform over the CTA) on timeout / abort
-__device__ __forceinline__ bool wait_geq(const int* p, int target, int* err, int* s_ok) {
+// thread 0 waits until *p has reached target (modulo 2^32); false (uniform over the CTA) on timeout / abort
+__device__ __forceinline__ bool wait_geq(const int* p, unsigned target, int* err, int limit, int* s_ok) {
   if (threadIdx.x == 0) {
     int ok = 1;
-    for (int it = 0; ld_acquire(p) < target; ++it) {
-      if (it > kSpinLimit || ((it & 31) == 31 && *(volatile int*)err)) {  // (a look at it delays the next poll)
+    for (int it = 0; (int)((unsigned)ld_acquire(p) - target) < 0; ++it) {
+      if (it > limit || ((it & 31) == 31 && *(volatile int*)err)) {  // (a look at it delays the next poll)
         atomicCAS(err, 0, 1);
         ok = 0;
         break;
@@ -135,12 +138,12 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
     for (int t = p0; t < p1; ++t) {
       const int j0 = ps[t], wt = ps[t + 1] - j0;
       stamp(a.trace, t, 0);
-      if (t > 0 && !wait_geq(critcnt + t, a.epoch * wt, a.err, &s_ok)) return false;
+      if (t > 0 && !wait_geq(critcnt + t, a.epoch * wt, a.err, a.limit, &s_ok)) return false;
       stamp(a.trace, t, 1);
       blk_panel_factor<T, true>(ab + j0 * SG + j0 * sj, SG, sj, j0, wt, REV ? a.n - j0 : j0 + 1, SG, C.blk_end + j0,
                                 perm_all + (size_t)t * kBlkW, rdiag + j0, a.info, s_l, s_p);
       __syncthreads();
-      if (tid == 0) st_release(pdone + t, a.epoch);
+      if (tid == 0) st_release(pdone + t, (int)a.epoch);
       stamp(a.trace, t, 2);
     }
     return true;
@@ -210,7 +213,7 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
     if (cfirst >= cend && !is_rhs) continue;
     const bool tr_owner = !TWO && p + 1 < npan && me == j1 % GW;
     if (tr_owner) stamp(a.trace, p + 1, 3);
-    if (p > 0 && !wait_geq(a21cnt + p, a.epoch * w, a.err, &s_ok)) return false;
+    if (p > 0 && !wait_geq(a21cnt + p, a.epoch * w, a.err, a.limit, &s_ok)) return false;
     const int nch = (R - w + 31) / 32;  // 32-row chunks below the diagonal block
     // columns of this panel: the one of panel p + 1 first, then the others, then the right-hand side
     const int nown = cfirst < cend ? (int)((cend - 1 - cfirst) / GW) + 1 : 0;
@@ -255,7 +258,7 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
       }
     };
     issue_cols(0, min(a.nslot, ncol), true);
-    if (!wait_geq(pdone + p, a.epoch, a.err, &s_ok)) {
+    if (!wait_geq(pdone + p, a.epoch, a.err, a.limit, &s_ok)) {
       wait_bar(s_bar, ph);  // no copy in flight when the CTA ends
       return false;
     }
@@ -412,7 +415,7 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
         __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) atomicAdd(a.bdone, 1);
-        if (!wait_geq(a.bdone, a.bdone_target, a.err, &s_ok)) return;
+        if (!wait_geq(a.bdone, a.bdone_target, a.err, a.limit, &s_ok)) return;
         if (rev) {
           role = kWorker;
           me += a.split - nx;
@@ -510,6 +513,7 @@ int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersi
   a.a21cnt = S.d_a21cnt + after;
   a.epoch = S.epoch[two] + 1;
   a.err = err;
+  a.limit = S.limit > 0 ? S.limit : kSpinLimit;
   a.trace = two ? nullptr : trace;
   void* args[] = {(void*)&a};
   const void* fn = two ? (const void*)blk_factor_persist_kernel<T, true> : (const void*)blk_factor_persist_kernel<T, false>;
@@ -517,6 +521,25 @@ int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersi
   S.epoch[two] = a.epoch;
   if (two) S.bdone = a.bdone_target;
   return 1;
+}
+
+cudaError_t blk_persist_count(const BlkPlan& B, BlkPersist& S, unsigned count, unsigned missing, cudaStream_t st) {
+  const std::vector<int>* ps[3] = {&B.ps, &B.ps0, &B.ps1};
+  std::vector<unsigned> v[2];  // pdone; critcnt and a21cnt
+  for (const auto* q : ps)
+    for (size_t t = 0; t + 1 < q->size(); ++t) {
+      v[0].push_back(count);
+      v[1].push_back(count * (unsigned)((*q)[t + 1] - (*q)[t]));
+    }
+  S.epoch[0] = S.epoch[1] = S.bdone = count;
+  const unsigned met = count - missing;
+  cudaError_t e = cudaMemcpyAsync(S.d_bdone, &met, sizeof met, cudaMemcpyHostToDevice, st);
+  int* dst[3] = {S.d_pdone, S.d_critcnt, S.d_a21cnt};
+  for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
+    const auto& w = v[k > 0];
+    e = cudaMemcpyAsync(dst[k], w.data(), w.size() * sizeof(unsigned), cudaMemcpyHostToDevice, st);
+  }
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
 }
 
 template int blk_persist_setup<double>(const BandLayout&, const BlkPlan&, BlkPersist&);

@@ -192,6 +192,7 @@ struct BlkPlan {
   std::vector<int> ps;   // panel starts; ps.back() == n
   int* d_ps = nullptr;   // device copy of ps
   const int* d_blk_end = nullptr;  // per unknown: one past the last unknown of its block
+  std::vector<int> ps0, ps1;  // panel starts of the two chains
   BlkChain one;          // the whole band as one forward chain
   // The same as two chains (blk_two_plan): two[0] eliminates the unknowns from the
   // first, two[1] from the last up to unknown mid, beside it; two[0] then goes on
@@ -239,7 +240,7 @@ template <class V, class T>
 int blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
                  V* inv, cudaStream_t st);
 template <class T>
-int blk_backward(const T* ab, const BlkPlan& B, bool two, double* y, SolveWord* xch, int& epoch, int* err, int grid,
+int blk_backward(const T* ab, const BlkPlan& B, bool two, double* y, SolveWord* xch, int64_t& epoch, int* err, int grid,
                  cudaStream_t st, WaitTest wt = WaitTest(), const int* gate = nullptr);
 template <class T>
 int blk_backward_grid();
@@ -247,7 +248,7 @@ int blk_backward_grid();
 // blk_backward.  Returns the kernels launched, or -1 if a launch was refused.
 template <class T>
 int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const double* inv, double* b,
-                     SolveWord* xch, int& epoch, int* err, int grid, cudaStream_t st, WaitTest wt = WaitTest(),
+                     SolveWord* xch, int64_t& epoch, int* err, int grid, cudaStream_t st, WaitTest wt = WaitTest(),
                      const int* gate = nullptr);
 // Persistent cooperative factorisation (band_lu_persist.cu): launch shape and
 // per-panel flags.  Flags are zeroed once; epochs make them reusable.  The arrays
@@ -259,8 +260,9 @@ struct BlkPersist {
   int min_two = 0;         // fewest CTAs of the two-chain form (0: not available)
   int nslot2 = 0;          // two chains: columns a worker stages at once
   size_t smem = 0, smem2 = 0;  // shared memory as one chain, as two
-  int epoch[2] = {0, 0};   // factorisations so far: as one chain, as two
-  int bdone = 0;           // *d_bdone once the last two-chain factorisation is done
+  unsigned epoch[2] = {0, 0};  // factorisations so far: as one chain, as two (modulo 2^32, as all counters)
+  unsigned bdone = 0;          // *d_bdone once the last two-chain factorisation is done
+  int limit = 0;               // polls before a wait gives up (0: kSpinLimit); tests only
   int* d_bdone = nullptr;  // counts the CTAs that are done with what the two chains do apart
   int* d_pdone = nullptr;
   int* d_critcnt = nullptr;
@@ -279,6 +281,10 @@ template <class T>
 // One chain only.  two: eliminate from both ends (needs B.has_two and grid >= min_two).
 int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersist& S, bool two, int* perm_all,
                           T* rdiag, int* info, T* rhs, int* err, cudaStream_t st, long long* trace = nullptr);
+// The counters as after `count` factorisations of either form, the meeting's short of
+// `missing` arrivals; waits for st.  count 0: as new, after a wait that ran out has
+// left them behind (0 missing).  Other values: tests.
+cudaError_t blk_persist_count(const BlkPlan& B, BlkPersist& S, unsigned count, unsigned missing, cudaStream_t st);
 template <class V, class T>
 void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, cudaStream_t st);
 }  // namespace mafem
