@@ -409,7 +409,7 @@ int mafem_set_wait_test(mafem_handle* h, int32_t limit_polls, int32_t withhold_p
  * meeting of the two chains `missing` arrivals short, as after a factorisation that
  * gave up, and let its waits give up after limit_polls polls (0: the default, 2^22).
  * A factorisation whose wait runs out leaves the state unchanged and returns
- * MAFEM_ERR_CUDA.
+ * MAFEM_ERR_CUDA; the counters then start afresh and the next call runs normally.
  * MAFEM_ERR_UNSUPPORTED for a handle without that factorisation. */
 int mafem_set_lu_count(mafem_handle* h, uint32_t count, uint32_t missing, int32_t limit_polls);
 

@@ -809,6 +809,15 @@ static int assemble(mafem_handle* h, double time, double dt, bool both_bands = f
   return MAFEM_OK;
 }
 
+// A wait of the handle's own kernels for another CTA ran out: report it, and start the
+// persistent factorisation's counters afresh -- one that gave up has left them short
+// of what the next one would wait for.
+static int wait_ran_out(mafem_handle* h, const char* where) {
+  if (h->pers.max_grid > 0) CK(blk_persist_count(h->blk, h->pers, 0, 0, h->st));
+  h->err = std::string(where) + ": a bounded wait for another CTA ran out";
+  return MAFEM_ERR_CUDA;
+}
+
 // Launch the node-block factorisation (persistent kernel, or per-panel launches)
 // without waiting for it; `info` tells later whether a block had no usable pivot.
 // The panels' triangle inverses for the cooperative forward substitution, formed
@@ -876,10 +885,7 @@ static int factor(mafem_handle* h, double* x, const double* rhs0) {
     CK(cudaMemcpyAsync(info2, h->d_info, sizeof info2, cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     const int info = info2[0];
-    if (info2[1]) {
-      h->err = "banded LU: a bounded wait for another CTA ran out";
-      return MAFEM_ERR_CUDA;
-    }
+    if (info2[1]) return wait_ran_out(h, "banded LU");
     if (info == 0) {
       h->factored = true;
       h->last_blk = true;
@@ -967,10 +973,7 @@ static void blk_fwd_solve(mafem_handle* h, double* y, const int* gate = nullptr)
 static int check_info(mafem_handle* h) {
   int info[2] = {0, 0};
   std::memcpy(info, h->h_out + 5, sizeof info);
-  if (info[1]) {
-    h->err = "back substitution: a bounded wait for another CTA ran out";
-    return MAFEM_ERR_CUDA;
-  }
+  if (info[1]) return wait_ran_out(h, "banded LU or substitution");
   if (info[0]) {
     h->err = "zero pivot in column " + std::to_string(info[0]);
     return MAFEM_ZERO_PIVOT;

@@ -24,7 +24,7 @@
 // Flags and counters go on across factorisations: pdone[t] holds the epoch that set
 // it, critcnt[t] / a21cnt[t] reach epoch * w(t), modulo 2^32; a wait compares
 // differences, so they may wrap.  All waits are bounded (kSpinLimit polls) and abort
-// every CTA through *err.
+// every CTA through *err; the host then starts the counters afresh (blk_persist_count).
 //
 // From both ends (FP64 with a right-hand side; blk_two_plan).  A panel takes ~24 us of
 // dependent steps however narrow the band is, so the number of panels in a row is
