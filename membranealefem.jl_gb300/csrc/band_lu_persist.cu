@@ -439,10 +439,17 @@ static size_t persist_smem(const BandLayout& L, int wmax, int nslot, bool two) {
   return ((two ? 64 : 0) + (size_t)wmax * ldp + 64 + nslot * (ldp + 32)) * sizeof(T);
 }
 
+// The kernel's limit of dynamic shared memory belongs to the process, not to a handle:
+// it is always set to all that the device has (cap) beside the kernel's static part, so
+// that no handle's set-up takes away what another one's launches ask for.
 template <class T, bool TWO>
-static bool persist_fits(size_t sm) {
+static bool persist_fits(size_t sm, int cap) {
   int per = 0;
-  return cudaFuncSetAttribute(blk_factor_persist_kernel<T, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) ==
+  cudaFuncAttributes fa;
+  if (cudaFuncGetAttributes(&fa, blk_factor_persist_kernel<T, TWO>) != cudaSuccess) return false;
+  const int dyn = cap - (int)fa.sharedSizeBytes;
+  return sm <= (size_t)dyn &&
+         cudaFuncSetAttribute(blk_factor_persist_kernel<T, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ==
              cudaSuccess &&
          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, blk_factor_persist_kernel<T, TWO>, 256, sm) ==
              cudaSuccess &&
@@ -459,7 +466,7 @@ int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   S.smem = persist_smem<T>(L, B.wmax, 4, false);
   if (!coop || S.smem + 12 * 1024 > (size_t)cap || B.wmax > kBlkW) return 0;  // + static shared memory
-  if (!persist_fits<T, false>(S.smem)) return 0;
+  if (!persist_fits<T, false>(S.smem, cap)) return 0;
   // workers need at most kMinCols columns each per panel (columns c of the
   // trailing range, owned by c mod (G - 1), plus the right-hand side)
   constexpr int kMinCols = 8;
@@ -476,7 +483,7 @@ int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
     if (!B.has_two) break;
     S.nslot2 = nslot;
     S.smem2 = persist_smem<T>(L, B.wmax, nslot, true);
-    if (S.smem2 + 12 * 1024 <= (size_t)cap && persist_fits<T, true>(S.smem2)) {
+    if (S.smem2 + 12 * 1024 <= (size_t)cap && persist_fits<T, true>(S.smem2, cap)) {
       S.min_two = 2 * (std::max((int)((B.kuf + B.wmax + 1 + kMaxCols - 1) / kMaxCols), B.wmax) + 2);
       break;
     }
