@@ -573,8 +573,15 @@ int band_lu_factor(T* ab, const BandLayout& L, int* ipiv, int* perm_all, int rma
 
 template <class T, class V>
 cudaError_t band_solve_setup(const BandLayout& L) {
-  return cudaFuncSetAttribute(forward_solve_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(((size_t)L.nb + L.kl) * sizeof(V)));
+  int dev = 0, cap = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaFuncAttributes fa;
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, forward_solve_kernel<T, V>);
+  if (e != cudaSuccess) return e;
+  const int dyn_cap = cap - (int)fa.sharedSizeBytes;  // process-wide, as in band_lu_setup
+  if (((size_t)L.nb + L.kl) * sizeof(V) > (size_t)dyn_cap) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(forward_solve_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_cap);
 }
 template <class T, class V>
 void band_forward(const T* ab, const BandLayout& L, const int* perm_all, int rmax, V* b, cudaStream_t st) {
