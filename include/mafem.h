@@ -72,7 +72,8 @@ enum mafem_lu_form_kind {
   MAFEM_FORM_FULL = 1,      /* full partial pivoting */
   MAFEM_FORM_PANELS = 2,    /* node-block pivoting, per-panel launches */
   MAFEM_FORM_ONE_CHAIN = 3, /* node-block pivoting, one persistent launch, from the first unknown to the last */
-  MAFEM_FORM_BOTH_ENDS = 4  /* the same from both ends: two chains of panels that meet in the middle */
+  MAFEM_FORM_BOTH_ENDS = 4  /* the same from both ends: two chains of panels that meet in the middle
+                               (side by side, or on few CTAs one after the other, with the same results) */
 };
 
 /* Params (src/input/Params.jl:36-55), field for field. */

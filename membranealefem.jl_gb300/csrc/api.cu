@@ -838,8 +838,8 @@ static int factor_enqueue(mafem_handle* h, double* x) {
   CK(cudaMemsetAsync(h->d_info, 0, sizeof(int), h->st));
   bool launched = false;
   if (h->pers.grid > 0 && h->lu_path == MAFEM_LU_AUTO) {
-    // from both ends where the grid allows (blk_two_plan)
-    const bool two = (x || !fp64) && h->pers.min_two > 0 && h->pers.grid >= h->pers.min_two && h->bwd_grid > 0;
+    // from both ends where the band is long enough (blk_two_plan), on any number of CTAs
+    const bool two = (x || !fp64) && h->pers.min_two > 0 && h->bwd_grid > 0;
     const int nl = fp64 ? blk_lu_factor_persist<double>((double*)h->d_band, h->L, h->blk, h->pers, two, h->d_perm,
                                                         (double*)h->d_rdiag, h->d_info, x, h->d_info + 1, h->st)
                         : blk_lu_factor_persist<float>((float*)h->d_band, h->L, h->blk, h->pers, two, h->d_perm,

@@ -57,7 +57,7 @@ template <class T>
 struct PersistArgs {
   T* ab;
   BlkChain c[2];              // TWO: c[0] forward on CTAs [0, split), c[1] backward on the others
-  int split;
+  int split;                  // 0: one chain after the other on all CTAs, c[1] first
   int n, off, kl, kuf;
   int rmax, wmax, nslot;      // rmax = wmax + kl: rows of a staged panel column
   int pm;
@@ -399,7 +399,12 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
     // first each chain on its own CTAs, the forward one up to panel pm, then the rest on all of them; the
     // forward chain's factorising CTA goes on without the meeting: of its panels pm alone can come before
     // it (later ones wait for columns that are updated after it), and pm's block is out of c[1]'s reach
-    const bool rev = me >= a.split;
+    // On too few CTAs for that (split 0) all of them run the backward chain, meet, and run the forward one.
+    // Every entry sees the same updates in the same order as side by side: the results do not depend on
+    // the number of CTAs.  (A batch keeps its patches on their smallest grids; one step of a batch of FP64
+    // patches against the one chain there: 24 of 8 x 8 to 16 x 16 56 -> 29 ms, 12 of 17 x 17 ALEVB 55.6 ->
+    // 51.4 ms, 8 of 32 x 32 375 -> 334 ms.)
+    const bool turn = a.split == 0, rev = me >= a.split;
     const int G0 = rev ? G - a.split : a.split;
     const int nx = a.rhs ? 2 : 1;  // CTAs of a chain that own no columns
     if (rev) me -= a.split;
@@ -416,12 +421,12 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
         __syncthreads();
         if (threadIdx.x == 0) atomicAdd(a.bdone, 1);
         if (!wait_geq(a.bdone, a.bdone_target, a.err, a.limit, &s_ok)) return;
-        if (rev) {
+        if (rev && !turn) {
           role = kWorker;
           me += a.split - nx;
         }
       }
-      const int p0 = half == 1 && role != kFactor ? a.pm : 0, p1 = half == 0 ? a.pm : a.c[0].npan;
+      const int p0 = half == 1 && role != kFactor && !turn ? a.pm : 0, p1 = half == 0 ? a.pm : a.c[0].npan;
       if (!persist_panels<T, false, true>(a, a.c[0], p0, p1, me, half == 0 ? a.split - nx : G - nx, role, smem_raw, &s_bar,
                                           ph))
         return;
@@ -477,7 +482,8 @@ int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
   S.min_grid = std::max((int)((B.kuf + B.wmax + 1 + kMinCols - 1) / kMinCols), B.wmax) + 2;
   if (S.grid < S.min_grid) return S.grid = 0;
   S.max_grid = S.grid;
-  // two chains: each on half of the CTAs, a worker with up to kMaxCols columns per panel
+  // two chains: each on half of the CTAs, a worker with up to kMaxCols columns per panel (on fewer CTAs one
+  // chain after the other); not where the device is too small for them to run side by side
   S.min_two = 0;
   for (int nslot : {8, 4}) {
     if (!B.has_two) break;
@@ -485,6 +491,7 @@ int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
     S.smem2 = persist_smem<T>(L, B.wmax, nslot, true);
     if (S.smem2 + 12 * 1024 <= (size_t)cap && persist_fits<T, true>(S.smem2, cap)) {
       S.min_two = 2 * (std::max((int)((B.kuf + B.wmax + 1 + kMaxCols - 1) / kMaxCols), B.wmax) + 2);
+      if (S.min_two > S.max_grid) S.min_two = 0;
       break;
     }
   }
@@ -500,7 +507,7 @@ int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersi
   a.c[0] = two ? B.two[0] : B.one;
   a.c[1] = B.two[1];
   const int after = two ? B.npan() : 0;  // the two chains' flags stand after the one chain's
-  a.split = two ? (S.grid + 1) / 2 : S.grid;
+  a.split = !two ? S.grid : S.grid >= S.min_two ? (S.grid + 1) / 2 : 0;
   a.n = (int)L.n;
   a.off = (int)L.off;
   a.kl = L.kl;
@@ -510,7 +517,7 @@ int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersi
   a.nslot = two ? S.nslot2 : 4;
   a.pm = B.pm;
   a.bdone = S.d_bdone;
-  a.bdone_target = S.bdone + S.grid - 1;  // all CTAs but the forward chain's factorising one
+  a.bdone_target = S.bdone + S.grid - (a.split ? 1 : 0);  // all CTAs, side by side but the forward chain's factorising one
   a.perm_all = perm_all;
   a.rdiag = rdiag;
   a.info = info;

@@ -257,7 +257,7 @@ struct BlkPersist {
   int grid = 0;            // CTAs of the launch: min_grid <= grid <= max_grid
   int min_grid = 0;        // fewest CTAs that give every worker <= kMaxCols columns per panel
   int max_grid = 0;        // the device's SM count
-  int min_two = 0;         // fewest CTAs of the two-chain form (0: not available)
+  int min_two = 0;         // fewest CTAs that run the two chains side by side (0: form not available)
   int nslot2 = 0;          // two chains: columns a worker stages at once
   size_t smem = 0, smem2 = 0;  // shared memory as one chain, as two
   unsigned epoch[2] = {0, 0};  // factorisations so far: as one chain, as two (modulo 2^32, as all counters)
@@ -278,7 +278,7 @@ template <class T>
 // published; for the owner of t's first column: [3] it starts step t - 1,
 // [4] panel t - 1 is published, [5] the copies issued before are there, [6] its
 // columns are solved, [7] the rows t reads are written, [8] the rest of the rows.
-// One chain only.  two: eliminate from both ends (needs B.has_two and grid >= min_two).
+// One chain only.  two: eliminate from both ends (needs B.has_two and min_two > 0).
 int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersist& S, bool two, int* perm_all,
                           T* rdiag, int* info, T* rhs, int* err, cudaStream_t st, long long* trace = nullptr);
 // The counters as after `count` factorisations of either form, the meeting's short of
