@@ -414,6 +414,13 @@ int mafem_set_wait_test(mafem_handle* h, int32_t limit_polls, int32_t withhold_p
  * MAFEM_ERR_UNSUPPORTED for a handle without that factorisation. */
 int mafem_set_lu_count(mafem_handle* h, uint32_t count, uint32_t missing, int32_t limit_polls);
 
+/* Test hook: the handle's cooperative launches count as refused -- factor != 0: the
+ * persistent factorisation's (per-panel launches take over); solve >= 0: of every
+ * substitution's launches those from number `solve` on (single-CTA kernels take over),
+ * -1: none.  As after a real refusal the handle keeps to the other kernels until
+ * mafem_set_launch_ctas is called. */
+int mafem_set_coop_test(mafem_handle* h, int32_t factor, int32_t solve);
+
 /* FP32 form: FP64 iterative refinement of each linear solve stops at tol
  * (default 1e-10) or fails after max_sweeps sweeps (default 30) or when it stops
  * converging (MAFEM_REFINE_STALLED).  A handle stepped on its own stops when

@@ -839,7 +839,7 @@ static int factor_enqueue(mafem_handle* h, double* x) {
   bool launched = false;
   if (h->pers.grid > 0 && h->lu_path == MAFEM_LU_AUTO) {
     // from both ends where the band is long enough (blk_two_plan), on any number of CTAs
-    const bool two = (x || !fp64) && h->pers.min_two > 0 && h->bwd_grid > 0;
+    const bool two = (x || !fp64) && h->pers.min_two > 0;
     const int nl = fp64 ? blk_lu_factor_persist<double>((double*)h->d_band, h->L, h->blk, h->pers, two, h->d_perm,
                                                         (double*)h->d_rdiag, h->d_info, x, h->d_info + 1, h->st)
                         : blk_lu_factor_persist<float>((float*)h->d_band, h->L, h->blk, h->pers, two, h->d_perm,
@@ -933,40 +933,20 @@ static int factor(mafem_handle* h, double* x, const double* rhs0) {
   return MAFEM_OK;
 }
 
-// Back substitution with the node-block factors, in place on y (device).
+// Back and forward substitution with the node-block factors, in place on y (device):
+// the cooperative multi-CTA kernels where the device allows them (a refused launch
+// sets bwd_grid to 0: single-CTA kernels from then on).
 template <class T>
 static void blk_back_solve(mafem_handle* h, double* y, const int* gate = nullptr) {
-  if (h->bwd_grid > 0) {
-    const int nl = blk_backward<T>((const T*)h->d_band, h->blk, h->last_two, y, h->d_xch, h->epoch,
-                                           h->d_info + 1, h->bwd_grid, h->st, h->wait_test, gate);
-    if (nl > 0 || h->last_two) {  // the factors of the two chains are for the cooperative kernel alone:
-      h->launches += std::max(nl, 0);  // a refused launch stays as the CUDA error that the caller reports
-      return;
-    }
-    cudaGetLastError();
-    h->bwd_grid = 0;  // cooperative launch refused: use the single-CTA kernel from now on
-  }
-  blk_backward_1cta<double, T>((const T*)h->d_band, h->L, h->blk, y, h->st);
-  h->launches += 1;
+  h->launches += blk_backward<T>((const T*)h->d_band, h->blk, h->last_two, y, h->d_xch, h->epoch, h->d_info + 1,
+                                 h->bwd_grid, h->st, h->wait_test, gate);
 }
-
-// Forward substitution with the node-block factors, in place on y (device):
-// the cooperative multi-CTA kernel where the device allows it.
 template <class T>
 static void blk_fwd_solve(mafem_handle* h, double* y, const int* gate = nullptr) {
-  if (h->bwd_grid > 0) {
-    blk_need_inverses(h);
-    const int nl = blk_forward_coop<T>((const T*)h->d_band, h->L, h->blk, h->last_two, h->d_pinv, y, h->d_xch, h->epoch,
-                                       h->d_info + 1, h->bwd_grid, h->st,
-                                               h->wait_test, gate);
-    if (nl > 0 || h->last_two) {
-      h->launches += std::max(nl, 0);
-      return;
-    }
-    cudaGetLastError();
-  }
-  blk_forward<double, T>((const T*)h->d_band, h->L, h->blk, h->d_perm, (const T*)h->d_rdiag, y, h->st);
-  h->launches += 1;
+  if (h->bwd_grid > 0) blk_need_inverses(h);
+  h->launches += blk_forward<T>((const T*)h->d_band, h->L, h->blk, h->last_two, h->d_perm, (const T*)h->d_rdiag,
+                                h->d_pinv, y, h->d_xch, h->epoch, h->d_info + 1, h->bwd_grid, h->st, h->wait_test,
+                                gate);
 }
 
 // info[0]: zero-pivot column, info[1]: a bounded device wait ran out (h_out + 5 holds both)
@@ -2894,6 +2874,13 @@ extern "C" int mafem_set_dirichlet_scale(mafem_handle* h, double scale) {
   launch_dirichlet_scale(h->P.cps, h->d_dir_idx, h->d_dir_val, h->n_dir, scale, h->st);
   h->launches += h->n_dir > 0 ? 1 : 0;
   CK(cudaGetLastError());
+  return MAFEM_OK;
+}
+
+extern "C" int mafem_set_coop_test(mafem_handle* h, int32_t factor, int32_t solve) {
+  if (!h || solve < -1) return MAFEM_ERR_ARG;
+  h->pers.refuse = factor != 0;
+  h->wait_test.refuse = solve;
   return MAFEM_OK;
 }
 

@@ -214,95 +214,108 @@ __global__ void __launch_bounds__(128) blk_apply_col_kernel(T* __restrict__ ab, 
   for (int r = tid; r < w; r += 128) ab[bix(L, j0 + r, c)] = s[r];
 }
 
-// ---------------------------------------------------------------------------
-// Forward substitution with the stored panels, one CTA (re-solves and the
-// refinement sweeps of the FP32 form).
-template <class T, class V>
-__global__ void __launch_bounds__(1024) blk_forward_kernel(const T* __restrict__ ab, BandLayout L,
-                                                           const int* __restrict__ ps, int npan,
-                                                           const int* __restrict__ perm_all,
-                                                           const T* __restrict__ rdiag, V* __restrict__ b) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  V* s = reinterpret_cast<V*>(smem_raw);  // [R]
-  __shared__ V Ls[32][33];
-  __shared__ V y[32];
-  __shared__ V rd[32];
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int pnl = 0; pnl < npan; ++pnl) {
-    const int64_t j0 = ps[pnl];
-    const int w = ps[pnl + 1] - ps[pnl];
-    const int R = (int)min64b(L.n - j0, (int64_t)w + L.kl);
-    const int* pm = perm_all + (size_t)pnl * kBlkW;
-    for (int r = tid; r < R; r += nt) s[r] = b[j0 + (r < w ? pm[r] : r)];
-    for (int k = tid; k < w * w; k += nt) {
-      const int c = k / w, i = k - c * w;
-      Ls[c][i] = V(ab[bix(L, j0 + i, j0 + c)]);
-    }
-    if (tid < w) rd[tid] = V(rdiag[j0 + tid]);
-    __syncthreads();
-    if (tid < 32) {
-      V x = tid < w ? s[tid] : V(0);
-      for (int k = 0; k < w; ++k) {
-        const V xk = __shfl_sync(kFull, x, k);
-        if (tid > k && tid < w) x -= Ls[k][tid] * xk;
-      }
-      V v = x;
-      for (int k = w - 1; k >= 0; --k) {
-        V yk = tid == k ? v * rd[k] : V(0);
-        yk = __shfl_sync(kFull, yk, k);
-        if (tid == k) v = yk;
-        if (tid < k) v -= Ls[k][tid] * yk;
-      }
-      if (tid < w) s[tid] = v;
-      y[tid] = tid < w ? v : V(0);
-    }
-    __syncthreads();
-    for (int r = w + tid; r < R; r += nt) {
-      V acc = s[r];
-      const T* row = ab + bix(L, j0 + r, j0);  // A(j0 + r, j0 + k) = row[k * (ldb - 1)]
-#pragma unroll 8
-      for (int k = 0; k < w; ++k) acc -= V(row[(int64_t)k * (L.ldb - 1)]) * y[k];
-      s[r] = acc;
-    }
-    __syncthreads();
-    for (int r = tid; r < R; r += nt) b[j0 + r] = s[r];
-    __syncthreads();
-  }
-}
+// A launch covers panels [p0, p1) of one chain, or of two chains side by side (CTAs
+// below `split` the first): the columns right of panel p1 - 1 (backward) or the panels
+// before p0 (forward) belong to an earlier launch.
+struct BlkSpan {
+  BlkChain c;
+  int p0, p1;
+};
 
-// Back substitution x1 = z - Y x2, one CTA, panels in reverse; Y has kuf
-// super-diagonals.
-template <class T, class V>
-__global__ void __launch_bounds__(1024) blk_backward_kernel(const T* __restrict__ ab, BandLayout L, int kuf,
-                                                            const int* __restrict__ ps, int npan, V* __restrict__ y) {
-  __shared__ V part[32][33];
+// ---------------------------------------------------------------------------
+// Substitutions by one CTA, over the spans of the cooperative ones (below) in the same
+// order, where a cooperative launch is not possible.  Forward: z(p) = A11^-1 (b(p) -
+// the panels before it), pulled, so that either kernel can go on after the other.
+template <class T>
+__global__ void __launch_bounds__(1024) blk_forward_kernel(const T* __restrict__ ab, int kl, BlkSpan S,
+                                                           const int* __restrict__ perm_all,
+                                                           const T* __restrict__ rdiag_all, double* bv,
+                                                           const int* __restrict__ gate) {
+  __shared__ double part[32][33], Ls[32][33], xs[32];
+  if (gate && *gate) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  for (int pnl = npan - 1; pnl >= 0; --pnl) {
-    const int64_t j0 = ps[pnl];
-    const int w = ps[pnl + 1] - ps[pnl];
-    const int64_t j1 = j0 + w;
-    const int64_t jend = min64b(L.n, j1 + kuf);
-    V acc = V(0);
+  const int64_t si = S.c.si, sj = S.c.sj;
+  const T* __restrict__ A = ab + S.c.org;  // element (i, j) at A[i si + j sj]
+  double* b = bv + S.c.vorg;               // element i at b[i si]
+  for (int p = S.p0; p < S.p1; ++p) {
+    const int j0 = S.c.ps[p], w = S.c.ps[p + 1] - j0;
+    for (int k = tid; k < w * w; k += blockDim.x) {
+      const int c = k / w, i = k - c * w;
+      Ls[c][i] = (double)A[(j0 + i) * si + (j0 + c) * sj];
+    }
+    double acc = 0.0;
+    const int r = j0 + lane;
     if (lane < w) {
-      int64_t c = j1 + warp;
-      for (; c + 7 * nw < jend; c += 8 * nw) {
-        V u[8], xv[8];
+      int c = max(0, r - kl) + warp;  // the row's first stored column
+      for (; c + 7 * nw < j0; c += 8 * nw) {
+        double a[8], z[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          u[q] = V(ab[bix(L, j0 + lane, c + q * nw)]);
-          xv[q] = y[c + q * nw];
+          a[q] = (double)A[r * si + (c + q * nw) * sj];
+          z[q] = b[(c + q * nw) * si];
         }
 #pragma unroll
-        for (int q = 0; q < 8; ++q) acc += u[q] * xv[q];
+        for (int q = 0; q < 8; ++q) acc = fma(a[q], z[q], acc);
       }
-      for (; c < jend; c += nw) acc += V(ab[bix(L, j0 + lane, c)]) * y[c];
+      for (; c < j0; c += nw) acc = fma((double)A[r * si + c * sj], b[c * si], acc);
     }
     part[warp][lane] = acc;
     __syncthreads();
     if (warp == 0) {
-      V sum = V(0);
+      double sum = 0.0;
       for (int k = 0; k < nw; ++k) sum += part[k][lane];
-      if (lane < w) y[j0 + lane] -= sum;
+      xs[lane] = lane < w ? b[r * si] - sum : 0.0;
+      __syncwarp();
+      double x = lane < w ? xs[perm_all[(size_t)(S.c.pbase + p) * kBlkW + lane]] : 0.0;
+      for (int k = 0; k < w; ++k) {
+        const double xk = __shfl_sync(kFull, x, k);
+        if (lane > k && lane < w) x -= Ls[k][lane] * xk;
+      }
+      const double rd = lane < w ? (double)rdiag_all[S.c.rbase + r] : 0.0;
+      for (int k = w - 1; k >= 0; --k) {
+        const double yk = __shfl_sync(kFull, x * rd, k);
+        if (lane == k) x = yk;
+        if (lane < k) x -= Ls[k][lane] * yk;
+      }
+      if (lane < w) b[r * si] = x;
+    }
+    __syncthreads();
+  }
+}
+
+// Back substitution x1 = z - Y x2, panels in reverse; Y has kuf super-diagonals.
+template <class T>
+__global__ void __launch_bounds__(1024) blk_backward_kernel(const T* __restrict__ ab, int kuf, BlkSpan S, double* yv,
+                                                            const int* __restrict__ gate) {
+  __shared__ double part[32][33];
+  if (gate && *gate) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int64_t si = S.c.si, sj = S.c.sj;
+  double* y = yv + S.c.vorg;
+  for (int p = S.p1 - 1; p >= S.p0; --p) {
+    const int j0 = S.c.ps[p], j1 = S.c.ps[p + 1], w = j1 - j0, jend = min(S.c.n, j1 + kuf);
+    const T* __restrict__ row = ab + S.c.org + (j0 + lane) * si;  // A(j0 + lane, c) at row[c sj]
+    double acc = 0.0;
+    if (lane < w) {
+      int c = j1 + warp;
+      for (; c + 7 * nw < jend; c += 8 * nw) {
+        double u[8], xv[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          u[q] = (double)row[(c + q * nw) * sj];
+          xv[q] = y[(c + q * nw) * si];
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc = fma(u[q], xv[q], acc);
+      }
+      for (; c < jend; c += nw) acc = fma((double)row[c * sj], y[c * si], acc);
+    }
+    part[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0) {
+      double sum = 0.0;
+      for (int k = 0; k < nw; ++k) sum += part[k][lane];
+      if (lane < w) y[(j0 + lane) * si] -= sum;
     }
     __syncthreads();
   }
@@ -423,13 +436,6 @@ __device__ __forceinline__ bool fetch(const SolveWord* X, int cg, int nc, long l
   }
 }
 
-// A launch covers panels [p0, p1) of one chain, or of two chains side by side (CTAs
-// below `split` the first): the columns right of panel p1 - 1 (backward) or the panels
-// before p0 (forward) belong to an earlier launch.
-struct BlkSpan {
-  BlkChain c;
-  int p0, p1;
-};
 constexpr int kSolveThreads = 128;
 
 // Back substitution x1 = z - Y x2.
@@ -678,8 +684,6 @@ int blk_lu_setup(const BandLayout& L) {
   if (cudaFuncSetAttribute(blk_apply_kernel<T, kApplyNR>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap) !=
           cudaSuccess ||
       cudaFuncSetAttribute(blk_apply_col_kernel<T, kColNR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           cap - 10 * 1024) != cudaSuccess ||
-      cudaFuncSetAttribute(blk_forward_kernel<T, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            cap - 10 * 1024) != cudaSuccess)
     return 0;
   return wmax;
@@ -761,12 +765,6 @@ int blk_lu_factor(T* ab, const BandLayout& L, const BlkPlan& B, int* perm_all, T
 }
 
 template <class V, class T>
-void blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, const int* perm_all, const T* rdiag, V* b,
-                 cudaStream_t st) {
-  const size_t sm = ((size_t)B.wmax + L.kl) * sizeof(V);
-  blk_forward_kernel<T, V><<<1, 1024, sm, st>>>(ab, L, B.d_ps, B.npan(), perm_all, rdiag, b);
-}
-template <class V, class T>
 int blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
                  V* inv, cudaStream_t st) {
   const BlkChain &c0 = two ? B.two[0] : B.one, &c1 = B.two[1];
@@ -774,61 +772,78 @@ int blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, c
   blk_inverses_kernel<T, V><<<b0 + b1, 128, 0, st>>>(ab, c0, c1, b0, L.kl, perm_all, rdiag, inv);
   return 1;
 }
-// One cooperative launch over spans a and (optionally) b, its CTAs shared out by their panels.
-template <class F>
-static int coop_spans(F&& launch, const BlkSpan& a, const BlkSpan* b, int grid) {
+// One cooperative launch over spans a and (optionally) b, its CTAs shared out by their
+// panels.  Where it is refused (then *coop = false) or *coop is false already: one(a),
+// one(b), single-CTA launches.  Returns the launches.
+template <class F, class G>
+static int coop_spans(F&& launch, G&& one, const BlkSpan& a, const BlkSpan* b, int grid, bool* coop) {
   const int na = a.p1 - a.p0, nb = b ? b->p1 - b->p0 : 0;
   if (na + nb <= 0) return 0;
-  if (nb > 0 && grid < 2) {  // one after the other
-    const int ra = coop_spans(launch, a, nullptr, grid), rb = coop_spans(launch, *b, nullptr, grid);
-    return ra < 0 || rb < 0 ? -1 : ra + rb;
+  if (*coop && nb > 0 && grid < 2)  // one after the other
+    return coop_spans(launch, one, a, nullptr, grid, coop) + coop_spans(launch, one, *b, nullptr, grid, coop);
+  if (*coop) {
+    const int ga = std::min(na, nb > 0 ? grid / 2 : grid), gb = std::min(nb, grid - ga);
+    if (launch(a, b ? *b : a, ga, ga + gb) == cudaSuccess) return 1;
+    cudaGetLastError();
+    *coop = false;
   }
-  const int ga = std::min(na, nb > 0 ? grid / 2 : grid), gb = std::min(nb, grid - ga);
-  return launch(a, b ? *b : a, ga, ga + gb) == cudaSuccess ? 1 : -1;
+  one(a);
+  if (nb > 0) one(*b);
+  return nb > 0 ? 2 : 1;
 }
 template <class T>
-int blk_backward(const T* ab, const BlkPlan& B, bool two, double* y, SolveWord* xch, int64_t& epoch, int* err, int grid,
-                 cudaStream_t st, WaitTest wt, const int* gate) {
-  int kuf = B.kuf;
+int blk_backward(const T* ab, const BlkPlan& B, bool two, double* y, SolveWord* xch, int64_t& epoch, int* err,
+                 int& grid, cudaStream_t st, WaitTest wt, const int* gate) {
+  int kuf = B.kuf, through = 0;
+  bool coop = grid > 0;
   auto launch = [&](BlkSpan a, BlkSpan b, int split, int ctas) {
+    if (wt.refuse >= 0 && through++ >= wt.refuse) return cudaErrorCooperativeLaunchTooLarge;
     ++epoch;
     void* args[] = {(void*)&ab,    (void*)&kuf, (void*)&a,  (void*)&b,   (void*)&split, (void*)&y, (void*)&xch,
                     (void*)&epoch, (void*)&err, (void*)&wt, (void*)&gate};
     return cudaLaunchCooperativeKernel((const void*)blk_backward_coop_kernel<T>, dim3(ctas), dim3(kSolveThreads), args, 0,
                                        st);
   };
-  if (!two) return coop_spans(launch, BlkSpan{B.one, 0, B.one.npan}, nullptr, grid);
-  // the unknowns between the chains, then both chains side by side
-  const int r1 = coop_spans(launch, BlkSpan{B.two[0], B.pm, B.two[0].npan}, nullptr, grid);
-  if (r1 < 0) return r1;
-  const BlkSpan b1{B.two[1], 0, B.two[1].npan};
-  const int r2 = coop_spans(launch, BlkSpan{B.two[0], 0, B.pm}, &b1, grid);
-  return r2 < 0 ? r2 : r1 + r2;
-}
-// single-CTA back substitution (used when a cooperative launch is not possible)
-template <class V, class T>
-void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, cudaStream_t st) {
-  blk_backward_kernel<T, V><<<1, 1024, 0, st>>>(ab, L, B.kuf, B.d_ps, B.npan(), y);
+  auto one = [&](const BlkSpan& s) { blk_backward_kernel<T><<<1, 1024, 0, st>>>(ab, kuf, s, y, gate); };
+  int nl;
+  if (!two) {
+    nl = coop_spans(launch, one, BlkSpan{B.one, 0, B.one.npan}, nullptr, grid, &coop);
+  } else {
+    // the unknowns between the chains, then both chains side by side
+    nl = coop_spans(launch, one, BlkSpan{B.two[0], B.pm, B.two[0].npan}, nullptr, grid, &coop);
+    const BlkSpan b1{B.two[1], 0, B.two[1].npan};
+    nl += coop_spans(launch, one, BlkSpan{B.two[0], 0, B.pm}, &b1, grid, &coop);
+  }
+  if (!coop) grid = 0;
+  return nl;
 }
 template <class T>
-int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const double* inv, double* b,
-                     SolveWord* xch, int64_t& epoch, int* err, int grid, cudaStream_t st, WaitTest wt, const int* gate) {
-  int kl = L.kl;
+int blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
+                const double* inv, double* b, SolveWord* xch, int64_t& epoch, int* err, int& grid, cudaStream_t st,
+                WaitTest wt, const int* gate) {
+  int kl = L.kl, through = 0;
+  bool coop = grid > 0;
   auto launch = [&](BlkSpan s0, BlkSpan s1, int split, int ctas) {
+    if (wt.refuse >= 0 && through++ >= wt.refuse) return cudaErrorCooperativeLaunchTooLarge;
     ++epoch;
     void* args[] = {(void*)&ab, (void*)&kl,  (void*)&s0,    (void*)&s1,  (void*)&split, (void*)&inv,
                     (void*)&b,  (void*)&xch, (void*)&epoch, (void*)&err, (void*)&wt,    (void*)&gate};
     return cudaLaunchCooperativeKernel((const void*)blk_forward_coop_kernel<T>, dim3(ctas), dim3(kSolveThreads), args, 0,
                                        st);
   };
-  if (!two) return coop_spans(launch, BlkSpan{B.one, 0, B.one.npan}, nullptr, grid);
-  const BlkSpan s1{B.two[1], 0, B.two[1].npan};
-  const int r1 = coop_spans(launch, BlkSpan{B.two[0], 0, B.pm}, &s1, grid);
-  if (r1 < 0) return r1;
-  const int lo = std::max(0, B.mid - L.kl);
-  blk_forward_mid_kernel<T, double><<<(B.mid - lo + 7) / 8, 256, 0, st>>>(ab, L, B.mid, lo, b, gate);
-  const int r2 = coop_spans(launch, BlkSpan{B.two[0], B.pm, B.two[0].npan}, nullptr, grid);
-  return r2 < 0 ? r2 : r1 + 1 + r2;
+  auto one = [&](const BlkSpan& s) { blk_forward_kernel<T><<<1, 1024, 0, st>>>(ab, kl, s, perm_all, rdiag, b, gate); };
+  int nl;
+  if (!two) {
+    nl = coop_spans(launch, one, BlkSpan{B.one, 0, B.one.npan}, nullptr, grid, &coop);
+  } else {
+    const BlkSpan s1{B.two[1], 0, B.two[1].npan};
+    nl = coop_spans(launch, one, BlkSpan{B.two[0], 0, B.pm}, &s1, grid, &coop);
+    const int lo = std::max(0, B.mid - L.kl);
+    blk_forward_mid_kernel<T, double><<<(B.mid - lo + 7) / 8, 256, 0, st>>>(ab, L, B.mid, lo, b, gate);
+    nl += 1 + coop_spans(launch, one, BlkSpan{B.two[0], B.pm, B.two[0].npan}, nullptr, grid, &coop);
+  }
+  if (!coop) grid = 0;
+  return nl;
 }
 // CTAs of the cooperative back substitution that can be resident at once
 template <class T>
@@ -847,27 +862,21 @@ template int blk_lu_factor<double>(double*, const BandLayout&, const BlkPlan&, i
                                    cudaStream_t, cudaStream_t, cudaEvent_t*, cudaEvent_t*);
 template int blk_lu_factor<float>(float*, const BandLayout&, const BlkPlan&, int*, float*, int*, float*, cudaStream_t,
                                   cudaStream_t, cudaEvent_t*, cudaEvent_t*);
-template void blk_forward<double, double>(const double*, const BandLayout&, const BlkPlan&, const int*, const double*,
-                                          double*, cudaStream_t);
-template void blk_forward<double, float>(const float*, const BandLayout&, const BlkPlan&, const int*, const float*,
-                                         double*, cudaStream_t);
 template int blk_inverses<double, double>(const double*, const BandLayout&, const BlkPlan&, bool, const int*,
                                           const double*, double*, cudaStream_t);
 template int blk_inverses<double, float>(const float*, const BandLayout&, const BlkPlan&, bool, const int*, const float*,
                                          double*, cudaStream_t);
-template int blk_backward<double>(const double*, const BlkPlan&, bool, double*, SolveWord*, int64_t&, int*, int, cudaStream_t,
-                                  WaitTest, const int*);
-template int blk_backward<float>(const float*, const BlkPlan&, bool, double*, SolveWord*, int64_t&, int*, int, cudaStream_t,
-                                 WaitTest, const int*);
-template void blk_backward_1cta<double, double>(const double*, const BandLayout&, const BlkPlan&, double*,
-                                                cudaStream_t);
-template void blk_backward_1cta<double, float>(const float*, const BandLayout&, const BlkPlan&, double*,
-                                               cudaStream_t);
+template int blk_backward<double>(const double*, const BlkPlan&, bool, double*, SolveWord*, int64_t&, int*, int&,
+                                  cudaStream_t, WaitTest, const int*);
+template int blk_backward<float>(const float*, const BlkPlan&, bool, double*, SolveWord*, int64_t&, int*, int&,
+                                 cudaStream_t, WaitTest, const int*);
 template int blk_backward_grid<double>();
 template int blk_backward_grid<float>();
-template int blk_forward_coop<double>(const double*, const BandLayout&, const BlkPlan&, bool, const double*, double*,
-                                      SolveWord*, int64_t&, int*, int, cudaStream_t, WaitTest, const int*);
-template int blk_forward_coop<float>(const float*, const BandLayout&, const BlkPlan&, bool, const double*, double*,
-                                     SolveWord*, int64_t&, int*, int, cudaStream_t, WaitTest, const int*);
+template int blk_forward<double>(const double*, const BandLayout&, const BlkPlan&, bool, const int*, const double*,
+                                 const double*, double*, SolveWord*, int64_t&, int*, int&, cudaStream_t, WaitTest,
+                                 const int*);
+template int blk_forward<float>(const float*, const BandLayout&, const BlkPlan&, bool, const int*, const float*,
+                                const double*, double*, SolveWord*, int64_t&, int*, int&, cudaStream_t, WaitTest,
+                                const int*);
 
 }  // namespace mafem

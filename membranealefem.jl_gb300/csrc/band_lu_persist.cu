@@ -502,6 +502,7 @@ int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
 template <class T>
 int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersist& S, bool two, int* perm_all,
                           T* rdiag, int* info, T* rhs, int* err, cudaStream_t st, long long* trace) {
+  if (S.refuse) return -1;
   PersistArgs<T> a;
   a.ab = ab;
   a.c[0] = two ? B.two[0] : B.one;

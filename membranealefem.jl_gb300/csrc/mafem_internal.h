@@ -215,41 +215,42 @@ int blk_lu_setup(const BandLayout& L);
 template <class T>
 int blk_lu_factor(T* ab, const BandLayout& L, const BlkPlan& B, int* perm_all, T* rdiag, int* info, T* rhs,
                   cudaStream_t st, cudaStream_t st2, cudaEvent_t* ev_pool, cudaEvent_t* prof);
-template <class V, class T>
-void blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, const int* perm_all, const T* rdiag, V* b,
-                 cudaStream_t st);
-// Back substitution x1 = z - Y x2 in place on many SMs (cooperative launches of at
-// most `grid` CTAs, grid <= blk_backward_grid()).  xch: npan_max x 32 words; epoch: a
-// value that no word's tag holds yet is taken per launch; err: nonzero after a bounded
-// wait ran out.  two: the factors of the two-chain elimination.  Returns the
-// kernels launched, or -1 if a launch failed.
+// What the panels of a cooperative substitution hand on.
 struct alignas(16) SolveWord {
   double v;
   long long tag;
 };
-// Failure-detection test hook of the cooperative substitutions: limit = polls
-// before a wait gives up (<= 0: the default), withhold = k: the back
-// substitution never publishes the flag of panel npan - 1 - k (-1: none).
+// Test hook of the cooperative substitutions: limit = polls before a wait gives up
+// (<= 0: the default), withhold = k: the back substitution never publishes the
+// solution of panel npan - 1 - k (-1: none); refuse = k: of a substitution's
+// cooperative launches the k-th and later ones count as refused (-1: none).
 struct WaitTest {
   int limit = 0;
   int withhold = -1;
+  int refuse = -1;
 };
 // Per panel the inverse of its diagonal block and its product with the rows of the
 // panel before (inv: npan_max x 2 x 32 x 32) for the cooperative forward substitution.
 template <class V, class T>
 int blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
                  V* inv, cudaStream_t st);
+// Back substitution x1 = z - Y x2 in place on many SMs (cooperative launches of at
+// most `grid` CTAs, grid <= blk_backward_grid()).  xch: npan_max x 32 words; epoch: a
+// value that no word's tag holds yet is taken per launch; err: nonzero after a bounded
+// wait ran out.  two: the factors of the two-chain elimination.  With grid 0, and from
+// a refused cooperative launch on (grid is then set to 0), by single-CTA kernels.
+// Returns the kernels launched.
 template <class T>
-int blk_backward(const T* ab, const BlkPlan& B, bool two, double* y, SolveWord* xch, int64_t& epoch, int* err, int grid,
-                 cudaStream_t st, WaitTest wt = WaitTest(), const int* gate = nullptr);
+int blk_backward(const T* ab, const BlkPlan& B, bool two, double* y, SolveWord* xch, int64_t& epoch, int* err,
+                 int& grid, cudaStream_t st, WaitTest wt = WaitTest(), const int* gate = nullptr);
 template <class T>
 int blk_backward_grid();
 // Forward substitution (P, L11, A21 of the stored panels), in place on b; the rest as for
-// blk_backward.  Returns the kernels launched, or -1 if a launch was refused.
+// blk_backward.  inv: blk_inverses' (read by the cooperative launches alone).
 template <class T>
-int blk_forward_coop(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const double* inv, double* b,
-                     SolveWord* xch, int64_t& epoch, int* err, int grid, cudaStream_t st, WaitTest wt = WaitTest(),
-                     const int* gate = nullptr);
+int blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
+                const double* inv, double* b, SolveWord* xch, int64_t& epoch, int* err, int& grid, cudaStream_t st,
+                WaitTest wt = WaitTest(), const int* gate = nullptr);
 // Persistent cooperative factorisation (band_lu_persist.cu): launch shape and
 // per-panel flags.  Flags are zeroed once; epochs make them reusable.  The arrays
 // hold the one chain's npan panels, then the two chains'.
@@ -263,6 +264,7 @@ struct BlkPersist {
   unsigned epoch[2] = {0, 0};  // factorisations so far: as one chain, as two (modulo 2^32, as all counters)
   unsigned bdone = 0;          // *d_bdone once the last two-chain factorisation is done
   int limit = 0;               // polls before a wait gives up (0: kSpinLimit); tests only
+  bool refuse = false;         // tests only: its launches count as refused
   int* d_bdone = nullptr;  // counts the CTAs that are done with what the two chains do apart
   int* d_pdone = nullptr;
   int* d_critcnt = nullptr;
@@ -285,8 +287,6 @@ int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersi
 // `missing` arrivals; waits for st.  count 0: as new, after a wait that ran out has
 // left them behind (0 missing).  Other values: tests.
 cudaError_t blk_persist_count(const BlkPlan& B, BlkPersist& S, unsigned count, unsigned missing, cudaStream_t st);
-template <class V, class T>
-void blk_backward_1cta(const T* ab, const BandLayout& L, const BlkPlan& B, V* y, cudaStream_t st);
 }  // namespace mafem
 
 namespace mafem {

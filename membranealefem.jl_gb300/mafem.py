@@ -176,6 +176,7 @@ def lib():
         L.mafem_launch_count.restype = C.c_int64
         L.mafem_set_lu_path.argtypes = [vp, C.c_int32]
         L.mafem_lu_form.argtypes = [vp]
+        L.mafem_set_coop_test.argtypes = [vp, C.c_int32, C.c_int32]
         L.mafem_set_lu_count.argtypes = [vp, C.c_uint32, C.c_uint32, C.c_int32]
         L.mafem_two_chain_plan.argtypes = [C.POINTER(MeshDesc), C.c_int32, C.c_int32, _P64, C.c_int64]
         L.mafem_set_patch_ctas.argtypes = [vp, C.c_int32]
@@ -542,6 +543,11 @@ class Solver:
         give up after limit_polls polls; the back substitution withholds the flag of
         the panel withhold_panel places before the last.  (0, -1) restores the default."""
         _raise(lib().mafem_set_wait_test(self.h, limit_polls, withhold_panel), self.h)
+
+    def set_coop_test(self, factor: bool = False, solve: int = -1) -> None:
+        """Test hook: cooperative launches count as refused -- the factorisation's, and a
+        substitution's from number `solve` on (-1: none)."""
+        _raise(lib().mafem_set_coop_test(self.h, int(factor), solve), self.h)
 
     def set_lu_count(self, count: int = 0, missing: int = 0, limit_polls: int = 0) -> None:
         """Test hook: the persistent factorisation's counters as after `count` factorisations,
