@@ -521,7 +521,7 @@ struct RefineSmem {
   float ring[kRing][2][kBlkW * kBlkW];  // forward: A21's rows of the next panel, the next panel's Ai; backward: Y's columns
   float zb[2][kBlkW];                   // z of the current panel, by parity
   float bb[kBlkW];
-  float part[2][kRT / 32][kBlkW];       // backward: the update warps' sums, by parity
+  alignas(16) float part[2][kRT / 32][kBlkW];  // backward: the update warps' sums, by parity
   double red[kRT / 32];
 };
 size_t patch_refine_smem(int64_t n, int npan) {
@@ -895,9 +895,6 @@ __device__ __forceinline__ double residual_rows(const PatchJob& J, const float2*
   }
   return ss;
 }
-__device__ double patch_residual(const PatchJob& J, const float2* xs, double* red) {
-  return sqrt(block_sum(residual_rows(J, xs, threadIdx.x >> 5, kRT / 32), red));
-}
 // The residual after a sweep on kResC CTAs per patch: partial sums of its squares to J.rs + 8.
 constexpr int kResC = 8, kResT = 256;
 __global__ void __launch_bounds__(kResT) patch_residual_kernel(const PatchJob* __restrict__ jobs,
@@ -915,6 +912,24 @@ __global__ void __launch_bounds__(kResT) patch_residual_kernel(const PatchJob* _
     for (int q = 0; q < kResT / 32; ++q) t += red[q];
     J.rs[8 + c] = t;
   }
+}
+// The same by one CTA of kRT threads, its norm summed in the same order: a patch's sweeps give the same bits
+// in either kernel, whichever group of a round it is in.  red: kResC * kResT / 32 doubles of shared memory.
+__device__ double patch_residual(const PatchJob& J, const float2* xs, double* red) {
+  constexpr int kW = kResT / 32;  // warps of a CTA of patch_residual_kernel
+  for (int q = threadIdx.x >> 5; q < kResC * kW; q += kRT / 32) {
+    double ss = residual_rows(J, xs, q, kResC * kW);
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(kFull, ss, o);
+    if ((threadIdx.x & 31) == 0) red[q] = ss;
+  }
+  __syncthreads();
+  double s = 0.0;
+  for (int c = 0; c < kResC; ++c) {
+    double t = 0.0;
+    for (int q = 0; q < kW; ++q) t += red[c * kW + q];
+    s += t;
+  }
+  return sqrt(s);
 }
 
 
@@ -1027,7 +1042,7 @@ __global__ void __launch_bounds__(kRT, 1) patch_refine_kernel(const PatchJob* __
     double dd = 0.0, xx = 0.0;
     for (int64_t i = tid; i < n; i += kRT) {
       const double d = rn * (double)v[i];
-      const double x = J.x[i] + d;
+      const double x = fma(rn, (double)v[i], J.x[i]);
       J.x[i] = x;
       const float xh = (float)x;
       xs[i] = make_float2(xh, (float)(x - (double)xh));
@@ -1061,7 +1076,8 @@ __global__ void __launch_bounds__(kRT, 1) patch_refine_kernel(const PatchJob* __
       }
       return;
     } else {
-      rn = patch_residual(J, xs, red);  // block_sum orders the x / xs writes before it
+      // block_sum orders the x / xs writes before it; the update warps' sums are not in use
+      rn = patch_residual(J, xs, reinterpret_cast<double*>(S.part));
       if (!after_residual(k, dn, xn)) return;
       prev_dn = dn;
     }
