@@ -282,17 +282,84 @@ static std::vector<int> pivot_blocks(const std::vector<int>& unk_node) {
   return blk_end;
 }
 
+// Node of every unknown (-1: none) from a mesh's ID; false if an entry is out of range.
+static bool nodes_of_unknowns(const mafem_mesh_desc* d, std::vector<int>& unk_node) {
+  unk_node.assign(d->nmdf, -1);
+  for (int64_t k = 0; k < d->ndf * d->numnp; ++k) {
+    if (d->ID[k] < 0 || d->ID[k] > d->nmdf) return false;
+    if (d->ID[k] > 0) unk_node[d->ID[k] - 1] = (int)(k / d->ndf);
+  }
+  return true;
+}
+
+// Element counts of the arrays of a handle that depend on its elimination plan: what
+// mafem_create allocates and mafem_footprint_bytes adds up.
+struct PlanSizes {
+  size_t perm, xch = 0, pinv = 0, flags = 0, inv = 0, a21 = 0;
+};
+static PlanSizes plan_sizes(const BandLayout& L, const BlkPlan& B, bool use_blk, bool patch) {
+  PlanSizes s;
+  s.perm = (size_t)((L.n + L.nb - 1) / L.nb) * ((size_t)L.nb + L.kl);
+  if (!use_blk) return s;
+  const size_t npx = (size_t)B.npan_max();
+  s.perm = std::max(s.perm, npx * kBlkW);
+  s.xch = npx * kBlkW;
+  s.pinv = npx * 2 * kBlkW * kBlkW;
+  s.flags = (size_t)B.npan() + (size_t)B.two[0].npan + (size_t)B.two[1].npan;
+  if (patch) {
+    s.inv = (size_t)B.npan() * kBlkW * kBlkW;
+    s.a21 = patch_a21_elems(patch_a21_rows(L.kl));
+  }
+  return s;
+}
+constexpr size_t kPartials = 4096;  // partial sums: of an update (2 x 1024), of a residual (2048)
+
+// The batched FP32 form serves a handle: its refinement residual reads every band
+// window without bounds checks, which needs nb >= 32 rows of padding, and its kernels
+// have `dyn` bytes of shared memory.
+static bool patch_fits(const BandLayout& L, const BlkPlan& B, int dyn) {
+  return L.nb >= 32 && dyn > 0 && patch_factor_smem() <= (size_t)dyn &&
+         patch_refine_smem(L.n, B.npan()) <= (size_t)dyn;
+}
+
+// Bytes of device memory mafem_create allocates for a mesh.
 static int64_t footprint(const mafem_mesh_desc* d, int precision, int64_t kl) {
+  const bool fp64 = precision == MAFEM_PLAIN_FP64;
+  const int64_t n = d->nmdf, nq = 9 * d->ndf, esz = fp64 ? 8 : 4;
   const int nb = choose_nb((int)kl, precision);
-  BandLayout L = make_band_layout(d->nmdf, (int)kl, (int)kl, nb ? nb : 8);
-  const int64_t esz = precision == MAFEM_PLAIN_FP64 ? 8 : 4;
-  const int64_t nq = 9 * d->ndf;
-  int64_t b = L.ldb * d->nmdf * esz * (precision == MAFEM_PLAIN_FP64 ? 1 : 2);  // band (+ unfactored copy)
-  b += d->numel * nq * nq * esz + d->numel * nq * 8;                             // element staging
-  b += d->numnp * (3 + d->ndf) * 8 + d->nmdf * 8 * 6;                           // state + vectors
-  b += ((d->nmdf + nb - 1) / std::max(nb, 1)) * ((int64_t)nb + kl) * 4;           // panel permutations
-  b += d->nmdf * (esz + 4);                                                      // pivot reciprocals, blocks
-  b += (d->nmdf / 24 + 1) * 2 * 32 * 32 * 8;                                     // panel triangle inverses
+  const BandLayout L = make_band_layout(n, (int)kl, (int)kl, nb ? nb : 8);
+  int dev = 0, cap = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+    cudaGetLastError();
+    cap = 227 * 1024;  // no device here: a GB300's
+  }
+  BlkPlan B;
+  std::vector<int> unk_node, ps0, ps1, end1;
+  bool mono = true, use_blk = false;
+  if (nodes_of_unknowns(d, unk_node)) {
+    for (int64_t q = 1; q < n; ++q) mono &= unk_node[q] >= unk_node[q - 1];
+    const std::vector<int> blk_end = pivot_blocks(unk_node);
+    const int wmax = fp64 ? blk_panel_width<double>(L, cap) : blk_panel_width<float>(L, cap);
+    use_blk = wmax && blk_plan(blk_end, wmax, (int)kl, B);
+    if (use_blk && blk_two_plan(blk_end, L, B, ps0, ps1, end1)) {
+      B.has_two = true;
+      B.two[0].npan = (int)ps0.size() - 1;
+      B.two[1].npan = (int)ps1.size() - 1;
+    }
+  }
+  const PlanSizes S = plan_sizes(L, B, use_blk, !fp64 && use_blk && patch_fits(L, B, patch_dyn_smem(cap)));
+  int64_t b = L.ldb * n * esz * (fp64 ? 1 : 2);                        // band (+ unfactored copy)
+  b += d->numel * nq * nq * esz + d->numel * nq * 8;                   // element blocks
+  b += d->numnp * (3 + d->ndf) * 8 + n * 8 * 4 + n * (esz + 4);        // state, vectors, reciprocals, pivot rows
+  b += (int64_t)(S.perm * 4 + S.xch * sizeof(SolveWord) + S.pinv * 8 + S.inv * 4 + S.a21 * 4 + kPartials * 8);
+  b += use_blk ? (int64_t)(S.flags * 3 + 1 + B.ps.size() + ps0.size() + ps1.size() + end1.size()) * 4 : 0;
+  b += n * 4 * 3 + d->numnp * d->ndf * 4 + (mono ? (d->numnp + 1) * 4 : 0);  // unknowns' nodes, dofs and blocks
+  int64_t rows = 0;
+  for (int k = 0; k < 4; ++k) rows += d->bdry_n_uel[k];
+  b += d->n_uel * (9 * kTab + 81) * 8 + std::max<int64_t>(rows, 1) * 3 * kTab * 8;  // Gauss-point tables
+  b += d->numel * (9 + nq + 1 + 4) * 4;                                             // element maps
+  b += 25 * (4 + nq * 8) + 2 * std::max<int64_t>(d->n_dir, 1) * 12 + 16 * 8 + 4 * 4 + 4 * 4;
   return b;
 }
 
@@ -310,11 +377,8 @@ extern "C" int mafem_two_chain_plan(const mafem_mesh_desc* d, int32_t precision,
   const int kl = (int)half_bandwidth(*d), nb = choose_nb(kl, precision);
   if (!nb || width > nb) return MAFEM_ERR_UNSUPPORTED;
   const BandLayout L = make_band_layout(n, kl, kl, nb);
-  std::vector<int> unk_node(n, -1);
-  for (int64_t k = 0; k < d->ndf * d->numnp; ++k) {
-    if (d->ID[k] < 0 || d->ID[k] > n) return MAFEM_ERR_ARG;
-    if (d->ID[k] > 0) unk_node[d->ID[k] - 1] = (int)(k / d->ndf);
-  }
+  std::vector<int> unk_node;
+  if (!nodes_of_unknowns(d, unk_node)) return MAFEM_ERR_ARG;
   const std::vector<int> blk_end = pivot_blocks(unk_node);
   BlkPlan B;
   std::vector<int> ps0, ps1, blk_end1;
@@ -589,10 +653,10 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
         b.pbase = a.npan;
         b.rbase = h->blk.mid;
       }
-      const size_t npx = (size_t)h->blk.npan_max();
-      AL(h->d_xch, npx * kBlkW);
-      AL(h->d_pinv, npx * 2 * kBlkW * kBlkW);
-      cudaMemset(h->d_xch, 0, npx * kBlkW * sizeof(SolveWord));
+      const PlanSizes S = plan_sizes(h->L, h->blk, true, false);
+      AL(h->d_xch, S.xch);
+      AL(h->d_pinv, S.pinv);
+      cudaMemset(h->d_xch, 0, S.xch * sizeof(SolveWord));
       h->bwd_grid = precision == MAFEM_PLAIN_FP64 ? blk_backward_grid<double>() : blk_backward_grid<float>();
       h->bwd_max = h->bwd_grid;
       cudaGetLastError();
@@ -600,7 +664,7 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
                                                    : blk_persist_setup<float>(h->L, h->blk, h->pers);
       cudaGetLastError();
       if (pg > 0) {
-        const size_t np = (size_t)h->blk.npan() + (size_t)h->blk.two[0].npan + (size_t)h->blk.two[1].npan;
+        const size_t np = S.flags;
         AL(h->pers.d_bdone, 1);
         cudaMemset(h->pers.d_bdone, 0, sizeof(int));
         AL(h->pers.d_pdone, np);
@@ -628,10 +692,10 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
   AL(h->d_x, n);
   AL(h->d_res, n);
   AL(h->d_dx, n);
-  AL(h->d_part, 4096);  // partial sums: of an update (2 x 1024), of a residual (2048)
+  AL(h->d_part, kPartials);
   AL(h->d_out, 16);
   AL(h->d_ipiv, n);
-  AL(h->d_perm, std::max((size_t)h->npan * h->rmax, (size_t)h->blk.npan_max() * kBlkW));
+  AL(h->d_perm, plan_sizes(h->L, h->blk, h->use_blk, false).perm);
   AL(h->d_rstate, 4);
   AL(h->d_info, 4);  // [0] zero-pivot column (1-based), [1] nonzero: a bounded device wait ran out
   cudaMemset(h->d_info, 0, 4 * sizeof(int));
@@ -663,16 +727,15 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
     mafem_destroy(hp.release());
     return MAFEM_ERR_OOM;
   }
-  // (the refinement residual reads every band window without bounds checks:
-  // it needs nb >= 32 rows of padding)
-  if (precision != MAFEM_PLAIN_FP64 && h->use_blk && h->L.nb >= 32) {
+  if (precision != MAFEM_PLAIN_FP64 && h->use_blk) {
     const int dyn = patch_solve_setup();
     cudaGetLastError();
-    if (dyn > 0 && patch_factor_smem() <= (size_t)dyn && patch_refine_smem(n, h->blk.npan()) <= (size_t)dyn) {
-      AL(h->d_inv, (size_t)h->blk.npan() * kBlkW * kBlkW);
+    if (patch_fits(h->L, h->blk, dyn)) {
+      const PlanSizes S = plan_sizes(h->L, h->blk, true, true);
+      AL(h->d_inv, S.inv);
       PatchJob& J = h->job;
       J.a21_rows = patch_a21_rows(h->L.kl);
-      AL(J.a21, (size_t)8 * 4 * 2 * J.a21_rows * 4);
+      AL(J.a21, S.a21);
       J.band = (float*)h->d_band;
       J.band0 = (const float*)h->d_band0;
       J.inv = h->d_inv;
@@ -2285,8 +2348,8 @@ extern "C" int mafem_server_submit(mafem_server* s, const mafem_request* r, int6
     return MAFEM_ERR_ARG;
   const int64_t fp = mafem_footprint_bytes(r->mesh, r->precision);
   if (fp < 0) return MAFEM_ERR_ARG;
-  // the footprint estimate plus the FP32 form's per-panel inverses and slack
-  const int64_t est = fp + fp / 8 + (16LL << 20);
+  // slack for the allocations' granularity
+  const int64_t est = fp + fp / 32 + (15LL << 20);
   if (est > s->budget) {
     set_global_error("request needs about " + std::to_string(est) + " device bytes, more than the server's budget of " +
                      std::to_string(s->budget));

@@ -668,18 +668,21 @@ bool blk_two_plan(const std::vector<int>& blk_end, const BandLayout& L, BlkPlan&
 }
 
 template <class T>
+int blk_panel_width(const BandLayout& L, int cap) {
+  for (int w : {32, 24, 16, 8}) {
+    if (w > L.nb) continue;
+    if (blk_apply_smem<T>(L, w) <= (size_t)cap && ((size_t)w + L.kl) * sizeof(double) + 10 * 1024 <= (size_t)cap)
+      return w;
+  }
+  return 0;
+}
+
+template <class T>
 int blk_lu_setup(const BandLayout& L) {
   int dev = 0, cap = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
-  int wmax = 0;
-  for (int w : {32, 24, 16, 8}) {
-    if (w > L.nb) continue;
-    if (blk_apply_smem<T>(L, w) <= (size_t)cap && ((size_t)w + L.kl) * sizeof(double) + 10 * 1024 <= (size_t)cap) {
-      wmax = w;
-      break;
-    }
-  }
+  const int wmax = blk_panel_width<T>(L, cap);
   if (!wmax) return 0;
   if (cudaFuncSetAttribute(blk_apply_kernel<T, kApplyNR>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap) !=
           cudaSuccess ||
@@ -856,6 +859,8 @@ int blk_backward_grid() {
   return std::max(0, sms * std::min(std::min(back, forw), 1));
 }
 
+template int blk_panel_width<double>(const BandLayout&, int);
+template int blk_panel_width<float>(const BandLayout&, int);
 template int blk_lu_setup<double>(const BandLayout&);
 template int blk_lu_setup<float>(const BandLayout&);
 template int blk_lu_factor<double>(double*, const BandLayout&, const BlkPlan&, int*, double*, int*, double*,

@@ -60,6 +60,7 @@ size_t patch_factor_smem() { return kFactorSmem; }
 // Rows of the split-A21 buffer per part (hi, lo) and rank: the most rows below
 // a panel's diagonal block (kl), rounded up to whole M tiles.
 int patch_a21_rows(int kl) { return (kl + kMT - 1) / kMT * kMT; }
+size_t patch_a21_elems(int rows) { return (size_t)8 * 4 * 2 * rows * 4; }  // k-quads, ranks, parts, rows, k % 4
 
 // x = hi + lo with hi, lo TF32 (round to nearest): the 3xTF32 split
 __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
@@ -1117,7 +1118,7 @@ int patch_solve_setup() {
   int dev = 0, cap = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
-  const int dyn = cap - 2 * 1024;  // room for the kernels' static shared memory
+  const int dyn = patch_dyn_smem(cap);
   if (cudaFuncSetAttribute(patch_factor_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
       cudaFuncSetAttribute(patch_factor_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
       cudaFuncSetAttribute(patch_factor_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||

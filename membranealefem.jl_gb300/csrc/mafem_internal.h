@@ -209,7 +209,10 @@ bool blk_two_plan(const std::vector<int>& blk_end, const BandLayout& L, BlkPlan&
                   std::vector<int>& ps1, std::vector<int>& blk_end1);
 // Host: panel starts for blocks `blk_end` (false if a block is wider than wmax).
 bool blk_plan(const std::vector<int>& blk_end, int wmax, int ku, BlkPlan& out);
-// Widest panel (<= kBlkW, <= L.nb) whose kernels fit the device's shared memory; 0 if none.
+// Widest panel (<= kBlkW, <= L.nb) whose kernels fit `cap` bytes of shared memory per CTA; 0 if none.
+template <class T>
+int blk_panel_width(const BandLayout& L, int cap);
+// The same for the current device, its kernels set up.
 template <class T>
 int blk_lu_setup(const BandLayout& L);
 template <class T>
@@ -386,11 +389,14 @@ struct PatchJob {
 };
 // Rows per part of a patch's split-A21 buffer for half bandwidth kl.
 int patch_a21_rows(int kl);
+size_t patch_a21_elems(int rows);  // floats of the split-A21 buffer
 // Encodes J.a21_map over J.a21 (J.a21, J.a21_rows set); returns false if the
 // driver refuses the tensor map.
 bool patch_a21_map(PatchJob& J);
 size_t patch_factor_smem();
 size_t patch_refine_smem(int64_t n, int npan);
+// Dynamic shared memory the kernels may use, of `cap` bytes per CTA.
+constexpr int patch_dyn_smem(int cap) { return cap - 2 * 1024; }  // room for their static shared memory
 // Sets the kernels' shared-memory limits; returns the dynamic bytes available (0: unusable).
 int patch_solve_setup();
 // Trailing columns per chunk of the factorisation (at most).
