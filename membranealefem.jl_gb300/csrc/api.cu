@@ -130,6 +130,7 @@ struct mafem_handle {
   float* d_inv = nullptr;
   double* d_pinv = nullptr;  // npan_max x 2 x 32 x 32 (blk_inverses)
   bool patch_ok = false;
+  size_t patch_smem = 0;  // dynamic shared memory of its refinement
   bool ss_patch = false;  // the iteration in progress ran through a batch's patch solve
   PatchJob job{};
   WaitTest wait_test;                   // mafem_set_wait_test (failure-detection tests)
@@ -316,10 +317,12 @@ constexpr size_t kPartials = 4096;  // partial sums: of an update (2 x 1024), of
 
 // The batched FP32 form serves a handle: its refinement residual reads every band
 // window without bounds checks, which needs nb >= 32 rows of padding, and its kernels
-// have `dyn` bytes of shared memory.
+// have `dyn` bytes of shared memory.  It takes as many unknowns as make up one CTA's
+// shared memory as floats (57.6 k); longer bands, strips of hundreds of elements
+// above all, keep their own solver.
 static bool patch_fits(const BandLayout& L, const BlkPlan& B, int dyn) {
-  return L.nb >= 32 && dyn > 0 && patch_factor_smem() <= (size_t)dyn &&
-         patch_refine_smem(L.n, B.npan()) <= (size_t)dyn;
+  return L.nb >= 32 && dyn > 0 && patch_factor_smem() <= (size_t)dyn && 4 * L.n <= dyn &&
+         patch_refine_smem(L.n, B.npan(), dyn) <= (size_t)dyn;
 }
 
 // Bytes of device memory mafem_create allocates for a mesh.
@@ -747,6 +750,9 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
       J.x = h->d_x;
       J.res = h->d_res;
       J.rs = h->d_part + 2048;  // free while a batched solve runs
+      // (d_ipiv, n ints, is full partial pivoting's)
+      if (!patch_vector_fits(n, h->blk.npan(), dyn)) J.vg = reinterpret_cast<float*>(h->d_ipiv);
+      h->patch_smem = patch_refine_smem(n, h->blk.npan(), dyn);
       J.xs = reinterpret_cast<float2*>(h->d_dx);  // d_dx: n doubles, unused by this form
       J.L = h->L;
       J.kuf = h->blk.kuf;
@@ -1591,7 +1597,7 @@ static PatchGroups order_patch_jobs(std::vector<mafem_handle*>& hv, std::vector<
     const int g = nr(k) == 4 ? 0 : nr(k) == 2 ? 1 : 2;
     G.n4 += g == 0;
     G.n2 += g == 1;
-    G.wide[g] |= patch_wide(hv[k]->L.kl, hv[k]->blk.kuf);
+    G.form[g] = std::max(G.form[g], patch_form(hv[k]->job));
   }
   return G;
 }
@@ -1829,7 +1835,7 @@ extern "C" int mafem_batch_create(mafem_handle* const* hs, int32_t n, int32_t ct
       jobs.push_back(h->job);
       b->cost.push_back((double)h->blk.npan() * h->L.kl * h->blk.kuf);
       b->smem_f = std::max(b->smem_f, patch_factor_smem());
-      b->smem_r = std::max(b->smem_r, patch_refine_smem(h->L.n, h->blk.npan()));
+      b->smem_r = std::max(b->smem_r, h->patch_smem);
     } else {
       b->slot.push_back(-1);
     }
@@ -2427,7 +2433,7 @@ extern "C" int mafem_server_round(mafem_server* s, int32_t* n_active, int32_t* n
     q->h = h;
     q->bytes = h->bytes;
     s->used += h->bytes;
-    if (h->patch_ok && s->smem_dyn >= patch_factor_smem() && s->smem_dyn >= patch_refine_smem(h->L.n, h->blk.npan()) &&
+    if (h->patch_ok && s->smem_dyn >= patch_factor_smem() && s->smem_dyn >= h->patch_smem &&
         !s->free_slots.empty()) {
       q->slot = s->free_slots.back();
       s->free_slots.pop_back();
@@ -2540,7 +2546,7 @@ extern "C" int mafem_server_round(mafem_server* s, int32_t* n_active, int32_t* n
       dscale[k] = q->dscale;
       pj[k] = k;
       smf = std::max(smf, patch_factor_smem());
-      smr = std::max(smr, patch_refine_smem(h->L.n, h->blk.npan()));
+      smr = std::max(smr, h->patch_smem);
       max_sw = std::max(max_sw, h->max_refine);
       tol = std::min(tol, h->refine_tol);
       if (q->start) cudaStreamWaitEvent(L.st, h->ev[5], 0);  // the handle's own work before the step
@@ -2753,10 +2759,9 @@ extern "C" int mafem_trace_patch_solve(mafem_handle* h, double time, double dt, 
   const int dyn = patch_solve_setup();
   cudaEventRecord(e0, h->st);
   const int nr = patch_ctas(h);  // as a batch would run it
-  patch_solve_stage(d_job, d_ord, 1, nr, patch_factor_smem(), 0, false, 0, 0.0, h->st);
+  patch_solve_stage(d_job, d_ord, 1, nr, patch_factor_smem(), 0, 0, 0, 0.0, h->st);
   cudaEventRecord(e1, h->st);
-  patch_solve_stage(d_job, d_ord, 1, 1, 0, patch_refine_smem(h->L.n, h->blk.npan()),
-                    patch_wide(h->L.kl, h->blk.kuf), h->max_refine, h->refine_tol, h->st);
+  patch_solve_stage(d_job, d_ord, 1, 1, 0, h->patch_smem, patch_form(h->job), h->max_refine, h->refine_tol, h->st);
   cudaEventRecord(e2, h->st);
   std::vector<long long> tr((size_t)ntr);
   CK(cudaMemcpyAsync(tr.data(), d_tr, tr.size() * sizeof(long long), cudaMemcpyDeviceToHost, h->st));

@@ -525,8 +525,12 @@ struct RefineSmem {
   alignas(16) float part[2][kRT / 32][kBlkW];  // backward: the update warps' sums, by parity
   double red[kRT / 32];
 };
-size_t patch_refine_smem(int64_t n, int npan) {
-  return sizeof(RefineSmem) + sizeof(float) * (size_t)n + sizeof(int) * ((size_t)npan + 1);
+static size_t refine_smem_base(int npan) { return sizeof(RefineSmem) + sizeof(int) * ((size_t)npan + 1); }
+bool patch_vector_fits(int64_t n, int npan, int dyn) {
+  return refine_smem_base(npan) + sizeof(float) * (size_t)n <= (size_t)dyn;
+}
+size_t patch_refine_smem(int64_t n, int npan, int dyn) {
+  return refine_smem_base(npan) + (patch_vector_fits(n, npan, dyn) ? sizeof(float) * (size_t)n : 0);
 }
 
 __device__ __forceinline__ long long gtime() {
@@ -943,16 +947,20 @@ __device__ double patch_residual(const PatchJob& J, const float2* xs, double* re
 // 1.96 ms, 48 x 48 1740 -> 383 us and 8.8 -> 5.4 ms.  What a sweep hands on stands in J.rs: [0] |r0|, [1] the last
 // correction's norm, [2] and [3] the norms of the current one and of x, [4] nonzero
 // once the patch is done, [8 ..] the residual's partial sums.
+// GV: patches whose working vector of n floats does not fit the shared memory beside
+// the rest (from 47 k unknowns: 110 x 110 LAG) keep it in global memory, in L1 and L2.
+// The arithmetic is that of the other forms.
 constexpr int kSplit = 3;
-template <int RPT, bool MONO>
+template <int RPT, bool MONO, bool GV = false>
 __global__ void __launch_bounds__(kRT, 1) patch_refine_kernel(const PatchJob* __restrict__ jobs,
                                                              const int* __restrict__ order, int k0, int max_sweeps,
                                                              double tol) {
   const PatchJob& J = jobs[order[blockIdx.x]];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RefineSmem& S = *reinterpret_cast<RefineSmem*>(smem_raw);
-  float* v = reinterpret_cast<float*>(smem_raw + sizeof(RefineSmem));  // [n]
-  int* ps = reinterpret_cast<int*>(v + J.L.n);                         // [npan + 1]
+  int* ps = reinterpret_cast<int*>(smem_raw + sizeof(RefineSmem));  // [npan + 1]
+  float* vs = reinterpret_cast<float*>(ps + J.npan + 1);            // [n]
+  float* v = GV && J.vg ? J.vg : vs;
   double* red = S.red;
   const int tid = threadIdx.x;
   const int64_t n = J.L.n;
@@ -1125,7 +1133,9 @@ int patch_solve_setup() {
       cudaFuncSetAttribute(patch_refine_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
       cudaFuncSetAttribute(patch_refine_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
       cudaFuncSetAttribute(patch_refine_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
-      cudaFuncSetAttribute(patch_refine_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
+      cudaFuncSetAttribute(patch_refine_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
+      cudaFuncSetAttribute(patch_refine_kernel<2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
+      cudaFuncSetAttribute(patch_refine_kernel<2, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
     return 0;
   return dyn;
 }
@@ -1155,31 +1165,33 @@ static cudaError_t launch_factor(const PatchJob* d_jobs, const int* d_order, int
                  : cudaLaunchKernelEx(&cfg, patch_factor_kernel<2>, d_jobs, d_order);
 }
 
-// Whether a band needs the refinement's two register sets per thread: more rows
-// or columns beyond a panel than one set of the update warps holds.
-bool patch_wide(int kl, int kuf) { return kl > kRowT || kuf > kRowT; }
-static cudaError_t launch_refine(const PatchJob* d_jobs, const int* d_order, int njobs, bool wide, size_t smem,
+// A band is wide for the refinement (two register sets per thread) with more rows or
+// columns beyond a panel than one set of the update warps holds.
+int patch_form(const PatchJob& J) { return J.vg ? 2 : J.L.kl > kRowT || J.kuf > kRowT ? 1 : 0; }
+static cudaError_t launch_refine(const PatchJob* d_jobs, const int* d_order, int njobs, int form, size_t smem,
                                  int max_sweeps, double tol, cudaStream_t st, bool apart = true) {
   auto sweeps = [&](auto kern, int k0) { kern<<<njobs, kRT, smem, st>>>(d_jobs, d_order, k0, max_sweeps, tol); };
   const int split = apart ? std::min(kSplit, max_sweeps) : 0;
   for (int k = 0; k < split; ++k) {
-    if (wide) sweeps(patch_refine_kernel<2, false>, k);
+    if (form == 2) sweeps(patch_refine_kernel<2, false, true>, k);
+    else if (form == 1) sweeps(patch_refine_kernel<2, false>, k);
     else sweeps(patch_refine_kernel<1, false>, k);
     patch_residual_kernel<<<njobs * kResC, kResT, 0, st>>>(d_jobs, d_order);
   }
-  if (wide) sweeps(patch_refine_kernel<2, true>, split);
+  if (form == 2) sweeps(patch_refine_kernel<2, true, true>, split);
+  else if (form == 1) sweeps(patch_refine_kernel<2, true>, split);
   else sweeps(patch_refine_kernel<1, true>, split);
   return cudaGetLastError();
 }
 
 cudaError_t patch_solve_stage(const PatchJob* d_jobs, const int* d_order, int njobs, int nr, size_t smem_factor,
-                              size_t smem_refine, bool wide, int max_sweeps, double tol, cudaStream_t st) {
+                              size_t smem_refine, int form, int max_sweeps, double tol, cudaStream_t st) {
   if (njobs <= 0) return cudaSuccess;
   if (smem_factor) {
     const cudaError_t e = launch_factor(d_jobs, d_order, njobs, nr, smem_factor, st);
     if (e != cudaSuccess) return e;
   }
-  if (smem_refine) return launch_refine(d_jobs, d_order, njobs, wide, smem_refine, max_sweeps, tol, st);
+  if (smem_refine) return launch_refine(d_jobs, d_order, njobs, form, smem_refine, max_sweeps, tol, st);
   return cudaGetLastError();
 }
 
@@ -1256,12 +1268,12 @@ cudaError_t patch_solve(const PatchJob* d_jobs, const int* d_order, const PatchG
     e = launch_factor(d_jobs, d_order + off, cnt[g], nrs[g], smem_factor, g == first ? st : st2);
     off += cnt[g];
     if (g == first && e == cudaSuccess)
-      e = launch_refine(d_jobs, d_order, cnt[g], G.wide[g], smem_refine, max_sweeps, tol, st);
+      e = launch_refine(d_jobs, d_order, cnt[g], G.form[g], smem_refine, max_sweeps, tol, st);
   }
   if (fork && e == cudaSuccess) {
-    bool wide = false;
-    for (int g = first + 1; g < 3; ++g) wide |= cnt[g] > 0 && G.wide[g];
-    e = launch_refine(d_jobs, d_order + cnt[first], njobs - cnt[first], wide, smem_refine, max_sweeps, tol, st2, false);
+    int form = 0;
+    for (int g = first + 1; g < 3; ++g) form = std::max(form, G.form[g]);
+    e = launch_refine(d_jobs, d_order + cnt[first], njobs - cnt[first], form, smem_refine, max_sweeps, tol, st2, false);
   }
   if (fork && e == cudaSuccess) e = cudaEventRecord(ev_join, st2);
   if (fork && e == cudaSuccess) e = cudaStreamWaitEvent(st, ev_join, 0);

@@ -375,6 +375,7 @@ struct PatchJob {
   double* x;            // [n] solution
   double* res;          // [n] FP64 residual (workspace)
   float2* xs;           // [n] x as two floats (workspace)
+  float* vg;            // [n] the sweeps' FP32 working vector in global memory; null: in shared memory
   double* rs;           // [16] the refinement's state between its launches (patch_refine_kernel)
   BandLayout L;
   int kuf, npan;
@@ -394,7 +395,10 @@ size_t patch_a21_elems(int rows);  // floats of the split-A21 buffer
 // driver refuses the tensor map.
 bool patch_a21_map(PatchJob& J);
 size_t patch_factor_smem();
-size_t patch_refine_smem(int64_t n, int npan);
+// `dyn` bytes available: with the working vector (n floats) in shared memory where that
+// fits, else without it (then PatchJob::vg).
+size_t patch_refine_smem(int64_t n, int npan, int dyn);
+bool patch_vector_fits(int64_t n, int npan, int dyn);
 // Dynamic shared memory the kernels may use, of `cap` bytes per CTA.
 constexpr int patch_dyn_smem(int cap) { return cap - 2 * 1024; }  // room for their static shared memory
 // Sets the kernels' shared-memory limits; returns the dynamic bytes available (0: unusable).
@@ -407,20 +411,21 @@ int patch_cluster_ctas(int kuf);
 // The factor kernel alone (smem_refine == 0; nr = CTAs per patch, 1, 2 or 4) or
 // the refine kernel alone (smem_factor == 0).
 cudaError_t patch_solve_stage(const PatchJob* d_jobs, const int* d_order, int njobs, int nr, size_t smem_factor,
-                              size_t smem_refine, bool wide, int max_sweeps, double tol, cudaStream_t st);
+                              size_t smem_refine, int form, int max_sweeps, double tol, cudaStream_t st);
 // Time (ms, CUDA events) of factoring job d_order1[0] on a cluster of nr CTAs,
 // on a synthetic band of its shape written over the job's band (which the
 // next assembly rewrites); synchronises st.
 cudaError_t patch_time_factor(const PatchJob* d_jobs, const int* d_order1, int nr, size_t smem, cudaStream_t st,
                               float* ms);
-// Whether a patch's band is wide for the refinement kernel (two register sets per thread).
-bool patch_wide(int kl, int kuf);
+// The refinement kernel's form a patch needs: 0, or 1 for a wide band (two register
+// sets per thread), or 2 for that with the working vector in global memory.
+int patch_form(const PatchJob& J);
 // The jobs of a round by cluster size: the first n4 on four CTAs, the next n2 on
-// two; wide[g]: group g (4, 2, 1 CTAs) holds a wide band.
+// two; form[g]: the largest patch_form in group g (4, 2, 1 CTAs).
 struct PatchGroups {
   int n4 = 0, n2 = 0;
-  bool wide[3] = {false, false, false};
-  int64_t key() const { return n4 | ((int64_t)n2 << 24) | ((int64_t)wide[0] << 48) | ((int64_t)wide[1] << 49) | ((int64_t)wide[2] << 50); }
+  int form[3] = {0, 0, 0};
+  int64_t key() const { return n4 | ((int64_t)n2 << 24) | ((int64_t)(form[0] + 4 * form[1] + 16 * form[2]) << 48); }
 };
 // kernel launches patch_solve makes for these group sizes
 int patch_solve_launches(const PatchGroups& G, int njobs, int max_sweeps);
