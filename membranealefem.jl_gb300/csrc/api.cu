@@ -896,9 +896,9 @@ static void blk_need_inverses(mafem_handle* h) {
   if (h->pinv_ready) return;
   h->pinv_ready = true;
   h->launches += h->precision == MAFEM_PLAIN_FP64
-                     ? blk_inverses<double, double>((const double*)h->d_band, h->L, h->blk, h->last_two,
+                     ? blk_inverses<double>((const double*)h->d_band, h->L, h->blk, h->last_two,
                                                     h->d_perm, (const double*)h->d_rdiag, h->d_pinv, h->st)
-                     : blk_inverses<double, float>((const float*)h->d_band, h->L, h->blk, h->last_two,
+                     : blk_inverses<float>((const float*)h->d_band, h->L, h->blk, h->last_two,
                                                    h->d_perm, (const float*)h->d_rdiag, h->d_pinv, h->st);
 }
 

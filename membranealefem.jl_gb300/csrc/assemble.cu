@@ -291,9 +291,7 @@ __global__ void axpy_norms_kernel(int64_t n, const double* __restrict__ dx, doub
   }
 }
 // out[0] = |dx|, out[1] = |x| from the block partial sums
-__global__ void sqrt_pair_kernel(const double* __restrict__ part, int nblk, double* __restrict__ out,
-                                 const int* __restrict__ gate) {
-  if (gate && *gate) return;
+__global__ void sqrt_pair_kernel(const double* __restrict__ part, int nblk, double* __restrict__ out) {
   const double a = sum_partials(part, nblk, 2), b = sum_partials(part + 1, nblk, 2);
   if (threadIdx.x == 0) {
     out[0] = sqrt(a);
@@ -468,7 +466,7 @@ void launch_axpy_partials(int64_t n, const double* dx, double* x, double* part, 
 }
 void launch_axpy_norms(int64_t n, const double* dx, double* x, double* part, double* out, cudaStream_t st) {
   launch_axpy_partials(n, dx, x, part, st, nullptr);
-  sqrt_pair_kernel<<<1, 32, 0, st>>>(part, norm_blocks(n), out, nullptr);
+  sqrt_pair_kernel<<<1, 32, 0, st>>>(part, norm_blocks(n), out);
 }
 
 // ---- device-side stopping test of one handle's iterative refinement ----------------

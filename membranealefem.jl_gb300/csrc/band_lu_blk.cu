@@ -328,12 +328,12 @@ __global__ void __launch_bounds__(1024) blk_backward_kernel(const T* __restrict_
 // W z(p - 1) can be formed before z(p - 1) is there.  Element (i, k) at k * 32 + i,
 // zero outside the panel's rows and columns; inv[p] = Ai then W.  One warp per panel
 // (four per CTA), lane c forming column c of both.
-template <class T, class V>
+template <class T>
 __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__ ab, BlkChain c0, BlkChain c1, int split,
                                                            int kl,
                                                            const int* __restrict__ perm_all,
-                                                           const T* __restrict__ rdiag_all, V* __restrict__ inv) {
-  __shared__ V S[4][32][33];  // per warp: S[k][i] = A(j0 + i, j0 + k) of its panel, then Ai
+                                                           const T* __restrict__ rdiag_all, double* __restrict__ inv) {
+  __shared__ double S[4][32][33];  // per warp: S[k][i] = A(j0 + i, j0 + k) of its panel, then Ai
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool second = (int)blockIdx.x >= split;
   const BlkChain& c = second ? c1 : c0;
@@ -342,25 +342,25 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
   const int j0 = c.ps[p], w = c.ps[p + 1] - j0;
   const T* blk = ab + c.org + j0 * c.si + j0 * c.sj;
   const T* rdiag = rdiag_all + c.rbase;
-  for (int k = 0; k < 32; ++k) S[warp][k][lane] = (k < w && lane < w) ? V(blk[lane * c.si + k * c.sj]) : V(0);
-  const V rd = lane < w ? V(rdiag[j0 + lane]) : V(0);
+  for (int k = 0; k < 32; ++k) S[warp][k][lane] = (k < w && lane < w) ? (double)blk[lane * c.si + k * c.sj] : 0.0;
+  const double rd = lane < w ? (double)rdiag[j0 + lane] : 0.0;
   const int pr = lane < w ? perm_all[(size_t)(c.pbase + p) * kBlkW + lane] : -1;
   __syncwarp();
-  V* Ai = inv + (size_t)(c.pbase + p) * 2 * kBlkW * kBlkW;
-  V* W = Ai + kBlkW * kBlkW;
+  double* Ai = inv + (size_t)(c.pbase + p) * 2 * kBlkW * kBlkW;
+  double* W = Ai + kBlkW * kBlkW;
   // column `lane`: L11 y = P e_lane forward, U11 x = y backward
-  V x[32];
+  double x[32];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) x[i] = __shfl_sync(kFull, pr, i) == lane ? V(1) : V(0);
+  for (int i = 0; i < 32; ++i) x[i] = __shfl_sync(kFull, pr, i) == lane ? 1.0 : 0.0;
 #pragma unroll
   for (int k = 0; k < 32; ++k) {
-    const V xk = x[k];
+    const double xk = x[k];
 #pragma unroll
     for (int i = k + 1; i < 32; ++i) x[i] = fma(-S[warp][k][i], xk, x[i]);
   }
 #pragma unroll
   for (int k = 31; k >= 0; --k) {
-    const V xk = x[k] * __shfl_sync(kFull, rd, k);
+    const double xk = x[k] * __shfl_sync(kFull, rd, k);
     x[k] = xk;
 #pragma unroll
     for (int i = 0; i < k; ++i) x[i] = fma(-S[warp][k][i], xk, x[i]);
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
   __syncwarp();
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
-    const V v = (lane < w && i < w) ? x[i] : V(0);
+    const double v = (lane < w && i < w) ? x[i] : 0.0;
     Ai[lane * 32 + i] = v;
     S[warp][lane][i] = v;
   }
@@ -376,9 +376,9 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
   const int q0 = p > 0 ? c.ps[p - 1] : j0;  // column q0 + lane of the panel before
   const T* col = ab + c.org + j0 * c.si + (q0 + lane) * c.sj;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) x[i] = V(0);
+  for (int i = 0; i < 32; ++i) x[i] = 0.0;
   for (int m = 0; m < w; ++m) {
-    const V am = q0 + lane < j0 && j0 + m - (q0 + lane) <= kl ? V(col[m * c.si]) : V(0);
+    const double am = q0 + lane < j0 && j0 + m - (q0 + lane) <= kl ? (double)col[m * c.si] : 0.0;
 #pragma unroll
     for (int i = 0; i < 32; ++i) x[i] = fma(S[warp][m][i], am, x[i]);
   }
@@ -581,15 +581,15 @@ __global__ void __launch_bounds__(kSolveThreads)
 // The backward chain's contributions to the rows [lo, mid) above it, before the
 // forward chain goes on through them: b[i] -= sum_j A(i, j) z(j) over the columns
 // j >= mid that reach row i (physical numbering; z stands in b).  A warp per row.
-template <class T, class V>
+template <class T>
 __global__ void __launch_bounds__(256) blk_forward_mid_kernel(const T* __restrict__ ab, BandLayout L, int mid, int lo,
-                                                              V* __restrict__ b, const int* __restrict__ gate) {
+                                                              double* __restrict__ b, const int* __restrict__ gate) {
   if (gate && *gate) return;
   const int i = lo + blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= mid) return;
   const int jend = (int)min64b(L.n, (int64_t)i + L.ku + 1);
-  V s = V(0);
-  for (int j = mid + lane; j < jend; j += 32) s += V(ab[bix(L, i, j)]) * b[j];
+  double s = 0.0;
+  for (int j = mid + lane; j < jend; j += 32) s += (double)ab[bix(L, i, j)] * b[j];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
   if (lane == 0) b[i] -= s;
 }
@@ -767,12 +767,12 @@ int blk_lu_factor(T* ab, const BandLayout& L, const BlkPlan& B, int* perm_all, T
   return launches;
 }
 
-template <class V, class T>
+template <class T>
 int blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
-                 V* inv, cudaStream_t st) {
+                 double* inv, cudaStream_t st) {
   const BlkChain &c0 = two ? B.two[0] : B.one, &c1 = B.two[1];
   const int b0 = (c0.npan + 3) / 4, b1 = two ? (c1.npan + 3) / 4 : 0;
-  blk_inverses_kernel<T, V><<<b0 + b1, 128, 0, st>>>(ab, c0, c1, b0, L.kl, perm_all, rdiag, inv);
+  blk_inverses_kernel<T><<<b0 + b1, 128, 0, st>>>(ab, c0, c1, b0, L.kl, perm_all, rdiag, inv);
   return 1;
 }
 // One cooperative launch over spans a and (optionally) b, its CTAs shared out by their
@@ -842,7 +842,7 @@ int blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, co
     const BlkSpan s1{B.two[1], 0, B.two[1].npan};
     nl = coop_spans(launch, one, BlkSpan{B.two[0], 0, B.pm}, &s1, grid, &coop);
     const int lo = std::max(0, B.mid - L.kl);
-    blk_forward_mid_kernel<T, double><<<(B.mid - lo + 7) / 8, 256, 0, st>>>(ab, L, B.mid, lo, b, gate);
+    blk_forward_mid_kernel<T><<<(B.mid - lo + 7) / 8, 256, 0, st>>>(ab, L, B.mid, lo, b, gate);
     nl += 1 + coop_spans(launch, one, BlkSpan{B.two[0], B.pm, B.two[0].npan}, nullptr, grid, &coop);
   }
   if (!coop) grid = 0;
@@ -867,9 +867,9 @@ template int blk_lu_factor<double>(double*, const BandLayout&, const BlkPlan&, i
                                    cudaStream_t, cudaStream_t, cudaEvent_t*, cudaEvent_t*);
 template int blk_lu_factor<float>(float*, const BandLayout&, const BlkPlan&, int*, float*, int*, float*, cudaStream_t,
                                   cudaStream_t, cudaEvent_t*, cudaEvent_t*);
-template int blk_inverses<double, double>(const double*, const BandLayout&, const BlkPlan&, bool, const int*,
+template int blk_inverses<double>(const double*, const BandLayout&, const BlkPlan&, bool, const int*,
                                           const double*, double*, cudaStream_t);
-template int blk_inverses<double, float>(const float*, const BandLayout&, const BlkPlan&, bool, const int*, const float*,
+template int blk_inverses<float>(const float*, const BandLayout&, const BlkPlan&, bool, const int*, const float*,
                                          double*, cudaStream_t);
 template int blk_backward<double>(const double*, const BlkPlan&, bool, double*, SolveWord*, int64_t&, int*, int&,
                                   cudaStream_t, WaitTest, const int*);

@@ -36,7 +36,6 @@ namespace mafem {
 
 constexpr int kPT = 512;   // threads per CTA of the factorisation (16 warps)
 constexpr int kRT = 512;   // threads per CTA of the refinement (16 warps)
-constexpr int kEpi = 1;    // batches of 16 columns of A22 whose loads run ahead of the subtraction (2: +3 %, 3: +10 % time)
 constexpr int kNCH = 256;  // trailing columns per chunk at most (the MMA's N <= 256)
 constexpr int kMT = 128;   // rows of A22 per tensor-core tile (the MMA's M)
 constexpr int kIS = 36;    // shared-memory row stride of the 32 x 32 inverse (16-byte rows)
@@ -395,8 +394,9 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
       const int q = warp & 3, grp = warp >> 2;
       const int cpg = ((ncp >> 2) + 7) & ~7;
       const int cs = min(ncp, grp * cpg), ce = min(ncp, cs + cpg), lim = min(ce, nc);
-      // the steps of this warp: tile t, columns c .. c + 15 of its group; each
-      // buffer's loads are issued kEpi steps before their use
+      // the steps of this warp: tile t, columns c .. c + 15 of its group; the next
+      // step's loads are issued after the current one's use (two steps ahead: +3 %
+      // time, three: +10 %)
       auto next = [&](int& t, int& c) MAFEM_INLINE {
         c += 16;
         if (c >= lim) {
@@ -435,46 +435,37 @@ __global__ void __launch_bounds__(kPT, 1) patch_factor_kernel(const PatchJob* __
         __syncthreads();  // the accumulator is read before the MMAs of tile t + 2 overwrite it
       };
       if (cs < lim) {
-        float va[kEpi][16];
-        int t = 0, c = cs, tl = 0, cl = cs;  // the step at hand, the next to load
-#pragma unroll
-        for (int u = 0; u < kEpi; ++u) {
-          load_a22(va[u], tl, cl);
-          next(tl, cl);
-        }
+        float va[16];
+        int t = 0, c = cs;
+        load_a22(va, t, c);
         while (t < ntile) {
+          if (c == cs) tile_begin(t);
+          const int row = w + t * kMT + 32 * q + lane;  // panel row of this thread
+          const uint32_t dt = tmem + ((uint32_t)(32 * q) << 16) + (t & 1) * kNCH;
+          float d0[8], d1[8];
+          tc::ld8(dt + c, d0);
+          if (c + 8 < ce) tc::ld8(dt + c + 8, d1);
+          tc::wait_ld();
+          if (row < R) {
+            float* pa = ab + bix(L, j0 + row, j1 + cb + c);  // A(j0 + row, j1 + cb + c), + ldm: the next column
+            if (c + 16 <= lim) {
 #pragma unroll
-          for (int u = 0; u < kEpi; ++u) {
-            if (t < ntile) {  // warp-uniform
-              if (c == cs) tile_begin(t);
-              const int row = w + t * kMT + 32 * q + lane;  // panel row of this thread
-              const uint32_t dt = tmem + ((uint32_t)(32 * q) << 16) + (t & 1) * kNCH;
-              float d0[8], d1[8];
-              tc::ld8(dt + c, d0);
-              if (c + 8 < ce) tc::ld8(dt + c + 8, d1);
-              tc::wait_ld();
-              if (row < R) {
-                float* pa = ab + bix(L, j0 + row, j1 + cb + c);  // A(j0 + row, j1 + cb + c), + ldm: the next column
-                if (c + 16 <= lim) {
-#pragma unroll
-                  for (int k = 0; k < 16; ++k) {
-                    *pa = va[u][k] - (k < 8 ? d0[k] : d1[k - 8]);
-                    pa += ldm;
-                  }
-                } else {
-#pragma unroll
-                  for (int k = 0; k < 16; ++k) {
-                    if (c + k < lim) *pa = va[u][k] - (k < 8 ? d0[k] : d1[k - 8]);
-                    pa += ldm;
-                  }
-                }
+              for (int k = 0; k < 16; ++k) {
+                *pa = va[k] - (k < 8 ? d0[k] : d1[k - 8]);
+                pa += ldm;
               }
-              load_a22(va[u], tl, cl);
-              next(tl, cl);
-              if (c + 16 >= lim) tile_end();
-              next(t, c);
+            } else {
+#pragma unroll
+              for (int k = 0; k < 16; ++k) {
+                if (c + k < lim) *pa = va[k] - (k < 8 ? d0[k] : d1[k - 8]);
+                pa += ldm;
+              }
             }
           }
+          const bool last = c + 16 >= lim;
+          next(t, c);
+          load_a22(va, t, c);
+          if (last) tile_end();
         }
       } else {  // no columns for this warp: the tiles' barriers only
         for (int t = 0; t < ntile; ++t) {
@@ -1092,8 +1083,6 @@ __global__ void __launch_bounds__(kRT, 1) patch_refine_kernel(const PatchJob* __
     }
   }
 }
-
-int patch_chunk_cols() { return kNCH; }
 
 // The split-A21 buffer as a 3-D tensor (k % 4, row, k / 4) of FP32 with strides
 // 16 bytes (rows) and 8 a21_rows x 16 bytes (k-quad planes); one 4 x 128 x 8 box

@@ -234,9 +234,9 @@ struct WaitTest {
 };
 // Per panel the inverse of its diagonal block and its product with the rows of the
 // panel before (inv: npan_max x 2 x 32 x 32) for the cooperative forward substitution.
-template <class V, class T>
+template <class T>
 int blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
-                 V* inv, cudaStream_t st);
+                 double* inv, cudaStream_t st);
 // Back substitution x1 = z - Y x2 in place on many SMs (cooperative launches of at
 // most `grid` CTAs, grid <= blk_backward_grid()).  xch: npan_max x 32 words; epoch: a
 // value that no word's tag holds yet is taken per launch; err: nonzero after a bounded
@@ -403,8 +403,6 @@ bool patch_vector_fits(int64_t n, int npan, int dyn);
 constexpr int patch_dyn_smem(int cap) { return cap - 2 * 1024; }  // room for their static shared memory
 // Sets the kernels' shared-memory limits; returns the dynamic bytes available (0: unusable).
 int patch_solve_setup();
-// Trailing columns per chunk of the factorisation (at most).
-int patch_chunk_cols();
 // CTAs that factor a patch with kuf trailing columns: 4 (a cluster, one chunk
 // per CTA) above two chunks, 2 above one chunk, else 1.
 int patch_cluster_ctas(int kuf);
