@@ -4,15 +4,16 @@ infrastructure: a numerical model, never the thing measured or shipped).
 It restates, in float32 numpy, the algorithm the batched FP32 form runs one
 CTA per patch.  Per panel of whole node blocks (at most 32 columns):
 
-1. Factor the w x w diagonal block with node-block pivoting.  The pivot of
-   column k is the largest entry among the not-yet-eliminated rows of k's
-   node block; rows below the panel never pivot.
-2. Form explicit inverses Li = L11^-1, Ui = U11^-1 and Mi = Ui Li.
-3. Form U12 = Li P A12 and Y = Mi P A12, and update A22 -= A21 Y with the raw
-   A21 (FP32 accumulation).
+1. Ai = A11^-1 of the w x w diagonal block by one in-place Gauss-Jordan sweep
+   (`gauss_jordan`).  The pivot of column k is the largest entry, to the bits
+   its search key keeps, among the not-yet-used rows of k's node block; rows
+   below the panel never pivot.
+2. Y = Ai A12 in place of A12, and A22 -= A21 Y with the raw A21 (FP32
+   accumulation).
 
-The FP32 substitutions use the same stored quantities.  The refinement
-repeats x += LU^-1 (b - A0 x), with the residual taken in FP64 against the
+The FP32 substitutions use the same stored quantities: z = Ai b1, b2 -= A21 z
+forward and x1 = z - Y x2 backward, no triangle.  The refinement repeats
+x += K^-1 (b - A0 x), with the residual taken in FP64 against the
 FP32 tangent A0.  It stops when the last correction is at most tol |x|.
 
 `double_float_residual` restates how the batched refinement forms that
@@ -26,7 +27,6 @@ Dense float32 storage: meant for patches up to 32 x 32 elements.
 from __future__ import annotations
 
 import numpy as np
-import scipy.linalg as sl
 
 
 def band_matvec(ab: np.ndarray, kl: int, x: np.ndarray) -> np.ndarray:
@@ -86,8 +86,49 @@ def panels_of(blk_end: np.ndarray, wmax: int = 32) -> tuple[list[int], int]:
     return ps, ndfp
 
 
+def _pivot_row(col: np.ndarray, cand: np.ndarray) -> int:
+    """The kernel's pivot search (warp_inverse in band_lu_patch.cu): the largest key
+    among the candidates, a key being the bits of |v| without its lowest six (17 bits
+    of the significand are left); of equal keys the first row.  -1 if no candidate is
+    usable."""
+    b = np.abs(col.astype(np.float32)).view(np.uint32)
+    key = np.where(b >= np.uint32(0x7F800000), np.uint32(0), b) & np.uint32(0xFFFFFFC0)
+    r = int(cand[np.argmax(key[cand])])
+    return r if key[r] else -1
+
+
+def gauss_jordan(D: np.ndarray, bend: np.ndarray) -> np.ndarray:
+    """The inverse of the float32 block D as warp_inverse forms it: step k exchanges
+    column k for the pivot row p_k (rows k's node block ends at bend[k]); rows are
+    never moved, and a row's scaling by -1 / pivot at its own step is applied at the
+    end.  Raises ZeroDivisionError (the step) where a column has no usable pivot."""
+    f32 = np.float32
+    w = len(D)
+    S = D.astype(f32).copy()
+    sc = np.ones(w, f32)
+    pos, rows = np.zeros(w, int), np.zeros(w, int)
+    free = np.ones(w, bool)
+    for k in range(w):
+        p = _pivot_row(S[:, k], np.nonzero(free & (np.arange(w) < bend[k]))[0])
+        if p < 0:
+            raise ZeroDivisionError(k)
+        r = f32(1.0) / S[p, k]
+        m = -(S[:, k] * r).astype(f32)
+        m[p] = 0.0
+        free[p], pos[p], rows[k], sc[p] = False, k, p, -r
+        piv = S[p].copy()
+        S = _fma32(np.broadcast_to(m[:, None], S.shape), np.broadcast_to(piv, S.shape), S)
+        S[:, k] = -m
+        S[p, k] = -1.0
+    inv = np.zeros((w, w), f32)
+    inv[pos[:, None], rows[None, :]] = (sc[:, None] * S).astype(f32)
+    return inv
+
+
 class PatchLU:
-    """The FP32 factors of one patch's tangent."""
+    """The FP32 factors of one patch's tangent.  growth: the largest entry met in
+    the diagonal blocks and in the rows right of them when their panel's turn has
+    come."""
 
     def __init__(self, ab0: np.ndarray, kl: int, blk_end: np.ndarray):
         A = dense_from_band(ab0, kl, np.float32)
@@ -100,47 +141,26 @@ class PatchLU:
             j0, j1 = ps[p], ps[p + 1]
             w = j1 - j0
             R, C = min(n - j0, w + kl), min(n, j1 + kuf) - j1
-            D = A[j0:j1, j0:j1].copy()
-            eliminated = np.zeros(w, bool)
-            perm = np.zeros(w, int)
-            bend = np.asarray(blk_end[j0:j1]) - j0
-            for k in range(w):
-                cand = np.nonzero(~eliminated & (np.arange(w) < bend[k]))[0]
-                pr = cand[np.argmax(np.abs(D[cand, k]))]
-                if D[pr, k] == 0.0 or not np.isfinite(D[pr, k]):
-                    raise ZeroDivisionError(f"no usable pivot in column {j0 + k}")
-                perm[k] = pr
-                eliminated[pr] = True
-                act = ~eliminated
-                l = D[act, k] / D[pr, k]
-                D[act, k + 1:] -= np.outer(l, D[pr, k + 1:]).astype(f32)
-                D[act, k] = l
-            PD = D[perm]
-            L11 = np.tril(PD, -1) + np.eye(w, dtype=f32)
-            U11 = np.triu(PD)
-            eye = np.eye(w, dtype=f32)
-            Li = sl.solve_triangular(L11, eye, lower=True, unit_diagonal=True).astype(f32)
-            Ui = sl.solve_triangular(U11, eye, lower=False).astype(f32)
-            Mi = (Ui @ Li).astype(f32)
-            a = A[j0:j1, j1:j1 + C][perm]
-            U12 = (Li @ a).astype(f32)
-            Y = (Mi @ a).astype(f32)
+            try:
+                Ai = gauss_jordan(A[j0:j1, j0:j1], np.asarray(blk_end[j0:j1]) - j0)
+            except ZeroDivisionError as e:
+                raise ZeroDivisionError(f"no usable pivot in column {j0 + e.args[0]}") from None
+            A12 = A[j0:j1, j1:j1 + C]
+            self.growth = max(self.growth, float(np.abs(A[j0:j1, j0:j1 + C]).max()))
+            Y = (Ai @ A12).astype(f32)
             A21 = A[j1:j0 + R, j0:j1].copy()
             A[j1:j0 + R, j1:j1 + C] -= (A21 @ Y).astype(f32)
-            A[j0:j1, j1:j1 + C] = U12
-            self.growth = max(self.growth, float(np.abs(U11).max()), float(np.abs(U12).max()) if C else 0.0)
-            self.panels.append((j0, j1, R, C, perm, Li, Ui, U12, A21))
+            self.panels.append((j0, j1, R, C, Ai, Y, A21))
 
     def solve(self, b: np.ndarray) -> np.ndarray:
-        """LU^-1 b in FP32 with the stored inverses (forward, then backward)."""
+        """K^-1 b in FP32 with the stored factors (forward, then backward)."""
         f32 = np.float32
         z = b.astype(f32)
-        for (j0, j1, R, C, perm, Li, Ui, U12, A21) in self.panels:
-            y = (Li @ z[j0:j1][perm]).astype(f32)
-            z[j1:j0 + R] -= (A21 @ (Ui @ y).astype(f32)).astype(f32)
-            z[j0:j1] = y
-        for (j0, j1, R, C, perm, Li, Ui, U12, A21) in reversed(self.panels):
-            z[j0:j1] = (Ui @ (z[j0:j1] - U12 @ z[j1:j1 + C]).astype(f32)).astype(f32)
+        for (j0, j1, R, C, Ai, Y, A21) in self.panels:
+            z[j0:j1] = (Ai @ z[j0:j1]).astype(f32)
+            z[j1:j0 + R] -= (A21 @ z[j0:j1]).astype(f32)
+        for (j0, j1, R, C, Ai, Y, A21) in reversed(self.panels):
+            z[j0:j1] -= (Y @ z[j1:j1 + C]).astype(f32)
         return z.astype(np.float64)
 
 
