@@ -1385,9 +1385,17 @@ static cudaError_t launch_elem_f(const DevPatch& Pt, const PhysParams& pp, doubl
                                  float* K_el, cudaStream_t st) {
   const cudaError_t e = launch_resid_t<MOTION>(Pt, pp, time, dt, r_el, st);
   if (e) return e;
-  // one element per CTA while all of them are resident at once (two CTAs on each of 152 SMs)
-  return Pt.numel <= 304 ? launch_elem_t<float, false, MOTION, 1>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0)
-                         : launch_elem_t<float, false, MOTION, 2>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0);
+  // One element per CTA while all of them are resident at once, else two (one wave less
+  // of serial phases).  On 152 SMs, assembly with its gathers, one element -> two: LAG
+  // (four CTAs per SM) 289 elements 93 -> 99 us, 400 100 -> 107, 600 104 -> 111, 900
+  // 117 -> 114; ALEVB (two) 289 125 -> 132, 400 149 -> 151, 484 155 -> 153.
+  int dev = 0, sms = 0;
+  cudaError_t e2 = cudaGetDevice(&dev);
+  if (e2 == cudaSuccess) e2 = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e2 != cudaSuccess) return e2;
+  return Pt.numel <= Lay<MOTION>::template ctas<float>() * sms
+             ? launch_elem_t<float, false, MOTION, 1>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0)
+             : launch_elem_t<float, false, MOTION, 2>(Pt, pp, time, dt, r_el, K_el, st, nullptr, 0, 0);
 }
 template <>
 cudaError_t launch_elem<float>(const DevPatch& Pt, const PhysParams& pp, double time, double dt, double* r_el,
