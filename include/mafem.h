@@ -362,8 +362,9 @@ int mafem_trace_factor(mafem_handle* h, double time, double dt, int64_t* out, in
  * chunk's Y, its trailing update, panel done), then
  * the factor and refine kernels' event times in ns, then 4 stamps per
  * refinement sweep for up to 32 sweeps (start, substitutions done, x updated,
- * residual done; 0 where not reached), then 16 phase sums (ns) of the first
- * sweep's substitutions (patch_solve_pass), then the relative residual
+ * residual done; 0 where not reached), then 16 words of which the first two
+ * are the first sweep's forward and backward substitution in ns, the others 0,
+ * then the relative residual
  * |r - A0 x| / |r| after each sweep (up to 32, as double bit patterns), then
  * the refinement's status and sweep count.  cap >= 6 npan + 182.
  * Returns npan, or MAFEM_ERR_UNSUPPORTED if the handle cannot use that solve. */

@@ -105,7 +105,7 @@ struct mafem_handle {
   bool last_two = false;  // node-block factors: of the elimination from both ends
   int lu_form = MAFEM_FORM_NONE;  // form of the last factorisation (mafem_lu_form)
   bool last_blk = false;  // which factorisation the band currently holds
-  bool pinv_ready = false;  // d_pinv holds the inverses of its panels' triangles
+  bool pinv_ready = false;  // d_pinv holds its panels' matrices (blk_inverses)
   BlkPlan blk;
   int* d_blk_end = nullptr;
   SolveWord* d_xch = nullptr;  // what the panels of the cooperative substitutions hand on: npan_max x 32
@@ -887,11 +887,10 @@ static int wait_ran_out(mafem_handle* h, const char* where) {
   return MAFEM_ERR_CUDA;
 }
 
-// Launch the node-block factorisation (persistent kernel, or per-panel launches)
-// without waiting for it; `info` tells later whether a block had no usable pivot.
-// The panels' triangle inverses for the cooperative forward substitution, formed
+// The panels' inverses for the cooperative forward substitution (blk_inverses), formed
 // when a factorisation is first solved with again (a time step's right-hand side
-// rides along its factorisation and needs none; the kernel takes 50 us).
+// rides along its factorisation and needs none; the kernel takes 97 us for 32 x 32
+// ALEVB).
 static void blk_need_inverses(mafem_handle* h) {
   if (h->pinv_ready) return;
   h->pinv_ready = true;
@@ -902,6 +901,8 @@ static void blk_need_inverses(mafem_handle* h) {
                                                    h->d_perm, (const float*)h->d_rdiag, h->d_pinv, h->st);
 }
 
+// Launch the node-block factorisation (persistent kernel, or per-panel launches)
+// without waiting for it; `info` tells later whether a block had no usable pivot.
 static int factor_enqueue(mafem_handle* h, double* x) {
   const bool fp64 = h->precision == MAFEM_PLAIN_FP64;
   CK(cudaMemsetAsync(h->d_info, 0, sizeof(int), h->st));
@@ -1436,9 +1437,6 @@ extern "C" int mafem_set_launch_ctas(mafem_handle* h, int32_t ctas) {
   return h->pers.max_grid > 0 ? h->pers.grid : h->bwd_grid;
 }
 
-// Order of a round's batched solves: the patches factored on four-CTA
-// clusters first, then those on two-CTA clusters, then the single-CTA ones,
-// each group largest first.  Returns the groups.
 // CTAs that factor the handle's patch in the batched FP32 form: the caller's
 // choice, else the autotuner's for this round, else by band width
 static int patch_ctas(const mafem_handle* h) {
@@ -1585,6 +1583,9 @@ static int tan_epb(const mafem_handle* h) {
 static int tan_tune(mafem_handle* h, const AsmJob* d_ajobs, int slot, unsigned char* d_buf, unsigned char* h_buf,
                     cudaStream_t st);
 
+// Order of a round's batched solves: the patches factored on four-CTA
+// clusters first, then those on two-CTA clusters, then the single-CTA ones,
+// each group largest first.  Returns the groups.
 static PatchGroups order_patch_jobs(std::vector<mafem_handle*>& hv, std::vector<int>& idx) {
   auto nr = [&](int k) { return patch_ctas(hv[k]); };
   auto cost = [&](int k) { return (double)hv[k]->blk.npan() * hv[k]->L.kl * hv[k]->blk.kuf; };

@@ -8,27 +8,29 @@
 // per panel.
 //
 // Per panel p every worker with columns in p's trailing range:
-//   1. waits for pdone[p] (panel p factorised) and a21cnt[p] (every column of
-//      p has its rows below the diagonal block final),
-//   2. stages panel p (L11\U11, A21, permutation, 1/U(j,j)) in shared memory,
-//   3. loads its columns and runs the triangular solves (one warp each),
+//   1. waits for a21cnt[p] (every column of p has its rows below the diagonal
+//      block final) and has p's A21 and its own columns copied to shared memory,
+//      beside the panel's factorisation,
+//   2. waits for pdone[p] (panel p factorised) and loads a row of L11\U11 per
+//      lane, with the permutation and 1/U(j,j), into registers,
+//   3. runs its columns' triangular solves (one warp each),
 //   4. for its column of panel p + 1 (at most one): updates the 32 rows the
 //      next factorisation reads, bumps critcnt[p + 1], then the rows below,
 //      bumps a21cnt[p + 1],
 //   5. updates the rows of its other columns.
 // The factorising CTA waits for critcnt[p + 1] = w(p + 1), factorises panel
 // p + 1 in registers and publishes pdone[p + 1].  So the critical path per
-// panel is: stage, one triangular solve, 32 rows of one column, the panel
-// factorisation, and two flag hand-overs -- no kernel launches.
+// panel is: the block's load, one triangular solve, 32 rows of one column, the
+// panel factorisation, and two flag hand-overs -- no kernel launches.
 //
 // Flags and counters go on across factorisations: pdone[t] holds the epoch that set
 // it, critcnt[t] / a21cnt[t] reach epoch * w(t), modulo 2^32; a wait compares
 // differences, so they may wrap.  All waits are bounded (kSpinLimit polls) and abort
 // every CTA through *err; the host then starts the counters afresh (blk_persist_count).
 //
-// From both ends (FP64 with a right-hand side; blk_two_plan).  A panel takes ~24 us of
-// dependent steps however narrow the band is, so the number of panels in a row is
-// what bounds narrow bands, and a band's last unknowns can be eliminated beside its
+// From both ends (FP64 with a right-hand side, and FP32; blk_two_plan).  A panel takes
+// 19.2 us of dependent steps in FP64 (15 us in FP32) however narrow the band is, so
+// the number of panels in a row is what bounds narrow bands, and a band's last unknowns can be eliminated beside its
 // first ones: two chains, each on half of the CTAs with its own factorising CTA,
 // meet in the middle.  The second numbers rows and columns from the last unknown,
 // so it is the same code on descending addresses (its fill and Y lie below the
@@ -472,14 +474,13 @@ int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
   S.smem = persist_smem<T>(L, B.wmax, 4, false);
   if (!coop || S.smem + 12 * 1024 > (size_t)cap || B.wmax > kBlkW) return 0;  // + static shared memory
   if (!persist_fits<T, false>(S.smem, cap)) return 0;
-  // workers need at most kMinCols columns each per panel (columns c of the
-  // trailing range, owned by c mod (G - 1), plus the right-hand side)
-  constexpr int kMinCols = 8;
+  // The smallest grid: workers with at most kFewCols columns each per panel (columns c
+  // of the trailing range, owned by c mod GW, plus the right-hand side), and at least
+  // one per column of the widest panel (a worker owns at most one column of the next
+  // panel); + the right-hand-side CTA + the factorising CTA
+  constexpr int kFewCols = 8;
   S.grid = sms;
-  // workers: <= kMinCols columns each per panel, and at least one per column of
-  // the widest panel (a worker owns at most one column of the next panel);
-  // + the right-hand-side CTA + the factorising CTA
-  S.min_grid = std::max((int)((B.kuf + B.wmax + 1 + kMinCols - 1) / kMinCols), B.wmax) + 2;
+  S.min_grid = std::max((int)((B.kuf + B.wmax + 1 + kFewCols - 1) / kFewCols), B.wmax) + 2;
   if (S.grid < S.min_grid) return S.grid = 0;
   S.max_grid = S.grid;
   // two chains: each on half of the CTAs, a worker with up to kMaxCols columns per panel (on fewer CTAs one

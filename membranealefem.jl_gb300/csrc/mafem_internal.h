@@ -259,7 +259,7 @@ int blk_forward(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, co
 // hold the one chain's npan panels, then the two chains'.
 struct BlkPersist {
   int grid = 0;            // CTAs of the launch: min_grid <= grid <= max_grid
-  int min_grid = 0;        // fewest CTAs that give every worker <= kMaxCols columns per panel
+  int min_grid = 0;        // fewest CTAs that give every worker <= 8 columns per panel (blk_persist_setup)
   int max_grid = 0;        // the device's SM count
   int min_two = 0;         // fewest CTAs that run the two chains side by side (0: form not available)
   int nslot2 = 0;          // two chains: columns a worker stages at once
