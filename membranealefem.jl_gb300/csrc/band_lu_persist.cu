@@ -36,13 +36,13 @@
 // so it is the same code on descending addresses (its fill and Y lie below the
 // diagonal).  Up to panel pm of the first one the two touch different entries; there
 // all CTAs meet (*bdone) and share the columns of what is left, 2 kuf unknowns.
-// The chain of dependent panels is n / 2 + kuf unknowns long instead of n.  Factor
-// and back substitution, ms per Newton iteration, one chain -> two:
-//   ALEVB 17 x 17 (n 2410, kuf 310)     1.88 + 0.24 -> 1.18 + 0.16
-//   ALEVB 32 x 32 (n 8410, kuf 550)     7.37 + 0.69 -> 6.10 + 0.44
-//   ALEVB 64 x 64 (n 33242, kuf 1062)   98.9 + 5.1  -> 83.4 + 3.4
-// The last two are bound by the FP64 units (1.25 TFLOP/s: 4.0 and 60 ms for the
-// 2 n kl kuf operations): there the gain is that one chain's hand-overs hide behind
+// The chain of dependent panels is n / 2 + kuf unknowns long instead of n.
+// Factorisation, ms, one chain -> two (FP64; FP32):
+//   ALEVB 17 x 17 (n 2410, kuf 310)     1.50 -> 1.01; 1.02 -> 0.65
+//   ALEVB 32 x 32 (n 8410, kuf 550)     6.77 -> 5.86; 3.58 -> 2.21
+//   ALEVB 64 x 64 (n 33242, kuf 1062)   94.3 -> 81.6
+// In FP64 the last two are bound by the FP64 units (1.25 TFLOP/s: 4.0 and 60 ms for
+// the 2 n kl kuf operations): there the gain is that one chain's hand-overs hide behind
 // the other's updates.  A worker has twice the columns while the chains run beside
 // each other (kMaxCols, and eight staged at once where shared memory allows).
 //
@@ -58,8 +58,8 @@ namespace {
 template <class T>
 struct PersistArgs {
   T* ab;
-  BlkChain c[2];              // TWO: c[0] forward on CTAs [0, split), c[1] backward on the others
-  int split;                  // 0: one chain after the other on all CTAs, c[1] first
+  BlkChain c[2];              // two chains: c[0] forward, side by side on CTAs [0, split), c[1] backward on the others
+  int split;
   int n, off, kl, kuf;
   int rmax, wmax, nslot;      // rmax = wmax + kl: rows of a staged panel column
   int pm;
@@ -379,11 +379,21 @@ __device__ __forceinline__ bool persist_panels(const PersistArgs<T>& a, const Bl
 
 // With a right-hand side the last CTA but one of a chain carries it alone (its extra
 // column would otherwise make one worker late every few panels); the last factorises.
-template <class T, bool TWO>
+// kSideBySide: each chain on its own CTAs, the forward one up to panel pm, then the rest on all of them.
+// kInTurn, on too few CTAs for that: all of them run the backward chain, meet, and run the forward one.  Every
+// entry sees the same updates in the same order as side by side: the results do not depend on the number of
+// CTAs.  (A batch keeps its patches on their smallest grids; one step of a batch of FP64 patches against the
+// one chain there: 24 of 8 x 8 to 16 x 16 56 -> 29 ms, 12 of 17 x 17 ALEVB 55.6 -> 51.4 ms, 8 of 32 x 32 375 ->
+// 334 ms.)  A kernel of its own: with both forms in one, side by side cost 64 x 64 ALEVB 82.5 instead of 81.6 ms
+// and the FP32 32 x 32 patch 2.30 instead of 2.21.
+enum Form { kOneChain, kSideBySide, kInTurn };
+template <class T, Form FORM>
 __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_bar;  // completion of the TMA copies
+  [[maybe_unused]] __shared__ int s_ok;
   const int G = (int)gridDim.x;
+  const int nx = a.rhs ? 2 : 1;  // CTAs of a chain that own no columns
   int me = blockIdx.x;
   if (threadIdx.x == 0) {
     mbar_init(&s_bar, 1);
@@ -391,44 +401,42 @@ __global__ void __launch_bounds__(256, 1) blk_factor_persist_kernel(PersistArgs<
   }
   __syncthreads();
   uint32_t ph = 0;
-  if constexpr (!TWO) {
-    const int GW = G - 1 - (a.rhs ? 1 : 0);
-    persist_panels<T, false, false>(a, a.c[0], 0, a.c[0].npan, me, GW,
-                                    me == G - 1 ? kFactor : a.rhs && me == G - 2 ? kRhs : kWorker, smem_raw, &s_bar,
-                                    ph);
+  auto role_of = [&](int i, int ctas) { return i == ctas - 1 ? kFactor : a.rhs && i == ctas - 2 ? kRhs : kWorker; };
+  // between the chains: each side reads what the other one updated
+  [[maybe_unused]] auto meet = [&]() {
+    fence_proxy_async_global();
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(a.bdone, 1);
+    return wait_geq(a.bdone, a.bdone_target, a.err, a.limit, &s_ok);
+  };
+  if constexpr (FORM == kOneChain) {
+    persist_panels<T, false, false>(a, a.c[0], 0, a.c[0].npan, me, G - nx, role_of(me, G), smem_raw, &s_bar, ph);
+  } else if constexpr (FORM == kInTurn) {
+    const Role role = role_of(me, G);
+    if (!persist_panels<T, true, true>(a, a.c[1], 0, a.c[1].npan, me, G - nx, role, smem_raw, &s_bar, ph)) return;
+    if (!meet()) return;
+    persist_panels<T, false, true>(a, a.c[0], 0, a.c[0].npan, me, G - nx, role, smem_raw, &s_bar, ph);
   } else {
-    __shared__ int s_ok;
-    // first each chain on its own CTAs, the forward one up to panel pm, then the rest on all of them; the
-    // forward chain's factorising CTA goes on without the meeting: of its panels pm alone can come before
-    // it (later ones wait for columns that are updated after it), and pm's block is out of c[1]'s reach
-    // On too few CTAs for that (split 0) all of them run the backward chain, meet, and run the forward one.
-    // Every entry sees the same updates in the same order as side by side: the results do not depend on
-    // the number of CTAs.  (A batch keeps its patches on their smallest grids; one step of a batch of FP64
-    // patches against the one chain there: 24 of 8 x 8 to 16 x 16 56 -> 29 ms, 12 of 17 x 17 ALEVB 55.6 ->
-    // 51.4 ms, 8 of 32 x 32 375 -> 334 ms.)
-    const bool turn = a.split == 0, rev = me >= a.split;
+    const bool rev = me >= a.split;
     const int G0 = rev ? G - a.split : a.split;
-    const int nx = a.rhs ? 2 : 1;  // CTAs of a chain that own no columns
     if (rev) me -= a.split;
-    Role role = me == G0 - 1 ? kFactor : a.rhs && me == G0 - 2 ? kRhs : kWorker;
+    Role role = role_of(me, G0);
     if (rev) {
       if (!persist_panels<T, true, true>(a, a.c[1], 0, a.c[1].npan, me, G0 - nx, role, smem_raw, &s_bar, ph)) return;
     }
+    // the forward chain's factorising CTA goes on without the meeting: of its panels pm alone can come before
+    // it (later ones wait for columns that are updated after it), and pm's block is out of c[1]'s reach
 #pragma unroll 1
     for (int half = rev || role == kFactor ? 1 : 0; half < 2; ++half) {
       if (half == 1 && (rev || role != kFactor)) {
-        // the columns change hands, and each side reads what the other one updated
-        fence_proxy_async_global();
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) atomicAdd(a.bdone, 1);
-        if (!wait_geq(a.bdone, a.bdone_target, a.err, a.limit, &s_ok)) return;
-        if (rev && !turn) {
+        if (!meet()) return;
+        if (rev) {  // the columns change hands
           role = kWorker;
           me += a.split - nx;
         }
       }
-      const int p0 = half == 1 && role != kFactor && !turn ? a.pm : 0, p1 = half == 0 ? a.pm : a.c[0].npan;
+      const int p0 = half == 1 && role != kFactor ? a.pm : 0, p1 = half == 0 ? a.pm : a.c[0].npan;
       if (!persist_panels<T, false, true>(a, a.c[0], p0, p1, me, half == 0 ? a.split - nx : G - nx, role, smem_raw, &s_bar,
                                           ph))
         return;
@@ -449,16 +457,16 @@ static size_t persist_smem(const BandLayout& L, int wmax, int nslot, bool two) {
 // The kernel's limit of dynamic shared memory belongs to the process, not to a handle:
 // it is always set to all that the device has (cap) beside the kernel's static part, so
 // that no handle's set-up takes away what another one's launches ask for.
-template <class T, bool TWO>
+template <class T, Form FORM>
 static bool persist_fits(size_t sm, int cap) {
   int per = 0;
   cudaFuncAttributes fa;
-  if (cudaFuncGetAttributes(&fa, blk_factor_persist_kernel<T, TWO>) != cudaSuccess) return false;
+  if (cudaFuncGetAttributes(&fa, blk_factor_persist_kernel<T, FORM>) != cudaSuccess) return false;
   const int dyn = cap - (int)fa.sharedSizeBytes;
   return sm <= (size_t)dyn &&
-         cudaFuncSetAttribute(blk_factor_persist_kernel<T, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ==
+         cudaFuncSetAttribute(blk_factor_persist_kernel<T, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ==
              cudaSuccess &&
-         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, blk_factor_persist_kernel<T, TWO>, 256, sm) ==
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, blk_factor_persist_kernel<T, FORM>, 256, sm) ==
              cudaSuccess &&
          per >= 1;
 }
@@ -473,7 +481,7 @@ int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   S.smem = persist_smem<T>(L, B.wmax, 4, false);
   if (!coop || S.smem + 12 * 1024 > (size_t)cap || B.wmax > kBlkW) return 0;  // + static shared memory
-  if (!persist_fits<T, false>(S.smem, cap)) return 0;
+  if (!persist_fits<T, kOneChain>(S.smem, cap)) return 0;
   // The smallest grid: workers with at most kFewCols columns each per panel (columns c
   // of the trailing range, owned by c mod GW, plus the right-hand side), and at least
   // one per column of the widest panel (a worker owns at most one column of the next
@@ -490,7 +498,8 @@ int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
     if (!B.has_two) break;
     S.nslot2 = nslot;
     S.smem2 = persist_smem<T>(L, B.wmax, nslot, true);
-    if (S.smem2 + 12 * 1024 <= (size_t)cap && persist_fits<T, true>(S.smem2, cap)) {
+    if (S.smem2 + 12 * 1024 <= (size_t)cap && persist_fits<T, kSideBySide>(S.smem2, cap) &&
+        persist_fits<T, kInTurn>(S.smem2, cap)) {
       S.min_two = 2 * (std::max((int)((B.kuf + B.wmax + 1 + kMaxCols - 1) / kMaxCols), B.wmax) + 2);
       if (S.min_two > S.max_grid) S.min_two = 0;
       break;
@@ -509,7 +518,8 @@ int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersi
   a.c[0] = two ? B.two[0] : B.one;
   a.c[1] = B.two[1];
   const int after = two ? B.npan() : 0;  // the two chains' flags stand after the one chain's
-  a.split = !two ? S.grid : S.grid >= S.min_two ? (S.grid + 1) / 2 : 0;
+  const Form form = !two ? kOneChain : S.grid >= S.min_two ? kSideBySide : kInTurn;
+  a.split = (S.grid + 1) / 2;
   a.n = (int)L.n;
   a.off = (int)L.off;
   a.kl = L.kl;
@@ -519,7 +529,7 @@ int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersi
   a.nslot = two ? S.nslot2 : 4;
   a.pm = B.pm;
   a.bdone = S.d_bdone;
-  a.bdone_target = S.bdone + S.grid - (a.split ? 1 : 0);  // all CTAs, side by side but the forward chain's factorising one
+  a.bdone_target = S.bdone + S.grid - (form == kSideBySide);  // all CTAs, side by side but the forward chain's factorising one
   a.perm_all = perm_all;
   a.rdiag = rdiag;
   a.info = info;
@@ -532,7 +542,9 @@ int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersi
   a.limit = S.limit > 0 ? S.limit : kSpinLimit;
   a.trace = two ? nullptr : trace;
   void* args[] = {(void*)&a};
-  const void* fn = two ? (const void*)blk_factor_persist_kernel<T, true> : (const void*)blk_factor_persist_kernel<T, false>;
+  const void* fn = form == kOneChain     ? (const void*)blk_factor_persist_kernel<T, kOneChain>
+                   : form == kSideBySide ? (const void*)blk_factor_persist_kernel<T, kSideBySide>
+                                         : (const void*)blk_factor_persist_kernel<T, kInTurn>;
   if (cudaLaunchCooperativeKernel(fn, dim3(S.grid), dim3(256), args, two ? S.smem2 : S.smem, st) != cudaSuccess) return -1;
   S.epoch[two] = a.epoch;
   if (two) S.bdone = a.bdone_target;
