@@ -322,12 +322,19 @@ __global__ void __launch_bounds__(1024) blk_backward_kernel(const T* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// Two 32 x 32 matrices per panel for the cooperative forward substitution:
-// Ai = U11^-1 L11^-1 P, and W = Ai A(p, p - 1), the panel's rows of the panel before
-// it, so that of z(p) = Ai (b - sum over q < p of A(p, q) z(q)) everything but
-// W z(p - 1) can be formed before z(p - 1) is there.  Element (i, k) at k * 32 + i,
-// zero outside the panel's rows and columns; inv[p] = Ai then W.  One warp per panel
+// Two 32 x 32 matrices per panel for the cooperative forward substitution, element
+// (i, k) at k * 32 + i, zero outside the panel's rows and columns.  One warp per panel
 // (four per CTA), lane c forming column c of both.
+// FP32 factors: Ai = U11^-1 L11^-1 P, and W = Ai A(p, p - 1), the panel's rows of the
+// panel before it, so that of z(p) = Ai (b - sum over q < p of A(p, q) z(q)) everything
+// but W z(p - 1) can be formed before z(p - 1) is there.  Formed and applied in FP64,
+// their rounding, of the size of A11's condition, stays far below the factors' own.
+// FP64 factors: L11^-1 P and U11^-1, each applied by itself: on tangents whose diagonal
+// blocks are ill-conditioned (strips of the ALE motions) Ai and W left backward errors
+// of up to 2e-4 (median 2e-15, nine in ten below 3e-11) where the triangles' inverses
+// stay at the level of the triangles' solves, 2e-16.
+template <class T>
+constexpr bool kTriangles = sizeof(T) == 8;
 template <class T>
 __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__ ab, BlkChain c0, BlkChain c1, int split,
                                                            int kl,
@@ -348,7 +355,7 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
   __syncwarp();
   double* Ai = inv + (size_t)(c.pbase + p) * 2 * kBlkW * kBlkW;
   double* W = Ai + kBlkW * kBlkW;
-  // column `lane`: L11 y = P e_lane forward, U11 x = y backward
+  // column `lane`: L11 y = P e_lane forward, U11 x = y (triangles: e_lane) backward
   double x[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) x[i] = __shfl_sync(kFull, pr, i) == lane ? 1.0 : 0.0;
@@ -358,12 +365,24 @@ __global__ void __launch_bounds__(128) blk_inverses_kernel(const T* __restrict__
 #pragma unroll
     for (int i = k + 1; i < 32; ++i) x[i] = fma(-S[warp][k][i], xk, x[i]);
   }
+  if constexpr (kTriangles<T>) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      Ai[lane * 32 + i] = (lane < w && i < w) ? x[i] : 0.0;
+      x[i] = i == lane ? 1.0 : 0.0;
+    }
+  }
 #pragma unroll
   for (int k = 31; k >= 0; --k) {
     const double xk = x[k] * __shfl_sync(kFull, rd, k);
     x[k] = xk;
 #pragma unroll
     for (int i = 0; i < k; ++i) x[i] = fma(-S[warp][k][i], xk, x[i]);
+  }
+  if constexpr (kTriangles<T>) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) W[lane * 32 + i] = (lane < w && i < w) ? x[i] : 0.0;
+    return;
   }
   __syncwarp();
 #pragma unroll
@@ -501,14 +520,16 @@ __global__ void __launch_bounds__(kSolveThreads)
   }
 }
 
-// Forward substitution z(p) = Ai(p) (b(p) - sum over q < p of A(p, q) z(q)), each panel's
-// contributions pulled from the panels before it; the last of them by W (above).
+// Forward substitution z(p) = A11^-1 (b(p) - sum over q < p of A(p, q) z(q)), each panel's
+// contributions pulled from the panels before it; FP32 factors: the last of them by W,
+// FP64 factors: L11^-1 P and U11^-1 after it (blk_inverses_kernel).
 template <class T>
 __global__ void __launch_bounds__(kSolveThreads)
     blk_forward_coop_kernel(const T* __restrict__ ab, int kl, BlkSpan s0, BlkSpan s1, int split,
                             const double* __restrict__ inv_all, double* bv, SolveWord* xch, long long epoch, int* err,
                             WaitTest wt, const int* gate) {
   __shared__ double xs[2][32];
+  [[maybe_unused]] __shared__ double ys[32];
   if (gate && *gate) return;
   const int lane = threadIdx.x & 31, row = 8 * (threadIdx.x >> 5) + (lane & 7), cg = lane >> 3;
   const bool second = (int)blockIdx.x >= split;
@@ -527,7 +548,7 @@ __global__ void __launch_bounds__(kSolveThreads)
     const T* arow = ab + S.c.org + r * si;
     const double br = row < w ? b[r * si] : 0.0;
     const double* Ip = inv_all + (size_t)(S.c.pbase + p) * 2 * kBlkW * kBlkW;
-    double Ai[8], W[8];
+    double Ai[8], W[8];  // (FP64 factors: L11^-1 P, U11^-1)
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       Ai[i] = Ip[(cg + 4 * i) * 32 + row];
@@ -545,12 +566,13 @@ __global__ void __launch_bounds__(kSolveThreads)
         an[i] = c < ce && r - c <= kl ? arow[c * sj] : T(0);  // inside that panel's band rows
       }
     };
-    if (q < p - 1) load(q);
-    for (; ok && q < p - 1; ++q) {
+    const int qe = kTriangles<T> ? p : p - 1;
+    if (q < qe) load(q);
+    for (; ok && q < qe; ++q) {
       double av[8], zv[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) av[i] = (double)an[i];
-      if (q + 1 < p - 1) load(q + 1);
+      if (q + 1 < qe) load(q + 1);
       ok = fetch(X + (size_t)q * kBlkW, cg, ps[q + 1] - ps[q], q >= S.p0 ? epoch : 0, q < p - 3, zv, err, wt.limit);
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i & 1] = fma(av[i], zv[i], acc[i & 1]);
@@ -563,7 +585,16 @@ __global__ void __launch_bounds__(kSolveThreads)
     double u[2] = {0.0, 0.0};
 #pragma unroll
     for (int i = 0; i < 8; ++i) u[i & 1] = fma(Ai[i], xs[par][cg + 4 * i], u[i & 1]);
-    if (p > 0) {
+    if constexpr (kTriangles<T>) {
+      double y = u[0] + u[1];
+      y += __shfl_xor_sync(kFull, y, 8);
+      y += __shfl_xor_sync(kFull, y, 16);
+      if (cg == 0) ys[row] = y;
+      __syncthreads();  // (ys is written again after the next panel's first barrier)
+      u[0] = u[1] = 0.0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) u[i & 1] = fma(W[i], ys[cg + 4 * i], u[i & 1]);
+    } else if (p > 0) {
       double zv[8];
       ok = fetch(X + (size_t)(p - 1) * kBlkW, cg, j0 - ps[p - 1], p - 1 >= S.p0 ? epoch : 0, false, zv, err, wt.limit);
 #pragma unroll

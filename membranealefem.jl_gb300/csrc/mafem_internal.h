@@ -232,8 +232,9 @@ struct WaitTest {
   int withhold = -1;
   int refuse = -1;
 };
-// Per panel the inverse of its diagonal block and its product with the rows of the
-// panel before (inv: npan_max x 2 x 32 x 32) for the cooperative forward substitution.
+// Per panel two matrices for the cooperative forward substitution (inv: npan_max x 2 x
+// 32 x 32): the inverse of its diagonal block and its product with the rows of the
+// panel before (FP32 factors), or the inverses of its two triangles (FP64 factors).
 template <class T>
 int blk_inverses(const T* ab, const BandLayout& L, const BlkPlan& B, bool two, const int* perm_all, const T* rdiag,
                  double* inv, cudaStream_t st);
