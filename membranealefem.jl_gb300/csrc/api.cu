@@ -638,10 +638,12 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
         h->blk.ps0 = ps0;
         h->blk.ps1 = ps1;
         BlkChain &a = h->blk.two[0], &b = h->blk.two[1];
-        int *d_ps0 = nullptr, *d_ps1 = nullptr, *d_end1 = nullptr;
-        UP(d_ps0, ps0);
-        UP(d_ps1, ps1);
-        UP(d_end1, blk_end1);
+        std::vector<int> all(ps0);
+        all.insert(all.end(), ps1.begin(), ps1.end());
+        all.insert(all.end(), blk_end1.begin(), blk_end1.end());
+        int* d_ps0 = nullptr;
+        UP(d_ps0, all);
+        const int *d_ps1 = d_ps0 + ps0.size(), *d_end1 = d_ps1 + ps1.size();
         a = b = one;
         a.ps = d_ps0;
         a.npan = (int)ps0.size() - 1;
@@ -668,14 +670,11 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
       cudaGetLastError();
       if (pg > 0) {
         const size_t np = S.flags;
-        AL(h->pers.d_bdone, 1);
-        cudaMemset(h->pers.d_bdone, 0, sizeof(int));
-        AL(h->pers.d_pdone, np);
-        AL(h->pers.d_critcnt, np);
-        AL(h->pers.d_a21cnt, np);
-        cudaMemset(h->pers.d_pdone, 0, np * sizeof(int));
-        cudaMemset(h->pers.d_critcnt, 0, np * sizeof(int));
-        cudaMemset(h->pers.d_a21cnt, 0, np * sizeof(int));
+        AL(h->pers.d_pdone, 3 * np + 1);  // all counters in one piece
+        h->pers.d_critcnt = h->pers.d_pdone + np;
+        h->pers.d_a21cnt = h->pers.d_critcnt + np;
+        h->pers.d_bdone = h->pers.d_a21cnt + np;
+        cudaMemset(h->pers.d_pdone, 0, (3 * np + 1) * sizeof(int));
       } else {
         h->pers.grid = 0;
       }
