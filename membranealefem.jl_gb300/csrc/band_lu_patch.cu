@@ -835,16 +835,20 @@ __device__ __forceinline__ void residual_run(const float* a, int64_t ldm, const 
 // them: at most two runs per grid row.  The columns skipped hold stored
 // zeros, whose products leave the pair unchanged: the sums equal a walk of
 // the whole band window.
-__device__ __forceinline__ double residual_rows(const PatchJob& J, const float2* xs, int w0, int nw) {
+// The 32-row blocks w0, w0 + nw, ... of a warp; the squares of the k-th one's entries go to ss[k mod NS].
+template <int NS>
+__device__ __forceinline__ void residual_rows(const PatchJob& J, const float2* xs, int w0, int nw, double (&ss)[NS]) {
   const BandLayout L = J.L;
   const int lane = threadIdx.x & 31;
   const int64_t ldm = L.ldb - 1;
-  double ss = 0.0;
+#pragma unroll
+  for (int u = 0; u < NS; ++u) ss[u] = 0.0;
+  int k = 0;
   // With nb >= 32 every (i, j) of the band window [rb - ku, rb + 32 + kl) lies
   // inside the band's storage, where the entries outside the band are stored
   // zeros, so A0(i, j) = a[j * ldm + lane] with a at row rb of column 0 needs
   // no guard but i < n; the runs are clipped to that window.
-  for (int64_t rb = (int64_t)w0 * 32; rb < L.n; rb += (int64_t)nw * 32) {
+  for (int64_t rb = (int64_t)w0 * 32; rb < L.n; rb += (int64_t)nw * 32, ++k) {
     const int64_t i = rb + lane;
     const bool live = i < L.n;
     const int64_t jlo = rb - L.ku > 0 ? rb - L.ku : 0;
@@ -886,10 +890,11 @@ __device__ __forceinline__ double residual_rows(const PatchJob& J, const float2*
     if (live) {
       const double r = J.rhs[i] - ((double)sh + (double)sl);
       J.res[i] = r;
-      ss = fma(r, r, ss);
+#pragma unroll
+      for (int u = 0; u < NS; ++u)
+        if (NS == 1 || k % NS == u) ss[u] = fma(r, r, ss[u]);
     }
   }
-  return ss;
 }
 // The residual after a sweep on kResC CTAs per patch: partial sums of its squares to J.rs + 8.
 constexpr int kResC = 8, kResT = 256;
@@ -899,9 +904,10 @@ __global__ void __launch_bounds__(kResT) patch_residual_kernel(const PatchJob* _
   const int c = blockIdx.x % kResC;
   if (J.rs[4] != 0.0) return;  // this patch's refinement has ended
   __shared__ double red[kResT / 32];
-  double ss = residual_rows(J, J.xs, c * (kResT / 32) + (threadIdx.x >> 5), kResC * kResT / 32);
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(kFull, ss, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  double ss[1];
+  residual_rows(J, J.xs, c * (kResT / 32) + (threadIdx.x >> 5), kResC * kResT / 32, ss);
+  for (int o = 16; o > 0; o >>= 1) ss[0] += __shfl_xor_sync(kFull, ss[0], o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss[0];
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
@@ -910,13 +916,18 @@ __global__ void __launch_bounds__(kResT) patch_residual_kernel(const PatchJob* _
   }
 }
 // The same by one CTA of kRT threads, its norm summed in the same order: a patch's sweeps give the same bits
-// in either kernel, whichever group of a round it is in.  red: kResC * kResT / 32 doubles of shared memory.
+// in either kernel, whichever group of a round it is in.  A warp holds the sums of the kNS warps there whose
+// blocks it takes.  red: kResC * kResT / 32 doubles of shared memory.
 __device__ double patch_residual(const PatchJob& J, const float2* xs, double* red) {
   constexpr int kW = kResT / 32;  // warps of a CTA of patch_residual_kernel
-  for (int q = threadIdx.x >> 5; q < kResC * kW; q += kRT / 32) {
-    double ss = residual_rows(J, xs, q, kResC * kW);
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(kFull, ss, o);
-    if ((threadIdx.x & 31) == 0) red[q] = ss;
+  constexpr int kNS = kResC * kW / (kRT / 32);
+  static_assert(kNS * (kRT / 32) == kResC * kW, "whole shares");
+  double ss[kNS];
+  residual_rows(J, xs, threadIdx.x >> 5, kRT / 32, ss);
+#pragma unroll
+  for (int u = 0; u < kNS; ++u) {
+    for (int o = 16; o > 0; o >>= 1) ss[u] += __shfl_xor_sync(kFull, ss[u], o);
+    if ((threadIdx.x & 31) == 0) red[(threadIdx.x >> 5) + u * (kRT / 32)] = ss[u];
   }
   __syncthreads();
   double s = 0.0;
