@@ -732,7 +732,8 @@ extern "C" int mafem_create(const mafem_mesh_desc* d, const mafem_params* p, con
   if (precision != MAFEM_PLAIN_FP64 && h->use_blk) {
     const int dyn = patch_solve_setup();
     cudaGetLastError();
-    if (patch_fits(h->L, h->blk, dyn)) {
+    if (patch_fits(h->L, h->blk, dyn) &&
+        (patch_vector_fits(n, h->blk.npan(), dyn) || patch_vector_setup(dyn))) {
       const PlanSizes S = plan_sizes(h->L, h->blk, true, true);
       AL(h->d_inv, S.inv);
       PatchJob& J = h->job;

@@ -1133,11 +1133,15 @@ int patch_solve_setup() {
       cudaFuncSetAttribute(patch_refine_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
       cudaFuncSetAttribute(patch_refine_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
       cudaFuncSetAttribute(patch_refine_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
-      cudaFuncSetAttribute(patch_refine_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
-      cudaFuncSetAttribute(patch_refine_kernel<2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
-      cudaFuncSetAttribute(patch_refine_kernel<2, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
+      cudaFuncSetAttribute(patch_refine_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
     return 0;
   return dyn;
+}
+bool patch_vector_setup(int dyn) {
+  return cudaFuncSetAttribute(patch_refine_kernel<2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ==
+             cudaSuccess &&
+         cudaFuncSetAttribute(patch_refine_kernel<2, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ==
+             cudaSuccess;
 }
 
 int patch_cluster_ctas(int kuf) { return kuf > 2 * kNCH ? 4 : kuf > kNCH ? 2 : 1; }

@@ -498,8 +498,7 @@ int blk_persist_setup(const BandLayout& L, const BlkPlan& B, BlkPersist& S) {
     if (!B.has_two) break;
     S.nslot2 = nslot;
     S.smem2 = persist_smem<T>(L, B.wmax, nslot, true);
-    if (S.smem2 + 12 * 1024 <= (size_t)cap && persist_fits<T, kSideBySide>(S.smem2, cap) &&
-        persist_fits<T, kInTurn>(S.smem2, cap)) {
+    if (S.smem2 + 12 * 1024 <= (size_t)cap && persist_fits<T, kSideBySide>(S.smem2, cap)) {
       S.min_two = 2 * (std::max((int)((B.kuf + B.wmax + 1 + kMaxCols - 1) / kMaxCols), B.wmax) + 2);
       if (S.min_two > S.max_grid) S.min_two = 0;
       break;
@@ -519,6 +518,14 @@ int blk_lu_factor_persist(T* ab, const BandLayout& L, const BlkPlan& B, BlkPersi
   a.c[1] = B.two[1];
   const int after = two ? B.npan() : 0;  // the two chains' flags stand after the one chain's
   const Form form = !two ? kOneChain : S.grid >= S.min_two ? kSideBySide : kInTurn;
+  if (form == kInTurn && !S.turn_ready) {  // not at every handle's creation: the kernel is loaded by its first use
+    int dev = 0, cap = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        !persist_fits<T, kInTurn>(S.smem2, cap))
+      return -1;
+    S.turn_ready = true;
+  }
   a.split = (S.grid + 1) / 2;
   a.n = (int)L.n;
   a.off = (int)L.off;

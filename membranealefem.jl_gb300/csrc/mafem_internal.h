@@ -264,6 +264,7 @@ struct BlkPersist {
   int max_grid = 0;        // the device's SM count
   int min_two = 0;         // fewest CTAs that run the two chains side by side (0: form not available)
   int nslot2 = 0;          // two chains: columns a worker stages at once
+  bool turn_ready = false; // the kernel of the two chains in turn is set up
   size_t smem = 0, smem2 = 0;  // shared memory as one chain, as two
   unsigned epoch[2] = {0, 0};  // factorisations so far: as one chain, as two (modulo 2^32, as all counters)
   unsigned bdone = 0;          // *d_bdone once the last two-chain factorisation is done
@@ -404,6 +405,8 @@ bool patch_vector_fits(int64_t n, int npan, int dyn);
 constexpr int patch_dyn_smem(int cap) { return cap - 2 * 1024; }  // room for their static shared memory
 // Sets the kernels' shared-memory limits; returns the dynamic bytes available (0: unusable).
 int patch_solve_setup();
+// The same for the kernels of patches with PatchJob::vg (loaded by the first such patch).
+bool patch_vector_setup(int dyn);
 // CTAs that factor a patch with kuf trailing columns: 4 (a cluster, one chunk
 // per CTA) above two chunks, 2 above one chunk, else 1.
 int patch_cluster_ctas(int kuf);
